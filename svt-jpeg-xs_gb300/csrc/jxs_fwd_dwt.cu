@@ -11,9 +11,9 @@
  *                and the int32 LL plane for the next level.
  *  fwd_h_kernel  the horizontal-only levels below the last vertical level
  *                (or all levels of a component without vertical
- *                decomposition): one warp per row, every level in shared
- *                memory, the high band of each level and the final LL band
- *                emitted as coefficients + GCLIs.
+ *                decomposition): one warp per chunk of a row, every level in
+ *                registers, the high band of each level and the final LL
+ *                band emitted as coefficients + GCLIs.
  *
  * Arithmetic (bit-exact with the reference):
  *  - input scaling: v = ((x & (2^d - 1)) << (20 - d)) - 2^19 (NltEnc.c:33-72);
@@ -61,27 +61,18 @@ DEV int mirror1(int i, int n) {
     return (unsigned)m < (unsigned)n ? m : mirror_far(i, n);
 }
 
-DEV uint32_t to_sm(int32_t v) {
-    const uint32_t m = ((uint32_t)abs(v) + 128u) >> 8;
-    return m ? (m | (((uint32_t)v >> 16) & 0x8000u)) : 0u;
+/* Two values as 16-bit sign-magnitude, the first in the low half: m = (|v| +
+ * 128) >> 8 (bytes 1 and 2 of the sum), the sign only where m is not zero.
+ * m stays below 2^15, so that m + 0x7fff has bit 15 set exactly where m > 0. */
+DEV uint32_t sm_pair(int32_t v0, int32_t v1) {
+    const uint32_t m = __byte_perm((uint32_t)abs(v0) + 128u, (uint32_t)abs(v1) + 128u, 0x6521);
+    const uint32_t sign = __byte_perm((uint32_t)v0, (uint32_t)v1, 0x7733);
+    return m | ((m + 0x7fff7fffu) & sign & 0x80008000u);
 }
-
-template <int SRC>
-DEV int32_t scale_in(uint32_t raw, int depth) {
-    if (SRC == SRC_I32) return (int32_t)raw;
-    const uint32_t mask = (1u << depth) - 1u;
-    return (int32_t)((raw & mask) << (20 - depth)) - (1 << 19);
-}
-
-/* one sample of the level input at (row y, column x), both in range */
-template <int SRC>
-DEV int32_t load1(const void* src, long long pitch, int chan, int depth, int y, int x) {
-    const long long row = (long long)y * pitch;
-    if (SRC == SRC_I32) return ((const int32_t*)src)[row + x];
-    if (SRC == SRC_U8) return scale_in<SRC>(((const uint8_t*)src)[row + x], depth);
-    if (SRC == SRC_U16) return scale_in<SRC>(((const uint16_t*)src)[row + x], depth);
-    if (SRC == SRC_PK8) return scale_in<SRC>(((const uint8_t*)src)[row + 3 * x + chan], depth);
-    return scale_in<SRC>(((const uint16_t*)src)[row + 3 * x + chan], depth);
+/* GCLI of a group of two pairs */
+DEV uint32_t gcli_of(uint32_t c01, uint32_t c23) {
+    const uint32_t o = c01 | c23;
+    return 32u - (uint32_t)__clz((int)((o | (o >> 16)) & 0x7fffu));
 }
 
 /* One lane's 4-coefficient group of a band row: coefficients j..j+3 (j a
@@ -104,50 +95,9 @@ DEV BandRow band_row(const jxs_band_t& bd, int row, uint16_t* coef, uint8_t* gcl
 }
 DEV void emit4(const BandRow& b, int j, int32_t v0, int32_t v1, int32_t v2, int32_t v3) {
     if ((j >> 2) >= b.gw) return;
-    const uint32_t c0 = to_sm(v0), c1 = j + 1 < b.w ? to_sm(v1) : 0u, c2 = j + 2 < b.w ? to_sm(v2) : 0u,
-                   c3 = j + 3 < b.w ? to_sm(v3) : 0u;
-    *(uint2*)(b.crow + j) = make_uint2(c0 | (c1 << 16), c2 | (c3 << 16));
-    const uint32_t m = (c0 | c1 | c2 | c3) & 0x7fffu;
-    b.grow[j >> 2] = (uint8_t)(32 - __clz(m));
-}
-
-/* One horizontal lifting pass of a row held in shared memory, by one warp.
- * x points at sample 0 of the pass; x[-2], x[-1] and the samples past the
- * last pair needed hold the (mirrored or neighbouring-tile) halo.  Output
- * pairs (s[j], d[j]) for j in [0, npairs) are produced; lane l of iteration
- * it owns j = 128*it + 4l .. +3 and passes them to out(j, s[4], d[4]).
- * Reads x[-2 .. 8 * ceil(npairs / 4) + 7] at most; outputs past the valid
- * width may depend on samples past x[2 * npairs + 1] and are discarded by
- * the caller.  x must be 16-byte aligned. */
-template <typename Out>
-DEV void warp_lift_fwd(const int32_t* x, int npairs, Out out) {
-    const int lane = threadIdx.x & 31;
-    int32_t carry = x[-1] - ((x[-2] + x[0]) >> 1); /* d[-1] */
-    for (int base = 0; base < npairs; base += 128) {
-        const int j = base + 4 * lane;
-        int4 a = make_int4(0, 0, 0, 0), b = a;
-        /* the lane just past the last pair still loads: its first sample is
-         * the right neighbour of the previous lane */
-        if (j <= npairs) {
-            a = *(const int4*)(x + 2 * j);
-            b = *(const int4*)(x + 2 * j + 4);
-        }
-        int32_t nxt = __shfl_down_sync(FULL, a.x, 1);
-        if (lane == 31) nxt = j < npairs ? x[2 * j + 8] : 0;
-        int32_t d[4], sv[4];
-        d[0] = a.y - ((a.x + a.z) >> 1);
-        d[1] = a.w - ((a.z + b.x) >> 1);
-        d[2] = b.y - ((b.x + b.z) >> 1);
-        d[3] = b.w - ((b.z + nxt) >> 1);
-        int32_t dm = __shfl_up_sync(FULL, d[3], 1);
-        if (lane == 0) dm = carry;
-        carry = __shfl_sync(FULL, d[3], 31);
-        sv[0] = a.x + ((dm + d[0] + 2) >> 2);
-        sv[1] = a.z + ((d[0] + d[1] + 2) >> 2);
-        sv[2] = b.x + ((d[1] + d[2] + 2) >> 2);
-        sv[3] = b.z + ((d[2] + d[3] + 2) >> 2);
-        if (j < npairs) out(j, sv, d);
-    }
+    const uint32_t c01 = sm_pair(v0, j + 1 < b.w ? v1 : 0), c23 = sm_pair(j + 2 < b.w ? v2 : 0, j + 3 < b.w ? v3 : 0);
+    *(uint2*)(b.crow + j) = make_uint2(c01, c23);
+    b.grow[j >> 2] = (uint8_t)gcli_of(c01, c23);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -282,9 +232,9 @@ template <bool FAST>
 DEV void fv_emit(const FvBand& b, int j, const int32_t* v) {
     if constexpr (FAST) {
         /* the whole group inside the band */
-        const uint32_t c0 = to_sm(v[0]), c1 = to_sm(v[1]), c2 = to_sm(v[2]), c3 = to_sm(v[3]);
-        *(uint2*)(b.crow + j) = make_uint2(c0 | (c1 << 16), c2 | (c3 << 16));
-        b.grow[j >> 2] = (uint8_t)(32 - __clz((c0 | c1 | c2 | c3) & 0x7fffu));
+        const uint32_t c01 = sm_pair(v[0], v[1]), c23 = sm_pair(v[2], v[3]);
+        *(uint2*)(b.crow + j) = make_uint2(c01, c23);
+        b.grow[j >> 2] = (uint8_t)gcli_of(c01, c23);
     } else {
         emit4(BandRow{b.crow, b.grow, b.w, b.gw}, j, v[0], v[1], v[2], v[3]);
     }
@@ -400,62 +350,217 @@ __global__ void __launch_bounds__(FV_THREADS) fwd_v_kernel(const __grid_constant
 /* ------------------------------------------------------------------------ */
 /* horizontal-only levels                                                    */
 /* ------------------------------------------------------------------------ */
+/* A warp transforms one chunk of one row through every level in registers:
+ * lane l holds the 16 input columns c0 = first - 16 halo + 16 l .. c0 + 15,
+ * so that a level leaves 8, 4, 2, 1 low and high values per lane and, at
+ * level 5, one pair per two lanes.  The neighbours come by shuffles.  A low
+ * value of level e reaches 2^(e+1) - 2 input columns to either side, so the
+ * outer 1 (up to 3 levels), 2 (4 levels) or 4 lanes (5 levels) on each side
+ * are halo, and a chunk yields 480, 448 or 384 columns, always whole
+ * 4-coefficient groups of every band.
+ *
+ * Bound by memory: 4 bytes read and 2 1/4 written per column.  The form
+ * before kept whole rows in shared memory, one warp per row, which left 8
+ * warps on an SM for the 3840-column rows of an 8K frame with one vertical
+ * level: 8 such frames took 650 us, now 250 (1.24 GB; encode 3308 -> 2907
+ * us). */
 #define FH_MAX_WARPS 4
+#define FH_COLS 16
 
-/* fills the 2-sample halo on both sides of a row of n samples at x */
-DEV void fill_halo(int32_t* x, int n, int lane) {
-    if (lane < 4) {
-        const int i = lane < 2 ? -2 + lane : n + lane - 2;
-        x[i] = x[mirror_idx(i, n)];
+/* columns a warp's chunk yields */
+static inline __host__ __device__ int fh_halo_lanes(int nh) { return nh >= 5 ? 4 : nh == 4 ? 2 : 1; }
+static inline __host__ __device__ int fh_net_cols(int nh) { return FH_COLS * (32 - 2 * fh_halo_lanes(nh)); }
+
+/* One level over the lane's N inputs x (the row's samples i0 .. i0 + N - 1,
+ * `rel` = row length - i0): N / 2 low and high values.  EDGE: the chunk
+ * touches an end of the row, where the symmetric extension holds: past the
+ * last pair's even sample the sample itself, before the first high value
+ * the first and past the last one the last. */
+template <int N, bool EDGE>
+DEV void fh_level(const int32_t* x, int i0, int rel, int32_t* s, int32_t* d) {
+    const int P = N / 2;
+    const int32_t nx = __shfl_down_sync(FULL, x[0], 1);
+#pragma unroll
+    for (int q = 0; q < P; q++) {
+        int32_t next = q + 1 < P ? x[2 * q + 2] : nx;
+        if (EDGE && 2 * q + 2 >= rel) next = x[2 * q];
+        d[q] = x[2 * q + 1] - ((x[2 * q] + next) >> 1);
     }
+    int32_t dm = __shfl_up_sync(FULL, d[P - 1], 1);
+    if (EDGE) {
+        if (i0 == 0) dm = rel > 1 ? d[0] : 0;
+#pragma unroll
+        for (int q = 0; q < P; q++)
+            if (2 * q + 1 >= rel) d[q] = q ? d[q - 1] : dm;
+    }
+#pragma unroll
+    for (int q = 0; q < P; q++) s[q] = x[2 * q] + (((q ? d[q - 1] : dm) + d[q] + 2) >> 2);
+}
+/* The level with one input per lane: the pairs are lanes 2k, 2k + 1 and the
+ * results belong to lane 2k. */
+template <bool EDGE>
+DEV void fh_level_lanes(int32_t x, int i0, int rel, int32_t& s, int32_t& d) {
+    const int32_t xo = __shfl_down_sync(FULL, x, 1);
+    int32_t next = __shfl_down_sync(FULL, x, 2);
+    if (EDGE && 2 >= rel) next = x;
+    d = xo - ((x + next) >> 1);
+    int32_t dm = __shfl_up_sync(FULL, d, 2);
+    if (EDGE) {
+        if (i0 == 0) dm = rel > 1 ? d : 0;
+        if (1 >= rel) d = dm;
+    }
+    s = x + ((dm + d + 2) >> 2);
+}
+
+/* K coefficients j .. j + K - 1 of a band row per lane (j a multiple of K)
+ * with the GCLIs of their groups.  Lanes that share a group OR their
+ * magnitudes down to the group's first lane.  Coefficients past the band
+ * width are zero, nothing is written past the last group. */
+template <int K, bool EDGE>
+DEV void fh_emit(const BandRow& b, int j, const int32_t* v, bool out_lane) {
+    int32_t t[K];
+#pragma unroll
+    for (int q = 0; q < K; q++) t[q] = !EDGE || j + q < b.w ? v[q] : 0;
+    const int g = j >> 2;
+    const bool ok = out_lane && (!EDGE || g < b.gw);
+    if constexpr (K >= 4) {
+#pragma unroll
+        for (int h = 0; h < K; h += 8) {
+            const uint32_t c0 = sm_pair(t[h], t[h + 1]), c1 = sm_pair(t[h + 2], t[h + 3]);
+            if constexpr (K >= 8) {
+                const uint32_t c2 = sm_pair(t[h + 4], t[h + 5]), c3 = sm_pair(t[h + 6], t[h + 7]);
+                const int gh = g + (h >> 2);
+                if (out_lane && (!EDGE || gh + 1 < b.gw)) {
+                    *(uint4*)(b.crow + j + h) = make_uint4(c0, c1, c2, c3);
+                    *(uint16_t*)(b.grow + gh) = (uint16_t)(gcli_of(c0, c1) | (gcli_of(c2, c3) << 8));
+                } else if (EDGE && out_lane && gh < b.gw) {
+                    *(uint2*)(b.crow + j + h) = make_uint2(c0, c1);
+                    b.grow[gh] = (uint8_t)gcli_of(c0, c1);
+                }
+            } else if (ok) {
+                *(uint2*)(b.crow + j) = make_uint2(c0, c1);
+                b.grow[g] = (uint8_t)gcli_of(c0, c1);
+            }
+        }
+    } else if constexpr (K == 2) {
+        const uint32_t c = sm_pair(t[0], t[1]);
+        const uint32_t m = c | __shfl_down_sync(FULL, c, 1);
+        if (ok) {
+            *(uint32_t*)(b.crow + j) = c;
+            if (!(j & 3)) b.grow[g] = (uint8_t)gcli_of(m, 0u);
+        }
+    } else {
+        const uint32_t c = sm_pair(t[0], 0);
+        uint32_t m = c | __shfl_down_sync(FULL, c, 1);
+        m |= __shfl_down_sync(FULL, m, 2);
+        if (ok) {
+            b.crow[j] = (uint16_t)c;
+            if (!(j & 3)) b.grow[g] = (uint8_t)gcli_of(m, 0u);
+        }
+    }
+}
+/* one coefficient j per lane 2k */
+template <bool EDGE>
+DEV void fh_emit_lanes(const BandRow& b, int j, int32_t v, bool out_lane) {
+    const uint32_t c = sm_pair(!EDGE || j < b.w ? v : 0, 0);
+    uint32_t m = c | __shfl_down_sync(FULL, c, 2);
+    m |= __shfl_down_sync(FULL, m, 4);
+    if (out_lane && !(threadIdx.x & 1) && (!EDGE || (j >> 2) < b.gw)) {
+        b.crow[j] = (uint16_t)c;
+        if (!(j & 3)) b.grow[j >> 2] = (uint8_t)gcli_of(m, 0u);
+    }
+}
+
+/* The lane's 16 input columns; columns outside the row read as anything
+ * in it or as 0 (fh_level never lets them into a result). */
+template <int SRC, bool EDGE>
+DEV void fh_load(const FwdHJob& J, int row, int c0, int32_t* x) {
+    if constexpr (SRC == SRC_I32) {
+        /* rows are padded to a multiple of 4 */
+        const int32_t* r = (const int32_t*)J.src + (size_t)row * J.src_pitch;
+#pragma unroll
+        for (int k = 0; k < FH_COLS; k += 4) {
+            int4 a = make_int4(0, 0, 0, 0);
+            if (!EDGE || (c0 >= 0 && c0 + k < J.w)) a = *(const int4*)(r + c0 + k);
+            x[k] = a.x;
+            x[k + 1] = a.y;
+            x[k + 2] = a.z;
+            x[k + 3] = a.w;
+        }
+    } else {
+        const FvSrc S{(const char*)J.src, (size_t)J.src_pitch * src_elem<SRC>(), J.w, J.chan};
+        const uint32_t mask = (1u << J.depth) - 1u;
+        const int32_t mul = 1 << (20 - J.depth);
+#pragma unroll
+        for (int k = 0; k < FH_COLS; k += 8) {
+            const int c = c0 + k;
+            uint32_t q[4];
+            fv_load<SRC, false>(S, row, EDGE ? min(max(c, 0), J.w - 1) : c, J.vec && c >= 0 && c + 8 <= J.w, q);
+            fv_decode<SRC>(q, mask, mul, x + k);
+        }
+    }
+}
+
+template <int SRC, bool EDGE>
+DEV void fh_chunk(const FwdHJob& J, int row, int c0, bool out_lane) {
+    const int nh = J.nh;
+    int32_t x[16];
+    fh_load<SRC, EDGE>(J, row, c0, x);
+    int m = J.w, b = J.b_ll;
+    if (nh == 0) {
+        fh_emit<16, EDGE>(band_row(J.bands[b], row, J.coef, J.gcli), c0, x, out_lane);
+        return;
+    }
+    int32_t s1[8], d1[8];
+    fh_level<16, EDGE>(x, c0, m - c0, s1, d1);
+    fh_emit<8, EDGE>(band_row(J.bands[J.b_hf[0]], row, J.coef, J.gcli), c0 >> 1, d1, out_lane);
+    m = (m + 1) >> 1;
+    if (nh == 1) {
+        fh_emit<8, EDGE>(band_row(J.bands[b], row, J.coef, J.gcli), c0 >> 1, s1, out_lane);
+        return;
+    }
+    int32_t s2[4], d2[4];
+    fh_level<8, EDGE>(s1, c0 >> 1, m - (c0 >> 1), s2, d2);
+    fh_emit<4, EDGE>(band_row(J.bands[J.b_hf[1]], row, J.coef, J.gcli), c0 >> 2, d2, out_lane);
+    m = (m + 1) >> 1;
+    if (nh == 2) {
+        fh_emit<4, EDGE>(band_row(J.bands[b], row, J.coef, J.gcli), c0 >> 2, s2, out_lane);
+        return;
+    }
+    int32_t s3[2], d3[2];
+    fh_level<4, EDGE>(s2, c0 >> 2, m - (c0 >> 2), s3, d3);
+    fh_emit<2, EDGE>(band_row(J.bands[J.b_hf[2]], row, J.coef, J.gcli), c0 >> 3, d3, out_lane);
+    m = (m + 1) >> 1;
+    if (nh == 3) {
+        fh_emit<2, EDGE>(band_row(J.bands[b], row, J.coef, J.gcli), c0 >> 3, s3, out_lane);
+        return;
+    }
+    int32_t s4[1], d4[1];
+    fh_level<2, EDGE>(s3, c0 >> 3, m - (c0 >> 3), s4, d4);
+    fh_emit<1, EDGE>(band_row(J.bands[J.b_hf[3]], row, J.coef, J.gcli), c0 >> 4, d4, out_lane);
+    m = (m + 1) >> 1;
+    if (nh == 4) {
+        fh_emit<1, EDGE>(band_row(J.bands[b], row, J.coef, J.gcli), c0 >> 4, s4, out_lane);
+        return;
+    }
+    int32_t s5, d5;
+    fh_level_lanes<EDGE>(s4[0], c0 >> 4, m - (c0 >> 4), s5, d5);
+    fh_emit_lanes<EDGE>(band_row(J.bands[J.b_hf[4]], row, J.coef, J.gcli), c0 >> 5, d5, out_lane);
+    fh_emit_lanes<EDGE>(band_row(J.bands[b], row, J.coef, J.gcli), c0 >> 5, s5, out_lane);
 }
 
 template <int SRC, int NJ>
 __global__ void __launch_bounds__(FH_MAX_WARPS * 32) fwd_h_kernel(const __grid_constant__ FwdHLaunchN<NJ> L) {
-    extern __shared__ __align__(16) int32_t hsm[];
     const FwdHJob& J = L.job[find_job<NJ>(L.job, L.njobs, (int)blockIdx.x)];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int row = (blockIdx.x - J.first_block) * L.rows_per_block + warp;
-    if (row >= J.h) return;
-    const int n = J.w;
-    /* per warp: buffer A (n + 8 words) and buffer B (n/2 + 8 words) */
-    int32_t* bufA = hsm + warp * L.warp_words + 4;
-    int32_t* bufB = bufA + ((n + 8 + 3) & ~3);
-    for (int x = lane; x < n; x += 32) bufA[x] = load1<SRC>(J.src, J.src_pitch, J.chan, J.depth, row, x);
-    __syncwarp();
-    fill_halo(bufA, n, lane);
-    __syncwarp();
-    int32_t* cur = bufA;
-    int32_t* nxt = bufB;
-    int m = n;
-    for (int e = 0; e < J.nh; e++) {
-        if (m == 1) break; /* nothing left to split: the remaining high bands are empty */
-        const BandRow bd = band_row(J.bands[J.b_hf[e]], row, J.coef, J.gcli);
-        const int m1 = (m + 1) >> 1;
-        int32_t* dst = nxt;
-        warp_lift_fwd(cur, m1, [&](int j, const int32_t* sv, const int32_t* d) {
-            emit4(bd, j, d[0], d[1], d[2], d[3]);
-            if (j + 3 < m1) {
-                *(int4*)(dst + j) = make_int4(sv[0], sv[1], sv[2], sv[3]);
-            } else {
-                for (int q = 0; q < 4; q++)
-                    if (j + q < m1) dst[j + q] = sv[q];
-            }
-        });
-        __syncwarp();
-        fill_halo(dst, m1, lane);
-        __syncwarp();
-        nxt = cur;
-        cur = dst;
-        m = m1;
-    }
-    /* final low band */
-    const BandRow bl = band_row(J.bands[J.b_ll], row, J.coef, J.gcli);
-    for (int j = 4 * lane; j < m; j += 128) {
-        int32_t v[4];
-        for (int q = 0; q < 4; q++) v[q] = j + q < m ? cur[j + q] : 0;
-        emit4(bl, j, v[0], v[1], v[2], v[3]);
-    }
+    const int unit = (blockIdx.x - J.first_block) * L.rows_per_block + warp;
+    const int row = unit / J.chunks, ch = unit - row * J.chunks;
+    if (row >= J.h) return; /* the whole warp */
+    const int halo = fh_halo_lanes(J.nh), first = ch * fh_net_cols(J.nh) - FH_COLS * halo;
+    const int c0 = first + FH_COLS * lane;
+    const bool out_lane = lane >= halo && lane < 32 - halo && c0 < J.w;
+    if (first >= 0 && first + 32 * FH_COLS <= J.w) fh_chunk<SRC, false>(J, row, c0, out_lane);
+    else fh_chunk<SRC, true>(J, row, c0, out_lane);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -464,6 +569,7 @@ __global__ void __launch_bounds__(FH_MAX_WARPS * 32) fwd_h_kernel(const __grid_c
 extern "C" int jxs_fwd_v_tile_rows(void) { return FV_ROWPAIRS; }
 extern "C" int jxs_fwd_v_tile_cols(void) { return FV_COLS; }
 extern "C" int jxs_fwd_h_max_rows_per_block(void) { return FH_MAX_WARPS; }
+extern "C" int jxs_fwd_h_chunk_cols(int nh) { return fh_net_cols(nh); }
 
 template <int SRC, int NJ>
 static cudaError_t launch_v(const FwdVLaunchN<NJ>* L, int grid_per_sm, cudaStream_t st) {
@@ -493,12 +599,8 @@ extern "C" cudaError_t jxs_launch_fwd_v_batch(const FwdVLaunchB* L, int src_kind
 
 template <int SRC, int NJ>
 static cudaError_t launch_h(const FwdHLaunchN<NJ>* L, int nblocks, cudaStream_t st) {
-    const size_t smem = (size_t)L->warp_words * L->rows_per_block * sizeof(int32_t);
-    static std::atomic<int> attr[JXS_MAX_DEV];
-    cudaError_t e = jxs_smem_attr(fwd_h_kernel<SRC, NJ>, (int)smem, attr);
-    if (e != cudaSuccess) return e;
     if (nblocks <= 0) return cudaSuccess;
-    fwd_h_kernel<SRC, NJ><<<nblocks, L->rows_per_block * 32, smem, st>>>(*L);
+    fwd_h_kernel<SRC, NJ><<<nblocks, L->rows_per_block * 32, 0, st>>>(*L);
     return cudaGetLastError();
 }
 

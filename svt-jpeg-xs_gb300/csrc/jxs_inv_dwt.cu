@@ -1,11 +1,11 @@
 /*
  * Inverse 5/3 wavelet transform for sm_103a.
  *
- *  inv_h_kernel  the horizontal-only levels, deepest first: one warp per row
- *                combines the final LL band with the high band of each level
- *                (in shared memory) and writes the row of the last vertical
- *                level's low band, or, for a component without vertical
- *                levels, the output samples.
+ *  inv_h_kernel  the horizontal-only levels, deepest first: one warp per
+ *                chunk of a row combines the final LL band with the high band
+ *                of each level (in registers) and writes the row of the last
+ *                vertical level's low band, or, for a component without
+ *                vertical levels, the output samples.
  *  inv_v_kernel  one vertical level: each warp streams down a strip of 240
  *                output columns (8 per lane, plus one halo lane on either
  *                side) for 8 row pairs.  Every step rebuilds a low row (LL +
@@ -29,8 +29,6 @@
 
 #define DEV __device__ __forceinline__
 #define FULL 0xffffffffu
-
-DEV int32_t dq(int16_t c, int fq) { return (int32_t)((uint32_t)(int32_t)c << fq); }
 
 /* linear_output_scaling (NltDec.c:242-264).  The reference adds 2^(Bw-1) in
  * int32, then rounds (v + 2^(zeta-1)) >> zeta in int64 and clamps to
@@ -68,139 +66,198 @@ DEV CoefRow coef_row(const jxs_band_t& bd, int r, const int16_t* coef) {
     return c;
 }
 
-/* Inverse horizontal lifting of one row by one warp, 4 pairs per lane.
- * sget(i) / dget(i) return the low / high band value i for i in [0, n1) /
- * [0, n2) (any value outside); get4(...) variants load four at once.  Pairs
- * j in [j0, j0 + npairs) are produced (j0 a multiple of 4) and passed to
- * out(j, xe[4], xo[4]): x[2j + 2q] = xe[q], x[2j + 2q + 1] = xo[q]. */
-template <typename S4, typename D4, typename S1, typename D1, typename Out>
-DEV void warp_lift_inv(int j0, int npairs, int n1, int n2, S4 s4, D4 d4, S1 s1, D1 d1, Out out) {
-    const int lane = threadIdx.x & 31;
-    /* symmetric extension of the high band: d[-1] = d[0], d[n2] = d[n2-1] */
-    auto dm = [&](int i) { return n2 == 0 ? 0 : d1(i < 0 ? 0 : (i >= n2 ? n2 - 1 : i)); };
-    int32_t carry = dm(j0 - 1);
-    for (int base = 0; base < npairs; base += 128) {
-        const int j = j0 + base + 4 * lane;
-        int32_t s[4], d[4];
-        s4(j, s);
-        d4(j, d);
-        /* high values past the band: mirrored */
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-            if (j + q >= n2) d[q] = dm(j + q);
-        int32_t dp = __shfl_up_sync(FULL, d[3], 1);
-        if (lane == 0) dp = carry;
-        carry = __shfl_sync(FULL, d[3], 31);
-        int32_t xe[4], xo[4];
-        xe[0] = s[0] - ((dp + d[0] + 2) >> 2);
-        xe[1] = s[1] - ((d[0] + d[1] + 2) >> 2);
-        xe[2] = s[2] - ((d[1] + d[2] + 2) >> 2);
-        xe[3] = s[3] - ((d[2] + d[3] + 2) >> 2);
-        int32_t xn = __shfl_down_sync(FULL, xe[0], 1);
-        if (lane == 31 && j + 4 < n1) xn = s1(j + 4) - ((d[3] + dm(j + 4) + 2) >> 2);
-        /* x[n] = x[n-2] for even widths: the last even sample is its own
-         * right neighbour */
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            const int32_t nx = (j + q + 1 >= n1) ? xe[q] : (q < 3 ? xe[q + 1] : xn);
-            xo[q] = d[q] + ((xe[q] + nx) >> 1);
-        }
-        if (j < j0 + npairs) out(j, xe, xo);
-    }
-}
-
 /* ------------------------------------------------------------------------ */
 /* horizontal-only levels                                                    */
 /* ------------------------------------------------------------------------ */
+/* A warp rebuilds one chunk of one row through every level in registers:
+ * lane l ends with the 16 output columns c0 = first - 16 halo + 16 l .. c0 +
+ * 15, so that a level takes 8, 4, 2, 1 low and high values per lane and, at
+ * level 5, one pair per two lanes.  A sample needs the high value before its
+ * pair (left lane) and the next pair's even sample (right lane), which in
+ * turn needs only the first values of that lane and the high value before
+ * them: one halo lane on either side, or two where level 5 pairs lanes.  A
+ * chunk yields 480 or 448 columns.
+ *
+ * Bound by memory: 2 bytes read and 4 written per column.  The form before
+ * kept whole rows in shared memory, one warp per row, which left few warps
+ * on an SM for wide rows: 8 8K frames with one vertical level (3840-column
+ * rows) took 1050 us, now 220 (1.2 GB; decode 3081 -> 2249 us). */
 #define IH_MAX_WARPS 4
+#define IH_COLS 16
 
-template <int OUT>
-DEV void store_row8(const InvHJob& J, int row, int x0, int w, const int32_t* v, const OutScale& os) {
-    if (OUT == 0) {
-        int32_t* dst = (int32_t*)J.dst + (long long)row * J.dst_pitch + x0;
-        if (x0 + 7 < w) {
-            *(int4*)dst = make_int4(v[0], v[1], v[2], v[3]);
-            *(int4*)(dst + 4) = make_int4(v[4], v[5], v[6], v[7]);
+static inline __host__ __device__ int ih_halo_lanes(int nh) { return nh >= 5 ? 2 : 1; }
+static inline __host__ __device__ int ih_net_cols(int nh) { return IH_COLS * (32 - 2 * ih_halo_lanes(nh)); }
+
+/* K coefficients j .. j + K - 1 of a band row (j a multiple of K) as int32
+ * << fq; indices outside the band read as 0 or as row padding (ih_level
+ * never lets them into a result). */
+template <int K, bool EDGE>
+DEV void ih_load(const CoefRow& b, int j, int fq, int32_t* v) {
+    uint32_t w[(K + 1) / 2];
+#pragma unroll
+    for (int k = 0; k < (K + 1) / 2; k++) w[k] = 0u;
+    if constexpr (K >= 8) {
+        /* rows are padded to a multiple of 8 */
+#pragma unroll
+        for (int h = 0; h < K; h += 8)
+            if (!EDGE || (j >= 0 && j + h < b.w)) {
+                const uint4 a = *(const uint4*)(b.row + j + h);
+                w[h / 2] = a.x;
+                w[h / 2 + 1] = a.y;
+                w[h / 2 + 2] = a.z;
+                w[h / 2 + 3] = a.w;
+            }
+    } else if (!EDGE || (j >= 0 && j < b.w)) {
+        if constexpr (K == 4) {
+            const uint2 a = *(const uint2*)(b.row + j);
+            w[0] = a.x;
+            w[1] = a.y;
+        } else if constexpr (K == 2) {
+            w[0] = *(const uint32_t*)(b.row + j);
         } else {
-            for (int q = 0; q < 8; q++)
-                if (x0 + q < w) dst[q] = v[q];
-        }
-    } else {
-        for (int q = 0; q < 8; q++) {
-            if (x0 + q >= w) break;
-            const uint32_t o = out_sample(v[q], os);
-            const long long idx = (long long)row * J.dst_pitch + x0 + q;
-            if (OUT == 1) ((uint8_t*)J.dst)[idx] = (uint8_t)o;
-            else ((uint16_t*)J.dst)[idx] = (uint16_t)o;
+            w[0] = (uint16_t)b.row[j];
         }
     }
+#pragma unroll
+    for (int k = 0; k < K; k++) v[k] = (k & 1) ? (int32_t)(w[k >> 1] & 0xffff0000u) >> (16 - fq) : (int32_t)(w[k >> 1] << 16) >> (16 - fq);
+}
+
+/* One level: the lane's P low and high values (pairs j0 .. j0 + P - 1 of n1
+ * even and n2 odd samples) to its 2 P samples.  EDGE: the chunk touches an
+ * end of the row, where the symmetric extension holds: high values past
+ * either end are the nearest one, past the last even sample it is its own
+ * right neighbour. */
+template <int P, bool EDGE>
+DEV void ih_level(const int32_t* s, int32_t* d, int j0, int n1, int n2, int32_t* x) {
+    int32_t dm = __shfl_up_sync(FULL, d[P - 1], 1);
+    if (EDGE) {
+        if (j0 == 0) dm = n2 > 0 ? d[0] : 0;
+#pragma unroll
+        for (int q = 0; q < P; q++)
+            if (j0 + q >= n2) d[q] = q ? d[q - 1] : dm;
+    }
+#pragma unroll
+    for (int q = 0; q < P; q++) x[2 * q] = s[q] - (((q ? d[q - 1] : dm) + d[q] + 2) >> 2);
+    const int32_t xn = __shfl_down_sync(FULL, x[0], 1);
+#pragma unroll
+    for (int q = 0; q < P; q++) {
+        int32_t next = q + 1 < P ? x[2 * q + 2] : xn;
+        if (EDGE && j0 + q + 1 >= n1) next = x[2 * q];
+        x[2 * q + 1] = d[q] + ((x[2 * q] + next) >> 1);
+    }
+}
+/* The level with one pair (index j) per lanes 2k, 2k + 1, held by both: lane
+ * 2k gets the even sample, lane 2k + 1 the odd one. */
+template <bool EDGE>
+DEV int32_t ih_level_lanes(int32_t s, int32_t d, int j, int n1, int n2) {
+    int32_t dm = __shfl_up_sync(FULL, d, 2);
+    if (EDGE) {
+        if (j == 0) dm = n2 > 0 ? d : 0;
+        if (j >= n2) d = dm;
+    }
+    const int32_t xe = s - ((dm + d + 2) >> 2);
+    int32_t next = __shfl_down_sync(FULL, xe, 2);
+    if (EDGE && j + 1 >= n1) next = xe;
+    return (threadIdx.x & 1) ? d + ((xe + next) >> 1) : xe;
+}
+
+/* The lane's 16 samples of row `row` from column c0 (c0 < w). */
+template <int OUT, bool EDGE>
+DEV void ih_store(const InvHJob& J, int row, int c0, const int32_t* x, const OutScale& os) {
+    if constexpr (OUT == 0) {
+        /* rows are padded to a multiple of 4 */
+        int32_t* dst = (int32_t*)J.dst + (size_t)row * J.dst_pitch + c0;
+#pragma unroll
+        for (int k = 0; k < IH_COLS; k += 4)
+            if (!EDGE || c0 + k < J.w) *(int4*)(dst + k) = make_int4(x[k], x[k + 1], x[k + 2], x[k + 3]);
+    } else {
+        /* samples: vector stores where the rows are aligned */
+        const int esz = OUT;
+        uint8_t* dst = (uint8_t*)J.dst + ((size_t)row * J.dst_pitch + c0) * esz;
+        const bool vec = (((uintptr_t)J.dst | ((size_t)J.dst_pitch * esz)) & 15) == 0;
+        uint32_t o[16];
+#pragma unroll
+        for (int k = 0; k < IH_COLS; k++) o[k] = out_sample(x[k], os);
+        if (vec && (!EDGE || c0 + IH_COLS <= J.w)) {
+            uint32_t w[4 * OUT];
+#pragma unroll
+            for (int k = 0; k < 4 * OUT; k++)
+                w[k] = OUT == 1 ? o[4 * k] | (o[4 * k + 1] << 8) | (o[4 * k + 2] << 16) | (o[4 * k + 3] << 24)
+                                : o[2 * k] | (o[2 * k + 1] << 16);
+#pragma unroll
+            for (int k = 0; k < 4 * OUT; k += 4) *(uint4*)(dst + 4 * k) = make_uint4(w[k], w[k + 1], w[k + 2], w[k + 3]);
+        } else {
+#pragma unroll
+            for (int k = 0; k < IH_COLS; k++) {
+                if (EDGE && c0 + k >= J.w) break;
+                if constexpr (OUT == 1) dst[k] = (uint8_t)o[k];
+                else ((uint16_t*)dst)[k] = (uint16_t)o[k];
+            }
+        }
+    }
+}
+
+template <int OUT, bool EDGE>
+DEV void ih_chunk(const InvHJob& J, int row, int c0, bool out_lane, const OutScale& os) {
+    const int fq = J.fq, nh = J.nh;
+    auto brow = [&](int b) { return coef_row(J.bands[b], row, J.coef); };
+    int m[6]; /* the row's length at every level */
+    m[0] = J.w;
+#pragma unroll
+    for (int e = 0; e < 5; e++) m[e + 1] = (m[e] + 1) >> 1;
+    int32_t x[16];
+    if (nh == 0) {
+        ih_load<16, EDGE>(brow(J.b_ll), c0, fq, x);
+    } else {
+        int32_t d1[8], s1[8];
+        ih_load<8, EDGE>(brow(J.b_hf[0]), c0 >> 1, fq, d1);
+        if (nh == 1) {
+            ih_load<8, EDGE>(brow(J.b_ll), c0 >> 1, fq, s1);
+        } else {
+            int32_t d2[4], s2[4];
+            ih_load<4, EDGE>(brow(J.b_hf[1]), c0 >> 2, fq, d2);
+            if (nh == 2) {
+                ih_load<4, EDGE>(brow(J.b_ll), c0 >> 2, fq, s2);
+            } else {
+                int32_t d3[2], s3[2];
+                ih_load<2, EDGE>(brow(J.b_hf[2]), c0 >> 3, fq, d3);
+                if (nh == 3) {
+                    ih_load<2, EDGE>(brow(J.b_ll), c0 >> 3, fq, s3);
+                } else {
+                    int32_t d4[1], s4[1];
+                    ih_load<1, EDGE>(brow(J.b_hf[3]), c0 >> 4, fq, d4);
+                    if (nh == 4) {
+                        ih_load<1, EDGE>(brow(J.b_ll), c0 >> 4, fq, s4);
+                    } else {
+                        int32_t d5[1], s5[1];
+                        ih_load<1, EDGE>(brow(J.b_hf[4]), c0 >> 5, fq, d5);
+                        ih_load<1, EDGE>(brow(J.b_ll), c0 >> 5, fq, s5);
+                        s4[0] = ih_level_lanes<EDGE>(s5[0], d5[0], c0 >> 5, m[5], m[4] >> 1);
+                    }
+                    ih_level<1, EDGE>(s4, d4, c0 >> 4, m[4], m[3] >> 1, s3);
+                }
+                ih_level<2, EDGE>(s3, d3, c0 >> 3, m[3], m[2] >> 1, s2);
+            }
+            ih_level<4, EDGE>(s2, d2, c0 >> 2, m[2], m[1] >> 1, s1);
+        }
+        ih_level<8, EDGE>(s1, d1, c0 >> 1, m[1], m[0] >> 1, x);
+    }
+    if (out_lane) ih_store<OUT, EDGE>(J, row, c0, x, os);
 }
 
 template <int OUT, int NJ>
 __global__ void __launch_bounds__(IH_MAX_WARPS * 32) inv_h_kernel(const __grid_constant__ InvHLaunchN<NJ> L) {
-    extern __shared__ __align__(16) int32_t ism[];
     const InvHJob& J = L.job[find_job<NJ>(L.job, L.njobs, (int)blockIdx.x)];
-    const jxs_band_t* __restrict__ bands = J.bands;
-    const int16_t* __restrict__ coef = J.coef;
-    const int warp = threadIdx.x >> 5;
-    const int row = (blockIdx.x - J.first_block) * L.rows_per_block + warp;
-    if (row >= J.h) return;
-    const int fq = J.fq;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int unit = (blockIdx.x - J.first_block) * L.rows_per_block + warp;
+    const int row = unit / J.chunks, ch = unit - row * J.chunks;
+    if (row >= J.h) return; /* the whole warp */
+    const int halo = ih_halo_lanes(J.nh), first = ch * ih_net_cols(J.nh) - IH_COLS * halo;
+    const int c0 = first + IH_COLS * lane;
+    const bool out_lane = lane >= halo && lane < 32 - halo && c0 < J.w;
     const OutScale os = out_scale(J.bw, J.depth);
-    int32_t* bufA = ism + warp * L.warp_words;
-    int32_t* bufB = bufA + L.warp_words / 2;
-    /* widths of every level's input, m[0] = row width */
-    int m[6];
-    m[0] = J.w;
-    for (int e = 0; e < J.nh; e++) m[e + 1] = (m[e] + 1) >> 1;
-    const CoefRow llr = coef_row(bands[J.b_ll], row, coef);
-    const int32_t* cur = nullptr; /* int32 low band of the level being rebuilt (null: the LL band) */
-    int32_t* nxt = bufA;
-    for (int e = J.nh - 1; e >= -1; e--) {
-        if (e == -1) {
-            /* no horizontal-only level: the LL band is the row */
-            if (J.nh > 0) break;
-            const int w = J.w;
-            for (int x0 = 8 * (threadIdx.x & 31); x0 < w; x0 += 256) {
-                int32_t v[8];
-                for (int q = 0; q < 8; q++) v[q] = x0 + q < w ? dq(llr.row[x0 + q], fq) : 0;
-                store_row8<OUT>(J, row, x0, w, v, os);
-            }
-            break;
-        }
-        const int n = m[e], n1 = m[e + 1], n2 = n >> 1;
-        const CoefRow hr = coef_row(bands[J.b_hf[e]], row, coef);
-        const int32_t* sc = cur;
-        auto s4 = [&](int j, int32_t* s) {
-            if (sc) {
-                for (int q = 0; q < 4; q++) s[q] = j + q < n1 ? sc[j + q] : 0;
-            } else {
-                for (int q = 0; q < 4; q++) s[q] = j + q < n1 ? dq(llr.row[j + q], fq) : 0;
-            }
-        };
-        auto s1 = [&](int j) { return sc ? sc[j] : dq(llr.row[j], fq); };
-        auto d4 = [&](int j, int32_t* d) {
-            for (int q = 0; q < 4; q++) d[q] = j + q < n2 ? dq(hr.row[j + q], fq) : 0;
-        };
-        auto d1 = [&](int j) { return dq(hr.row[j], fq); };
-        if (e > 0) {
-            int32_t* dst = nxt;
-            warp_lift_inv(0, n1, n1, n2, s4, d4, s1, d1, [&](int j, const int32_t* xe, const int32_t* xo) {
-                for (int q = 0; q < 4; q++) {
-                    if (2 * (j + q) < n) dst[2 * (j + q)] = xe[q];
-                    if (2 * (j + q) + 1 < n) dst[2 * (j + q) + 1] = xo[q];
-                }
-            });
-            __syncwarp();
-            cur = dst;
-            nxt = (dst == bufA) ? bufB : bufA;
-        } else {
-            warp_lift_inv(0, n1, n1, n2, s4, d4, s1, d1, [&](int j, const int32_t* xe, const int32_t* xo) {
-                const int32_t v[8] = {xe[0], xo[0], xe[1], xo[1], xe[2], xo[2], xe[3], xo[3]};
-                store_row8<OUT>(J, row, 2 * j, n, v, os);
-            });
-        }
-    }
+    if (first >= 0 && first + 32 * IH_COLS <= J.w) ih_chunk<OUT, false>(J, row, c0, out_lane, os);
+    else ih_chunk<OUT, true>(J, row, c0, out_lane, os);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -484,6 +541,7 @@ __global__ void __launch_bounds__(IV_THREADS) inv_v_kernel(const __grid_constant
 extern "C" int jxs_inv_v_tile_rows(void) { return IV_ROWPAIRS; }
 extern "C" int jxs_inv_v_tile_cols(void) { return IV_COLS; }
 extern "C" int jxs_inv_h_max_rows_per_block(void) { return IH_MAX_WARPS; }
+extern "C" int jxs_inv_h_chunk_cols(int nh) { return ih_net_cols(nh); }
 
 template <int OUT, int NJ>
 static cudaError_t launch_iv(const InvVLaunchN<NJ>* L, int nblocks, cudaStream_t st) {
@@ -505,12 +563,8 @@ extern "C" cudaError_t jxs_launch_inv_v_batch(const InvVLaunchB* L, int out_kind
 
 template <int OUT, int NJ>
 static cudaError_t launch_ih(const InvHLaunchN<NJ>* L, int nblocks, cudaStream_t st) {
-    const size_t smem = (size_t)L->warp_words * L->rows_per_block * sizeof(int32_t);
-    static std::atomic<int> attr[JXS_MAX_DEV];
-    cudaError_t e = jxs_smem_attr(inv_h_kernel<OUT, NJ>, (int)smem, attr);
-    if (e != cudaSuccess) return e;
     if (nblocks <= 0) return cudaSuccess;
-    inv_h_kernel<OUT, NJ><<<nblocks, L->rows_per_block * 32, smem, st>>>(*L);
+    inv_h_kernel<OUT, NJ><<<nblocks, L->rows_per_block * 32, 0, st>>>(*L);
     return cudaGetLastError();
 }
 

@@ -78,12 +78,15 @@ typedef FwdVLaunchN<JXS_MAXC> FwdVLaunch;
 typedef FwdVLaunchN<JXS_BATCH_JOBS> FwdVLaunchB;
 
 /* Forward transform, horizontal-only levels: rows [0, h) of a w-wide
- * plane, rows_per_block rows (one warp each) per block. */
+ * plane, each in `chunks` chunks of one warp; rows_per_block warps per
+ * block. */
 struct FwdHJob {
     const void* src;
     long long src_pitch;
     int chan;
+    int vec;                /* as FwdVJob.vec */
     int w, h;
+    int chunks;
     int first_block;
     int nh;                 /* levels */
     int b_hf[5];            /* high band of each level */
@@ -96,7 +99,6 @@ struct FwdHJob {
 template <int NJ> struct FwdHLaunchN {
     int njobs;
     int rows_per_block;
-    int warp_words;         /* shared-memory words per warp */
     FwdHJob job[NJ];
 };
 typedef FwdHLaunchN<JXS_MAXC> FwdHLaunch;
@@ -124,9 +126,11 @@ template <int NJ> struct InvVLaunchN {
 typedef InvVLaunchN<JXS_MAXC> InvVLaunch;
 typedef InvVLaunchN<JXS_BATCH_JOBS> InvVLaunchB;
 
-/* Inverse transform, horizontal-only levels: rows [0, h) of width w. */
+/* Inverse transform, horizontal-only levels: rows [0, h) of width w, each
+ * in `chunks` chunks of one warp. */
 struct InvHJob {
     int w, h;
+    int chunks;
     int first_block;
     int nh;
     int b_hf[5], b_ll;
@@ -138,7 +142,7 @@ struct InvHJob {
 };
 template <int NJ> struct InvHLaunchN {
     int njobs;
-    int rows_per_block, warp_words;
+    int rows_per_block;
     InvHJob job[NJ];
 };
 typedef InvHLaunchN<JXS_MAXC> InvHLaunch;

@@ -24,6 +24,7 @@ extern "C" cudaError_t jxs_launch_fwd_h_batch(const FwdHLaunchB* L, int src_kind
 extern "C" int jxs_fwd_v_tile_rows(void);
 extern "C" int jxs_fwd_v_tile_cols(void);
 extern "C" int jxs_fwd_h_max_rows_per_block(void);
+extern "C" int jxs_fwd_h_chunk_cols(int nh);
 extern "C" cudaError_t jxs_launch_rc(const jxs_cfg_t* dcfg, uint32_t np, uint32_t nslices, const uint8_t* gcli,
                                      const uint16_t* coef, uint32_t* cost, uint32_t* slice_done, PrecRC* rc, int* status,
                                      int modes, cudaStream_t st);
@@ -52,6 +53,7 @@ extern "C" cudaError_t jxs_launch_star_tetrix(const StParams* P, cudaStream_t st
 extern "C" int jxs_inv_v_tile_rows(void);
 extern "C" int jxs_inv_v_tile_cols(void);
 extern "C" int jxs_inv_h_max_rows_per_block(void);
+extern "C" int jxs_inv_h_chunk_cols(int nh);
 
 static const size_t kSmemMax = 220 * 1024;
 
@@ -269,11 +271,13 @@ static inline int plan_fwd_h(const jxs_cfg_t* c, const jxs_cfg_t* dcfg, const Fr
             J.src = in.p[packed ? 0 : k];
             J.src_pitch = in.pitch[packed ? 0 : k];
             J.chan = packed ? (int)k : 0;
+            J.vec = !packed && ((uintptr_t)J.src % (8 * bytes_per_sample(c))) == 0 && (J.src_pitch % 8) == 0;
         }
         DwtJob bj;
         memset(&bj, 0, sizeof(bj));
         job_bands(c, (int)k, cp.dv > 0 ? (int)cp.dv - 1 : 0, &bj);
         J.nh = bj.nh;
+        J.chunks = (int)div_up(w, (uint32_t)jxs_fwd_h_chunk_cols(J.nh));
         for (int e = 0; e < 5; e++) J.b_hf[e] = bj.b_hf[e];
         J.b_ll = bj.b_ll;
         J.depth = (int)c->depth;
@@ -305,6 +309,7 @@ static inline int plan_inv_h(const jxs_cfg_t* c, const jxs_cfg_t* dcfg, const Fr
         memset(&bj, 0, sizeof(bj));
         job_bands(c, (int)k, cp.dv > 0 ? (int)cp.dv - 1 : 0, &bj);
         J.nh = bj.nh;
+        J.chunks = (int)div_up(w, (uint32_t)jxs_inv_h_chunk_cols(J.nh));
         for (int e = 0; e < 5; e++) J.b_hf[e] = bj.b_hf[e];
         J.b_ll = bj.b_ll;
         if (cp.dv > c->proxy) {
@@ -367,41 +372,26 @@ static inline int plan_inv_v(const jxs_cfg_t* c, const jxs_cfg_t* dcfg, const Fr
     return n;
 }
 
-/* Shared-memory layout and block numbering of a horizontal-only launch:
- * rows_per_block is the largest power of two <= max_rpb whose buffers fit;
- * returns the block count, or -1 when one row does not fit. */
+/* Block numbering of a horizontal-only launch, rpb chunks (one warp each)
+ * per block; returns the block count, or -1 for a row of more than max_w
+ * columns. */
 template <class LT>
-static inline int fwd_h_layout(LT& L, int max_rpb) {
-    int maxw = 0;
-    for (int i = 0; i < L.njobs; i++) maxw = L.job[i].w > maxw ? L.job[i].w : maxw;
-    L.warp_words = 4 + ((maxw + 8 + 3) & ~3) + (((maxw + 1) / 2 + 8 + 3) & ~3) + 4;
-    int rpb = max_rpb;
-    while (rpb > 1 && (size_t)L.warp_words * rpb * 4 > kSmemMax) rpb >>= 1;
-    if ((size_t)L.warp_words * rpb * 4 > kSmemMax) return -1;
-    L.rows_per_block = rpb;
+static inline int h_layout(LT& L, int rpb, int max_w) {
     int blocks = 0;
+    L.rows_per_block = rpb;
     for (int i = 0; i < L.njobs; i++) {
+        if (L.job[i].w > max_w) return -1;
         L.job[i].first_block = blocks;
-        blocks += (int)div_up((uint32_t)L.job[i].h, (uint32_t)rpb);
+        blocks += (int)div_up((uint32_t)L.job[i].h * (uint32_t)L.job[i].chunks, (uint32_t)rpb);
     }
     return blocks;
 }
-
+/* The widest rows taken (larger frames are refused). */
+#define JXS_FWD_H_MAX_W 37528
+#define JXS_INV_H_MAX_W 56304
 template <class LT>
-static inline int inv_h_layout(LT& L, int max_rpb) {
-    int maxw = 0;
-    for (int i = 0; i < L.njobs; i++) maxw = L.job[i].w > maxw ? L.job[i].w : maxw;
-    L.warp_words = 2 * ((((maxw + 1) / 2) + 8 + 3) & ~3);
-    int rpb = max_rpb;
-    while (rpb > 1 && (size_t)L.warp_words * rpb * 4 > kSmemMax) rpb >>= 1;
-    if ((size_t)L.warp_words * rpb * 4 > kSmemMax) return -1;
-    L.rows_per_block = rpb;
-    int blocks = 0;
-    for (int i = 0; i < L.njobs; i++) {
-        L.job[i].first_block = blocks;
-        blocks += (int)div_up((uint32_t)L.job[i].h, (uint32_t)rpb);
-    }
-    return blocks;
-}
+static inline int fwd_h_layout(LT& L, int rpb) { return h_layout(L, rpb, JXS_FWD_H_MAX_W); }
+template <class LT>
+static inline int inv_h_layout(LT& L, int rpb) { return h_layout(L, rpb, JXS_INV_H_MAX_W); }
 
 #endif
