@@ -174,7 +174,7 @@ static uint64_t enc_work_layout(const jxs_cfg_t* c, uint8_t* base, EncWork* w) {
     uint64_t in_bytes = 0;
     memset(w->in_off, 0, sizeof(w->in_off));
     if (c->fmt == COLOUR_FORMAT_PACKED_YUV444_OR_RGB) {
-        in_bytes = (uint64_t)c->W * c->H * 3 * bps;
+        in_bytes = (uint64_t)stage_pitch(c->W * 3, bps) * c->H * bps;
     } else {
         for (uint32_t k = 0; k < c->nc; k++) {
             w->in_off[k] = in_bytes;
@@ -399,10 +399,14 @@ static int32_t plan_encode_chain(const std::vector<EncItem>& it, const std::vect
                 }
                 memset(L, 0, sizeof(*L));
             };
+            uint32_t warps = 0;
+            for (int f : fr)
+                if (v > 0 || enc_level0_kind(it[f].c) == kind) warps += v_warps(it[f].c, v, (uint32_t)jxs_fwd_v_tile_cols());
+            const int rp = v_rowpairs(warps);
             for (int f : fr) {
                 const EncItem& e = it[f];
                 if (v == 0 && enc_level0_kind(e.c) != kind) continue;
-                const int nj = plan_fwd_v(e.c, e.dcfg, e.w->fb, e.in, v, vj, tiles);
+                const int nj = plan_fwd_v(e.c, e.dcfg, e.w->fb, e.in, v, rp, vj, tiles);
                 for (int j = 0; j < nj; j++) {
                     if (L->njobs == JXS_BATCH_JOBS) flush();
                     vj[j].first_block = L->ntiles;
@@ -584,10 +588,15 @@ static int32_t plan_decode_chain(const std::vector<DecItem>& it, const std::vect
             };
             InvVJob vj[JXS_MAXC];
             int tiles[JXS_MAXC];
+            uint32_t warps = 0;
+            for (int f : fr)
+                if ((v > (int)it[f].c->proxy ? 0 : dec_sample_kind(it[f].c)) == ok)
+                    warps += v_warps(it[f].c, v, (uint32_t)jxs_inv_v_tile_cols());
+            const int rp = v_rowpairs(warps);
             for (int f : fr) {
                 const DecItem& d = it[f];
                 if ((v > (int)d.c->proxy ? 0 : dec_sample_kind(d.c)) != ok) continue;
-                const int nj = plan_inv_v(d.c, d.dcfg, d.w->fb, d.out, v, vj, tiles);
+                const int nj = plan_inv_v(d.c, d.dcfg, d.w->fb, d.out, v, rp, vj, tiles);
                 for (int j = 0; j < nj; j++) {
                     if (L->njobs == JXS_BATCH_JOBS) flush();
                     vj[j].first_block = blocks;
@@ -1123,7 +1132,7 @@ extern "C" int32_t jxs_gpu_batch_encode(jxs_gpu_batch_t* b, jxs_gpu_enc_t* const
                 e.in.pitch[k] = strides[i][k];
             } else {
                 uint8_t* d = w.in_stage + w.in_off[k];
-                const uint32_t sp = packed ? pw : stage_pitch(pw, bps);
+                const uint32_t sp = stage_pitch(pw, bps);
                 BCK(cudaMemcpy2DAsync(d, (size_t)sp * bps, planes[i][k], (size_t)strides[i][k] * bps, (size_t)pw * bps, ph,
                                       cudaMemcpyHostToDevice, st));
                 e.in.p[k] = d;

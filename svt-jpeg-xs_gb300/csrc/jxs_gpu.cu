@@ -281,7 +281,7 @@ static int32_t enc_slot_alloc(jxs_gpu_enc_t* e, EncSlot* s) {
     const uint32_t bps = bytes_per_sample(c);
     if (c->fmt == COLOUR_FORMAT_PACKED_YUV444_OR_RGB) {
         s->in_off[0] = 0;
-        in_bytes = (uint64_t)c->W * c->H * 3 * bps;
+        in_bytes = (uint64_t)stage_pitch(c->W * 3, bps) * c->H * bps;
     } else {
         for (uint32_t k = 0; k < c->nc; k++) {
             s->in_off[k] = in_bytes;
@@ -410,7 +410,7 @@ static int32_t enc_run(jxs_gpu_enc_t* e, EncSlot* s, void* const planes[4], cons
             pitch[k] = strides[k];
         } else {
             uint8_t* d = s->in_stage + s->in_off[k];
-            const uint32_t sp = packed ? w : stage_pitch(w, bps);
+            const uint32_t sp = stage_pitch(w, bps);
             cudaError_t ce = cudaSuccess;
             if (!jxs_gpu_is_page_locked(planes[k]) &&
                 host_copy_kernel(d, (size_t)sp * bps, planes[k], (size_t)strides[k] * bps, (size_t)w * bps, h, st, &ce, planes[k],
@@ -447,7 +447,7 @@ static int32_t enc_run(jxs_gpu_enc_t* e, EncSlot* s, void* const planes[4], cons
         FwdVLaunch L;
         memset(&L, 0, sizeof(L));
         int tiles[JXS_MAXC];
-        L.njobs = plan_fwd_v(c, e->dcfg, fb, in, v, L.job, tiles);
+        L.njobs = plan_fwd_v(c, e->dcfg, fb, in, v, v_rowpairs(v_warps(c, v, (uint32_t)jxs_fwd_v_tile_cols())), L.job, tiles);
         for (int i = 0; i < L.njobs; i++) {
             L.job[i].first_block = L.ntiles;
             L.ntiles += tiles[i];
@@ -887,7 +887,7 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
         InvVLaunch L;
         memset(&L, 0, sizeof(L));
         int tiles[JXS_MAXC], blocks = 0;
-        L.njobs = plan_inv_v(c, d->dcfg, fb, lout, v, L.job, tiles);
+        L.njobs = plan_inv_v(c, d->dcfg, fb, lout, v, v_rowpairs(v_warps(c, v, (uint32_t)jxs_inv_v_tile_cols())), L.job, tiles);
         for (int i = 0; i < L.njobs; i++) {
             L.job[i].first_block = blocks;
             blocks += tiles[i];

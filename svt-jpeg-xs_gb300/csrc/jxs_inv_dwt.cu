@@ -8,7 +8,7 @@
  *                vertical levels, the output samples.
  *  inv_v_kernel  one vertical level: each warp streams down a strip of 240
  *                output columns (8 per lane, plus one halo lane on either
- *                side) for 8 row pairs.  Every step rebuilds a low row (LL +
+ *                side) for a few row pairs.  Every step rebuilds a low row (LL +
  *                HL) and a high row (LH + HH) by inverse horizontal lifting
  *                across the warp, lifts vertically in registers and writes
  *                two rows of the next level's int32 low band or, for level 0,
@@ -263,87 +263,55 @@ __global__ void __launch_bounds__(IH_MAX_WARPS * 32) inv_h_kernel(const __grid_c
 /* ------------------------------------------------------------------------ */
 /* vertical level                                                            */
 /* ------------------------------------------------------------------------ */
-/* A tile is IV_COLS columns x IV_ROWPAIRS row pairs of the level's output;
- * its warps are stacked vertically, each working alone on IV_WROWPAIRS row
- * pairs of the tile's column strip.  Lane l holds the 8 output columns c0 =
- * first - 8 + 8 l .. c0 + 7 (band pairs j0 = c0 / 2 .. j0 + 3, one group of
- * every band): lanes 1 to 30 produce the strip, lanes 0 and 31 are the halo
- * the lifting needs on either side.  Each step rebuilds the next low row (LL
- * + HL) and high row (LH + HH) by inverse horizontal lifting across the warp
- * (the neighbours by two shuffles), lifts vertically in registers (the last
- * even row and high row are kept) and writes two output rows.  The band rows
- * of the step after are loaded while this one computes.  No shared memory,
- * no block barrier. */
-#define IV_WARPS 4
-#define IV_THREADS (32 * IV_WARPS)
+/* A block is one warp, working on a strip of IV_COLS columns x rp row pairs
+ * of the level's output.  Lane l holds the 8 output columns c0 = first - 8 +
+ * 8 l .. c0 + 7 (band pairs j0 = c0 / 2 .. j0 + 3, one group of every band):
+ * lanes 1 to 30 produce the strip, lanes 0 and 31 are the halo the lifting
+ * needs on either side.  Each step rebuilds the next low row (LL + HL) and
+ * high row (LH + HH) by inverse horizontal lifting across the warp (the
+ * neighbours by two shuffles), lifts vertically in registers (the last even
+ * row and high row are kept) and writes two output rows.  The band rows of
+ * the step after are loaded while this one computes.  No shared memory, no
+ * barrier; with one warp per block every row address is the same for the
+ * whole block and stays out of the lanes' registers. */
 #define IV_COLS 240                          /* output columns of a strip: lanes 1..30, 8 each */
-#define IV_WROWPAIRS 8                       /* row pairs per warp */
-#define IV_ROWPAIRS (IV_WROWPAIRS * IV_WARPS)
 
 DEV int clampi(int i, int n) { return i < 0 ? 0 : (i >= n ? n - 1 : i); }
 
-/* Raw band values of one low or high row for the lane's pairs j0 .. j0 + 3:
- * the low-pass values (int32 low band, or int16 coefficients of the LH band)
- * and the high-pass int16 coefficients (HL or HH), two per word. */
+/* Raw band values of the lane's pairs j0 .. j0 + 3 of a low row (int32 low
+ * band) and a high row (LH coefficients), each with its high-pass
+ * coefficients (HL, HH), two per word. */
 struct IvRaw {
-    int4 s;     /* int32 low band values */
-    uint2 sc;   /* or LH coefficients, two per word */
-    uint2 d;    /* HL / HH coefficients, two per word */
+    int4 s;
+    uint2 hl, lh, hh;
 };
+/* four int16 values of two words */
+DEV void unpack4(uint2 w, int32_t* v) {
+    v[0] = (int16_t)(w.x & 0xffffu);
+    v[1] = (int32_t)w.x >> 16;
+    v[2] = (int16_t)(w.y & 0xffffu);
+    v[3] = (int32_t)w.y >> 16;
+}
 
-/* int16 values j0 .. j0 + 3 of a band row of n (> 0) coefficients, two per
- * word; indices outside [0, n) read the nearest inside (FAST: all inside) */
-template <bool FAST>
-DEV uint2 iv_ld_coef(const int16_t* row, int j0, int n) {
-    if constexpr (FAST) {
-        return *(const uint2*)(row + j0);
-    } else {
-        if (j0 >= 0 && j0 + 4 <= n) return *(const uint2*)(row + j0);
-        uint32_t v[4];
+/* The lane's neighbours at the ends of a row (EDGE: the strip touches one):
+ * the high value before its first is the first one at the row's start, high
+ * values past the last are the last one. */
+template <bool EDGE>
+DEV int32_t iv_high_edge(int32_t* d, int j0, int w2) {
+    int32_t dm = __shfl_up_sync(FULL, d[3], 1);
+    if (EDGE) {
+        if (j0 == 0) dm = w2 > 0 ? d[0] : 0;
 #pragma unroll
-        for (int q = 0; q < 4; q++) v[q] = (uint16_t)row[clampi(j0 + q, n)];
-        return make_uint2(v[0] | (v[1] << 16), v[2] | (v[3] << 16));
+        for (int q = 0; q < 4; q++)
+            if (j0 + q >= w2) d[q] = q ? d[q - 1] : dm;
     }
-}
-template <bool FAST>
-DEV int4 iv_ld_low(const int32_t* row, int j0, int n) {
-    if (FAST || (j0 >= 0 && j0 + 4 <= n)) return *(const int4*)(row + j0);
-    return make_int4(row[clampi(j0, n)], row[clampi(j0 + 1, n)], row[clampi(j0 + 2, n)], row[clampi(j0 + 3, n)]);
-}
-/* two int16 values of a word as int32 << fq */
-DEV void iv_dq2(uint32_t w, int fq, int32_t& a, int32_t& b) {
-    a = (int32_t)(w << 16) >> (16 - fq);
-    b = (int32_t)(w & 0xffff0000u) >> (16 - fq);
+    return dm;
 }
 
-/* Inverse horizontal lifting of one row across the warp from the lane's low
- * values s[0..3] and high values d[0..3] (pairs j0 .. j0 + 3): x[2j] = s[j] -
- * ((d[j-1] + d[j] + 2) >> 2), x[2j+1] = d[j] + ((x[2j] + x[2j+2]) >> 1), with
- * x[2j] itself in place of x[2j+2] past the row (j + 1 >= w1).  The left
- * neighbour's last high value and the right neighbour's first even sample
- * come by shuffles.  x receives the lane's 8 samples. */
-template <bool FAST>
-DEV void iv_hrow(const int32_t* s, const int32_t* d, int j0, int w1, int32_t* x) {
-    const int32_t dm = __shfl_up_sync(FULL, d[3], 1);
-    const int32_t e0 = s[0] - ((dm + d[0] + 2) >> 2);
-    const int32_t e1 = s[1] - ((d[0] + d[1] + 2) >> 2);
-    const int32_t e2 = s[2] - ((d[1] + d[2] + 2) >> 2);
-    const int32_t e3 = s[3] - ((d[2] + d[3] + 2) >> 2);
-    const int32_t en = __shfl_down_sync(FULL, e0, 1);
-    x[0] = e0;
-    x[1] = d[0] + ((e0 + (FAST || j0 + 1 < w1 ? e1 : e0)) >> 1);
-    x[2] = e1;
-    x[3] = d[1] + ((e1 + (FAST || j0 + 2 < w1 ? e2 : e1)) >> 1);
-    x[4] = e2;
-    x[5] = d[2] + ((e2 + (FAST || j0 + 3 < w1 ? e3 : e2)) >> 1);
-    x[6] = e3;
-    x[7] = d[3] + ((e3 + (FAST || j0 + 4 < w1 ? en : e3)) >> 1);
-}
-
-/* linear_output_scaling of one sample with zeta >= 2: the rounded value
- * (u + 2^(zeta-1)) >> zeta (u = v + 2^(Bw-1), wrapping like the reference's
- * int32 addition) equals ((u >> 1) + 2^(zeta-2)) >> (zeta-1), which cannot
- * overflow; then the clamp to [0, 2^d - 1] */
+/* linear_output_scaling with zeta >= 2: the rounded value (u + 2^(zeta-1))
+ * >> zeta (u = v + 2^(Bw-1), wrapping like the reference's int32 addition)
+ * equals ((u >> 1) + 2^(zeta-2)) >> (zeta-1), which cannot overflow; then the
+ * clamp to [0, 2^d - 1] */
 struct OutScale8 {
     uint32_t half_bw;
     int32_t q;
@@ -366,56 +334,72 @@ DEV uint32_t out_sample8(int32_t v, const OutScale8& s) {
     return (uint32_t)min(max(((u >> 1) + s.q) >> s.zm1, 0), s.m);
 }
 
-/* One output row of the lane's 8 columns c0 .. c0 + 7 (c0 < w): vector
- * stores where the row is aligned and all 8 are inside. */
-template <int OUT, bool FAST>
-DEV void iv_store8(const InvVJob& J, int y, int c0, int w, bool vec, const int32_t* x, const OutScale8& os) {
-    const bool all8 = FAST || (vec && c0 + 8 <= w);
+/* How a strip writes its rows. */
+enum {
+    ST_ALL = 0,     /* every lane's 8 columns inside the row, aligned rows */
+    ST_WHOLE = 1,   /* every lane's 8 columns inside the row or all outside it, aligned rows */
+    ST_ANY = 2      /* sample by sample */
+};
+
+/* The lane's 8 columns c0 .. c0 + 7 (c0 < w) of output row y; samples already
+ * scaled. */
+template <int OUT, int ST>
+DEV void iv_store8(const InvVJob& J, int y, uint32_t c0, int left, const int32_t* x) {
     if constexpr (OUT == 0) {
+        /* rows are padded to a multiple of 4 */
         int32_t* d = (int32_t*)J.dst + (size_t)y * J.dst_pitch + c0;
-        if (all8) {
-            *(int4*)d = make_int4(x[0], x[1], x[2], x[3]);
-            *(int4*)(d + 4) = make_int4(x[4], x[5], x[6], x[7]);
+        *(int4*)d = make_int4(x[0], x[1], x[2], x[3]);
+        if (ST == ST_ALL || left > 4) *(int4*)(d + 4) = make_int4(x[4], x[5], x[6], x[7]);
+    } else if constexpr (OUT == 1) {
+        uint8_t* d = (uint8_t*)J.dst + (size_t)y * J.dst_pitch + c0;
+        if constexpr (ST != ST_ANY) {
+            const uint32_t a = __byte_perm(__byte_perm(x[0], x[1], 0x0040), __byte_perm(x[2], x[3], 0x0040), 0x5410);
+            const uint32_t b = __byte_perm(__byte_perm(x[4], x[5], 0x0040), __byte_perm(x[6], x[7], 0x0040), 0x5410);
+            *(uint2*)d = make_uint2(a, b);
         } else {
+#pragma unroll
             for (int q = 0; q < 8; q++)
-                if (c0 + q < w) d[q] = x[q];
+                if (q < left) d[q] = (uint8_t)x[q];
         }
     } else {
-        uint32_t o[8];
-#pragma unroll
-        for (int q = 0; q < 8; q++) o[q] = out_sample8(x[q], os);
-        if constexpr (OUT == 1) {
-            uint8_t* d = (uint8_t*)J.dst + (size_t)y * J.dst_pitch + c0;
-            if (all8) {
-                *(uint2*)d = make_uint2(o[0] | (o[1] << 8) | (o[2] << 16) | (o[3] << 24),
-                                        o[4] | (o[5] << 8) | (o[6] << 16) | (o[7] << 24));
-            } else {
-                for (int q = 0; q < 8; q++)
-                    if (c0 + q < w) d[q] = (uint8_t)o[q];
-            }
+        uint16_t* d = (uint16_t*)J.dst + (size_t)y * J.dst_pitch + c0;
+        if constexpr (ST != ST_ANY) {
+            *(uint4*)d = make_uint4(__byte_perm(x[0], x[1], 0x5410), __byte_perm(x[2], x[3], 0x5410), __byte_perm(x[4], x[5], 0x5410),
+                                    __byte_perm(x[6], x[7], 0x5410));
         } else {
-            uint16_t* d = (uint16_t*)J.dst + (size_t)y * J.dst_pitch + c0;
-            if (all8) {
-                *(uint4*)d = make_uint4(o[0] | (o[1] << 16), o[2] | (o[3] << 16), o[4] | (o[5] << 16), o[6] | (o[7] << 16));
-            } else {
-                for (int q = 0; q < 8; q++)
-                    if (c0 + q < w) d[q] = (uint16_t)o[q];
-            }
+#pragma unroll
+            for (int q = 0; q < 8; q++)
+                if (q < left) d[q] = (uint16_t)x[q];
         }
     }
 }
 
 /* One warp's strip: row pairs r0 .. rend - 1 of output columns c0 (this
- * lane) of job J.  FAST: the strip is away from the level's left and right
- * edges and its rows are aligned, so that no load or store needs a check. */
-template <int OUT, bool FAST>
-DEV void iv_strip(const InvVJob& J, int r0, int rend, int c0, bool vec) {
+ * lane) of job J.
+ *
+ * EXACT (Fq 6 or 8): the coefficients are multiples of 2^Fq and no rounding
+ * happens where only they meet, so that the high rows are kept as exact
+ * multiples, even columns E = 4 lh - (hh' + hh) of 2^(Fq-2) and odd ones O =
+ * 8 hh + E + E' of 2^(Fq-3), and the updates subtract their plain sums.  The
+ * output scaling's offset 2^(Bw-1) + 2^(zeta-1) is added once to the four low
+ * values of a lane: every lifting step passes a constant of the low band to
+ * all samples unchanged.  Nothing can overflow: with |c| < 2^15 the levels
+ * reach less than 16 2^(15+Fq) <= 2^27.  Otherwise (Fq 0) in the order of
+ * the standard, rounding at every step.
+ *
+ * Bound by memory latency at 24 warps per SM: 29 -> 19.6 thread
+ * instructions per sample against rounding at every step in 64-bit row
+ * pointers, and 8 4K 4:2:2 10-bit frames in 118 us instead of 174 (560 MB of
+ * DRAM traffic, 4.8 TB/s). */
+template <int OUT, int ST, bool EXACT>
+DEV void iv_strip(const InvVJob& J, int r0, int rend, int c0) {
+    constexpr bool EDGE = ST != ST_ALL;
     const int lane = threadIdx.x & 31;
     const int w = J.w, h = J.h, fq = J.fq;
-    const int n1 = (h + 1) >> 1, n2 = h >> 1;
-    const int w1 = (w + 1) >> 1, w2 = w >> 1;
-    const int j0 = c0 >> 1;
-    const bool out_lane = lane >= 1 && lane <= 30 && c0 < w;
+    const int n2 = h >> 1, w1 = (w + 1) >> 1, w2 = w >> 1;
+    const int j0 = c0 >> 1, left = w - c0;
+    const bool have = c0 >= 0 && left > 0, have2 = have && j0 < w2;
+    const bool out_lane = lane >= 1 && lane <= 30 && left > 0;
     const jxs_band_t& bHL = J.bands[J.b_hl];
     const jxs_band_t& bLH = J.bands[J.b_lh];
     const jxs_band_t& bHH = J.bands[J.b_hh];
@@ -426,76 +410,139 @@ DEV void iv_strip(const InvVJob& J, int r0, int rend, int c0, bool vec) {
     const int32_t* llb = J.ll;
     const int ll_p = J.ll_pitch;
     const OutScale8 os = out_scale8(J.bw, J.depth);
-    /* raw loads of low row i (i < n1) and high row i (clamped into [0, n2),
+    const int zeta = os.os.zeta, maxv = os.m;
+    const int32_t offset = EXACT && OUT != 0 ? (int32_t)(os.half_bw + os.os.half_z) : 0;
+    /* exact: scales of a coefficient, of E and O, and of their sums' quarters */
+    const int32_t kc = 1 << fq, kc4 = EXACT ? kc >> 2 : 1, ke = kc4, ko = EXACT ? kc >> 3 : 1, ke4 = EXACT ? kc >> 4 : 1,
+                  ko4 = EXACT ? kc >> 5 : 1;
+
+    /* raw loads of low row i (i < (h + 1) / 2) and high row i (clamped into [0, n2),
      * n2 > 0) */
     auto ld_low = [&](int i, IvRaw& r) {
-        r.s = iv_ld_low<FAST>(llb + (size_t)i * ll_p, j0, w1);
-        r.d = w2 ? iv_ld_coef<FAST>(hl + (size_t)i * hl_p, j0, w2) : make_uint2(0u, 0u);
+        r.s = make_int4(0, 0, 0, 0);
+        r.hl = make_uint2(0u, 0u);
+        if (!EDGE || have) r.s = *(const int4*)(llb + (size_t)i * ll_p + (uint32_t)j0);
+        if (!EDGE || have2) r.hl = *(const uint2*)(hl + (size_t)i * hl_p + (uint32_t)j0);
     };
     auto ld_high = [&](int i, IvRaw& r) {
         i = clampi(i, n2);
-        r.sc = iv_ld_coef<FAST>(lh + (size_t)i * lh_p, j0, w1);
-        r.d = w2 ? iv_ld_coef<FAST>(hh + (size_t)i * hh_p, j0, w2) : make_uint2(0u, 0u);
+        r.lh = make_uint2(0u, 0u);
+        r.hh = make_uint2(0u, 0u);
+        if (!EDGE || have) r.lh = *(const uint2*)(lh + (size_t)i * lh_p + (uint32_t)j0);
+        if (!EDGE || have2) r.hh = *(const uint2*)(hh + (size_t)i * hh_p + (uint32_t)j0);
     };
-    auto build = [&](const IvRaw& r, bool low, int32_t* x) {
-        int32_t sv[4], dv[4];
-        if (low) {
-            sv[0] = r.s.x; sv[1] = r.s.y; sv[2] = r.s.z; sv[3] = r.s.w;
-        } else {
-            iv_dq2(r.sc.x, fq, sv[0], sv[1]);
-            iv_dq2(r.sc.y, fq, sv[2], sv[3]);
+    /* a low row's 8 samples */
+    auto build_low = [&](const IvRaw& r, int32_t* x) {
+        const int32_t s[4] = {r.s.x + offset, r.s.y + offset, r.s.z + offset, r.s.w + offset};
+        int32_t d[4];
+        unpack4(r.hl, d);
+        if constexpr (!EXACT) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) d[q] = (int32_t)((uint32_t)d[q] << fq);
         }
-        iv_dq2(r.d.x, fq, dv[0], dv[1]);
-        iv_dq2(r.d.y, fq, dv[2], dv[3]);
-        iv_hrow<FAST>(sv, dv, j0, w1, x);
+        const int32_t dm = iv_high_edge<EDGE>(d, j0, w2);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int32_t t = (q ? d[q - 1] : dm) + d[q];
+            x[2 * q] = EXACT ? s[q] - t * kc4 : s[q] - ((t + 2) >> 2);
+        }
+        const int32_t xn = __shfl_down_sync(FULL, x[0], 1);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            int32_t next = q < 3 ? x[2 * q + 2] : xn;
+            if (EDGE && j0 + q + 1 >= w1) next = x[2 * q];
+            x[2 * q + 1] = (EXACT ? d[q] * kc : d[q]) + ((x[2 * q] + next) >> 1);
+        }
     };
+    /* a high row's 8 values (exact: scaled down by ke and ko) */
+    auto build_high = [&](const IvRaw& r, int32_t* x) {
+        int32_t s[4], d[4];
+        unpack4(r.lh, s);
+        unpack4(r.hh, d);
+        if constexpr (!EXACT) {
+#pragma unroll
+            for (int q = 0; q < 4; q++) {
+                s[q] = (int32_t)((uint32_t)s[q] << fq);
+                d[q] = (int32_t)((uint32_t)d[q] << fq);
+            }
+        }
+        const int32_t dm = iv_high_edge<EDGE>(d, j0, w2);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            const int32_t t = (q ? d[q - 1] : dm) + d[q];
+            x[2 * q] = EXACT ? 4 * s[q] - t : s[q] - ((t + 2) >> 2);
+        }
+        const int32_t xn = __shfl_down_sync(FULL, x[0], 1);
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            int32_t next = q < 3 ? x[2 * q + 2] : xn;
+            if (EDGE && j0 + q + 1 >= w1) next = x[2 * q];
+            x[2 * q + 1] = EXACT ? 8 * d[q] + (x[2 * q] + next) : d[q] + ((x[2 * q] + next) >> 1);
+        }
+    };
+    auto update = [&](int k, int32_t low, int32_t ha, int32_t hb) { /* an even row's sample */
+        return EXACT ? low - (ha + hb) * ((k & 1) ? ko4 : ke4) : low - ((ha + hb + 2) >> 2);
+    };
+    auto high = [&](int k, int32_t v) { return EXACT ? v * ((k & 1) ? ko : ke) : v; };
+    auto store = [&](int y, const int32_t* x) {
+        if constexpr (OUT == 0) {
+            iv_store8<OUT, ST>(J, y, (uint32_t)c0, left, x);
+        } else {
+            int32_t o[8];
+#pragma unroll
+            for (int k = 0; k < 8; k++) o[k] = EXACT ? __vimin_s32_relu(x[k] >> zeta, maxv) : (int32_t)out_sample8(x[k], os);
+            iv_store8<OUT, ST>(J, y, (uint32_t)c0, left, o);
+        }
+    };
+
     /* x[2 r0] = low[r0] - ((high[r0 - 1] + high[r0] + 2) >> 2) */
     int32_t xe[8], hc[8];
-    IvRaw nl, nh; /* the next step's low and high rows, in flight */
+    IvRaw nx; /* the next step's low and high rows, in flight */
     {
-        IvRaw a, b, c;
+        IvRaw a, b;
         ld_low(r0, a);
         if (n2) {
             ld_high(r0 - 1, b);
-            ld_high(r0, c);
+            ld_high(r0, a);
         }
-        if (r0 + 1 < n1 && 2 * r0 + 2 < h) {
-            ld_low(r0 + 1, nl);
-            if (n2) ld_high(r0 + 1, nh);
+        if (2 * r0 + 2 < h) {
+            ld_low(r0 + 1, nx);
+            if (n2) ld_high(r0 + 1, nx);
         }
         int32_t hp[8];
-        build(a, true, xe);
+        build_low(a, xe);
         if (n2) {
-            build(b, false, hp);
-            build(c, false, hc);
+            build_high(b, hp);
+            build_high(a, hc);
         } else {
 #pragma unroll
             for (int k = 0; k < 8; k++) hp[k] = hc[k] = 0;
         }
 #pragma unroll
-        for (int k = 0; k < 8; k++) xe[k] -= (hp[k] + hc[k] + 2) >> 2;
+        for (int k = 0; k < 8; k++) xe[k] = update(k, xe[k], hp[k], hc[k]);
     }
+#pragma unroll 2
     for (int i = r0; i < rend; i++) {
         const int y = 2 * i;
         int32_t xo[8], xn[8];
         if (y + 2 < h) {
             /* x[2i + 2] from the next low and high rows */
             int32_t hn[8];
-            build(nl, true, xn);
+            build_low(nx, xn);
             if (n2) {
-                build(nh, false, hn);
+                build_high(nx, hn);
             } else {
 #pragma unroll
                 for (int k = 0; k < 8; k++) hn[k] = 0;
             }
             if (i + 1 < rend && y + 4 < h) {
-                ld_low(i + 2, nl);
-                if (n2) ld_high(i + 2, nh);
+                ld_low(i + 2, nx);
+                if (n2) ld_high(i + 2, nx);
             }
 #pragma unroll
             for (int k = 0; k < 8; k++) {
-                xn[k] -= (hc[k] + hn[k] + 2) >> 2;
-                xo[k] = hc[k] + ((xe[k] + xn[k]) >> 1);
+                xn[k] = update(k, xn[k], hc[k], hn[k]);
+                xo[k] = high(k, hc[k]) + ((xe[k] + xn[k]) >> 1);
                 hc[k] = hn[k];
             }
         } else {
@@ -503,42 +550,53 @@ DEV void iv_strip(const InvVJob& J, int r0, int rend, int c0, bool vec) {
 #pragma unroll
             for (int k = 0; k < 8; k++) {
                 xn[k] = xe[k];
-                xo[k] = hc[k] + xe[k];
+                xo[k] = high(k, hc[k]) + xe[k];
             }
         }
         if (out_lane) {
-            iv_store8<OUT, FAST>(J, y, c0, w, vec, xe, os);
-            if (y + 1 < h) iv_store8<OUT, FAST>(J, y + 1, c0, w, vec, xo, os);
+            store(y, xe);
+            if (y + 1 < h) store(y + 1, xo);
         }
 #pragma unroll
         for (int k = 0; k < 8; k++) xe[k] = xn[k];
     }
 }
 
+template <int OUT, int ST>
+DEV void iv_strip_any(const InvVJob& J, int r0, int rend, int c0) {
+    if (J.fq >= 6) iv_strip<OUT, ST, true>(J, r0, rend, c0);
+    else iv_strip<OUT, ST, false>(J, r0, rend, c0);
+}
+
 template <int OUT, int NJ>
-__global__ void __launch_bounds__(IV_THREADS) inv_v_kernel(const __grid_constant__ InvVLaunchN<NJ> L) {
+__global__ void __launch_bounds__(32, 24) inv_v_kernel(const __grid_constant__ InvVLaunchN<NJ> L) {
     const InvVJob& J = L.job[find_job<NJ>(L.job, L.njobs, (int)blockIdx.x)];
     const int t = blockIdx.x - J.first_block;
     const int ty = t / J.col_tiles, tx = t - ty * J.col_tiles;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int n1 = (J.h + 1) >> 1;
-    const int r0 = (ty * IV_WARPS + warp) * IV_WROWPAIRS;
-    if (r0 >= n1) return; /* the whole warp */
-    const int rend = min(r0 + IV_WROWPAIRS, n1);
-    const int first = tx * IV_COLS, c0 = first - 8 + 8 * lane;
+    const int r0 = ty * J.rp, rend = min(r0 + J.rp, n1);
+    const int first = tx * IV_COLS, c0 = first - 8 + 8 * (int)threadIdx.x;
     const int esz = OUT == 0 ? 4 : OUT;
-    const bool vec = ((uintptr_t)J.dst & 15) == 0 && (((size_t)J.dst_pitch * esz) & 15) == 0;
+    const bool vec = (((uintptr_t)J.dst | ((size_t)J.dst_pitch * esz)) & (8 * esz - 1) & 15) == 0;
     /* the strip's 256 columns first - 8 .. first + 247 (band pairs up to
      * first / 2 + 123) all inside, aligned rows: the whole warp takes the
      * path without checks */
-    if (vec && first >= 8 && first + IV_COLS + 8 <= J.w) iv_strip<OUT, true>(J, r0, rend, c0, vec);
-    else iv_strip<OUT, false>(J, r0, rend, c0, vec);
+    const bool inner = first >= 8 && first + IV_COLS + 8 <= J.w;
+    if (OUT == 0) {
+        if (inner) iv_strip_any<OUT, ST_ALL>(J, r0, rend, c0);
+        else iv_strip_any<OUT, ST_WHOLE>(J, r0, rend, c0);
+    } else if (vec && inner) {
+        iv_strip_any<OUT, ST_ALL>(J, r0, rend, c0);
+    } else if (vec && (J.w & 7) == 0) {
+        iv_strip_any<OUT, ST_WHOLE>(J, r0, rend, c0);
+    } else {
+        iv_strip_any<OUT, ST_ANY>(J, r0, rend, c0);
+    }
 }
 
 /* ------------------------------------------------------------------------ */
 /* launchers                                                                 */
 /* ------------------------------------------------------------------------ */
-extern "C" int jxs_inv_v_tile_rows(void) { return IV_ROWPAIRS; }
 extern "C" int jxs_inv_v_tile_cols(void) { return IV_COLS; }
 extern "C" int jxs_inv_h_max_rows_per_block(void) { return IH_MAX_WARPS; }
 extern "C" int jxs_inv_h_chunk_cols(int nh) { return ih_net_cols(nh); }
@@ -546,7 +604,7 @@ extern "C" int jxs_inv_h_chunk_cols(int nh) { return ih_net_cols(nh); }
 template <int OUT, int NJ>
 static cudaError_t launch_iv(const InvVLaunchN<NJ>* L, int nblocks, cudaStream_t st) {
     if (nblocks <= 0) return cudaSuccess;
-    inv_v_kernel<OUT, NJ><<<nblocks, IV_THREADS, 0, st>>>(*L);
+    inv_v_kernel<OUT, NJ><<<nblocks, 32, 0, st>>>(*L);
     return cudaGetLastError();
 }
 

@@ -52,14 +52,15 @@ struct DwtJob {
 #define JXS_BATCH_FRAMES 64
 
 /* Forward transform, one vertical level (jxs_fwd_dwt.cu): one component's
- * share of the launch; its tiles are blocks [first_block, first_block +
- * row_tiles * col_tiles). */
+ * share of the launch; its tiles, strips of one warp each, are blocks
+ * [first_block, first_block + row_tiles * col_tiles). */
 struct FwdVJob {
     const void* src;        /* level input: samples (level 0) or the int32 low band of the previous level */
     long long src_pitch;    /* elements */
     int chan;               /* packed input: channel of this component */
-    int vec;                /* rows may be read 8 samples per vector load (aligned planar source) */
+    int vec;                /* rows may be read 8 samples by vector loads (aligned source) */
     int w, h;               /* level input size */
+    int rp;                 /* row pairs per warp */
     int col_tiles, first_block;
     int32_t* ll;            /* int32 low band written for the next level */
     int ll_pitch;           /* elements, a multiple of 4 */
@@ -108,13 +109,13 @@ typedef FwdHLaunchN<JXS_BATCH_JOBS> FwdHLaunchB;
  * w x h level input from the int32 low band ll and the HL, LH, HH bands. */
 struct InvVJob {
     int w, h;
+    int rp;                 /* row pairs per warp */
     const int32_t* ll;
     int ll_pitch;           /* elements, a multiple of 4 */
     int b_hl, b_lh, b_hh;
     int col_tiles, first_block;
     void* dst;              /* int32 low band of the next level up, or the output plane */
     long long dst_pitch;    /* elements */
-    int vec;                /* two adjacent output samples may be stored at once */
     int depth, bw, fq;
     const jxs_band_t* bands;
     const int16_t* coef;

@@ -21,7 +21,6 @@ extern "C" cudaError_t jxs_launch_fwd_v(const FwdVLaunch* L, int src_kind, int g
 extern "C" cudaError_t jxs_launch_fwd_v_batch(const FwdVLaunchB* L, int src_kind, int grid_per_sm, cudaStream_t st);
 extern "C" cudaError_t jxs_launch_fwd_h(const FwdHLaunch* L, int src_kind, int nblocks, cudaStream_t st);
 extern "C" cudaError_t jxs_launch_fwd_h_batch(const FwdHLaunchB* L, int src_kind, int nblocks, cudaStream_t st);
-extern "C" int jxs_fwd_v_tile_rows(void);
 extern "C" int jxs_fwd_v_tile_cols(void);
 extern "C" int jxs_fwd_h_max_rows_per_block(void);
 extern "C" int jxs_fwd_h_chunk_cols(int nh);
@@ -50,7 +49,6 @@ extern "C" cudaError_t jxs_launch_inv_h(const InvHLaunch* L, int out_kind, int n
 extern "C" cudaError_t jxs_launch_inv_h_batch(const InvHLaunchB* L, int out_kind, int nblocks, cudaStream_t st);
 extern "C" cudaError_t jxs_launch_nlt_out(const NltOut* P, cudaStream_t st);
 extern "C" cudaError_t jxs_launch_star_tetrix(const StParams* P, cudaStream_t st);
-extern "C" int jxs_inv_v_tile_rows(void);
 extern "C" int jxs_inv_v_tile_cols(void);
 extern "C" int jxs_inv_h_max_rows_per_block(void);
 extern "C" int jxs_inv_h_chunk_cols(int nh);
@@ -202,13 +200,47 @@ static inline uint64_t ll_layout(const jxs_cfg_t* c, int pitch[2][JXS_MAXC], uin
     return total;
 }
 
+/* 1: rows of sample planes may be read 8 samples by vector loads: 8 bytes
+ * per load for 8-bit samples, 16 for 16-bit ones (packed: three loads for 8
+ * samples of all components). */
+static inline int src_vec(const jxs_cfg_t* c, const void* p, long long pitch) {
+    const uint32_t bps = bytes_per_sample(c);
+    return (((uintptr_t)p | (uintptr_t)(pitch * bps)) & (8 * bps - 1)) == 0;
+}
+
+/* Warps of vertical level v of one frame at 8 row pairs each. */
+#define JXS_V_ROWPAIRS 8
+static inline uint32_t v_warps(const jxs_cfg_t* c, int v, uint32_t cols) {
+    uint32_t n = 0;
+    for (uint32_t k = 0; k < c->nc; k++) {
+        if ((int)c->comp[k].dv <= v) continue;
+        uint32_t w, h;
+        level_dims(c->comp[k], v, &w, &h);
+        n += div_up(w, cols) * div_up((h + 1) / 2, JXS_V_ROWPAIRS);
+    }
+    return n;
+}
+/* Row pairs per warp of a vertical level's launch with `warps` warps at 8
+ * each: 8 where that fills the device (32 warps on each of 152 SMs), fewer
+ * for smaller launches, down to one, where a warp's chain of steps is what
+ * takes the time.  Fewer cost rows read twice (3 per warp): at 8 / 4 / 2 row
+ * pairs 8 4K frames encode in 642 / 645 / 700 us and one frame in 155 / 147 /
+ * 150 us, a 256x64 frame there and back takes 174 us at 8 and 157 at 1. */
+static inline int v_rowpairs(uint32_t warps) {
+    int rp = JXS_V_ROWPAIRS;
+    while (rp > 1 && warps < 152 * 32) {
+        rp >>= 1;
+        warps <<= 1;
+    }
+    return rp;
+}
+
 /* Forward jobs of vertical level v of one frame (one per component that has
  * the level); *tiles receives each job's tile count. */
 static inline int plan_fwd_v(const jxs_cfg_t* c, const jxs_cfg_t* dcfg, const FrameBufs& b, const FramePlanes& in, int v,
-                             FwdVJob* jobs, int* tiles) {
+                             int rp, FwdVJob* jobs, int* tiles) {
     const int packed = c->fmt == COLOUR_FORMAT_PACKED_YUV444_OR_RGB;
-    const uint32_t bps = bytes_per_sample(c);
-    const uint32_t vcols = (uint32_t)jxs_fwd_v_tile_cols(), vrows = (uint32_t)jxs_fwd_v_tile_rows();
+    const uint32_t vcols = (uint32_t)jxs_fwd_v_tile_cols();
     int n = 0;
     for (uint32_t k = 0; k < c->nc; k++) {
         const jxs_comp_t& cp = c->comp[k];
@@ -224,8 +256,7 @@ static inline int plan_fwd_v(const jxs_cfg_t* c, const jxs_cfg_t* dcfg, const Fr
             J.src = in.p[pk];
             J.src_pitch = in.pitch[pk];
             J.chan = packed ? (int)k : 0;
-            /* 8 samples per vector load: 16 bytes (16-bit) or 8 bytes (8-bit) */
-            J.vec = !packed && ((uintptr_t)in.p[pk] % (8 * bps)) == 0 && (in.pitch[pk] % 8) == 0;
+            J.vec = src_vec(c, in.p[pk], in.pitch[pk]);
         } else {
             J.src = b.ll[v - 1][k];
             J.src_pitch = b.ll_pitch[v - 1][k];
@@ -237,12 +268,13 @@ static inline int plan_fwd_v(const jxs_cfg_t* c, const jxs_cfg_t* dcfg, const Fr
         J.b_hh = top;
         J.b_lh = top - 1;
         J.b_hl = top - 2;
+        J.rp = rp;
         J.col_tiles = (int)div_up(w, vcols);
         J.depth = (int)c->depth;
         J.bands = dev_bands(dcfg);
         J.coef = (uint16_t*)b.coef;
         J.gcli = b.gcli;
-        tiles[n] = J.col_tiles * (int)div_up((h + 1) / 2, vrows);
+        tiles[n] = J.col_tiles * (int)div_up((h + 1) / 2, (uint32_t)rp);
         n++;
     }
     return n;
@@ -271,7 +303,7 @@ static inline int plan_fwd_h(const jxs_cfg_t* c, const jxs_cfg_t* dcfg, const Fr
             J.src = in.p[packed ? 0 : k];
             J.src_pitch = in.pitch[packed ? 0 : k];
             J.chan = packed ? (int)k : 0;
-            J.vec = !packed && ((uintptr_t)J.src % (8 * bytes_per_sample(c))) == 0 && (J.src_pitch % 8) == 0;
+            J.vec = src_vec(c, J.src, J.src_pitch);
         }
         DwtJob bj;
         memset(&bj, 0, sizeof(bj));
@@ -332,9 +364,8 @@ static inline int plan_inv_h(const jxs_cfg_t* c, const jxs_cfg_t* dcfg, const Fr
  * or the samples for v = proxy, the output level); levels below the output
  * level have no jobs.  *tiles receives each job's block count. */
 static inline int plan_inv_v(const jxs_cfg_t* c, const jxs_cfg_t* dcfg, const FrameBufs& b, const FramePlanes& out, int v,
-                             InvVJob* jobs, int* tiles) {
-    const uint32_t bps = bytes_per_sample(c);
-    const uint32_t vcols = (uint32_t)jxs_inv_v_tile_cols(), vrows = (uint32_t)jxs_inv_v_tile_rows();
+                             int rp, InvVJob* jobs, int* tiles) {
+    const uint32_t vcols = (uint32_t)jxs_inv_v_tile_cols();
     int n = 0;
     for (uint32_t k = 0; k < c->nc; k++) {
         const jxs_comp_t& cp = c->comp[k];
@@ -351,14 +382,13 @@ static inline int plan_inv_v(const jxs_cfg_t* c, const jxs_cfg_t* dcfg, const Fr
         J.b_hh = top;
         J.b_lh = top - 1;
         J.b_hl = top - 2;
+        J.rp = rp;
         if (v > (int)c->proxy) {
             J.dst = b.ll[v - 1][k];
             J.dst_pitch = b.ll_pitch[v - 1][k];
-            J.vec = 1;
         } else {
             J.dst = out.p[k];
             J.dst_pitch = out.pitch[k];
-            J.vec = ((uintptr_t)J.dst % (2 * bps)) == 0 && (J.dst_pitch % 2) == 0;
         }
         J.depth = (int)c->depth;
         J.bw = (int)c->bw;
@@ -366,7 +396,7 @@ static inline int plan_inv_v(const jxs_cfg_t* c, const jxs_cfg_t* dcfg, const Fr
         J.bands = dev_bands(dcfg);
         J.coef = (const int16_t*)b.coef;
         J.col_tiles = (int)div_up(w, vcols);
-        tiles[n] = J.col_tiles * (int)div_up((h + 1) / 2, vrows);
+        tiles[n] = J.col_tiles * (int)div_up((h + 1) / 2, (uint32_t)rp);
         n++;
     }
     return n;
