@@ -92,52 +92,82 @@ DEV SliceSplit slice_split(const jxs_cfg_t* __restrict__ cfg, int s) {
     return o;
 }
 
-/* The precinct searches of rate_control_precinct (RateControl.c:1259-1333,
- * binary searches :889-1083), by one thread on tables in shared memory
- * ([q * nr + r]): the quantization by binary
- * search on T[q * nr]; with `scan` (full signs, vertical prediction) then
- * lower quantizations while TS fits, else the first higher one that fits
- * (:936-1015); the refinement by binary search on TS.  Returns an error
- * code, 0 when q, r and data (TS at (q, r)) are set. */
-DEV int prec_search(const uint32_t* T, const uint32_t* TS, int ld, int scan, int nr, int max_q, int max_r,
-                    const uint32_t* __restrict__ s_empty, uint32_t avail, int& q, int& r, uint32_t& data) {
-    BSearch bs;
-    int step = 6;
-    if (step > max_q) step = 0;
-    bs_init(bs, 0, max_q, 0, step);
-    int res, next = BS_BEGIN, v = 0;
-    while ((res = bs_next(bs, next, &v)) == BS_CONTINUE) {
-        if (s_empty[v] & 1u) next = BS_OUT_OF_RANGE;
-        else next = T[v * nr] > avail ? BS_TOO_SMALL : BS_TOO_BIG;
-    }
-    if (res != BS_FOUND) return JXS_E_ENC_FRAME;
-    q = v;
-    if (scan) {
-        int best = -1;
-        for (int qt = q - 1; qt >= 0; qt--) {
-            if ((s_empty[qt] & 1u) || TS[qt * ld] > avail) break;
-            best = qt;
+/* What the searches of a slice read of the configuration, held in
+ * registers by every lane of the searching warp. */
+struct RcParams {
+    int nr, max_q, max_r, rc_mode, signs;
+    uint32_t hdrs0, hdrs1, np, empty; /* empty: lane q's word of cfg->empty */
+};
+DEV RcParams rc_params(const jxs_cfg_t* __restrict__ cfg) {
+    RcParams P;
+    P.nr = cfg->max_r + 1;
+    P.max_q = cfg->max_q;
+    P.max_r = cfg->max_r;
+    P.rc_mode = (int)cfg->rc_mode;
+    P.signs = (int)cfg->signs;
+    P.hdrs0 = cfg->hdrs_bytes[0];
+    P.hdrs1 = cfg->hdrs_bytes[1];
+    P.np = cfg->np;
+    P.empty = cfg->empty[threadIdx.x & 31];
+    return P;
+}
+
+/* The reference's binary search (binary_search_next_step) over v in [0, n],
+ * n <= 31, with the answers of every v known: bit v of `small` is "too
+ * small" (the search moves up, the result with below = 1), of `big` "too
+ * big" (it moves down, the result with below = 0), neither "out of range" (it
+ * moves down).  Where exactly the lowest values are too small, every such
+ * search ends at the border; other patterns (a cost that does not fall with
+ * Q or grow with R) are searched step by step.  Returns the result or -1. */
+DEV int mask_search(uint32_t small, uint32_t big, int n, int below, int step) {
+    if (!(small & (small + 1u))) {
+        const int border = __popc(small);
+        if (below) {
+            if (border > 0) return border - 1;
+        } else if (border <= n && ((big >> border) & 1u)) {
+            return border;
         }
-        if (best < 0)
-            for (int qt = q; qt <= max_q; qt++)
-                if (!(s_empty[qt] & 1u) && TS[qt * ld] <= avail) {
-                    best = qt;
-                    break;
-                }
-        if (best < 0) return JXS_E_ENC_FRAME;
-        q = best;
     }
-    step = 6;
-    if (step >= max_r) step = 0;
-    bs_init(bs, 0, max_r, 1, step);
-    next = BS_BEGIN;
-    while ((res = bs_next(bs, next, &v)) == BS_CONTINUE) {
-        if ((s_empty[q] >> v) & 1u) next = BS_OUT_OF_RANGE;
-        else next = TS[q * ld + v] <= avail ? BS_TOO_SMALL : BS_TOO_BIG;
+    BSearch bs;
+    bs_init(bs, 0, n, below, step);
+    int res, next = BS_BEGIN, v = 0;
+    while ((res = bs_next(bs, next, &v)) == BS_CONTINUE)
+        next = (small >> v) & 1u ? BS_TOO_SMALL : (big >> v) & 1u ? BS_TOO_BIG : BS_OUT_OF_RANGE;
+    return res == BS_FOUND ? v : -1;
+}
+
+/* The precinct searches of rate_control_precinct (RateControl.c:1259-1333,
+ * binary searches :889-1083), by one warp on tables in shared memory
+ * ([q * ld + r]), a lane per candidate: the quantization by binary search on
+ * T[q * ld]; with `scan` (full signs, vertical prediction) then lower
+ * quantizations while TS fits, else the first higher one that fits
+ * (:936-1015); the refinement by binary search on TS.  Returns an error
+ * code, 0 when q, r and data (TS at (q, r)) are set; the same in every
+ * lane. */
+DEV int prec_search(const RcParams& P, const uint32_t* T, int ldt, const uint32_t* TS, int ld, int scan, uint32_t avail, int& q, int& r,
+                    uint32_t& data) {
+    const int lane = threadIdx.x & 31;
+    const bool inq = lane <= P.max_q;
+    const uint32_t none = __ballot_sync(FULL, inq && (P.empty & 1u)); /* every band truncated: out of range */
+    const uint32_t fit = __ballot_sync(FULL, inq && T[lane * ldt] <= avail) & ~none;
+    const uint32_t fulq = (2u << P.max_q) - 1u;
+    q = mask_search(fulq & ~fit & ~none, fit, P.max_q, 0, 6 > P.max_q ? 0 : 6);
+    if (q < 0) return JXS_E_ENC_FRAME;
+    if (scan) {
+        const uint32_t ok = __ballot_sync(FULL, inq && TS[lane * ld] <= avail) & ~none;
+        const uint32_t low = (1u << q) - 1u, gaps = low & ~ok;
+        const int run0 = gaps ? 32 - __clz((int)gaps) : 0; /* first of the run of fitting values that ends at q - 1 */
+        if (run0 < q) q = run0;
+        else if (ok & ~low) q = __ffs((int)(ok & ~low)) - 1;
+        else return JXS_E_ENC_FRAME;
     }
-    if (res != BS_FOUND) return JXS_E_ENC_FRAME;
-    r = v;
-    data = TS[q * ld + r];
+    const bool inr = lane <= P.max_r;
+    const uint32_t eq = __shfl_sync(FULL, P.empty, q);
+    const uint32_t row = inr ? TS[q * ld + lane] : 0xffffffffu;
+    const uint32_t fitr = __ballot_sync(FULL, inr && row <= avail) & ~eq;
+    r = mask_search(fitr, __ballot_sync(FULL, inr) & ~fitr & ~eq, P.max_r, 1, 6 >= P.max_r ? 0 : 6);
+    if (r < 0) return JXS_E_ENC_FRAME;
+    data = __shfl_sync(FULL, row, r);
     return 0;
 }
 
@@ -147,12 +177,11 @@ DEV int prec_search(const uint32_t* T, const uint32_t* TS, int ld, int scan, int
  * into `area`, one (Q, R) for the slice by the precinct searches, then the
  * budget of each precinct, kept in rc[p].total_bytes.  Run by a whole
  * block; returns the error (every thread). */
-DEV int slice_common(const jxs_cfg_t* __restrict__ cfg, int s, const SliceSplit& sp, const uint32_t* __restrict__ cost,
-                     uint32_t* area, const uint32_t* __restrict__ s_empty, PrecRC* __restrict__ rc, int* __restrict__ status) {
+DEV int slice_common(const RcParams& P, int s, const SliceSplit& sp, const uint32_t* __restrict__ cost, uint32_t* area,
+                     PrecRC* __restrict__ rc, int* __restrict__ status) {
     __shared__ int s_cerr;
-    const int nq = cfg->max_q + 1, nr = cfg->max_r + 1, nt = nq * nr;
-    const int max_q = cfg->max_q, max_r = cfg->max_r, rc_mode = (int)cfg->rc_mode;
-    const uint32_t np_all = cfg->np, hdrs0 = cfg->hdrs_bytes[0], hdrs1 = cfg->hdrs_bytes[1];
+    const int nr = P.nr, nt = (P.max_q + 1) * nr, rc_mode = P.rc_mode;
+    const uint32_t np_all = P.np, hdrs0 = P.hdrs0, hdrs1 = P.hdrs1;
     const uint32_t first_p = sp.first_p, nprec = sp.nprec, slice_budget = sp.slice_budget;
     __syncthreads();
     for (int e = threadIdx.x; e < nt; e += blockDim.x) {
@@ -162,7 +191,7 @@ DEV int slice_common(const jxs_cfg_t* __restrict__ cfg, int s, const SliceSplit&
         area[e] = sum;
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         int err = 0;
         uint32_t headers = 0;
         for (uint32_t i = 0; i < nprec; i++) headers += first_p + i + 1 >= np_all ? hdrs1 : hdrs0;
@@ -170,8 +199,8 @@ DEV int slice_common(const jxs_cfg_t* __restrict__ cfg, int s, const SliceSplit&
         else if (slice_budget <= headers) err = JXS_E_UNDEFINED;
         int q = 0, r = 0;
         uint32_t dsum = 0;
-        if (!err) err = prec_search(area, area, nr, 0, nr, max_q, max_r, s_empty, slice_budget - headers, q, r, dsum);
-        if (!err) {
+        if (!err) err = prec_search(P, area, nr, area, nr, 0, slice_budget - headers, q, r, dsum);
+        if (!err && threadIdx.x == 0) {
             /* each precinct its headers and data at (Q, R); the last also
              * the slice's remaining bytes */
             uint32_t pad_last = slice_budget - headers;
@@ -214,7 +243,7 @@ DEV int slice_common(const jxs_cfg_t* __restrict__ cfg, int s, const SliceSplit&
             if (pad_last > 0) {
                 /* the first precinct 10 % more (20 % with fast signs), the
                  * rest of the padding shared evenly */
-                uint32_t add_first = rc[first_p].total_bytes * (cfg->signs == 1 ? 20u : 10u) / 100;
+                uint32_t add_first = rc[first_p].total_bytes * (P.signs == 1 ? 20u : 10u) / 100;
                 if (add_first > pad_last) add_first = pad_last;
                 pad_last -= add_first;
                 rc[first_p + nprec - 1].total_bytes -= add_first;
@@ -226,111 +255,114 @@ DEV int slice_common(const jxs_cfg_t* __restrict__ cfg, int s, const SliceSplit&
                 }
             }
         }
-        if (err) {
+        if (err && threadIdx.x == 0) {
             printf("jxs rc: slice %d (common quantization): error 0x%x\n", s, (unsigned)err);
             JXS_STATUS_SET(status, err);
         }
-        s_cerr = err;
+        if (threadIdx.x == 0) s_cerr = err;
     }
     __syncthreads();
     return s_cerr;
 }
 
-/* One precinct's budget, searches and padding carry; thread 0.  `T` is the
- * table of the quantization search, `F` the exact-sign table (fast signs:
- * the bytes of the signs not sent are T - F at the chosen (Q, R)), `TS` the
- * table of the scan and the refinement search (row stride `ld`); all in
- * shared memory.
+/* One precinct's budget, searches and padding carry, by one warp.  `T` (row
+ * stride ldt) is the table of the quantization search, `F` the exact-sign
+ * table (fast signs: the bytes of the signs not sent are T - F at the chosen
+ * (Q, R)), `TS` (row stride ld) the table of the scan and the refinement
+ * search; all in shared memory.
  * Modes 1-3 carry the padding (and fast signs' unsent sign bytes) to the
  * next precinct of the slice; a slice's last precinct and mode 0 keep them
  * as zero bytes (PackStageProcess.c:293-333, 526-560,
- * PackPrecinct.c:513-536).  Returns an error code. */
-DEV int prec_select(const jxs_cfg_t* __restrict__ cfg, int s, uint32_t i, const SliceSplit& sp, const uint32_t* T,
-                    const uint32_t* F, const uint32_t* TS, int ld, int scan, const uint32_t* __restrict__ s_empty, uint32_t& carry,
-                    uint32_t& run, PrecRC* __restrict__ rc, int* __restrict__ status) {
+ * PackPrecinct.c:513-536).  Returns an error code; that, the carry, the
+ * running offset and q, r are the same in every lane. */
+DEV int prec_select(const RcParams& P, int s, uint32_t i, const SliceSplit& sp, const uint32_t* T, const uint32_t* F, int ldt,
+                    const uint32_t* TS, int ld, int scan, uint32_t& carry, uint32_t& run, int& q, int& r, PrecRC* __restrict__ rc,
+                    int* __restrict__ status) {
     const uint32_t p = sp.first_p + i;
-    const int last = (p + 1 >= cfg->np);
-    const uint32_t budget =
-        (cfg->rc_mode >= 2 ? rc[p].total_bytes : (i == 0 ? sp.first_b : sp.min_b) + (i < sp.left ? 1 : 0)) + carry;
-    const uint32_t hdr = cfg->hdrs_bytes[last];
-    const int nr = cfg->max_r + 1;
+    const uint32_t budget = (P.rc_mode >= 2 ? rc[p].total_bytes : (i == 0 ? sp.first_b : sp.min_b) + (i < sp.left ? 1 : 0)) + carry;
+    const uint32_t hdr = p + 1 >= P.np ? P.hdrs1 : P.hdrs0;
     int err = 0;
     if (budget > JXS_PREC_MAX_BYTES) err = JXS_E_ENC_FRAME;
     else if (budget <= hdr) err = JXS_E_UNDEFINED;
-    int q = 0, r = 0;
+    q = r = 0;
     uint32_t data = 0;
-    if (!err) err = prec_search(T, TS, ld, scan, nr, cfg->max_q, cfg->max_r, s_empty, budget - hdr, q, r, data);
+    if (!err) err = prec_search(P, T, ldt, TS, ld, scan, budget - hdr, q, r, data);
     if (!err) {
         const uint32_t padding = budget - hdr - data;
         uint32_t total = budget;
-        const uint32_t retrieve = cfg->signs == 1 ? T[q * nr + r] - F[q * nr + r] : 0u;
-        if (cfg->rc_mode >= 1 && i + 1 < sp.nprec) {
+        const uint32_t retrieve = P.signs == 1 ? T[q * ldt + r] - F[q * ldt + r] : 0u;
+        if (P.rc_mode >= 1 && i + 1 < sp.nprec) {
             total -= padding + retrieve;
             carry = padding + retrieve;
         } else {
             carry = 0;
         }
-        PrecRC o;
-        o.total_bytes = total;
-        o.offset = run;
-        o.data_bytes = data - retrieve; /* the sub-packet bytes packed */
-        o.q = (uint8_t)q;
-        o.r = (uint8_t)r;
-        o.first_in_slice = (uint8_t)(i == 0);
-        o.pad = 0;
-        rc[p] = o;
+        if ((threadIdx.x & 31) == 0) {
+            PrecRC o;
+            o.total_bytes = total;
+            o.offset = run;
+            o.data_bytes = data - retrieve; /* the sub-packet bytes packed */
+            o.q = (uint8_t)q;
+            o.r = (uint8_t)r;
+            o.first_in_slice = (uint8_t)(i == 0);
+            o.pad = 0;
+            rc[p] = o;
+        }
         run += total;
-    } else {
+    } else if ((threadIdx.x & 31) == 0) {
         printf("jxs rc: slice %d precinct %u budget %u: error 0x%x\n", s, p, budget, (unsigned)err);
         JXS_STATUS_SET(status, err);
     }
     return err;
 }
 
+/* Words of one [Q][R] table in the selection's shared memory: 32 rows of 36
+ * words, so that rows are written 16 bytes at a time and a column is read
+ * with 4-way conflicts. */
+#define RC_TLD 36
+#define RC_TWORDS (32 * RC_TLD)
+
 /* One slice's selection without vertical prediction, on the slice's cost
- * tables: the tables of up to `area_words / (nq * nr * tables)` precincts
- * are read (through L2) into `area` at a time; thread 0 then runs their
- * searches in order.  With sign handling each precinct has two tables:
- * signs counted the fast way (every coefficient of a group above gtli) and
+ * tables: as many precincts' tables as fit are read (through L2) into `area`
+ * at a time by the whole block; one warp then runs their searches in order, a
+ * lane per candidate.  With sign handling each precinct has two tables: signs
+ * counted the fast way (every coefficient of a group above gtli) and
  * exactly; the quantization search runs on the fast one, the full strategy
- * then scans and searches the refinement on the exact one. */
+ * then scans and searches the refinement on the exact one.
+ *
+ * A chain of one search after another, 4 per slice of 16 lines: by one
+ * thread, step by step, 24,000 cycles of the slice's last block, alone on
+ * the critical path of a single frame; now 5,000. */
 DEV void select_slice(const jxs_cfg_t* __restrict__ cfg, int s, const uint32_t* __restrict__ cost, uint32_t* area,
                       uint32_t area_words, PrecRC* __restrict__ rc, int* __restrict__ status) {
-    __shared__ uint32_t s_carry, s_run;
     __shared__ int s_err;
-    __shared__ uint32_t s_empty[32];
-    if (threadIdx.x < 32) s_empty[threadIdx.x] = cfg->empty[threadIdx.x];
+    const RcParams P = rc_params(cfg);
     const SliceSplit sp = slice_split(cfg, s);
-    if (threadIdx.x == 0) {
-        s_carry = 0;
-        s_run = cfg->slice_begin[s] + 6;
-        s_err = 0;
-    }
-    const int nq = cfg->max_q + 1, nr = cfg->max_r + 1, nt = nq * nr;
-    const uint32_t np_all = cfg->np, signs = cfg->signs;
+    uint32_t carry = 0, run = cfg->slice_begin[s] + 6;
+    if (threadIdx.x == 0) s_err = 0;
     __syncthreads();
-    if (cfg->rc_mode >= 2 && slice_common(cfg, s, sp, cost, area, s_empty, rc, status)) return;
-    const int ntab = signs ? 2 : 1;
-    const uint32_t chunk = area_words / (uint32_t)(nt * ntab);
+    if (P.rc_mode >= 2 && slice_common(P, s, sp, cost, area, rc, status)) return;
+    const uint32_t ntab = P.signs ? 2 : 1, chunk = area_words / (RC_TWORDS * ntab);
     for (uint32_t c0 = 0; c0 < sp.nprec; c0 += chunk) {
         const uint32_t cnt = min(chunk, sp.nprec - c0);
         __syncthreads();
         if (s_err) break;
-        for (int e = threadIdx.x; e < (int)cnt * nt * ntab; e += blockDim.x) {
-            const int i = e / (nt * ntab), rest = e - i * nt * ntab, tb = rest / nt, qr = rest - tb * nt, q = qr / nr,
-                      r = qr - q * nr;
-            area[e] = __ldcg(cost + ((uint64_t)tb * np_all + sp.first_p + c0 + i) * 1024 + q * 32 + r);
+        for (uint32_t e = threadIdx.x; e < cnt * ntab * 256; e += blockDim.x) {
+            /* 16 bytes of row q of table tb of precinct i */
+            const uint32_t i = e / (ntab * 256), tb = (e >> 8) - i * ntab, q = (e >> 3) & 31u, c = 4 * (e & 7u);
+            *(uint4*)(area + (e >> 8) * RC_TWORDS + q * RC_TLD + c) =
+                __ldcg((const uint4*)(cost + ((uint64_t)tb * P.np + sp.first_p + c0 + i) * 1024 + q * 32 + c));
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            for (uint32_t ii = 0; ii < cnt && !s_err; ii++) {
-                const uint32_t* T = area + ii * nt * ntab;
-                const uint32_t* F = signs ? T + nt : T; /* exact signs */
-                uint32_t carry = s_carry, run = s_run;
-                s_err = prec_select(cfg, s, c0 + ii, sp, T, F, signs == 2 ? F : T, nr, signs == 2, s_empty, carry, run, rc, status);
-                s_carry = carry;
-                s_run = run;
+        if (threadIdx.x < 32) {
+            int err = 0, q, r;
+            for (uint32_t ii = 0; ii < cnt && !err; ii++) {
+                const uint32_t* T = area + ii * RC_TWORDS * ntab;
+                const uint32_t* F = P.signs ? T + RC_TWORDS : T; /* exact signs */
+                err = prec_select(P, s, c0 + ii, sp, T, F, RC_TLD, P.signs == 2 ? F : T, RC_TLD, P.signs == 2, carry, run, q, r, rc,
+                                  status);
             }
+            if (err && threadIdx.x == 0) s_err = err;
         }
     }
 }
@@ -375,9 +407,7 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
                             int* __restrict__ status, Stage& stage_kind, const uint8_t* lgain, const uint8_t* lprio,
                             const uint8_t* lfb, const uint32_t* lsig, const uint32_t* lraw, const jxs_bline_t* bls,
                             const jxs_seg_t* segs, const uint8_t* s_pkbl0, const uint8_t* s_pknbl, const uint8_t* s_order) {
-    __shared__ uint32_t s_carry, s_run;
     __shared__ int s_err;
-    __shared__ uint32_t s_empty[32];
     __shared__ uint8_t s_gtop[JXS_MAXBL], s_bl0[JXS_MAXBL], s_bl1[JXS_MAXBL];
     __shared__ uint32_t s_methv[JXS_MAXBL]; /* per band: 2 bits per t */
     uint32_t(*vtfs)[16] = (uint32_t(*)[16])area;
@@ -391,19 +421,16 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
     uint32_t* Ts = area + 8 * RC_LT_REGION;
     uint32_t* Fs = area + 9 * RC_LT_REGION;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (threadIdx.x < 32) s_empty[threadIdx.x] = cfg->empty[threadIdx.x];
+    const RcParams P = rc_params(cfg);
     const SliceSplit sp = slice_split(cfg, s);
-    if (threadIdx.x == 0) {
-        s_carry = 0;
-        s_run = cfg->slice_begin[s] + 6;
-        s_err = 0;
-    }
+    uint32_t carry = 0, run = cfg->slice_begin[s] + 6; /* of warp 0 */
+    if (threadIdx.x == 0) s_err = 0;
     const int nq = cfg->max_q + 1, nr = cfg->max_r + 1, nt = nq * nr;
     const uint32_t np_all = cfg->np, signs = cfg->signs, fs = cfg->fs, SG = cfg->seg_groups, npk = cfg->npk;
     const uint32_t nbands = cfg->nbands, sig = cfg->sig;
     const int rm = cfg->rm;
     __syncthreads();
-    if (cfg->rc_mode >= 2 && slice_common(cfg, s, sp, cost, Ts, s_empty, rc, status)) return;
+    if (P.rc_mode >= 2 && slice_common(P, s, sp, cost, Ts, rc, status)) return;
     int kind_staged = -1;
     for (uint32_t i = 0; i < sp.nprec; i++) {
         const uint32_t p = sp.first_p + i;
@@ -563,14 +590,14 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
             }
         }
         __syncthreads();
-        if (threadIdx.x == 0) {
-            uint32_t carry = s_carry, run = s_run;
-            s_err = prec_select(cfg, s, i, sp, Ts, fs ? Fs : Ts, &dV[0][0], 32, 1, s_empty, carry, run, rc, status);
-            s_carry = carry;
-            s_run = run;
-            if (!s_err) {
-                const PrecRC o = rc[p];
-                for (uint32_t fb = 0; fb < nbands; fb++) s_gtop[fb] = jxs_truncation(cfg->band[fb].gain, cfg->band[fb].prio, o.q, o.r);
+        if (warp == 0) {
+            int q, r;
+            const int err = prec_select(P, s, i, sp, Ts, fs ? Fs : Ts, nr, &dV[0][0], 32, 1, carry, run, q, r, rc, status);
+            if (err) {
+                if (lane == 0) s_err = err;
+            } else {
+                for (uint32_t fb = lane; fb < nbands; fb += 32)
+                    s_gtop[fb] = jxs_truncation(cfg->band[fb].gain, cfg->band[fb].prio, (uint8_t)q, (uint8_t)r);
             }
         }
     }
@@ -627,15 +654,16 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
     uint32_t(*nzh)[16] = (uint32_t(*)[16])(s_area + (SIGNS ? 5 : 0) * JXS_MAXBLINES * 16); /* later: full sign bits per t */
     uint32_t(*tfs)[16] = hist;
     uint32_t(*tnz)[16] = nzh;
-    uint32_t(*dF)[32] = (uint32_t(*)[32])shist;
+    uint32_t(*dF)[33] = (uint32_t(*)[33])shist;
     /* SIGNS: the launch may hold frames with sign handling; VPRED: with
      * vertical prediction (compiled out otherwise) */
     const uint32_t fs = SIGNS ? cfg->fs : 0u, uniform = cfg->qpih;
     __shared__ uint32_t cn[JXS_MAXBL][16], cs[JXS_MAXBL][16];
-    __shared__ uint16_t meth[JXS_MAXBL];
     __shared__ uint8_t lgain[JXS_MAXBLINES], lprio[JXS_MAXBLINES], lfb[JXS_MAXBLINES];
     __shared__ uint32_t lsig[JXS_MAXBLINES], lraw[JXS_MAXPK];
-    __shared__ uint32_t dC[32][32]; /* per Q: cost at R = 0, then its changes at each R */
+    /* per Q: cost at R = 0, then its changes at each R; rows of 33 words, a
+     * lane per Q adds at one R (rows of 32 would put all lanes in one bank) */
+    __shared__ uint32_t dC[32][33];
     /* this precinct kind's tables, staged from the configuration */
     __shared__ jxs_seg_t s_seg[JXS_MAXSEG];
     __shared__ jxs_bline_t s_bl[JXS_MAXBLINES];
@@ -701,6 +729,13 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
      * value (lanes 0..15) or significance (16..31) words */
     const uint32_t hb = lane & 15u, hsh = 8u * ((hb >> 1) & 3u);
     uint32_t* htab = (lane < 16 ? &hist[0][0] : &shist[0][0]) + hb;
+    /* the first 4 groups of the lane in a segment, read one segment ahead */
+    auto first4 = [&](uint32_t sidx) {
+        const jxs_seg_t sg = segs[sidx];
+        const uint32_t g = sg.g0 + 4 * lane;
+        return g < min(sg.g0 + SG, bls[sg.bl].gcli_w) ? *(const uint32_t*)(gcli + s_grow[sg.bl] + g) : 0u;
+    };
+    uint32_t ahead = (uint32_t)warp < nseg ? first4(warp) : 0u;
     for (uint32_t sidx = warp; sidx < nseg; sidx += RC_WARPS) {
         const jxs_seg_t sg = segs[sidx];
         const uint32_t x = sg.bl;
@@ -711,10 +746,12 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
             const jxs_band_t& bd = cfg->band[lfb[x]];
             crow = coef + bd.coef_off + (uint64_t)(p * bd.lines + bls[x].line) * bd.pitch;
         }
+        const uint32_t cur = ahead;
+        if (sidx + RC_WARPS < nseg) ahead = first4(sidx + RC_WARPS);
         for (uint32_t base = sg.g0; base < gend; base += 128) {
             const uint32_t g = base + 4 * lane;
             const uint32_t nv = g < gend ? min(4u, gend - g) : 0u;
-            uint32_t w4 = nv ? *(const uint32_t*)(grow + g) : 0u;
+            uint32_t w4 = base == sg.g0 ? cur : nv ? *(const uint32_t*)(grow + g) : 0u;
             /* GCLIs past the line's end read as 0 and are taken off bin 0 */
             w4 &= nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
             uint32_t lo = nv - 4u, hi = 0u; /* bin 0 starts at -(4 - nv) */
@@ -739,9 +776,14 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
             /* bytes: even bins, odd bins of 0..7 and of 8..15 */
             const uint32_t M = 0x0f0f0f0fu;
             const uint32_t v0 = __reduce_add_sync(FULL, lo & M), v1 = __reduce_add_sync(FULL, (lo >> 4) & M);
-            const uint32_t v2 = __reduce_add_sync(FULL, hi & M), v3 = __reduce_add_sync(FULL, (hi >> 4) & M);
             const uint32_t s0 = __reduce_add_sync(FULL, slo & M), s1 = __reduce_add_sync(FULL, (slo >> 4) & M);
-            const uint32_t s2 = __reduce_add_sync(FULL, shi & M), s3 = __reduce_add_sync(FULL, (shi >> 4) & M);
+            uint32_t v2 = 0, v3 = 0, s2 = 0, s3 = 0;
+            if (__any_sync(FULL, hi)) {
+                v2 = __reduce_add_sync(FULL, hi & M);
+                v3 = __reduce_add_sync(FULL, (hi >> 4) & M);
+                s2 = __reduce_add_sync(FULL, shi & M);
+                s3 = __reduce_add_sync(FULL, (shi >> 4) & M);
+            }
             const uint32_t wv = hb >= 8 ? (hb & 1 ? v3 : v2) : (hb & 1 ? v1 : v0);
             const uint32_t ws = hb >= 8 ? (hb & 1 ? s3 : s2) : (hb & 1 ? s1 : s0);
             const uint32_t c = ((lane < 16 ? wv : ws) >> hsh) & 255u;
@@ -781,35 +823,46 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
     __syncthreads();
 
     /* per band line and gtli t: data bits, GCLI bits without / with
-     * significance coding */
-    for (uint32_t x = threadIdx.x; x < nbl; x += blockDim.x) {
-        const uint32_t N = bls[x].gcli_w;
-        int S0 = 0, S1 = 0;
-        uint32_t Z1 = 0;
-        for (int t = 15; t >= 0; t--) {
-            const int dsum = S1 - (t - 1) * S0; /* sum over v > t of (v - t + 1) h[v] */
-            const uint32_t h = hist[x][t];
+     * significance coding; half a warp per line, a lane per t, the sums over
+     * the larger and smaller GCLIs by shuffles */
+    for (uint32_t x0 = 2 * warp; x0 < nbl; x0 += 2 * RC_WARPS) {
+        const uint32_t x = min(x0 + (lane >> 4), nbl - 1);
+        const int t = lane & 15;
+        const int h = (int)hist[x][t], th = t * h;
+        const uint32_t zh = SIGNS ? nzh[x][t] : 0u;
+        int S0 = h, S1 = th;
+        uint32_t Z = shist[x][t], Z1 = zh;
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            const int a0 = __shfl_down_sync(FULL, S0, o, 16), a1 = __shfl_down_sync(FULL, S1, o, 16);
+            const uint32_t az = __shfl_up_sync(FULL, Z, o, 16);
+            if (t + o < 16) {
+                S0 += a0;
+                S1 += a1;
+            }
+            if (t >= o) Z += az; /* groups in significance groups whose maximum is <= t: no GCLI codes */
+            if (SIGNS) {
+                const uint32_t a2 = __shfl_down_sync(FULL, Z1, o, 16);
+                if (t + o < 16) Z1 += a2;
+            }
+        }
+        S0 -= h; /* over v > t */
+        S1 -= th;
+        const int dsum = S1 - (t - 1) * S0; /* sum over v > t of (v - t + 1) h[v] */
+        if (x == x0 + (lane >> 4)) {
             /* with sign handling the data leave out the sign nibbles
              * (RateControl.c:156-210): fast signs count 4 per group above
              * t, full signs the coefficients that stay non-zero */
+            const uint32_t nos = (uint32_t)dsum + bls[x].gcli_w - (uint32_t)S0, fb = lfb[x];
             tdat[x][t] = 4u * (uint32_t)(dsum - (fs ? S0 : 0));
-            tnos[x][t] = (uint32_t)dsum + N - (uint32_t)S0;
+            tnos[x][t] = nos;
+            tsig[x][t] = nos - Z;
             if (SIGNS) {
                 tfs[x][t] = 4u * (uint32_t)S0;
-                const uint32_t zh = nzh[x][t];
-                tnz[x][t] = Z1;
-                Z1 += zh;
+                tnz[x][t] = Z1 - zh;
             }
-            S0 += (int)h;
-            S1 += t * (int)h;
-        }
-        uint32_t Z = 0; /* groups in significance groups whose maximum is <= t: no GCLI codes */
-        const uint32_t fb = lfb[x];
-        for (int t = 0; t < 16; t++) {
-            Z += shist[x][t];
-            tsig[x][t] = tnos[x][t] - Z;
-            atomicAdd(&cn[fb][t], tnos[x][t]);
-            atomicAdd(&cs[fb][t], tsig[x][t] + lsig[x]);
+            atomicAdd(&cn[fb][t], nos);
+            atomicAdd(&cs[fb][t], nos - Z + lsig[x]);
         }
     }
     __syncthreads();
@@ -828,23 +881,24 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
         }
     }
     /* coding method per band and t: significance only if strictly cheaper
-     * (RateControl.c:528-575) */
-    for (uint32_t fb = threadIdx.x; fb < cfg->nbands; fb += blockDim.x) {
-        uint32_t m = 0;
-        if (cfg->sig)
-            for (int t = 0; t < 16; t++) m |= (cn[fb][t] > cs[fb][t] ? 1u : 0u) << t;
-        meth[fb] = (uint16_t)m;
+     * (RateControl.c:528-575); tnos becomes the GCLI bits of the method
+     * chosen, tsig its significance flags */
+    const int nq = cfg->max_q + 1, nr = cfg->max_r + 1;
+    const uint32_t sig = cfg->sig;
+    for (uint32_t i = threadIdx.x; i < nbl * 16; i += blockDim.x) {
+        const uint32_t x = i >> 4, t = i & 15, fb = lfb[x];
+        const bool m = sig && cn[fb][t] > cs[fb][t];
+        if (m) tnos[x][t] = tsig[x][t];
+        tsig[x][t] = m ? lsig[x] : 0u;
     }
-    __syncthreads();
-
     /* costs: band priorities are distinct, so raising R by one lowers the
      * gtli of one band only; each (Q, packet) thread adds its packet's cost
      * at R = 0 and its change at every R where one of its band lines drops,
      * and the table is a prefix sum over R */
-    const int nq = cfg->max_q + 1, nr = cfg->max_r + 1;
-    for (int e = threadIdx.x; e < nq * 32; e += blockDim.x) {
-        dC[e >> 5][e & 31] = 0;
-        if (SIGNS) dF[e >> 5][e & 31] = 0;
+    if (SIGNS) __syncthreads(); /* dF takes the place of shist */
+    for (int e = threadIdx.x; e < nq * 33; e += blockDim.x) {
+        (&dC[0][0])[e] = 0;
+        if (SIGNS) (&dF[0][0])[e] = 0;
     }
     __syncthreads();
     /* with sign handling each packet adds its sign sub-packet, rounded on
@@ -854,25 +908,20 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
      * are the same for the whole warp */
     for (uint32_t k = warp; k < npk; k += RC_WARPS) {
         const int q = lane;
-        const uint32_t b0 = s_pkbl0[k], nb = s_pknbl[k];
+        const uint32_t b0 = s_pkbl0[k], nb = s_pknbl[k], raw = lraw[k];
         if (!nb || q >= nq) continue;
         uint32_t db = 0, gb = 0, sb = 0, fb = 0, zb = 0;
         for (uint32_t x = b0; x < b0 + nb; x++) {
-            const int g = lgain[x];
-            const int t = q < g ? 0 : min(q - g, 15);
+            const int t = min(max(q - (int)lgain[x], 0), 15);
             db += tdat[x][t];
-            if ((meth[lfb[x]] >> t) & 1u) {
-                gb += tsig[x][t];
-                sb += lsig[x];
-            } else {
-                gb += tnos[x][t];
-            }
+            gb += tnos[x][t];
+            sb += tsig[x][t];
             if (fs) {
                 fb += tfs[x][t];
                 zb += tnz[x][t];
             }
         }
-        const uint32_t base = ((db + 7) >> 3) + min(lraw[k], ((sb + 7) >> 3) + ((gb + 7) >> 3));
+        const uint32_t base = ((db + 7) >> 3) + min(raw, ((sb + 7) >> 3) + ((gb + 7) >> 3));
         uint32_t c = base + (fs ? (fb + 7) >> 3 : 0u), cf = base + ((zb + 7) >> 3);
         atomicAdd(&dC[q][0], c);
         if (fs) atomicAdd(&dF[q][0], cf);
@@ -881,12 +930,11 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
             const int rf = lprio[x] + 1; /* the line's gtli drops by one for R >= priority + 1 */
             if (rf >= nr) break;
             const int g = lgain[x];
-            const int t0 = q < g ? 0 : min(q - g, 15), t1 = q < g + 1 ? 0 : min(q - g - 1, 15);
-            const uint32_t m0 = (meth[lfb[x]] >> t0) & 1u, m1 = (meth[lfb[x]] >> t1) & 1u;
+            const int t0 = min(max(q - g, 0), 15), t1 = min(max(q - g - 1, 0), 15);
             db += tdat[x][t1] - tdat[x][t0];
-            gb += (m1 ? tsig[x][t1] : tnos[x][t1]) - (m0 ? tsig[x][t0] : tnos[x][t0]);
-            sb += (m1 ? lsig[x] : 0u) - (m0 ? lsig[x] : 0u);
-            const uint32_t base1 = ((db + 7) >> 3) + min(lraw[k], ((sb + 7) >> 3) + ((gb + 7) >> 3));
+            gb += tnos[x][t1] - tnos[x][t0];
+            sb += tsig[x][t1] - tsig[x][t0];
+            const uint32_t base1 = ((db + 7) >> 3) + min(raw, ((sb + 7) >> 3) + ((gb + 7) >> 3));
             uint32_t c1 = base1;
             if (fs) {
                 fb += tfs[x][t1] - tfs[x][t0];
@@ -901,17 +949,23 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
         }
     }
     __syncthreads();
+    /* a warp per Q, a lane per R */
     uint32_t* out = cost + (uint64_t)p * 32 * 32;
     uint32_t* outf = cost + ((uint64_t)cfg->np + p) * 32 * 32;
-    for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-        uint32_t run = 0, runf = 0;
-        for (int r = 0; r < nr; r++) {
-            run += dC[q][r];
-            out[q * 32 + r] = run;
-            if (fs) {
-                runf += dF[q][r];
-                outf[q * 32 + r] = runf;
+    for (int q = warp; q < nq; q += RC_WARPS) {
+        uint32_t c = dC[q][lane], f = SIGNS && fs ? dF[q][lane] : 0u;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, c, o);
+            if (lane >= o) c += y;
+            if (SIGNS) {
+                const uint32_t yf = __shfl_up_sync(FULL, f, o);
+                if (lane >= o) f += yf;
             }
+        }
+        if (lane < nr) {
+            out[q * 32 + lane] = c;
+            if (SIGNS && fs) outf[q * 32 + lane] = f;
         }
     }
     /* the block that completes a slice runs the slice's selection: tables
