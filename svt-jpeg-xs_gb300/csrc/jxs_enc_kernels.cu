@@ -633,6 +633,14 @@ DEV uint32_t nz_levels(uint32_t m, uint32_t g, uint32_t uniform) {
  *   costs       per packet, data / significance / GCLI bytes rounded
  *               separately, raw fallback when cheaper; summed over packets
  *               for every (Q, R). */
+/* a << n, 0 for n >= 32 (the machine's shift, for which C++ has no
+ * expression without a comparison) */
+DEV uint32_t shl_or_0(uint32_t a, uint32_t n) {
+    uint32_t r;
+    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(n));
+    return r;
+}
+
 template <bool SIGNS, bool VPRED>
 __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ gcli,
                                              const uint16_t* __restrict__ coef, uint32_t* __restrict__ cost,
@@ -716,12 +724,16 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
 
     /* histograms: each lane 4 consecutive groups (one 4-byte load) in 4-bit
      * counters, one per GCLI value (at most 4, or 8 for a significance
-     * group's weight), widened to bytes and summed over the warp per 128
-     * groups (at most 128 per bin); then lane b < 16 holds the count of
-     * GCLI b and lane 16 + b that of significance-group maximum b, adds it
-     * to the band line's histogram and, for a segment of at most 128
-     * groups, stores it as byte b / 16 + b of the segment's histograms for
-     * packing */
+     * group's weight), values 0..7 in one word and 8..15 in another, each
+     * counter reached by a shift that gives 0 past the word; widened to
+     * bytes and summed over the warp per 128 groups (at most 128 per bin);
+     * then lane b < 16 holds the count of GCLI b and lane 16 + b that of
+     * significance-group maximum b, adds it to the band line's histogram
+     * and, for a segment of at most 128 groups, stores it as byte b / 16 + b
+     * of the segment's histograms for packing.  Groups without a GCLI of 8 or
+     * more skip the upper word.  Bound by instruction issue: 58 warp
+     * instructions per 128 groups fewer than counters picked by comparisons and
+     * 8-byte maxima (8 4K frames: 143 -> 132 us). */
     uint32_t* seghist = cost + jxs_seghist_word(cfg) + (uint64_t)p * jxs_seg_cap(cfg) * JXS_SEGHIST_WORDS;
     static_assert(JXS_SEGHIST_WORDS * 4 == 32, "a segment's histograms: one byte per lane");
     const bool export_hist = SG <= 128;
@@ -729,13 +741,6 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
      * value (lanes 0..15) or significance (16..31) words */
     const uint32_t hb = lane & 15u, hsh = 8u * ((hb >> 1) & 3u);
     uint32_t* htab = (lane < 16 ? &hist[0][0] : &shist[0][0]) + hb;
-    /* the first 4 groups of the lane in a segment, read one segment ahead */
-    auto first4 = [&](uint32_t sidx) {
-        const jxs_seg_t sg = segs[sidx];
-        const uint32_t g = sg.g0 + 4 * lane;
-        return g < min(sg.g0 + SG, bls[sg.bl].gcli_w) ? *(const uint32_t*)(gcli + s_grow[sg.bl] + g) : 0u;
-    };
-    uint32_t ahead = (uint32_t)warp < nseg ? first4(warp) : 0u;
     for (uint32_t sidx = warp; sidx < nseg; sidx += RC_WARPS) {
         const jxs_seg_t sg = segs[sidx];
         const uint32_t x = sg.bl;
@@ -746,47 +751,40 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
             const jxs_band_t& bd = cfg->band[lfb[x]];
             crow = coef + bd.coef_off + (uint64_t)(p * bd.lines + bls[x].line) * bd.pitch;
         }
-        const uint32_t cur = ahead;
-        if (sidx + RC_WARPS < nseg) ahead = first4(sidx + RC_WARPS);
         for (uint32_t base = sg.g0; base < gend; base += 128) {
             const uint32_t g = base + 4 * lane;
             const uint32_t nv = g < gend ? min(4u, gend - g) : 0u;
-            uint32_t w4 = base == sg.g0 ? cur : nv ? *(const uint32_t*)(grow + g) : 0u;
+            uint32_t w4 = nv ? *(const uint32_t*)(grow + g) : 0u;
             /* GCLIs past the line's end read as 0 and are taken off bin 0 */
             w4 &= nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
-            uint32_t lo = nv - 4u, hi = 0u; /* bin 0 starts at -(4 - nv) */
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                const uint32_t v = (w4 >> (8 * k)) & 15u;
-                const uint32_t inc = 1u << (4 * (v & 7u));
-                if (v & 8u) hi += inc;
-                else lo += inc;
-            }
-            const uint32_t m2 = __vmaxu4(w4, w4 >> 16), m = max(m2 & 255u, (m2 >> 8) & 255u);
             /* significance group: 8 groups in lanes 2i, 2i+1; its groups
              * (8, or fewer at the end of a line) counted at its maximum */
-            const uint32_t mx = max(m, __shfl_xor_sync(FULL, m, 1));
-            const uint32_t nvp = nv + __shfl_xor_sync(FULL, nv, 1);
-            uint32_t slo = 0u, shi = 0u;
-            if (!(lane & 1) && nv) {
-                const uint32_t si = nvp << (4 * (mx & 7u));
-                if (mx & 8u) shi = si;
-                else slo = si;
-            }
-            /* bytes: even bins, odd bins of 0..7 and of 8..15 */
+            uint32_t m = __vmaxu2(w4 & 0x00ff00ffu, (w4 >> 8) & 0x00ff00ffu);
+            m = __vmaxu2(m, m >> 16);
+            const uint32_t mx = __vmaxu2(m, __shfl_xor_sync(FULL, m, 1)) & 255u;
+            const uint32_t left = gend - base; /* groups of the segment from base on */
+            const uint32_t nvp = (lane & 1) || g >= gend ? 0u : min(8u, left - 4 * lane);
+            /* 4 GCLI per byte */
+            const uint32_t a4 = 4u * w4;
             const uint32_t M = 0x0f0f0f0fu;
+            const uint32_t lo = nv - 4u + shl_or_0(1u, a4 & 255u) + shl_or_0(1u, __byte_perm(a4, 0u, 0x4441)) +
+                                shl_or_0(1u, __byte_perm(a4, 0u, 0x4442)) + shl_or_0(1u, a4 >> 24); /* bin 0 starts at -(4 - nv) */
+            const uint32_t slo = shl_or_0(nvp, 4u * mx);
             const uint32_t v0 = __reduce_add_sync(FULL, lo & M), v1 = __reduce_add_sync(FULL, (lo >> 4) & M);
             const uint32_t s0 = __reduce_add_sync(FULL, slo & M), s1 = __reduce_add_sync(FULL, (slo >> 4) & M);
-            uint32_t v2 = 0, v3 = 0, s2 = 0, s3 = 0;
-            if (__any_sync(FULL, hi)) {
-                v2 = __reduce_add_sync(FULL, hi & M);
-                v3 = __reduce_add_sync(FULL, (hi >> 4) & M);
-                s2 = __reduce_add_sync(FULL, shi & M);
-                s3 = __reduce_add_sync(FULL, (shi >> 4) & M);
+            const uint32_t even = lane < 16 ? v0 : s0, odd = lane < 16 ? v1 : s1;
+            uint32_t word = hb >= 8 ? 0u : hb & 1 ? odd : even;
+            if (__any_sync(FULL, w4 & 0x08080808u)) {
+                /* the same for values 8..15 (shifts less 32) */
+                const uint32_t b4 = a4 ^ 0x20202020u; /* 4 v - 32 per byte, 32 or more below 8 */
+                const uint32_t hi = shl_or_0(1u, b4 & 255u) + shl_or_0(1u, __byte_perm(b4, 0u, 0x4441)) +
+                                    shl_or_0(1u, __byte_perm(b4, 0u, 0x4442)) + shl_or_0(1u, b4 >> 24);
+                const uint32_t shi = shl_or_0(nvp, 4u * mx - 32u);
+                const uint32_t v2 = __reduce_add_sync(FULL, hi & M), v3 = __reduce_add_sync(FULL, (hi >> 4) & M);
+                const uint32_t s2 = __reduce_add_sync(FULL, shi & M), s3 = __reduce_add_sync(FULL, (shi >> 4) & M);
+                if (hb >= 8) word = lane < 16 ? (hb & 1 ? v3 : v2) : (hb & 1 ? s3 : s2);
             }
-            const uint32_t wv = hb >= 8 ? (hb & 1 ? v3 : v2) : (hb & 1 ? v1 : v0);
-            const uint32_t ws = hb >= 8 ? (hb & 1 ? s3 : s2) : (hb & 1 ? s1 : s0);
-            const uint32_t c = ((lane < 16 ? wv : ws) >> hsh) & 255u;
+            const uint32_t c = (word >> hsh) & 255u;
             if (c) atomicAdd(htab + 16 * x, c);
             if (export_hist) ((uint8_t*)(seghist + sidx * JXS_SEGHIST_WORDS))[lane] = (uint8_t)c;
             if (fs) {
@@ -1003,10 +1001,11 @@ __device__ __forceinline__ uint32_t queue_next(uint32_t* ctr, int lane) {
     return __shfl_sync(0xffffffffu, v, 0);
 }
 
-/* OR the low `n` bits (1..64) of `v` into a big-endian bit string stored in
- * native byte order (byte i of the string is byte i of the buffer), at bit
- * `pos`.  Bits past the buffer's `nw` words are not written and set `ovf`
- * (the sizes would disagree with the rate control). */
+/* The precinct being packed is a bit string in 32-bit words, first bit in
+ * the most significant position; its bytes are swapped when it is copied
+ * out.  OR the low `n` bits (1..64) of `v` into it at bit `pos`.  Bits past
+ * the buffer's `nw` words are not written and set `ovf` (the sizes would
+ * disagree with the rate control). */
 DEV void put_bits(uint32_t* buf, uint32_t nw, uint32_t pos, uint64_t v, uint32_t n, int& ovf) {
     if (((pos + n - 1) >> 5) >= nw) {
         ovf = 1;
@@ -1015,19 +1014,38 @@ DEV void put_bits(uint32_t* buf, uint32_t nw, uint32_t pos, uint64_t v, uint32_t
     const uint64_t a = v << (64 - n); /* left-aligned */
     const uint32_t hi = (uint32_t)(a >> 32), lo = (uint32_t)a;
     const uint32_t w = pos >> 5, sh = pos & 31;
-    atomicOr(&buf[w], __byte_perm(hi >> sh, 0, 0x0123));
-    if (sh + n > 32) atomicOr(&buf[w + 1], __byte_perm(__funnelshift_r(lo, hi, sh), 0, 0x0123));
-    if (sh + n > 64) atomicOr(&buf[w + 2], __byte_perm(lo << (32 - sh), 0, 0x0123));
+    atomicOr(&buf[w], hi >> sh);
+    if (sh + n > 32) atomicOr(&buf[w + 1], __funnelshift_r(lo, hi, sh));
+    if (sh + n > 64) atomicOr(&buf[w + 2], lo << (32 - sh));
 }
+/* The same for at most 32 bits, left-aligned in `a` (zeros after them), that
+ * are known to lie inside the buffer. */
+DEV void put_left32(uint32_t* buf, uint32_t pos, uint32_t a) {
+    const uint32_t w = pos >> 5, sh = pos & 31, lo = __funnelshift_r(0u, a, sh);
+    atomicOr(&buf[w], a >> sh);
+    if (lo) atomicOr(&buf[w + 1], lo);
+}
+/* all ones in every byte whose top bit is set */
+DEV uint32_t sign_bytes(uint32_t x) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %1, 0xba98;" : "=r"(r) : "r"(x));
+    return r;
+}
+/* byte i of the bit string */
+DEV uint8_t& byte_at(uint32_t* buf, uint32_t i) { return ((uint8_t*)buf)[i ^ 3u]; }
 
-DEV uint32_t warp_excl_scan(uint32_t x, uint32_t* total) {
-    const int lane = threadIdx.x & 31;
-    uint32_t inc = x;
+/* Inclusive sum over the lanes up to this one (the shuffle's own predicate
+ * says whether there is a lane to add). */
+DEV uint32_t warp_incl_scan(uint32_t x) {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(FULL, inc, o);
-        if (lane >= o) inc += y;
-    }
+    for (int o = 1; o < 32; o <<= 1)
+        asm volatile("{.reg .u32 r; .reg .pred p; shfl.sync.up.b32 r|p, %0, %1, 0, 0xffffffff; @p add.u32 %0, %0, r;}"
+                     : "+r"(x)
+                     : "r"(o));
+    return x;
+}
+DEV uint32_t warp_excl_scan(uint32_t x, uint32_t* total) {
+    const uint32_t inc = warp_incl_scan(x);
     *total = __shfl_sync(FULL, inc, 31);
     return inc - x;
 }
@@ -1127,12 +1145,11 @@ DEV uint64_t data_chunk_signed(uint2 raw4, uint32_t v, uint32_t t, uint32_t unif
     return planes;
 }
 
-/* Per band line of the precinct being packed. */
-struct PkLine {
-    uint32_t sig_pos, gcli_pos, data_pos, sign_pos; /* bit positions in the shared-memory precinct */
-    uint32_t data, vlc, zero, nz; /* data bits, VLC bits without significance, groups in insignificant significance
-                                     groups, signs sent in the sign sub-packet */
-    uint8_t meth, raw, pad0, pad1;
+/* A segment as pass B reads it: bit positions of its first GCLI code and
+ * data bit, first group and group count, gtli | method << 4 | raw << 6 | band
+ * line << 8. */
+struct PkSeg {
+    uint32_t vpos, dpos, g0n, info;
 };
 
 /* pack_precinct (PackPrecinct.c:235-572) for one precinct row.
@@ -1147,53 +1164,57 @@ struct PkLine {
  *           per segment), or, with sign handling, vertical prediction or
  *           segments of more than 128 groups, from the GCLIs (warp per
  *           segment);
- *   layout  warp 0, lanes over band lines, bands, packets: coding method per
- *           band (significance only if strictly cheaper), packet headers, raw
- *           fallback, packet positions by a warp scan, sub-packet positions,
- *           each segment's start in its GCLI and data sub-packets;
+ *   layout  band totals (thread per segment); warp 0: coding method per band
+ *           (significance only if strictly cheaper), running sums over the
+ *           segments and lines in packet order, packet headers, raw
+ *           fallback, packet positions; then each segment's positions
+ *           (thread per segment): a segment's start in its sub-packet is the
+ *           running sum up to it less that at its packet's first segment;
  *   pass B  each lane 4 groups: significance flags and the unary GCLI
  *           codes at positions from a warp prefix sum; the groups above
  *           gtli listed per warp, each lane then packing one listed group's
  *           data bits; everything OR-ed into the buffer.
- * VPRED (frames with vertical prediction; compiled out otherwise): a
+ * SIGNS: the launch may hold frames with sign handling; VPRED: with vertical
+ * prediction (both compiled out otherwise).  With vertical prediction a
  * precinct row below another of its slice also sums, per segment, the
  * codes of its GCLIs predicted from the line above at its gtli (line 0:
  * from the row above, with that row's gtli) and the groups that need no
  * code; the layout chooses among the four codings per band like the rate
  * control (RateControl.c:526-676), and pass B writes the prediction codes
  * (pack_bitplane_count_vpred_*, PackPrecinct.c:47-74). */
-template <bool VPRED>
+template <bool SIGNS, bool VPRED>
 __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, const uint16_t* __restrict__ coef,
                                           const uint8_t* __restrict__ gcli, const PrecRC* __restrict__ rc,
                                           const uint32_t* __restrict__ cost, uint8_t* __restrict__ out, uint32_t cap_words,
                                           int* status, const int p) {
     extern __shared__ __align__(16) uint32_t buf[];
-    /* per segment: data bits, VLC bits, groups without codes, signs; in pass
-     * B the same words hold each warp's list of significant groups */
-    __shared__ uint32_t s_segw[4][JXS_MAXSEG];
+    /* per segment: data bits, VLC bits, groups without codes, signs, then
+     * running sums; in pass B the same words hold each warp's list of
+     * significant groups */
+    __shared__ uint32_t s_segw[4][JXS_MAXSEG + 4];
     uint32_t* s_data = s_segw[0];
     uint32_t* s_vlc = s_segw[1];
     uint32_t* s_zero = s_segw[2];
     uint32_t* s_nz = s_segw[3];
     static_assert(4 * JXS_MAXSEG >= 128 * PK_WARPS, "a list of 128 groups per warp");
-    __shared__ PkLine pl[JXS_MAXBLINES];
+    __shared__ __align__(16) PkSeg s_desc[JXS_MAXSEG];
+    __shared__ uint32_t s_nst[SIGNS ? JXS_MAXSEG : 1];                 /* per segment: first sign bit */
     __shared__ uint8_t s_meth[JXS_MAXBL];
     __shared__ uint32_t s_cn[JXS_MAXBL], s_cs[JXS_MAXBL];
     __shared__ uint32_t s_vn[VPRED ? JXS_MAXSEG : 1], s_vr[VPRED ? JXS_MAXSEG : 1]; /* per segment: prediction bits */
     __shared__ uint32_t s_cv[VPRED ? JXS_MAXBL : 1], s_cvs[VPRED ? JXS_MAXBL : 1];   /* per band: prediction totals */
     __shared__ int8_t s_gtt[VPRED ? JXS_MAXBLINES : 1];                            /* per line: gtli of the line above (-1: this row's) */
-    __shared__ uint32_t s_lvn[VPRED ? JXS_MAXBLINES : 1], s_lvr[VPRED ? JXS_MAXBLINES : 1]; /* per line: prediction bits */
     __shared__ uint32_t s_gp[VPRED ? JXS_MAXBLINES : 1];                           /* per line: GCLI row pitch */
-    __shared__ uint32_t s_lg[JXS_MAXBLINES], s_ls[JXS_MAXBLINES];       /* per line: GCLI / significance bits */
-    __shared__ uint32_t s_pks[JXS_MAXPK], s_pkg[JXS_MAXPK], s_pkd[JXS_MAXPK], s_pkn[JXS_MAXPK]; /* per packet: sub-packet starts */
+    __shared__ uint32_t s_lsx[JXS_MAXBLINES + 1], s_lrx[JXS_MAXBLINES + 1]; /* per line: significance / raw GCLI bits before it */
+    __shared__ uint32_t s_pks[JXS_MAXPK], s_pkg[JXS_MAXPK], s_pkd[JXS_MAXPK], s_pkn[JXS_MAXPK]; /* per packet: sub-packet starts less the running sums there */
     __shared__ uint8_t s_pkr[JXS_MAXPK];
-    __shared__ uint32_t s_vst[JXS_MAXSEG], s_dst[JXS_MAXSEG], s_nst[JXS_MAXSEG]; /* per segment: GCLI / data / sign bit starts */
     /* this precinct kind's tables, staged from the configuration */
     __shared__ jxs_seg_t s_seg[JXS_MAXSEG];
     __shared__ uint16_t s_ord[JXS_MAXSEG];                              /* work order of the segments */
     __shared__ uint32_t s_q[2];                                         /* work queues of passes A and B */
     __shared__ jxs_bline_t s_bl[JXS_MAXBLINES];
     __shared__ uint64_t s_grow[JXS_MAXBLINES], s_crow[JXS_MAXBLINES]; /* per line: GCLI / coefficient row offsets */
+    __shared__ uint32_t s_sigp[JXS_MAXBLINES];                         /* per line: bit position of its significance flags */
     __shared__ uint8_t s_lt[JXS_MAXBLINES];                            /* per line: gtli */
     __shared__ uint8_t s_pkbl0[JXS_MAXPK], s_pknbl[JXS_MAXPK];
     __shared__ uint32_t s_praw[JXS_MAXPK];
@@ -1222,7 +1243,7 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
         return;
     }
     int ovf = 0;
-    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) buf[i] = 0;
+    for (uint32_t i = threadIdx.x; i < words >> 2; i += blockDim.x) ((uint4*)buf)[i] = make_uint4(0u, 0u, 0u, 0u);
     for (uint32_t fb = threadIdx.x; fb < cfg->nbands; fb += blockDim.x) {
         s_cn[fb] = 0;
         s_cs[fb] = 0;
@@ -1233,7 +1254,7 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
     }
     /* vertical prediction applies below the first row of a slice */
     const int vp = VPRED && cfg->vpred && !R.first_in_slice;
-    const int rmode = cfg->rm;
+    const int rmode = VPRED ? (int)cfg->rm : 0;
     {
         const uint32_t ns = cfg->nseg[last], nl = cfg->nbline[last];
         for (uint32_t i = threadIdx.x; i < ns * (sizeof(jxs_seg_t) / 4); i += blockDim.x)
@@ -1283,7 +1304,7 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
     /* pass A: each lane 4 consecutive groups (one 4-byte GCLI load), a warp
      * 128 groups per step; with sign handling also the non-zero quantized
      * coefficients, whose signs go to the sign sub-packets */
-    const uint32_t fs = cfg->fs, uniform = cfg->qpih;
+    const uint32_t fs = SIGNS ? cfg->fs : 0u, uniform = cfg->qpih;
     if (!VPRED && !fs && SG <= 128) {
         /* from the rate control's histograms: data bits 4 (v - t + 1) and
          * codes of v - t + 1 bits for groups with GCLI v > t, 1-bit codes
@@ -1393,37 +1414,20 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
     }
     __syncthreads();
 
-    /* layout, by warp 0: lanes over band lines, bands, packets, segments */
+    /* layout: band totals of every coding */
+    for (uint32_t i = threadIdx.x; i < nseg; i += blockDim.x) {
+        const jxs_bline_t& B = bls[segs[i].bl];
+        const uint32_t sw = segs[i].g0 ? 0u : B.sig_w;
+        atomicAdd(&s_cn[B.fb], s_vlc[i]);
+        atomicAdd(&s_cs[B.fb], s_vlc[i] - s_zero[i] + sw);
+        if (VPRED && vp) {
+            atomicAdd(&s_cv[B.fb], s_vn[i]);
+            atomicAdd(&s_cvs[B.fb], s_vn[i] - s_vr[i] + sw);
+        }
+    }
+    __syncthreads();
     if (warp == 0) {
         const uint32_t nbl = s_nbl;
-        for (uint32_t b = lane; b < nbl; b += 32) {
-            const jxs_bline_t& B = bls[b];
-            uint32_t d = 0, v = 0, z = 0, n = 0;
-            for (uint32_t i = B.seg0; i < B.seg0 + B.nseg; i++) {
-                d += s_data[i];
-                v += s_vlc[i];
-                z += s_zero[i];
-                n += s_nz[i];
-            }
-            pl[b].data = d;
-            pl[b].vlc = v;
-            pl[b].zero = z;
-            pl[b].nz = n;
-            atomicAdd(&s_cn[B.fb], v);
-            atomicAdd(&s_cs[B.fb], v - z + B.sig_w);
-            if (VPRED && vp) {
-                uint32_t vn = 0, vr = 0;
-                for (uint32_t i = B.seg0; i < B.seg0 + B.nseg; i++) {
-                    vn += s_vn[i];
-                    vr += s_vr[i];
-                }
-                s_lvn[b] = vn;
-                s_lvr[b] = vr;
-                atomicAdd(&s_cv[B.fb], vn);
-                atomicAdd(&s_cvs[B.fb], vn - vr + B.sig_w);
-            }
-        }
-        __syncwarp();
         /* coding method per band, D[p,b] (bit 1 significance, bit 0
          * prediction): a later one only if strictly cheaper
          * (RateControl.c:526-676) */
@@ -1443,23 +1447,75 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
             s_meth[fb] = (uint8_t)m;
         }
         __syncwarp();
-        /* per line: GCLI and significance bits with the band's method */
-        for (uint32_t b = lane; b < nbl; b += 32) {
-            const uint8_t m = s_meth[bls[b].fb];
-            pl[b].meth = m;
-            s_lg[b] = m == 0 ? pl[b].vlc : m == 2 ? pl[b].vlc - pl[b].zero : m == 1 ? s_lvn[VPRED ? b : 0] : s_lvn[VPRED ? b : 0] - s_lvr[VPRED ? b : 0];
-            s_ls[b] = (m & 2) ? bls[b].sig_w : 0u;
+        /* data, GCLI and sign bits before every segment (into s_data, s_vlc,
+         * s_nz), each lane a run of them */
+        {
+            const uint32_t per = (nseg + 31) >> 5, i0 = min(nseg, per * lane), i1 = min(nseg, i0 + per);
+            uint32_t d = 0, g = 0, n = 0;
+            for (uint32_t i = i0; i < i1; i++) {
+                const uint32_t m = s_meth[bls[segs[i].bl].fb];
+                const uint32_t gi = m == 0 ? s_vlc[i] : m == 2 ? s_vlc[i] - s_zero[i] : m == 1 ? s_vn[VPRED ? i : 0] : s_vn[VPRED ? i : 0] - s_vr[VPRED ? i : 0];
+                s_zero[i] = gi;
+                d += s_data[i];
+                g += gi;
+                if (SIGNS) n += s_nz[i];
+            }
+            uint32_t td, tg, tn = 0;
+            d = warp_excl_scan(d, &td);
+            g = warp_excl_scan(g, &tg);
+            if (SIGNS) n = warp_excl_scan(n, &tn);
+            for (uint32_t i = i0; i < i1; i++) {
+                const uint32_t di = s_data[i], gi = s_zero[i];
+                s_data[i] = d;
+                s_vlc[i] = g;
+                d += di;
+                g += gi;
+                if (SIGNS) {
+                    const uint32_t ni = s_nz[i];
+                    s_nz[i] = n;
+                    n += ni;
+                }
+            }
+            if (lane == 0) {
+                s_data[nseg] = td;
+                s_vlc[nseg] = tg;
+                if (SIGNS) s_nz[nseg] = tn;
+            }
+        }
+        /* significance flags and raw GCLI bits before every line */
+        {
+            const uint32_t per = (nbl + 31) >> 5, x0 = min(nbl, per * lane), x1 = min(nbl, x0 + per);
+            uint32_t sg = 0, rw = 0;
+            for (uint32_t x = x0; x < x1; x++) {
+                sg += (s_meth[bls[x].fb] & 2) ? bls[x].sig_w : 0u;
+                rw += 4 * bls[x].gcli_w;
+            }
+            uint32_t tsg, trw;
+            sg = warp_excl_scan(sg, &tsg);
+            rw = warp_excl_scan(rw, &trw);
+            for (uint32_t x = x0; x < x1; x++) {
+                s_lsx[x] = sg;
+                s_lrx[x] = rw;
+                sg += (s_meth[bls[x].fb] & 2) ? bls[x].sig_w : 0u;
+                rw += 4 * bls[x].gcli_w;
+            }
+            if (lane == 0) {
+                s_lsx[nbl] = tsg;
+                s_lrx[nbl] = trw;
+            }
         }
         __syncwarp();
         /* one lane per packet: sub-packet sizes, raw fallback, header */
         const uint32_t k = lane;
         const uint32_t nb = k < s_npk ? s_pknbl[k] : 0u, b0 = k < s_npk ? s_pkbl0[k] : 0u;
-        uint32_t db = 0, gbits = 0, sbits = 0, nbits = 0;
-        for (uint32_t x = b0; x < b0 + nb; x++) {
-            db += pl[x].data;
-            gbits += s_lg[x];
-            sbits += s_ls[x];
-            nbits += pl[x].nz;
+        uint32_t db = 0, gbits = 0, sbits = 0, nbits = 0, i0 = 0;
+        if (nb) {
+            i0 = bls[b0].seg0;
+            const uint32_t i1 = bls[b0 + nb - 1].seg0 + bls[b0 + nb - 1].nseg;
+            db = s_data[i1] - s_data[i0];
+            gbits = s_vlc[i1] - s_vlc[i0];
+            sbits = s_lsx[b0 + nb] - s_lsx[b0];
+            if (SIGNS) nbits = s_nz[i1] - s_nz[i0];
         }
         const uint32_t dB = (db + 7) >> 3, gB = (gbits + 7) >> 3, sB = (sbits + 7) >> 3, nB = (nbits + 7) >> 3;
         const uint32_t rawB = nb ? s_praw[k] : 0u;
@@ -1473,73 +1529,39 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
         const int fits = start + hb <= words * 4;
         if (nb && fits) {
             /* packet header (PackHeaders.c:98-127) */
-            uint8_t* h = (uint8_t*)buf + start;
             if (s_short) {
-                h[0] = (uint8_t)((raw << 7) | ((dB >> 8) & 0x7f));
-                h[1] = (uint8_t)dB;
-                h[2] = (uint8_t)(gcl_bytes >> 5);
-                h[3] = (uint8_t)(((gcl_bytes & 0x1f) << 3) | ((nB >> 8) & 7));
-                h[4] = (uint8_t)nB;
+                byte_at(buf, start) = (uint8_t)((raw << 7) | ((dB >> 8) & 0x7f));
+                byte_at(buf, start + 1) = (uint8_t)dB;
+                byte_at(buf, start + 2) = (uint8_t)(gcl_bytes >> 5);
+                byte_at(buf, start + 3) = (uint8_t)(((gcl_bytes & 0x1f) << 3) | ((nB >> 8) & 7));
+                byte_at(buf, start + 4) = (uint8_t)nB;
             } else {
-                h[0] = (uint8_t)((raw << 7) | ((dB >> 13) & 0x7f));
-                h[1] = (uint8_t)(dB >> 5);
-                h[2] = (uint8_t)(((dB & 0x1f) << 3) | ((gcl_bytes >> 17) & 7));
-                h[3] = (uint8_t)(gcl_bytes >> 9);
-                h[4] = (uint8_t)(gcl_bytes >> 1);
-                h[5] = (uint8_t)(((gcl_bytes & 1) << 7) | ((nB >> 8) & 0x7f));
-                h[6] = (uint8_t)nB;
+                byte_at(buf, start) = (uint8_t)((raw << 7) | ((dB >> 13) & 0x7f));
+                byte_at(buf, start + 1) = (uint8_t)(dB >> 5);
+                byte_at(buf, start + 2) = (uint8_t)(((dB & 0x1f) << 3) | ((gcl_bytes >> 17) & 7));
+                byte_at(buf, start + 3) = (uint8_t)(gcl_bytes >> 9);
+                byte_at(buf, start + 4) = (uint8_t)(gcl_bytes >> 1);
+                byte_at(buf, start + 5) = (uint8_t)(((gcl_bytes & 1) << 7) | ((nB >> 8) & 0x7f));
+                byte_at(buf, start + 6) = (uint8_t)nB;
             }
-            /* sub-packet starts: significance, GCLIs, data, signs */
-            const uint32_t p0 = (start + hb) * 8;
-            s_pks[k] = p0;
-            s_pkg[k] = raw ? p0 : p0 + sB * 8;
-            s_pkd[k] = p0 + (raw ? rawB : sB + gB) * 8;
-            s_pkn[k] = s_pkd[k] + dB * 8;
+            /* sub-packet starts (significance, GCLIs, data, signs) less the
+             * running sums at the packet's first segment or line */
+            const uint32_t p0 = (start + hb) * 8, pd = p0 + (raw ? rawB : sB + gB) * 8;
+            s_pks[k] = p0 - s_lsx[b0];
+            s_pkg[k] = raw ? p0 - s_lrx[b0] : p0 + sB * 8 - s_vlc[i0];
+            s_pkd[k] = pd - s_data[i0];
+            if (SIGNS) s_pkn[k] = pd + dB * 8 - s_nz[i0];
             s_pkr[k] = (uint8_t)raw;
-        }
-        __syncwarp();
-        /* per line: positions inside its packet's sub-packets */
-        for (uint32_t x = lane; x < nbl; x += 32) {
-            const uint32_t kk = bls[x].pk, xb0 = s_pkbl0[kk];
-            uint32_t sp = 0, gp = 0, dp = 0, np = 0;
-            const int r = s_pkr[kk];
-            for (uint32_t y = xb0; y < x; y++) {
-                sp += s_ls[y];
-                gp += r ? 4 * bls[y].gcli_w : s_lg[y];
-                dp += pl[y].data;
-                np += pl[y].nz;
-            }
-            pl[x].raw = (uint8_t)r;
-            pl[x].sig_pos = s_pks[kk] + sp;
-            pl[x].gcli_pos = s_pkg[kk] + gp;
-            pl[x].data_pos = s_pkd[kk] + dp;
-            pl[x].sign_pos = s_pkn[kk] + np;
-        }
-        __syncwarp();
-        /* per segment: its start in its line's GCLI and data bits */
-        for (uint32_t i = lane; i < nseg; i += 32) {
-            const uint32_t x = segs[i].bl;
-            const uint8_t m = pl[x].meth;
-            uint32_t vp = pl[x].gcli_pos, dp = pl[x].data_pos, np = pl[x].sign_pos;
-            for (uint32_t j = bls[x].seg0; j < i; j++) {
-                vp += m == 0 ? s_vlc[j] : m == 2 ? s_vlc[j] - s_zero[j] : m == 1 ? s_vn[VPRED ? j : 0] : s_vn[VPRED ? j : 0] - s_vr[VPRED ? j : 0];
-                dp += s_data[j];
-                np += s_nz[j];
-            }
-            s_vst[i] = vp;
-            s_dst[i] = dp;
-            s_nst[i] = np;
         }
         /* precinct header: Lprc, Q, R as bytes first, then the 2-bit band
          * coding modes D[p,b] of every existing band */
         if (lane == 0) {
-            uint8_t* bytes = (uint8_t*)buf + lead;
             const uint32_t lprc = total - hdr;
-            bytes[0] = (uint8_t)(lprc >> 16);
-            bytes[1] = (uint8_t)(lprc >> 8);
-            bytes[2] = (uint8_t)lprc;
-            bytes[3] = R.q;
-            bytes[4] = R.r;
+            byte_at(buf, lead) = (uint8_t)(lprc >> 16);
+            byte_at(buf, lead + 1) = (uint8_t)(lprc >> 8);
+            byte_at(buf, lead + 2) = (uint8_t)lprc;
+            byte_at(buf, lead + 3) = R.q;
+            byte_at(buf, lead + 4) = R.r;
         }
         __syncwarp();
         uint32_t idx0 = 0;
@@ -1566,213 +1588,345 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
     }
     __syncthreads();
     if (!s_ok) return;
+    /* every segment's positions */
+    for (uint32_t i = threadIdx.x; i < nseg; i += blockDim.x) {
+        const jxs_seg_t sg = segs[i];
+        const jxs_bline_t& B = bls[sg.bl];
+        const uint32_t m = s_meth[B.fb], raw = s_pkr[B.pk];
+        PkSeg D;
+        D.vpos = s_pkg[B.pk] + (raw ? s_lrx[sg.bl] + 4 * sg.g0 : s_vlc[i]);
+        D.dpos = s_pkd[B.pk] + s_data[i];
+        D.g0n = sg.g0 | (min(SG, B.gcli_w - sg.g0) << 16);
+        D.info = s_lt[sg.bl] | (m << 4) | (raw << 6) | ((uint32_t)sg.bl << 8);
+        s_desc[i] = D;
+        if (SIGNS) s_nst[i] = s_pkn[B.pk] + s_nz[i];
+    }
+    for (uint32_t x = threadIdx.x; x < s_nbl; x += blockDim.x) s_sigp[x] = s_pks[bls[x].pk] + s_lsx[x];
+    __syncthreads();
 
-    /* pass B: each lane 4 consecutive groups; its unary codes are joined
-     * into one write, its data chunks into writes of up to 64 bits, its
-     * signs (with sign handling) into one write */
-    for (uint32_t qi = queue_next(&s_q[1], lane); qi < nseg; qi = queue_next(&s_q[1], lane)) {
-        const uint32_t sidx = s_ord[qi];
-        const jxs_seg_t sg = segs[sidx];
-        const jxs_bline_t B = bls[sg.bl];
-        const PkLine L = pl[sg.bl];
-        const uint32_t t = s_lt[sg.bl];
-        const uint8_t* grow = gcli + s_grow[sg.bl];
-        const uint16_t* crow = coef + s_crow[sg.bl];
-        const uint32_t gend = min(sg.g0 + SG, B.gcli_w);
-        uint32_t vpos = s_vst[sidx], dpos = s_dst[sidx], npos = s_nst[sidx];
-        for (uint32_t base = sg.g0; base < gend; base += 128) {
-            const uint32_t g = base + 4 * lane;
-            const uint32_t nv = g < gend ? min(4u, gend - g) : 0u;
-            /* the lane's GCLIs, one per byte (0 past the line's end) */
-            uint32_t w4 = nv ? *(const uint32_t*)(grow + g) : 0u;
-            w4 &= nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
-            uint4 c0 = make_uint4(0, 0, 0, 0), c1 = c0;
-            if (nv && fs) {
-                c0 = *(const uint4*)(crow + 4 * g);
-                c1 = *(const uint4*)(crow + 4 * g + 8);
+    if constexpr (!SIGNS && !VPRED) {
+        /* pass B.  Bound by instruction issue; per 128 groups about 200 warp
+         * instructions, of them 90 for the groups above gtli. */
+        uint32_t* list = &s_segw[0][0] + 128 * warp;
+        for (uint32_t qi = queue_next(&s_q[1], lane); qi < nseg; qi = queue_next(&s_q[1], lane)) {
+            const uint32_t sidx = s_ord[qi];
+            const PkSeg D = s_desc[sidx];
+            const uint32_t line = D.info >> 8, t = D.info & 15u, n = D.g0n >> 16;
+            const uint8_t* grow = gcli + s_grow[line] + (D.g0n & 0xffffu);
+            const uint16_t* crow = coef + s_crow[line] + 4 * (D.g0n & 0xffffu);
+            uint32_t vpos = D.vpos, dpos = D.dpos;
+            if ((D.info & 64u) && vpos + 4 * n > words * 32) {
+                ovf = 1;
+                continue;
             }
-            /* per byte: planes above gtli d = max(v - t, 0), and v > t */
-            const uint32_t t4 = t * 0x01010101u;
-            const uint32_t d4 = __vsubus4(w4, t4), s4 = __vcmpgtu4(w4, t4);
-            const uint32_t dsum = __vsadu4(d4, 0u), nsig = __popc(s4 & 0x01010101u);
-            uint32_t v[4];
-#pragma unroll
-            for (int k = 0; k < 4; k++) v[k] = (w4 >> (8 * k)) & 255u;
-            const uint32_t m2 = __vmaxu4(w4, w4 >> 16), m = max(m2 & 255u, (m2 >> 8) & 255u);
-            const uint32_t mx = max(m, __shfl_xor_sync(FULL, m, 1));
-            /* a significance group without codes: all GCLIs <= gtli, or with
-             * prediction the group's flag */
-            bool insig = mx <= t;
-            uint32_t n4[4] = {0, 0, 0, 0}; /* prediction: each GCLI's code length */
-            uint64_t vacc = 0;             /* otherwise: the lane's codes joined */
-            uint32_t vl = 0;
-            if (VPRED && (L.meth & 1) && !L.raw) {
-                /* codes predicted from the line above (vlc_encode,
-                 * PackPrecinct.h:41-65) */
-                const uint32_t wt = nv ? *(const uint32_t*)(grow - s_gp[VPRED ? sg.bl : 0] + g) : 0u;
-                const int gmax = max((int)t, (int)s_gtt[VPRED ? sg.bl : 0]);
-                uint32_t flag = 1;
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    if (k < (int)nv) {
-                        const int c = (int)v[k], tp = (int)((wt >> (8 * k)) & 255u);
-                        const int mt = max(tp, gmax), gv = max(c, (int)t);
-                        n4[k] = vlc_vp_bits(gv - mt, mt, (int)t) + 1;
-                        flag &= rmode ? (uint32_t)(c <= (int)t) : (uint32_t)(mt == gv);
-                    }
-                }
-                insig = (flag & __shfl_xor_sync(FULL, flag, 1)) != 0;
-            }
-            if (L.raw) {
-                /* raw GCLIs: the lane's nibbles in one write */
-                if (nv) put_bits(buf, words, L.gcli_pos + 4 * g, ((v[0] << 12) | (v[1] << 8) | (v[2] << 4) | v[3]) >> (4 * (4 - nv)), 4 * nv, ovf);
-            } else {
-                if (L.meth & 2) {
-                    /* significance flags, 1 = insignificant: even lanes lead a group of 8 */
-                    const uint32_t bal = __ballot_sync(FULL, nv && !(lane & 1) && insig);
-                    if (lane == 0) {
-                        /* the even lanes' votes compacted (bit i: group of 8
-                         * number i), then reversed: group 0 first */
-                        const uint32_t nsg = min(16u, (gend - base + 7) >> 3);
-                        uint32_t x = bal & 0x55555555u;
-                        x = (x | (x >> 1)) & 0x33333333u;
-                        x = (x | (x >> 2)) & 0x0f0f0f0fu;
-                        x = (x | (x >> 4)) & 0x00ff00ffu;
-                        x = (x | (x >> 8)) & 0x0000ffffu;
-                        const uint32_t bits = __brev(x) >> (32 - nsg);
-                        if (bits) put_bits(buf, words, L.sig_pos + (base >> 3), bits, nsg, ovf);
-                    }
-                }
-                if (!((L.meth & 2) && insig)) {
-                    if (VPRED && (L.meth & 1)) {
-#pragma unroll
-                        for (int k = 0; k < 4; k++) vl += n4[k];
-                    } else {
-                        /* unary codes: d ones then a zero for each present
-                         * group (PackPrecinct.h:25-39), two groups per word */
-                        uint32_t n[4], c[4];
-#pragma unroll
-                        for (int k = 0; k < 4; k++) {
-                            const uint32_t dk = (d4 >> (8 * k)) & 255u;
-                            n[k] = k < (int)nv ? dk + 1 : 0u;
-                            c[k] = ((1u << dk) - 1u) << 1;
+            for (uint32_t base = 0; base < n; base += 128) {
+                const uint32_t g = base + 4 * lane;
+                const uint32_t nv = g < n ? min(4u, n - g) : 0u;
+                /* the lane's GCLIs, one per byte (0 past the line's end) */
+                uint32_t w4 = nv ? *(const uint32_t*)(grow + g) : 0u;
+                const uint32_t keep = nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
+                w4 &= keep;
+                /* per byte: all ones for a group above gtli (v > t), and its
+                 * planes above gtli d = v - t */
+                const uint32_t y = (w4 | 0x80808080u) - (t + 1) * 0x01010101u;
+                const uint32_t above = sign_bytes(y), ones = above & 0x01010101u;
+                const uint32_t d4 = (y & above & 0x7f7f7f7fu) + ones;
+                /* code bits d + 1 of every group up to and with each byte's,
+                 * data nibbles d + 1 of every group above gtli likewise */
+                const uint32_t codes = (d4 + (keep & 0x01010101u)) * 0x01010101u, nibs = (d4 + ones) * 0x01010101u;
+                uint32_t vl = 0;
+                if (D.info & 64u) {
+                    /* raw GCLIs: the lane's nibbles in one write */
+                    const uint32_t h = ((w4 & 0x000f000fu) << 4) | ((w4 >> 8) & 0x000f000fu);
+                    if (nv) put_left32(buf, vpos + 4 * g, (h << 24) | (h & 0x00ff0000u));
+                } else {
+                    vl = codes >> 24;
+                    if (D.info & 32u) {
+                        /* significance flags, 1 = insignificant, of the groups
+                         * of 8 in lanes 2i, 2i + 1: the even votes compacted (bit
+                         * i: group of 8 number i), then reversed, group 0 first */
+                        const uint32_t bal = __ballot_sync(FULL, above != 0u), some = bal | (bal >> 1);
+                        if (lane == 0) {
+                            const uint32_t nsg = min(16u, (n - base + 7) >> 3), pos = s_sigp[line] + (((D.g0n & 0xffffu) + base) >> 3);
+                            uint32_t x = ~some & 0x55555555u;
+                            x = (x | (x >> 1)) & 0x33333333u;
+                            x = (x | (x >> 2)) & 0x0f0f0f0fu;
+                            x = (x | (x >> 4)) & 0x00ff00ffu;
+                            x = (x | (x >> 8)) & 0x0000ffffu;
+                            const uint32_t bits = (__brev(x) >> (32 - nsg)) << (32 - nsg);
+                            if (pos + nsg > words * 32) ovf = 1;
+                            else put_left32(buf, pos, bits);
                         }
-                        const uint32_t l23 = n[2] + n[3];
-                        vacc = ((uint64_t)((c[0] << n[1]) | c[1]) << l23) | ((c[2] << n[3]) | c[3]);
-                        vl = dsum + nv;
+                        if (!((some >> (lane & 30)) & 1u)) vl = 0;
                     }
                 }
+                /* one scan for three running sums: data nibbles (12 bits), code
+                 * bits (12 bits), listed groups */
+                const uint32_t own = (nibs >> 24) | (vl << 12) | ((uint32_t)__popc(ones) << 24);
+                const uint32_t inc = warp_incl_scan(own), ex = inc - own, tot = __shfl_sync(FULL, inc, 31);
+                const uint32_t tot_d = (tot & 0xfffu) << 2, tot_v = (tot >> 12) & 0xfffu, cnt = tot >> 24;
+                if (max(vpos + tot_v, dpos + tot_d) > words * 32) {
+                    ovf = 1;
+                    break;
+                }
+                if (vl) {
+                    /* unary codes: d ones then a zero for each present group
+                     * (PackPrecinct.h:25-39) */
+                    const uint32_t pos = vpos + ((ex >> 12) & 0xfffu);
+                    if (vl <= 32) {
+                        /* ones, and a zero where each code ends (absent groups
+                         * repeat the last end) */
+                        const uint32_t f = 0x20202020u - codes;
+                        const uint32_t z = (1u << (f & 255u)) | (1u << __byte_perm(f, 0u, 0x4441)) | (1u << __byte_perm(f, 0u, 0x4442)) |
+                                           (1u << (f >> 24));
+                        put_left32(buf, pos, (uint32_t)((int32_t)0x80000000 >> (vl - 1)) & ~z);
+                    } else {
+                        /* up to 64 bits, first code at the top */
+                        uint64_t z = 0;
+#pragma unroll
+                        for (int k = 0; k < 4; k++) z |= 1ull << (64 - ((codes >> (8 * k)) & 255u));
+                        const uint64_t a = (uint64_t)((int64_t)0x8000000000000000ll >> (vl - 1)) & ~z;
+                        put_bits(buf, words, pos, a >> (64 - vl), vl, ovf);
+                    }
+                }
+                /* the warp lists its groups above gtli (nibble offset in the
+                 * warp's data, group, GCLI), then each lane packs one listed
+                 * group at a time, its sign nibble and planes in one write of
+                 * at most 64 bits; the coefficients of the other groups are
+                 * never read */
+                {
+                    const uint32_t po = nibs << 8, pi = ones * 0x01010100u; /* before each byte's group */
+                    const uint32_t e0 = ((ex & 0xfffu) << 16) | ((uint32_t)lane << 6);
+                    uint32_t* slot = list + (ex >> 24);
+                    if (ones & 0x00000001u) slot[0] = e0 + (w4 & 255u);
+                    if (ones & 0x00000100u) slot[(pi >> 8) & 255u] = e0 + 0x10u + __byte_perm(w4, po, 0x4541);
+                    if (ones & 0x00010000u) slot[(pi >> 16) & 255u] = e0 + 0x20u + __byte_perm(w4, po, 0x4642);
+                    if (ones & 0x01000000u) slot[pi >> 24] = e0 + 0x30u + __byte_perm(w4, po, 0x4743);
+                }
+                __syncwarp();
+                for (uint32_t r = lane; r < cnt; r += 32) {
+                    const uint32_t e = list[r];
+                    const uint32_t gi = base + ((e >> 4) & 127u), np = (e & 15u) - t, pos = dpos + 4 * (e >> 16);
+                    /* the coefficients past the band width are stored as zero */
+                    const uint2 raw4 = *(const uint2*)(crow + 4 * gi);
+                    const uint64_t ch = data_chunk_signed(raw4, e & 15u, t, uniform);
+                    if (np < 8) put_left32(buf, pos, (uint32_t)ch << (28 - 4 * np));
+                    else put_bits(buf, words, pos, ch, 4 * (np + 1), ovf);
+                }
+                __syncwarp();
+                vpos += tot_v;
+                dpos += tot_d;
             }
-            /* data bits of the groups above gtli: 4 (d + 1) each (the sign
-             * nibble, unless signs go to their own sub-packet) */
-            const uint32_t dl4 = dsum + (fs ? 0u : nsig);
-            /* one scan for three running sums: data bits / 4 (12 bits), code
-             * bits (13 bits), listed groups (the exclusive sums, at most 124,
-             * in the top 7 bits) */
-            uint32_t tot;
-            const uint32_t ex = warp_excl_scan(dl4 | (vl << 12) | (nsig << 25), &tot);
-            const uint32_t ex_d = (ex & 0xfffu) << 2, ex_v = (ex >> 12) & 0x1fffu;
-            const uint32_t tot_d = (tot & 0xfffu) << 2, tot_v = (tot >> 12) & 0x1fffu;
-            if (vl) {
-                if (VPRED && (L.meth & 1)) {
-                    /* prediction codes (up to 31 bits each): n - 1 ones then
-                     * a zero, joined while they fit 64 bits */
-                    uint32_t pos = vpos + ex_v, an = 0;
-                    uint64_t acc = 0;
+        }
+    } else {
+        /* pass B with signs in a sub-packet of their own or predicted codes:
+         * each lane 4 consecutive groups; its unary codes are joined into one
+         * write, its data chunks into writes of up to 64 bits, its signs into
+         * one write */
+        for (uint32_t qi = queue_next(&s_q[1], lane); qi < nseg; qi = queue_next(&s_q[1], lane)) {
+            const uint32_t sidx = s_ord[qi];
+            const jxs_seg_t sg = segs[sidx];
+            const jxs_bline_t B = bls[sg.bl];
+            const PkSeg D = s_desc[sidx];
+            const uint32_t t = D.info & 15u, meth = (D.info >> 4) & 3u, raw = (D.info >> 6) & 1u;
+            const uint8_t* grow = gcli + s_grow[sg.bl];
+            const uint16_t* crow = coef + s_crow[sg.bl];
+            const uint32_t gend = min(sg.g0 + SG, B.gcli_w);
+            uint32_t vpos = D.vpos, dpos = D.dpos, npos = s_nst[SIGNS ? sidx : 0];
+            for (uint32_t base = sg.g0; base < gend; base += 128) {
+                const uint32_t g = base + 4 * lane;
+                const uint32_t nv = g < gend ? min(4u, gend - g) : 0u;
+                /* the lane's GCLIs, one per byte (0 past the line's end) */
+                uint32_t w4 = nv ? *(const uint32_t*)(grow + g) : 0u;
+                w4 &= nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
+                uint4 c0 = make_uint4(0, 0, 0, 0), c1 = c0;
+                if (nv && fs) {
+                    c0 = *(const uint4*)(crow + 4 * g);
+                    c1 = *(const uint4*)(crow + 4 * g + 8);
+                }
+                /* per byte: planes above gtli d = max(v - t, 0), and v > t */
+                const uint32_t t4 = t * 0x01010101u;
+                const uint32_t d4 = __vsubus4(w4, t4), s4 = __vcmpgtu4(w4, t4);
+                const uint32_t dsum = __vsadu4(d4, 0u), nsig = __popc(s4 & 0x01010101u);
+                uint32_t v[4];
+#pragma unroll
+                for (int k = 0; k < 4; k++) v[k] = (w4 >> (8 * k)) & 255u;
+                const uint32_t m2 = __vmaxu4(w4, w4 >> 16), m = max(m2 & 255u, (m2 >> 8) & 255u);
+                const uint32_t mx = max(m, __shfl_xor_sync(FULL, m, 1));
+                /* a significance group without codes: all GCLIs <= gtli, or with
+                 * prediction the group's flag */
+                bool insig = mx <= t;
+                uint32_t n4[4] = {0, 0, 0, 0}; /* prediction: each GCLI's code length */
+                uint64_t vacc = 0;             /* otherwise: the lane's codes joined */
+                uint32_t vl = 0;
+                if (VPRED && (meth & 1) && !raw) {
+                    /* codes predicted from the line above (vlc_encode,
+                     * PackPrecinct.h:41-65) */
+                    const uint32_t wt = nv ? *(const uint32_t*)(grow - s_gp[VPRED ? sg.bl : 0] + g) : 0u;
+                    const int gmax = max((int)t, (int)s_gtt[VPRED ? sg.bl : 0]);
+                    uint32_t flag = 1;
 #pragma unroll
                     for (int k = 0; k < 4; k++) {
-                        const uint32_t n = n4[k];
-                        if (n) {
+                        if (k < (int)nv) {
+                            const int c = (int)v[k], tp = (int)((wt >> (8 * k)) & 255u);
+                            const int mt = max(tp, gmax), gv = max(c, (int)t);
+                            n4[k] = vlc_vp_bits(gv - mt, mt, (int)t) + 1;
+                            flag &= rmode ? (uint32_t)(c <= (int)t) : (uint32_t)(mt == gv);
+                        }
+                    }
+                    insig = (flag & __shfl_xor_sync(FULL, flag, 1)) != 0;
+                }
+                if (raw) {
+                    /* raw GCLIs: the lane's nibbles in one write */
+                    if (nv) put_bits(buf, words, D.vpos + 4 * (g - sg.g0), ((v[0] << 12) | (v[1] << 8) | (v[2] << 4) | v[3]) >> (4 * (4 - nv)), 4 * nv, ovf);
+                } else {
+                    if (meth & 2) {
+                        /* significance flags, 1 = insignificant: even lanes lead a group of 8 */
+                        const uint32_t bal = __ballot_sync(FULL, nv && !(lane & 1) && insig);
+                        if (lane == 0) {
+                            /* the even lanes' votes compacted (bit i: group of 8
+                             * number i), then reversed: group 0 first */
+                            const uint32_t nsg = min(16u, (gend - base + 7) >> 3);
+                            uint32_t x = bal & 0x55555555u;
+                            x = (x | (x >> 1)) & 0x33333333u;
+                            x = (x | (x >> 2)) & 0x0f0f0f0fu;
+                            x = (x | (x >> 4)) & 0x00ff00ffu;
+                            x = (x | (x >> 8)) & 0x0000ffffu;
+                            const uint32_t bits = __brev(x) >> (32 - nsg);
+                            if (bits) put_bits(buf, words, s_sigp[sg.bl] + (base >> 3), bits, nsg, ovf);
+                        }
+                    }
+                    if (!((meth & 2) && insig)) {
+                        if (VPRED && (meth & 1)) {
+#pragma unroll
+                            for (int k = 0; k < 4; k++) vl += n4[k];
+                        } else {
+                            /* unary codes: d ones then a zero for each present
+                             * group (PackPrecinct.h:25-39), two groups per word */
+                            uint32_t n[4], c[4];
+#pragma unroll
+                            for (int k = 0; k < 4; k++) {
+                                const uint32_t dk = (d4 >> (8 * k)) & 255u;
+                                n[k] = k < (int)nv ? dk + 1 : 0u;
+                                c[k] = ((1u << dk) - 1u) << 1;
+                            }
+                            const uint32_t l23 = n[2] + n[3];
+                            vacc = ((uint64_t)((c[0] << n[1]) | c[1]) << l23) | ((c[2] << n[3]) | c[3]);
+                            vl = dsum + nv;
+                        }
+                    }
+                }
+                /* data bits of the groups above gtli: 4 (d + 1) each (the sign
+                 * nibble, unless signs go to their own sub-packet) */
+                const uint32_t dl4 = dsum + (fs ? 0u : nsig);
+                /* one scan for three running sums: data bits / 4 (12 bits), code
+                 * bits (13 bits), listed groups (the exclusive sums, at most 124,
+                 * in the top 7 bits) */
+                uint32_t tot;
+                const uint32_t ex = warp_excl_scan(dl4 | (vl << 12) | (nsig << 25), &tot);
+                const uint32_t ex_d = (ex & 0xfffu) << 2, ex_v = (ex >> 12) & 0x1fffu;
+                const uint32_t tot_d = (tot & 0xfffu) << 2, tot_v = (tot >> 12) & 0x1fffu;
+                if (vl) {
+                    if (VPRED && (meth & 1)) {
+                        /* prediction codes (up to 31 bits each): n - 1 ones then
+                         * a zero, joined while they fit 64 bits */
+                        uint32_t pos = vpos + ex_v, an = 0;
+                        uint64_t acc = 0;
+#pragma unroll
+                        for (int k = 0; k < 4; k++) {
+                            const uint32_t n = n4[k];
+                            if (n) {
+                                if (an + n > 64) {
+                                    put_bits(buf, words, pos, acc, an, ovf);
+                                    pos += an;
+                                    acc = 0;
+                                    an = 0;
+                                }
+                                acc = (acc << n) | (((1ull << (n - 1)) - 1) << 1);
+                                an += n;
+                            }
+                        }
+                        if (an) put_bits(buf, words, pos, acc, an, ovf);
+                    } else {
+                        put_bits(buf, words, vpos + ex_v, vacc, vl, ovf);
+                    }
+                }
+                uint32_t sbits = 0, sn = 0;
+                if (!fs) {
+                    /* signs with the data: the warp lists its groups with GCLI
+                     * > gtli (bit offset in the warp's data, group, GCLI), then
+                     * each lane packs one listed group at a time, its sign
+                     * nibble and planes in one write of at most 64 bits; the
+                     * coefficients of the other groups are never read */
+                    uint32_t* list = &s_segw[0][0] + 128 * warp;
+                    const uint32_t cnt = __reduce_add_sync(FULL, nsig);
+                    {
+                        /* per byte: 1 for a listed group, and its data nibbles
+                         * v - t + 1; their exclusive prefix sums over the
+                         * lane's bytes give each entry's slot and offset */
+                        const uint32_t one = s4 & 0x01010101u, dd = d4 + one;
+                        const uint32_t po = dd * 0x01010100u, pi = one * 0x01010100u;
+                        const uint32_t e0 = (ex_d << 11) | ((uint32_t)lane << 6), i0 = ex >> 25;
+#pragma unroll
+                        for (int k = 0; k < 4; k++)
+                            if ((one >> (8 * k)) & 1u)
+                                list[i0 + ((pi >> (8 * k)) & 255u)] = e0 + (((po >> (8 * k)) & 255u) << 13) + ((uint32_t)k << 4) + v[k];
+                    }
+                    __syncwarp();
+                    for (uint32_t r = lane; r < cnt; r += 32) {
+                        const uint32_t e = list[r];
+                        const uint32_t gi = base + ((e >> 4) & 127u), vv = e & 15u, np = vv - t;
+                        /* the coefficients past the band width are stored as zero */
+                        const uint2 raw4 = *(const uint2*)(crow + 4 * gi);
+                        put_bits(buf, words, dpos + (e >> 11), data_chunk_signed(raw4, vv, t, uniform), 4 * (np + 1), ovf);
+                    }
+                    __syncwarp();
+                } else if (dl4) {
+                    /* data bits of the groups with gcli > gtli (pack_data_c,
+                     * PackPrecinct.c:128-198), joined while they fit 64 bits */
+                    uint32_t pos = dpos + ex_d;
+                    uint64_t acc = 0;
+                    uint32_t an = 0;
+                    const uint2 cw[4] = {make_uint2(c0.x, c0.y), make_uint2(c0.z, c0.w), make_uint2(c1.x, c1.y), make_uint2(c1.z, c1.w)};
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        if (k < (int)nv && v[k] > t) {
+                            const uint32_t np = v[k] - t, n = 4 * (np + 1 - fs);
+                            uint32_t sgn, nzm;
+                            uint64_t ch = data_chunk(cw[k], (int)B.w - 4 * (int)(g + k), v[k], t, uniform, sgn, nzm);
+                            if (fs) {
+                                /* the signs of the non-zero magnitudes, coefficient 0 first */
+#pragma unroll
+                                for (int j = 3; j >= 0; j--) {
+                                    if ((nzm >> j) & 1u) {
+                                        sbits = (sbits << 1) | ((sgn >> j) & 1u);
+                                        sn++;
+                                    }
+                                }
+                            } else {
+                                ch |= (uint64_t)sgn << (4 * np);
+                            }
                             if (an + n > 64) {
                                 put_bits(buf, words, pos, acc, an, ovf);
                                 pos += an;
                                 acc = 0;
                                 an = 0;
                             }
-                            acc = (acc << n) | (((1ull << (n - 1)) - 1) << 1);
+                            acc = n == 64 ? ch : (acc << n) | ch;
                             an += n;
                         }
                     }
                     if (an) put_bits(buf, words, pos, acc, an, ovf);
-                } else {
-                    put_bits(buf, words, vpos + ex_v, vacc, vl, ovf);
                 }
-            }
-            uint32_t sbits = 0, sn = 0;
-            if (!fs) {
-                /* signs with the data: the warp lists its groups with GCLI
-                 * > gtli (bit offset in the warp's data, group, GCLI), then
-                 * each lane packs one listed group at a time, its sign
-                 * nibble and planes in one write of at most 64 bits; the
-                 * coefficients of the other groups are never read */
-                uint32_t* list = &s_segw[0][0] + 128 * warp;
-                const uint32_t cnt = __reduce_add_sync(FULL, nsig);
-                {
-                    /* per byte: 1 for a listed group, and its data nibbles
-                     * v - t + 1; their exclusive prefix sums over the
-                     * lane's bytes give each entry's slot and offset */
-                    const uint32_t one = s4 & 0x01010101u, dd = d4 + one;
-                    const uint32_t po = dd * 0x01010100u, pi = one * 0x01010100u;
-                    const uint32_t e0 = (ex_d << 11) | ((uint32_t)lane << 6), i0 = ex >> 25;
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        if ((one >> (8 * k)) & 1u)
-                            list[i0 + ((pi >> (8 * k)) & 255u)] = e0 + (((po >> (8 * k)) & 255u) << 13) + ((uint32_t)k << 4) + v[k];
+                vpos += tot_v;
+                dpos += tot_d;
+                if (fs) {
+                    /* sign sub-packet (pack_sign_c, PackPrecinct.c:200-233) */
+                    uint32_t stot;
+                    const uint32_t sx = warp_excl_scan(sn, &stot);
+                    if (sn) put_bits(buf, words, npos + sx, sbits, sn, ovf);
+                    npos += stot;
                 }
-                __syncwarp();
-                for (uint32_t r = lane; r < cnt; r += 32) {
-                    const uint32_t e = list[r];
-                    const uint32_t gi = base + ((e >> 4) & 127u), vv = e & 15u, np = vv - t;
-                    /* the coefficients past the band width are stored as zero */
-                    const uint2 raw4 = *(const uint2*)(crow + 4 * gi);
-                    put_bits(buf, words, dpos + (e >> 11), data_chunk_signed(raw4, vv, t, uniform), 4 * (np + 1), ovf);
-                }
-                __syncwarp();
-            } else if (dl4) {
-                /* data bits of the groups with gcli > gtli (pack_data_c,
-                 * PackPrecinct.c:128-198), joined while they fit 64 bits */
-                uint32_t pos = dpos + ex_d;
-                uint64_t acc = 0;
-                uint32_t an = 0;
-                const uint2 cw[4] = {make_uint2(c0.x, c0.y), make_uint2(c0.z, c0.w), make_uint2(c1.x, c1.y), make_uint2(c1.z, c1.w)};
-#pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    if (k < (int)nv && v[k] > t) {
-                        const uint32_t np = v[k] - t, n = 4 * (np + 1 - fs);
-                        uint32_t sgn, nzm;
-                        uint64_t ch = data_chunk(cw[k], (int)B.w - 4 * (int)(g + k), v[k], t, uniform, sgn, nzm);
-                        if (fs) {
-                            /* the signs of the non-zero magnitudes, coefficient 0 first */
-#pragma unroll
-                            for (int j = 3; j >= 0; j--) {
-                                if ((nzm >> j) & 1u) {
-                                    sbits = (sbits << 1) | ((sgn >> j) & 1u);
-                                    sn++;
-                                }
-                            }
-                        } else {
-                            ch |= (uint64_t)sgn << (4 * np);
-                        }
-                        if (an + n > 64) {
-                            put_bits(buf, words, pos, acc, an, ovf);
-                            pos += an;
-                            acc = 0;
-                            an = 0;
-                        }
-                        acc = n == 64 ? ch : (acc << n) | ch;
-                        an += n;
-                    }
-                }
-                if (an) put_bits(buf, words, pos, acc, an, ovf);
-            }
-            vpos += tot_v;
-            dpos += tot_d;
-            if (fs) {
-                /* sign sub-packet (pack_sign_c, PackPrecinct.c:200-233) */
-                uint32_t stot;
-                const uint32_t sx = warp_excl_scan(sn, &stot);
-                if (sn) put_bits(buf, words, npos + sx, sbits, sn, ovf);
-                npos += stot;
             }
         }
     }
@@ -1785,15 +1939,16 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
     }
     /* copy out: whole 16-byte chunks where the precinct covers them, single
      * bytes at its two ends; slice header, codestream header and EOC around */
-    const uint8_t* bytes = (const uint8_t*)buf;
     uint8_t* gbase = out + R.offset - lead;
     const uint32_t nbytes = lead + total;
     for (uint32_t c = threadIdx.x; c < (nbytes + 15) >> 4; c += blockDim.x) {
         const uint32_t b0 = c << 4;
         if (b0 >= lead && b0 + 16 <= nbytes) {
-            *(uint4*)(gbase + b0) = *(const uint4*)(bytes + b0);
+            const uint4 v = *(const uint4*)(buf + 4 * c);
+            *(uint4*)(gbase + b0) = make_uint4(__byte_perm(v.x, 0u, 0x0123), __byte_perm(v.y, 0u, 0x0123),
+                                               __byte_perm(v.z, 0u, 0x0123), __byte_perm(v.w, 0u, 0x0123));
         } else {
-            for (uint32_t i = max(b0, lead); i < min(b0 + 16, nbytes); i++) gbase[i] = bytes[i];
+            for (uint32_t i = max(b0, lead); i < min(b0 + 16, nbytes); i++) gbase[i] = byte_at(buf, i);
         }
     }
     if (threadIdx.x == 0) {
@@ -1830,18 +1985,18 @@ __global__ void __launch_bounds__(RC_THREADS, (SIGNS || VPRED) ? 3 : 4) rc_cost_
     rc_cost_body<SIGNS, VPRED>(F.cfg, F.gcli, F.coef, F.cost, F.slice_done, F.rc, F.status, (int)blockIdx.x - F.first_block);
 }
 
-template <bool VPRED>
+template <bool SIGNS, bool VPRED>
 __global__ void __launch_bounds__(PK_THREADS, 4) pack_kernel(const jxs_cfg_t* __restrict__ cfg, const uint16_t* __restrict__ coef,
                                                           const uint8_t* __restrict__ gcli, const PrecRC* __restrict__ rc,
                                                           const uint32_t* __restrict__ cost, uint8_t* __restrict__ out,
                                                           uint32_t cap_words, int* status) {
-    pack_body<VPRED>(cfg, coef, gcli, rc, cost, out, cap_words, status, (int)blockIdx.x);
+    pack_body<SIGNS, VPRED>(cfg, coef, gcli, rc, cost, out, cap_words, status, (int)blockIdx.x);
 }
 
-template <bool VPRED>
+template <bool SIGNS, bool VPRED>
 __global__ void __launch_bounds__(PK_THREADS, 4) pack_batch_kernel(const __grid_constant__ EncPrecLaunch L, uint32_t cap_words) {
     const EncPrecFrame& F = L.job[find_job<JXS_BATCH_FRAMES>(L.job, L.nframes, (int)blockIdx.x)];
-    pack_body<VPRED>(F.cfg, F.coef, F.gcli, F.rc, F.cost, F.out, cap_words, F.status, (int)blockIdx.x - F.first_block);
+    pack_body<SIGNS, VPRED>(F.cfg, F.coef, F.gcli, F.rc, F.cost, F.out, cap_words, F.status, (int)blockIdx.x - F.first_block);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -1885,23 +2040,24 @@ extern "C" cudaError_t jxs_launch_rc(const jxs_cfg_t* dcfg, uint32_t np, uint32_
     }
 }
 
-template <bool V>
+template <bool S, bool V>
 static cudaError_t pack_one(const jxs_cfg_t* dcfg, uint32_t np, const uint16_t* coef, const uint8_t* gcli, const PrecRC* rc,
                             const uint32_t* cost, uint8_t* out, uint32_t cap_words, int* status, cudaStream_t st) {
     const size_t smem = (size_t)cap_words * 4;
     static std::atomic<int> attr[JXS_MAX_DEV];
-    cudaError_t e = jxs_smem_attr(pack_kernel<V>, (int)smem, attr);
+    cudaError_t e = jxs_smem_attr(pack_kernel<S, V>, (int)smem, attr);
     if (e != cudaSuccess) return e;
-    pack_kernel<V><<<np, PK_THREADS, smem, st>>>(dcfg, coef, gcli, rc, cost, out, cap_words, status);
+    pack_kernel<S, V><<<np, PK_THREADS, smem, st>>>(dcfg, coef, gcli, rc, cost, out, cap_words, status);
     return cudaGetLastError();
 }
 
-/* `modes` bit 1: a frame of the launch has vertical prediction */
+/* `modes` as for the rate control */
 extern "C" cudaError_t jxs_launch_pack(const jxs_cfg_t* dcfg, uint32_t np, const uint16_t* coef, const uint8_t* gcli,
                                        const PrecRC* rc, const uint32_t* cost, uint8_t* out, uint32_t cap_words, int* status,
                                        int modes, cudaStream_t st) {
-    if (modes & 2) return pack_one<true>(dcfg, np, coef, gcli, rc, cost, out, cap_words, status, st);
-    return pack_one<false>(dcfg, np, coef, gcli, rc, cost, out, cap_words, status, st);
+    if (modes & 2) return pack_one<true, true>(dcfg, np, coef, gcli, rc, cost, out, cap_words, status, st);
+    if (modes & 1) return pack_one<true, false>(dcfg, np, coef, gcli, rc, cost, out, cap_words, status, st);
+    return pack_one<false, false>(dcfg, np, coef, gcli, rc, cost, out, cap_words, status, st);
 }
 
 extern "C" cudaError_t jxs_launch_rc_batch(const EncPrecLaunch* L, int modes, cudaStream_t st) {
@@ -1914,18 +2070,19 @@ extern "C" cudaError_t jxs_launch_rc_batch(const EncPrecLaunch* L, int modes, cu
     }
 }
 
-template <bool V>
+template <bool S, bool V>
 static cudaError_t pack_batch_one(const EncPrecLaunch* L, uint32_t cap_words, cudaStream_t st) {
     const size_t smem = (size_t)cap_words * 4;
     static std::atomic<int> attr[JXS_MAX_DEV];
-    cudaError_t e = jxs_smem_attr(pack_batch_kernel<V>, (int)smem, attr);
+    cudaError_t e = jxs_smem_attr(pack_batch_kernel<S, V>, (int)smem, attr);
     if (e != cudaSuccess) return e;
     if (L->nblocks <= 0) return cudaSuccess;
-    pack_batch_kernel<V><<<L->nblocks, PK_THREADS, smem, st>>>(*L, cap_words);
+    pack_batch_kernel<S, V><<<L->nblocks, PK_THREADS, smem, st>>>(*L, cap_words);
     return cudaGetLastError();
 }
 
 extern "C" cudaError_t jxs_launch_pack_batch(const EncPrecLaunch* L, uint32_t cap_words, int modes, cudaStream_t st) {
-    if (modes & 2) return pack_batch_one<true>(L, cap_words, st);
-    return pack_batch_one<false>(L, cap_words, st);
+    if (modes & 2) return pack_batch_one<true, true>(L, cap_words, st);
+    if (modes & 1) return pack_batch_one<true, false>(L, cap_words, st);
+    return pack_batch_one<false, false>(L, cap_words, st);
 }

@@ -472,7 +472,8 @@ static int32_t enc_run(jxs_gpu_enc_t* e, EncSlot* s, void* const planes[4], cons
     TMARK(3);
     const int out_dev = jxs_gpu_is_device_ptr(out);
     uint8_t* dst = out_dev ? out : s->out_stage;
-    CK(jxs_launch_pack(e->dcfg, c->np, s->coef, s->gcli, s->rc, s->cost, dst, e->cap_words, s->status, c->vpred ? 2 : 0, st));
+    CK(jxs_launch_pack(e->dcfg, c->np, s->coef, s->gcli, s->rc, s->cost, dst, e->cap_words, s->status,
+                       (c->fs ? 1 : 0) | (c->vpred ? 2 : 0), st));
     KMARK();
     publish_status_kernel<<<1, 32, 0, st>>>(s->status_hd, s->status);
     CK(cudaGetLastError());
