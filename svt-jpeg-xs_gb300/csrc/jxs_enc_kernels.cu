@@ -1110,20 +1110,18 @@ DEV uint64_t data_chunk(uint2 raw4, int wleft, uint32_t v, uint32_t t, uint32_t 
     return planes;
 }
 
-/* The same with the sign nibble leading the planes (signs with the data),
- * for a group whose coefficients past the band width are stored as zero:
- * the sign of every coefficient that stays non-zero enters as plane
- * v - t of its magnitude, and one transpose gives sign and planes. */
-DEV uint64_t data_chunk_signed(uint2 raw4, uint32_t v, uint32_t t, uint32_t uniform) {
+/* A group's quantized magnitudes as 16-bit pairs (coefficients 0 | 1 << 16
+ * and 2 | 3 << 16) with the sign of every coefficient that stays non-zero as
+ * plane v - t, above the magnitude: one transpose then gives the sign nibble
+ * and the planes.  For signs with the data and a group whose coefficients
+ * past the band width are stored as zero; uq: uniform quantization, t > 0
+ * (t = 0 is not quantized, and a deadzone shift by 0 is the same). */
+DEV void quantize_signed(uint2 raw4, uint32_t v, uint32_t t, bool uq, uint32_t& P01, uint32_t& P23) {
     const uint32_t c01 = raw4.x, c23 = raw4.y, np = v - t;
-    uint32_t P01, P23;
-    if (t == 0) {
-        P01 = c01 & 0x7fff7fffu;
-        P23 = c23 & 0x7fff7fffu;
-    } else if (!uniform) {
+    if (!uq) {
         const uint32_t keep = (0x7fffu >> t) * 0x00010001u;
-        P01 = ((c01 & 0x7fff7fffu) >> t) & keep;
-        P23 = ((c23 & 0x7fff7fffu) >> t) & keep;
+        P01 = (c01 >> t) & keep;
+        P23 = (c23 >> t) & keep;
     } else {
         uint32_t q[4];
         const uint32_t c[4] = {c01 & 0xffffu, c01 >> 16, c23 & 0xffffu, c23 >> 16};
@@ -1136,13 +1134,10 @@ DEV uint64_t data_chunk_signed(uint2 raw4, uint32_t v, uint32_t t, uint32_t unif
         P01 = q[0] | (q[1] << 16);
         P23 = q[2] | (q[3] << 16);
     }
-    /* sign bits (bits 15 and 31) of the non-zero magnitudes moved to bit np
-     * of each half (np <= 15) */
-    P01 |= (__vcmpne2(P01, 0u) & c01 & 0x80008000u) >> (15 - np);
-    P23 |= (__vcmpne2(P23, 0u) & c23 & 0x80008000u) >> (15 - np);
-    uint64_t planes = coefs_to_planes(__byte_perm(P01, P23, 0x0246));
-    if (np >= 8) planes |= (uint64_t)coefs_to_planes(__byte_perm(P01, P23, 0x1357)) << 32;
-    return planes;
+    /* magnitudes stay below 2^15: adding 0x7fff sets bit 15 of the non-zero
+     * ones; the sign moves to bit np (<= 15) */
+    P01 |= ((P01 + 0x7fff7fffu) & c01 & 0x80008000u) >> (15 - np);
+    P23 |= ((P23 + 0x7fff7fffu) & c23 & 0x80008000u) >> (15 - np);
 }
 
 /* A segment as pass B reads it: bit positions of its first GCLI code and
@@ -1611,6 +1606,7 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
         for (uint32_t qi = queue_next(&s_q[1], lane); qi < nseg; qi = queue_next(&s_q[1], lane)) {
             const uint32_t sidx = s_ord[qi];
             const PkSeg D = s_desc[sidx];
+            const bool uq = uniform && (D.info & 15u);
             const uint32_t line = D.info >> 8, t = D.info & 15u, n = D.g0n >> 16;
             const uint8_t* grow = gcli + s_grow[line] + (D.g0n & 0xffffu);
             const uint16_t* crow = coef + s_crow[line] + 4 * (D.g0n & 0xffffu);
@@ -1709,9 +1705,12 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
                     const uint32_t gi = base + ((e >> 4) & 127u), np = (e & 15u) - t, pos = dpos + 4 * (e >> 16);
                     /* the coefficients past the band width are stored as zero */
                     const uint2 raw4 = *(const uint2*)(crow + 4 * gi);
-                    const uint64_t ch = data_chunk_signed(raw4, e & 15u, t, uniform);
-                    if (np < 8) put_left32(buf, pos, (uint32_t)ch << (28 - 4 * np));
-                    else put_bits(buf, words, pos, ch, 4 * (np + 1), ovf);
+                    uint32_t P01, P23;
+                    quantize_signed(raw4, e & 15u, t, uq, P01, P23);
+                    const uint32_t low = coefs_to_planes(__byte_perm(P01, P23, 0x0246));
+                    if (np < 8) put_left32(buf, pos, low << (28 - 4 * np));
+                    else
+                        put_bits(buf, words, pos, (uint64_t)coefs_to_planes(__byte_perm(P01, P23, 0x1357)) << 32 | low, 4 * (np + 1), ovf);
                 }
                 __syncwarp();
                 vpos += tot_v;
@@ -1878,7 +1877,11 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
                         const uint32_t gi = base + ((e >> 4) & 127u), vv = e & 15u, np = vv - t;
                         /* the coefficients past the band width are stored as zero */
                         const uint2 raw4 = *(const uint2*)(crow + 4 * gi);
-                        put_bits(buf, words, dpos + (e >> 11), data_chunk_signed(raw4, vv, t, uniform), 4 * (np + 1), ovf);
+                        uint32_t P01, P23;
+                        quantize_signed(raw4, vv, t, uniform && t, P01, P23);
+                        uint64_t planes = coefs_to_planes(__byte_perm(P01, P23, 0x0246));
+                        if (np >= 8) planes |= (uint64_t)coefs_to_planes(__byte_perm(P01, P23, 0x1357)) << 32;
+                        put_bits(buf, words, dpos + (e >> 11), planes, 4 * (np + 1), ovf);
                     }
                     __syncwarp();
                 } else if (dl4) {
