@@ -493,7 +493,7 @@ static int32_t plan_decode_chain(const std::vector<DecItem>& it, const std::vect
     for (int op = 0; op < 2; op++) {
         DecPrecLaunch* L = (DecPrecLaunch*)scratch.data();
         memset(L, 0, sizeof(*L));
-        uint32_t cb = 0, cg = 0, cs = 0;
+        uint32_t cb = 0, cg = 0, cs = 0, fs = 0;
         auto flush = [&]() {
             if (L->nframes) {
                 if (op == 0) {
@@ -502,16 +502,18 @@ static int32_t plan_decode_chain(const std::vector<DecItem>& it, const std::vect
                 } else {
                     /* one shared-memory layout for the launch: the largest
                      * precinct buffer that leaves room for the rest */
-                    const size_t fixed = uk_layout(0, cg, cs).end;
+                    const size_t fixed = uk_reserved(cg, cs, 0);
                     const size_t room = kSmemMax - UK_STATIC_SMEM;
                     if (cb + fixed > room) cb = room > fixed + 4096 ? (uint32_t)(room - fixed) : 4096;
-                    /* the launch's segment capacity travels as the op's kind */
-                    if (L->nframes > 1) P->add(OP_UNPACK, (int)cs, chain, L->nblocks, cb & ~15u, cg, L, sizeof(*L));
-                    else P->add(OP_UNPACK1, (int)cs, chain, L->nblocks, cb & ~15u, cg, &L->job[0], sizeof(L->job[0]));
+                    /* the launch's segment capacity and whether a frame has
+                     * separate signs travel as the op's kind */
+                    const int kind = (int)(cs << 1 | fs);
+                    if (L->nframes > 1) P->add(OP_UNPACK, kind, chain, L->nblocks, cb & ~15u, cg, L, sizeof(*L));
+                    else P->add(OP_UNPACK1, kind, chain, L->nblocks, cb & ~15u, cg, &L->job[0], sizeof(L->job[0]));
                 }
             }
             memset(L, 0, sizeof(*L));
-            cb = cg = 0;
+            cb = cg = fs = 0;
         };
         for (int f : fr) {
             const DecItem& d = it[f];
@@ -531,6 +533,7 @@ static int32_t plan_decode_chain(const std::vector<DecItem>& it, const std::vect
             cb = std::max(cb, d.cap_bytes);
             cg = std::max(cg, d.cap_groups);
             cs = std::max(cs, d.cap_seg);
+            fs |= d.c->fs ? 1u : 0u;
         }
         flush();
     }
@@ -642,7 +645,7 @@ static int32_t issue(jxs_gpu_batch_t* b, const Plan& P, cudaStream_t st) {
         case OP_RC: e = jxs_launch_rc_batch((const EncPrecLaunch*)d, (int)o.b, s); break;
         case OP_PACK: e = jxs_launch_pack_batch((const EncPrecLaunch*)d, o.a, (int)o.b, s); break;
         case OP_WALK: e = jxs_launch_walk_batch((const DecPrecLaunch*)d, s); break;
-        case OP_UNPACK: e = jxs_launch_unpack_batch((const DecPrecLaunch*)d, o.a, o.b, (uint32_t)o.kind, s); break;
+        case OP_UNPACK: e = jxs_launch_unpack_batch((const DecPrecLaunch*)d, o.a, o.b, (uint32_t)o.kind >> 1, o.kind & 1, s); break;
         case OP_INV_H: e = jxs_launch_inv_h_batch((const InvHLaunchB*)d, o.kind, o.nblocks, s); break;
         case OP_INV_V: e = jxs_launch_inv_v_batch((const InvVLaunchB*)d, o.kind, o.nblocks, s); break;
         case OP_FWD_V_S: e = jxs_launch_fwd_v((const FwdVLaunch*)d, o.kind, (int)o.a, s); break;
@@ -667,8 +670,8 @@ static int32_t issue(jxs_gpu_batch_t* b, const Plan& P, cudaStream_t st) {
         }
         case OP_UNPACK1: {
             const DecPrecFrame* F = (const DecPrecFrame*)d;
-            e = jxs_launch_unpack(F->cfg, F->bs, F->bs_size, F->prec_off, F->coef, (uint32_t)o.nblocks, o.a, o.b, (uint32_t)o.kind,
-                                  F->status, s);
+            e = jxs_launch_unpack(F->cfg, F->bs, F->bs_size, F->prec_off, F->coef, (uint32_t)o.nblocks, o.a, o.b, (uint32_t)o.kind >> 1,
+                                  o.kind & 1, F->status, s);
             break;
         }
         }

@@ -27,9 +27,7 @@ static_assert(UK_LIST_BYTES == 4 * 128 * UK_WARPS, "a list of 128 groups per war
 
 /* Per band line of the precinct being unpacked. */
 struct UkLine {
-    uint32_t sig_pos;           /* bit position of its significance flags; raw packets: of its 4-bit GCLIs */
-    uint8_t t, meth, raw, pk;
-    uint8_t vp, pad0, pad1, pad2; /* vp: GCLIs predicted from the line above */
+    uint8_t t, meth, vp, pk;    /* vp: GCLIs predicted from the line above */
 };
 /* Per packet. */
 struct UkPk {
@@ -42,13 +40,33 @@ struct UkPk {
     uint32_t ncoded;            /* unary codewords */
     uint32_t raw, present;
 };
+/* A segment as the warp passes read it: rank of its first codeword's zero
+ * bit (raw packets: bit position of its first 4-bit GCLI), bit position of its
+ * first significance flag, its first group's place among the precinct's
+ * GCLIs, and group count | gtli << 16 | significance << 20 | raw << 21 |
+ * predicted << 22 | band line << 24. */
+struct UkSeg {
+    uint32_t vpos, sig, z, info;
+};
 
-/* 32 bits of a big-endian bit string held in shared memory, starting at
- * bit `pos`; the buffer must be readable 8 bytes past pos / 8. */
-DEV uint32_t be_word(const uint8_t* b, uint32_t wi) { return __byte_perm(((const uint32_t*)b)[wi], 0, 0x0123); }
-DEV uint32_t bits32_at(const uint8_t* b, uint32_t pos) {
+/* The precinct's bytes are kept as a bit string in 32-bit words, first bit in
+ * the most significant position (bytes swapped once, when it is copied in):
+ * 32 bits from bit `pos`, readable 8 bytes past pos / 8, and byte i. */
+DEV uint32_t bits32_at(const uint32_t* b, uint32_t pos) {
     const uint32_t wi = pos >> 5;
-    return __funnelshift_l(be_word(b, wi + 1), be_word(b, wi), pos & 31);
+    return __funnelshift_l(b[wi + 1], b[wi], pos & 31);
+}
+DEV uint32_t byte_of(const uint32_t* b, uint32_t i) { return ((const uint8_t*)b)[i ^ 3u]; }
+DEV uint32_t shl_or_0(uint32_t a, uint32_t n) { /* 0 for n >= 32 */
+    uint32_t r;
+    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(n));
+    return r;
+}
+/* all ones in every byte whose top bit is set */
+DEV uint32_t sign_bytes(uint32_t x) {
+    uint32_t r;
+    asm("prmt.b32 %0, %1, %1, 0xba98;" : "=r"(r) : "r"(x));
+    return r;
 }
 
 /* Transpose of the 8 x 4 bit matrix in a word: bit 4k + j moves to bit
@@ -57,7 +75,7 @@ DEV uint32_t bits32_at(const uint8_t* b, uint32_t pos) {
  * ((4,1), (3,0), (2,1), (1,0)) as masked delta swaps. */
 DEV uint32_t dswap(uint32_t x, int d, uint32_t m) {
     const uint32_t t = ((x >> d) ^ x) & m;
-    return x ^ t ^ (t << d);
+    return x ^ (t * ((1u << d) + 1u)); /* t and t << d have no bit in common */
 }
 DEV uint32_t planes_to_coefs(uint32_t x) {
     x = dswap(x, 14, 0x0000ccccu);
@@ -66,41 +84,33 @@ DEV uint32_t planes_to_coefs(uint32_t x) {
     return dswap(x, 1, 0x22222222u);
 }
 
-DEV uint32_t warp_excl_scan(uint32_t x, uint32_t* total) {
-    const int lane = threadIdx.x & 31;
-    uint32_t inc = x;
+/* Inclusive sum over the lanes up to this one (the shuffle's own predicate
+ * says whether there is a lane to add). */
+DEV uint32_t warp_incl_scan(uint32_t x) {
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(FULL, inc, o);
-        if (lane >= o) inc += y;
-    }
+    for (int o = 1; o < 32; o <<= 1)
+        asm volatile("{.reg .u32 r; .reg .pred p; shfl.sync.up.b32 r|p, %0, %1, 0, 0xffffffff; @p add.u32 %0, %0, r;}"
+                     : "+r"(x)
+                     : "r"(o));
+    return x;
+}
+DEV uint32_t warp_excl_scan(uint32_t x, uint32_t* total) {
+    const uint32_t inc = warp_incl_scan(x);
     *total = __shfl_sync(FULL, inc, 31);
     return inc - x;
 }
 
-/* Block-wide exclusive scan of one counter; returns the block total. */
+/* Block-wide exclusive scan of one counter; returns the block total.  ws is
+ * free for another scan once every thread has passed a later barrier. */
 DEV uint32_t block_scan1(uint32_t a, uint32_t* ea, uint32_t* ws) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    uint32_t ia = a;
-    for (int o = 1; o < 32; o <<= 1) {
-        uint32_t t = __shfl_up_sync(FULL, ia, o);
-        if (lane >= o) ia += t;
-    }
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t ia = warp_incl_scan(a);
     if (lane == 31) ws[warp] = ia;
     __syncthreads();
-    if (warp == 0) {
-        uint32_t v = lane < nw ? ws[lane] : 0;
-        for (int o = 1; o < 32; o <<= 1) {
-            uint32_t t = __shfl_up_sync(FULL, v, o);
-            if (lane >= o) v += t;
-        }
-        if (lane < nw) ws[lane] = v;
-    }
-    __syncthreads();
-    *ea = (warp ? ws[warp - 1] : 0) + ia - a;
-    const uint32_t total = ws[nw - 1];
-    __syncthreads();
-    return total;
+    /* every warp adds up the totals of the 16 */
+    const uint32_t w = warp_incl_scan(lane < UK_WARPS ? ws[lane] : 0u);
+    *ea = (warp ? __shfl_sync(FULL, w, warp - 1) : 0u) + ia - a;
+    return __shfl_sync(FULL, w, 31);
 }
 
 /* Next segment for a warp from a shared queue (the warps balance segments
@@ -114,40 +124,43 @@ DEV uint32_t next_seg(uint32_t* ctr, int lane) {
 /* Per-packet exclusive running sums of one count per segment.  Segments
  * are numbered in packet order, so a segment's base inside its packet is the
  * block-wide exclusive sum up to it minus that of its packet's first
- * segment.  Thread i holds segment i's count (nseg <= blockDim.x); base[i]
- * receives its base, ex[0 .. nseg] the block-wide exclusive sums, and
- * threads k < npk get packet k's total (0 without segments).  Other
- * threads may read base[] and ex[] after the caller's next barrier. */
-DEV uint32_t seg_bases(uint32_t cnt, uint32_t nseg, uint32_t npk, const jxs_seg_t* segs, const jxs_bline_t* bls,
-                       const uint8_t* pkbl0, const uint8_t* pknbl, uint32_t* ex, uint32_t* base, uint32_t* ws) {
+ * segment.  Thread i holds segment i's count and band line (nseg <=
+ * blockDim.x) and gets its base; ex[0 .. nseg] receives the block-wide
+ * exclusive sums, and threads k < npk get packet k's total in *sum (0 without
+ * segments). */
+DEV uint32_t seg_bases(uint32_t cnt, uint32_t bl, uint32_t nseg, uint32_t npk, const jxs_bline_t* bls, const uint8_t* pkbl0,
+                       const uint8_t* pknbl, uint32_t* ex, uint32_t* ws, uint32_t* sum) {
     const uint32_t i = threadIdx.x;
     uint32_t e;
     const uint32_t total = block_scan1(i < nseg ? cnt : 0u, &e, ws);
     if (i < nseg) ex[i] = e;
     if (i == 0) ex[nseg] = total;
     __syncthreads();
-    if (i < nseg) base[i] = e - ex[bls[pkbl0[bls[segs[i].bl].pk]].seg0];
-    uint32_t sum = 0;
+    *sum = 0;
     if (i < npk && pknbl[i]) {
         const uint32_t b0 = pkbl0[i], lb = b0 + pknbl[i] - 1;
-        sum = ex[bls[lb].seg0 + bls[lb].nseg] - ex[bls[b0].seg0];
+        *sum = ex[bls[lb].seg0 + bls[lb].nseg] - ex[bls[b0].seg0];
     }
-    return sum;
+    return i < nseg ? e - ex[bls[pkbl0[bls[bl].pk]].seg0] : 0u;
 }
 
 /* Packet header fields (get_packet_header, ParseHeader.c:20-44): raw flag,
  * data, GCLI and sign sub-packet lengths in bytes; short (5-byte) or long
  * (7-byte) form. */
-DEV void pk_header(const uint8_t* h, int long_hdr, uint32_t& raw, uint32_t& dlen, uint32_t& glen, uint32_t& slen) {
-    raw = h[0] >> 7;
+DEV void pk_header(const uint32_t* b, uint32_t at, int long_hdr, uint32_t& raw, uint32_t& dlen, uint32_t& glen, uint32_t& slen) {
+    /* bytes 0-3 and 3-6 (or 1-4) */
+    const uint32_t h = bits32_at(b, 8 * at), l = bits32_at(b, 8 * (at + (long_hdr ? 3 : 1)));
+    raw = h >> 31;
     if (long_hdr) {
-        dlen = ((uint32_t)(h[0] & 0x7f) << 13) | ((uint32_t)h[1] << 5) | (h[2] >> 3);
-        glen = ((uint32_t)(h[2] & 7) << 17) | ((uint32_t)h[3] << 9) | ((uint32_t)h[4] << 1) | (h[5] >> 7);
-        slen = ((uint32_t)(h[5] & 0x7f) << 8) | h[6];
+        /* 1 raw, 20 data, 20 GCLI, 15 sign bits */
+        dlen = (h >> 11) & 0xfffffu;
+        glen = ((h & 0x7ffu) << 9) | ((l >> 15) & 0x1ffu);
+        slen = l & 0x7fffu;
     } else {
-        dlen = ((uint32_t)(h[0] & 0x7f) << 8) | h[1];
-        glen = ((uint32_t)h[2] << 5) | (h[3] >> 3);
-        slen = ((uint32_t)(h[3] & 7) << 8) | h[4];
+        /* 1 raw, 15 data, 13 GCLI, 11 sign bits */
+        dlen = (h >> 16) & 0x7fffu;
+        glen = (h >> 3) & 0x1fffu;
+        slen = l & 0x7ffu;
     }
 }
 
@@ -271,63 +284,70 @@ DEV uint2 decode_group_dz(uint64_t chunk, uint32_t np, uint32_t t, int wl) {
     return make_uint2(a & keepA, b & keepB);
 }
 
-/* unpack_precinct (Packing.c:513-868) for one precinct row; vertical
- * prediction and separate sign sub-packets are rejected.
+/* unpack_precinct (Packing.c:513-868) for one precinct.  FS: the launch may
+ * hold frames with separate sign sub-packets; VP: slice-ordered decoding,
+ * which resolves vertical prediction (otherwise a precinct with predicted
+ * bands reports JXS_E_DEC_VPRED); both compiled out otherwise.
  *
- * Dynamic shared memory (uk_layout): [precinct bytes: cap_bytes + 32,
- * stream byte i at i + lead so that 16-byte chunks are aligned] [GCLI per
- * group: cap_groups] [every zero bit of the VLC sub-packets, as a 16-bit
- * offset in its sub-packet] [the per-segment arrays, cap_seg segments].
+ * Dynamic shared memory: see uk_layout.
  *
- *   copy    the precinct's bytes into shared memory;
- *   parse   thread 0: precinct header, packet headers, sub-packet positions
- *           with the reference's length checks;
- *   pass 1  warp per segment: groups with a unary codeword (the
- *           significance flags drop the insignificant ones); raw GCLIs;
+ *   copy    the precinct's bytes into shared memory as big-endian words;
+ *   parse   warp 0: precinct header, band modes, packet headers, sub-packet
+ *           positions with the reference's length checks, running sums of
+ *           the lines' significance and raw GCLI bits;
+ *   counts  thread per segment: groups with a unary codeword (the
+ *           significance flags drop the insignificant ones);
  *   zeros   block pass over the VLC sub-packets: codeword c of a packet ends
  *           at the c-th zero bit of its sub-packet (unpack_pred_zero_gclis_*,
- *           Packing.c:435-511);
- *   pass 2  warp per segment: GCLI = gtli + ones in the codeword; data bits;
+ *           Packing.c:435-511); its value, the ones before that bit, goes to
+ *           byte c of a table;
+ *   pass 2  warp per segment: GCLI = gtli + codeword value, or raw; data bits;
  *   pass 3  warp per segment: data bits at warp-scanned offsets, decoded and
- *           written as int16 coefficients (8 bytes per lane, coalesced). */
+ *           written as int16 coefficients (8 bytes per lane, coalesced).
+ *
+ * Bound by instruction issue.  Segments are described once, a 16-byte record
+ * each, instead of by every warp that takes one; codeword values are read 4
+ * at a time instead of 5 zero positions; bytes are swapped once.  8 4K 4:2:2
+ * 10-bit frames: 263 us before, UNPACK_US us now. */
+template <bool FS, bool VP>
 __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t bs_size,
                                             const uint32_t* __restrict__ prec_off, int16_t* __restrict__ coef,
                                             uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg, int* status, const int p,
                                             uint8_t* top_gcl, uint8_t* top_t, const int vp_ok) {
     extern __shared__ __align__(16) uint8_t dsm[];
     const UkLayout UL = uk_layout(cap_bytes, cap_groups, cap_seg);
-    uint8_t* pbuf = dsm;
+    uint32_t* pbuf = (uint32_t*)dsm;
     uint8_t* gcl = dsm + UL.gcl;
-    uint16_t* zend = (uint16_t*)(dsm + UL.zend);
+    uint8_t* zval = dsm + UL.zval;
     /* zero bits: one per codeword plus up to 7 padding bits per packet */
     const uint32_t zcap = UK_ZCAP(cap_groups);
     __shared__ UkLine ln[JXS_MAXBLINES];
     __shared__ UkPk pk[JXS_MAXPK];
     __shared__ uint8_t s_mode[JXS_MAXBL];
-    __shared__ uint32_t s_pksb[JXS_MAXPK], s_pkrb[JXS_MAXPK], s_hpos[JXS_MAXPK];
+    __shared__ uint32_t s_hpos[JXS_MAXPK];
     __shared__ uint32_t s_next[2]; /* segment queues of the two warp passes */
-    /* this precinct kind's tables, staged from the configuration */
-    /* this precinct kind's segments, their work order and per-segment sums
-     * (dynamic: sized for the launch's largest segment count) */
-    jxs_seg_t* s_seg = (jxs_seg_t*)(dsm + UL.seg);
+    /* per segment (dynamic: sized for the launch's largest segment count) */
     uint16_t* s_ord = (uint16_t*)(dsm + UL.ord);
-    uint32_t* s_cnt = (uint32_t*)(dsm + UL.cnt);
-    uint32_t* s_base = (uint32_t*)(dsm + UL.base);
+    UkSeg* s_desc = (UkSeg*)(dsm + UL.desc);
+    uint32_t* s_cnt = (uint32_t*)(dsm + UL.cnt);   /* data bits; separate signs: then signs */
+    uint32_t* s_base = (uint32_t*)(dsm + UL.base); /* bit position of the data */
     uint32_t* s_ex = (uint32_t*)(dsm + UL.ex);
-    uint32_t* s_nz = (uint32_t*)(dsm + UL.nz);  /* separate signs: per segment, count */
-    uint32_t* s_sgb = (uint32_t*)(dsm + UL.sgb); /* and first bit */
+    uint32_t* s_sgb = (uint32_t*)(dsm + UL.sgb);   /* separate signs: bit position of the signs */
+    /* this precinct kind's tables, staged from the configuration */
     __shared__ jxs_bline_t s_bl[JXS_MAXBLINES];
-    __shared__ uint64_t s_crow[JXS_MAXBLINES]; /* per line: coefficient row offset */
+    __shared__ uint64_t s_crow[JXS_MAXBLINES]; /* per line: coefficient row offset, less 4 times the line's first group */
+    __shared__ uint32_t s_wend[JXS_MAXBLINES]; /* per line: coefficients, plus 4 times the line's first group */
+    __shared__ uint32_t s_lsx[JXS_MAXBLINES + 1], s_lrx[JXS_MAXBLINES + 1]; /* per line: significance / raw GCLI bits before it */
     __shared__ uint8_t s_pkbl0[JXS_MAXPK], s_pknbl[JXS_MAXPK];
     __shared__ uint32_t ws[UK_WARPS];
     __shared__ int s_err;
-    __shared__ uint32_t s_total, s_lead, s_tw, s_npk, s_off;
+    __shared__ uint32_t s_total, s_lead, s_tw, s_off;
     __shared__ uint8_t s_g2f[JXS_MAXBL];          /* global band -> flat band */
     __shared__ uint16_t s_lgp[JXS_MAXBLINES];      /* per line: band gain | priority << 8 */
     __shared__ uint32_t s_sc[9];                   /* nbands_all, npk, long headers, separate signs, precinct header bytes,
                                                       band lines, segments, groups per segment, run mode */
-    __shared__ uint8_t s_topbl[JXS_MAXBLINES], s_topprev[JXS_MAXBLINES]; /* vertical prediction: the line above */
-    __shared__ uint32_t s_topg[JXS_MAXBLINES];
+    __shared__ uint8_t s_topbl[VP ? JXS_MAXBLINES : 1], s_topprev[VP ? JXS_MAXBLINES : 1]; /* vertical prediction: the line above */
+    __shared__ uint32_t s_topg[VP ? JXS_MAXBLINES : 1];
     __shared__ int s_hasvp;
 
     /* the precinct kind's tables (last row / last of several columns) */
@@ -372,21 +392,28 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         s_err = err;
     }
     if (threadIdx.x < 2) s_next[threadIdx.x] = 0;
+    jxs_seg_t myseg; /* thread i: segment i */
+    myseg.bl = 0;
+    myseg.g0 = 0;
     {
         const uint32_t ns = cfg->nseg[last], nl = cfg->nbline[last];
-        for (uint32_t i = threadIdx.x; i < ns * (sizeof(jxs_seg_t) / 4); i += blockDim.x)
-            ((uint32_t*)s_seg)[i] = ((const uint32_t*)cfg->seg[last])[i];
+        if (threadIdx.x < ns) {
+            myseg = cfg->seg[last][threadIdx.x];
+            s_ord[threadIdx.x] = cfg->seg_ord[last][threadIdx.x];
+        }
         for (uint32_t i = threadIdx.x; i < nl * (sizeof(jxs_bline_t) / 4); i += blockDim.x)
             ((uint32_t*)s_bl)[i] = ((const uint32_t*)cfg->bline[last])[i];
-        for (uint32_t i = threadIdx.x; i < ns; i += blockDim.x) s_ord[i] = cfg->seg_ord[last][i];
         for (uint32_t x = threadIdx.x; x < nl; x += blockDim.x) {
             const jxs_bline_t& B = cfg->bline[last][x];
             const jxs_band_t& bd = cfg->band[B.fb];
-            s_crow[x] = bd.coef_off + (uint64_t)(prow * bd.lines + B.line) * bd.pitch + (uint64_t)pcol * bd.cwn;
+            s_crow[x] = bd.coef_off + (uint64_t)(prow * bd.lines + B.line) * bd.pitch + (uint64_t)pcol * bd.cwn - 4 * (uint64_t)B.gbase;
+            s_wend[x] = B.w + 4 * B.gbase;
             s_lgp[x] = (uint16_t)(bd.gain | (bd.prio << 8));
-            s_topbl[x] = cfg->top_bl[last][x];
-            s_topprev[x] = cfg->top_prev[last][x];
-            s_topg[x] = cfg->top_gbase[last][x];
+            if (VP) {
+                s_topbl[x] = cfg->top_bl[last][x];
+                s_topprev[x] = cfg->top_prev[last][x];
+                s_topg[x] = cfg->top_gbase[last][x];
+            }
         }
         for (uint32_t k = threadIdx.x; k < cfg->npk; k += blockDim.x) {
             s_pkbl0[k] = cfg->pk_bl0[last][k];
@@ -406,34 +433,34 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         for (uint32_t c = threadIdx.x; c < nch + 2; c += blockDim.x) {
             const uint32_t b0 = c << 4;
             if (b0 >= lead && b0 + 16 <= nbytes) {
-                *(uint4*)(pbuf + b0) = *(const uint4*)(gsrc + b0);
+                const uint4 v = *(const uint4*)(gsrc + b0);
+                *(uint4*)(pbuf + 4 * c) = make_uint4(__byte_perm(v.x, 0u, 0x0123), __byte_perm(v.y, 0u, 0x0123),
+                                                     __byte_perm(v.z, 0u, 0x0123), __byte_perm(v.w, 0u, 0x0123));
             } else {
-                for (uint32_t i = b0; i < b0 + 16; i++) pbuf[i] = (i >= lead && i < nbytes) ? gsrc[i] : 0;
+                for (uint32_t i = b0; i < b0 + 16; i++) ((uint8_t*)pbuf)[i ^ 3u] = (i >= lead && i < nbytes) ? gsrc[i] : 0;
             }
         }
     }
     __syncthreads();
 
-    const uint32_t nbl = s_sc[5], nseg = s_sc[6], SG = s_sc[7];
+    const uint32_t nbl = s_sc[5], nseg = s_sc[6], SG = s_sc[7], npk = s_sc[1];
     const jxs_bline_t* bls = s_bl;
-    const jxs_seg_t* segs = s_seg;
     /* parse, by warp 0: band modes and per-line fields in parallel, the
-     * packet headers in order by lane 0, then every line's positions */
+     * packet headers in order by lane 0 */
     if (warp == 0) {
-        const uint8_t* h0 = pbuf + lead;
-        const uint8_t q = h0[3], r = h0[4];
+        const uint32_t q = byte_of(pbuf, lead + 3), r = byte_of(pbuf, lead + 4);
         int err = 0, vp_seen = 0;
         /* band coding modes D[p,b], 2 bits per existing band */
         uint32_t idx0 = 0;
-        const uint32_t nbands_all = s_sc[0], npk_c = s_sc[1];
+        const uint32_t nbands_all = s_sc[0];
         for (uint32_t gb0 = 0; gb0 < nbands_all; gb0 += 32) {
             const uint32_t gb = gb0 + lane;
             const int fb = gb < nbands_all ? s_g2f[gb] : JXS_NOBAND;
             const bool ex = fb != JXS_NOBAND;
             const uint32_t bal = __ballot_sync(FULL, ex);
             if (ex) {
-                const uint32_t pos = 40 + 2 * (idx0 + __popc(bal & ((1u << lane) - 1)));
-                s_mode[fb] = (uint8_t)((h0[pos >> 3] >> (6 - (pos & 7))) & 3);
+                const uint32_t pos = 8 * lead + 40 + 2 * (idx0 + __popc(bal & ((1u << lane) - 1)));
+                s_mode[fb] = (uint8_t)((pbuf[pos >> 5] >> (30 - (pos & 31))) & 3);
                 /* vertical prediction: resolved here when the precinct row
                  * above is known (slice-ordered decoding), else the frame is
                  * decoded again that way; never in a slice's first row */
@@ -442,63 +469,83 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
             idx0 += __popc(bal);
         }
         __syncwarp();
-        for (uint32_t x = lane; x < nbl; x += 32) {
-            ln[x].t = jxs_truncation((uint8_t)(s_lgp[x] & 255u), (uint8_t)(s_lgp[x] >> 8), q, r);
-            ln[x].meth = (s_mode[bls[x].fb] & 2) ? 1 : 0;
-            ln[x].vp = (s_mode[bls[x].fb] & 1) ? 1 : 0;
-            ln[x].pk = bls[x].pk;
-        }
-        __syncwarp();
-        /* per packet: significance bits and raw GCLI bits it must hold */
-        uint32_t sb = 0, rb = 0;
-        if (lane < (int)npk_c) {
-            const uint32_t b0 = s_pkbl0[lane], nb = s_pknbl[lane];
-            for (uint32_t x = b0; x < b0 + nb; x++) {
-                if (ln[x].meth) sb += bls[x].sig_w;
-                rb += 4 * bls[x].gcli_w;
+        /* per line, each lane a run of them: gtli and method, and the
+         * significance flags and raw GCLI bits before it */
+        {
+            const uint32_t per = (nbl + 31) >> 5, x0 = min(nbl, per * lane), x1 = min(nbl, x0 + per);
+            uint32_t sg = 0, rw = 0;
+            for (uint32_t x = x0; x < x1; x++) {
+                const uint32_t m = s_mode[bls[x].fb];
+                ln[x].t = jxs_truncation((uint8_t)(s_lgp[x] & 255u), (uint8_t)(s_lgp[x] >> 8), (uint8_t)q, (uint8_t)r);
+                ln[x].meth = (m & 2) ? 1 : 0;
+                ln[x].vp = (m & 1) ? 1 : 0;
+                ln[x].pk = bls[x].pk;
+                sg += (m & 2) ? bls[x].sig_w : 0u;
+                rw += 4 * bls[x].gcli_w;
             }
-            s_pksb[lane] = sb;
-            s_pkrb[lane] = rb;
+            uint32_t tsg, trw;
+            sg = warp_excl_scan(sg, &tsg);
+            rw = warp_excl_scan(rw, &trw);
+            for (uint32_t x = x0; x < x1; x++) {
+                s_lsx[x] = sg;
+                s_lrx[x] = rw;
+                sg += ln[x].meth ? bls[x].sig_w : 0u;
+                rw += 4 * bls[x].gcli_w;
+            }
+            if (lane == 0) {
+                s_lsx[nbl] = tsg;
+                s_lrx[nbl] = trw;
+            }
         }
         __syncwarp();
-        /* packet headers: lane 0 follows the chain of header positions
+        /* per packet: significance bytes and raw GCLI bits it must hold */
+        const bool here = lane < (int)npk && s_pknbl[lane];
+        uint32_t sB = 0, rb = 0;
+        if (here) {
+            const uint32_t b0 = s_pkbl0[lane], b1 = b0 + s_pknbl[lane];
+            sB = (s_lsx[b1] - s_lsx[b0] + 7) >> 3;
+            rb = s_lrx[b1] - s_lrx[b0];
+        }
+        /* packet headers: the warp follows the chain of header positions
          * only; one lane per packet then reads its header again and derives
          * its sub-packet positions with the reference's checks (every check
          * bounds the running position, so testing each packet's own end
          * against the precinct's end is equivalent) */
         const int long_hdr = (int)s_sc[2];
         const uint32_t hb = long_hdr ? 7u : 5u, pend_max = lead + total;
-        if (lane == 0) {
-            uint32_t bpos = lead + s_sc[4]; /* bytes */
-            for (uint32_t k = 0; k < npk_c; k++) {
-                if (!s_pknbl[k]) continue;
+        {
+            const uint32_t have = __ballot_sync(FULL, here);
+            uint32_t bpos = lead + s_sc[4], mine = 0; /* bytes */
+            for (uint32_t left = have; left; left &= left - 1) {
+                const int k = __ffs((int)left) - 1;
                 if (bpos + hb > pend_max) {
                     err = JXS_E_DEC_BITSTREAM;
                     break;
                 }
                 uint32_t raw, dlen, glen, slen;
-                pk_header(pbuf + bpos, long_hdr, raw, dlen, glen, slen);
-                s_hpos[k] = bpos;
-                bpos += hb + (raw ? 0u : (s_pksb[k] + 7) >> 3) + glen + dlen + slen;
+                pk_header(pbuf, bpos, long_hdr, raw, dlen, glen, slen);
+                if (lane == k) mine = bpos;
+                const uint32_t sBk = __shfl_sync(FULL, sB, k);
+                bpos += hb + (raw ? 0u : sBk) + glen + dlen + slen;
             }
+            if (lane < JXS_MAXPK) s_hpos[lane] = mine;
         }
-        err = __shfl_sync(FULL, err, 0);
         uint32_t nwords = 0;
-        if (lane < (int)npk_c) {
+        if (lane < (int)npk) {
             UkPk& P = pk[lane];
             P.present = 0;
             P.gbits = P.dbits = P.ncoded = P.nzero = 0;
             P.raw = 0;
-            if (!err && s_pknbl[lane]) {
+            if (!err && here) {
                 uint32_t raw, dlen, glen, slen;
                 const uint32_t b = s_hpos[lane] + hb;
-                pk_header(pbuf + s_hpos[lane], long_hdr, raw, dlen, glen, slen);
+                pk_header(pbuf, s_hpos[lane], long_hdr, raw, dlen, glen, slen);
                 uint32_t gp = b;
                 if (raw) {
-                    if (s_pkrb[lane] > glen * 8) err = JXS_E_DEC_BITSTREAM;
+                    if (rb > glen * 8) err = JXS_E_DEC_BITSTREAM;
                 } else {
-                    gp += (s_pksb[lane] + 7) >> 3;
-                    /* codeword ends are kept as 16-bit offsets in the sub-packet */
+                    gp += sB;
+                    /* unary codes longer than this are refused */
                     if (glen * 8 > 65535u) err = JXS_E_DEC_BITSTREAM;
                 }
                 if ((uint64_t)gp + glen + dlen + slen > pend_max) err = JXS_E_DEC_BITSTREAM;
@@ -517,37 +564,24 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         {
             uint32_t tw;
             const uint32_t wb = warp_excl_scan(nwords, &tw);
-            if (lane < (int)npk_c) {
+            if (lane < (int)npk) {
                 pk[lane].wbase = wb;
                 pk[lane].nwords = nwords;
             }
-            if (lane == 0) {
-                s_tw = tw;
-                s_npk = npk_c;
-            }
+            if (lane == 0) s_tw = tw;
         }
         err = __reduce_or_sync(FULL, (uint32_t)err) ? JXS_E_DEC_BITSTREAM : 0;
         if (!err && __any_sync(FULL, vp_seen)) {
-            if (!top_gcl) err = JXS_E_DEC_VPRED;
+            if (!VP) err = JXS_E_DEC_VPRED;
             else if (!vp_ok) err = JXS_E_DEC_BITSTREAM; /* no precinct row above to predict from */
         }
         __syncwarp();
-        /* line positions: significance flags, or raw GCLIs for raw packets */
-        if (!err && lane < (int)npk_c && pk[lane].present) {
-            const UkPk& P = pk[lane];
-            const uint32_t b0 = s_pkbl0[lane], nb = s_pknbl[lane];
-            uint32_t run = P.spos;
-            for (uint32_t x = b0; x < b0 + nb; x++) {
-                ln[x].raw = (uint8_t)P.raw;
-                if (P.raw) ln[x].vp = 0;
-                ln[x].sig_pos = run;
-                run += P.raw ? 4 * bls[x].gcli_w : (ln[x].meth ? bls[x].sig_w : 0u);
-            }
-        }
-        __syncwarp();
-        if (!err) {
+        if (VP && !err) {
             bool hv = false;
-            for (uint32_t x = lane; x < nbl; x += 32) hv |= ln[x].vp != 0;
+            for (uint32_t x = lane; x < nbl; x += 32) {
+                if (pk[ln[x].pk].raw) ln[x].vp = 0;
+                hv |= ln[x].vp != 0;
+            }
             if (__any_sync(FULL, hv) && lane == 0) s_hasvp = 1;
         }
         if (lane == 0) s_err = err;
@@ -561,20 +595,21 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
     /* codewords of every segment, one thread each: its groups minus those
      * in insignificant significance groups (flags: 1 = insignificant); then
      * the codeword base of every segment inside its packet */
-    const uint32_t tw = s_tw, npk = s_npk;
+    const uint32_t tw = s_tw;
+    uint32_t cwbase, sigpos = 0;
     {
         uint32_t cnt = 0;
         if (threadIdx.x < nseg) {
-            const jxs_seg_t sg = segs[threadIdx.x];
-            const jxs_bline_t& B = bls[sg.bl];
-            const UkLine& L = ln[sg.bl];
-            const uint32_t gend = min(sg.g0 + SG, B.gcli_w);
-            if (!L.raw) {
-                cnt = gend - sg.g0;
-                if (L.meth) {
-                    for (uint32_t s0 = sg.g0 >> 3; s0 < ((gend + 7) >> 3); s0 += 32) {
+            const jxs_bline_t& B = bls[myseg.bl];
+            const UkPk& P = pk[B.pk];
+            const uint32_t gend = min(myseg.g0 + SG, B.gcli_w);
+            if (!P.raw) {
+                cnt = gend - myseg.g0;
+                if (ln[myseg.bl].meth) {
+                    sigpos = P.spos + s_lsx[myseg.bl] - s_lsx[s_pkbl0[B.pk]] + (myseg.g0 >> 3);
+                    for (uint32_t s0 = myseg.g0 >> 3; s0 < ((gend + 7) >> 3); s0 += 32) {
                         const uint32_t ns = min(32u, ((gend + 7) >> 3) - s0);
-                        const uint32_t fl = bits32_at(pbuf, L.sig_pos + s0) >> (32 - ns);
+                        const uint32_t fl = bits32_at(pbuf, sigpos + s0 - (myseg.g0 >> 3)) >> (32 - ns);
                         cnt -= 8 * __popc(fl);
                         /* a flagged partial last group counts its own size */
                         if ((fl & 1u) && 8 * (s0 + ns) > B.gcli_w) cnt += 8 * (s0 + ns) - B.gcli_w;
@@ -582,14 +617,15 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
                 }
             }
         }
-        const uint32_t ncoded = seg_bases(cnt, nseg, npk, segs, bls, s_pkbl0, s_pknbl, s_ex, s_base, ws);
+        uint32_t ncoded;
+        cwbase = seg_bases(cnt, myseg.bl, nseg, npk, bls, s_pkbl0, s_pknbl, s_ex, ws, &ncoded);
         if (threadIdx.x < npk) pk[threadIdx.x].ncoded = ncoded;
         __syncthreads();
     }
 
-    /* zero bits of the VLC sub-packets: count, scan, record positions.  A
-     * thread's first word finds its packet by binary search over the
-     * packets' word ranges (contiguous, in packet order; a packet without
+    /* zero bits of the VLC sub-packets: count, scan, record the codeword
+     * values.  A thread's first word finds its packet by binary search over
+     * the packets' word ranges (contiguous, in packet order; a packet without
      * VLC words has an empty range), later words step forward. */
     const uint32_t per = (tw + blockDim.x - 1) / blockDim.x;
     const uint32_t wa = min(tw, threadIdx.x * per), we = min(tw, wa + per);
@@ -618,20 +654,31 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
     uint32_t z0;
     const uint32_t ztotal = block_scan1(zc, &z0, ws);
     {
-        uint32_t k = k0;
+        uint32_t k = k0, ones = 0; /* ones since the last zero bit */
         for (uint32_t wi = wa; wi < we; wi++) {
             while (k + 1 < npk && wi >= pk[k].wbase + pk[k].nwords) k++;
-            const uint32_t i = wi - pk[k].wbase;
-            if (i == 0) pk[k].zbase = z0;
-            const uint32_t valid = min(32u, pk[k].gbits - 32 * i);
-            uint32_t z = ~bits32_at(pbuf, pk[k].gpos + 32 * i);
-            if (valid < 32) z &= ~(0xffffffffu >> valid);
-            while (z) {
-                const uint32_t lz = __clz(z);
-                if (z0 < zcap) zend[z0] = (uint16_t)(32 * i + lz);
-                z0++;
-                z &= ~(0x80000000u >> lz);
+            const uint32_t i = wi - pk[k].wbase, at = pk[k].gpos + 32 * i;
+            if (i == 0) {
+                pk[k].zbase = z0;
+                ones = 0;
+            } else if (wi == wa) {
+                /* the end of the word before (32 ones: no valid codeword is
+                 * that long) */
+                const uint32_t zp = ~bits32_at(pbuf, at - 32);
+                ones = zp ? (uint32_t)__ffs((int)zp) - 1 : 32u;
             }
+            const uint32_t valid = min(32u, pk[k].gbits - 32 * i);
+            uint32_t z = ~bits32_at(pbuf, at);
+            if (valid < 32) z &= ~(0xffffffffu >> valid);
+            const uint32_t tail = z ? (uint32_t)__ffs((int)z) - 1 : min(ones + 32u, 64u);
+            while (z) {
+                const uint32_t run = __clz((int)z);
+                if (z0 < zcap) zval[z0] = (uint8_t)(ones + run);
+                z0++;
+                ones = 0;
+                z = shl_or_0(z, run + 1);
+            }
+            ones = tail;
         }
     }
     __syncthreads();
@@ -663,83 +710,81 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         if (threadIdx.x == 0) JXS_STATUS_SET(status, s_err);
         return;
     }
+    /* the segments' records */
+    if (threadIdx.x < nseg) {
+        const jxs_bline_t& B = bls[myseg.bl];
+        const UkLine L = ln[myseg.bl];
+        const UkPk& P = pk[B.pk];
+        UkSeg D;
+        D.vpos = P.raw ? P.spos + s_lrx[myseg.bl] - s_lrx[s_pkbl0[B.pk]] + 4 * myseg.g0 : P.zbase + cwbase;
+        D.sig = sigpos;
+        D.z = B.gbase + myseg.g0;
+        D.info = min(SG, B.gcli_w - myseg.g0) | ((uint32_t)L.t << 16) | ((P.raw ? 0u : (uint32_t)L.meth) << 20) | (P.raw << 21) |
+                 (VP ? (uint32_t)L.vp << 22 : 0u) | ((uint32_t)myseg.bl << 24);
+        s_desc[threadIdx.x] = D;
+    }
+    __syncthreads();
 
-    /* pass 2: GCLIs from codeword ends; data bits per segment.  Each lane
+    /* pass 2: GCLIs from codeword values; data bits per segment.  Each lane
      * takes 4 consecutive groups: they share one significance flag, so
      * either all of them carry a codeword or none (only the segment's last
      * lane may hold fewer than 4 groups, and no lane after it holds any). */
     int bad = 0;
     const uint32_t lt_mask = (1u << lane) - 1u;
     /* a group's data: its sign nibble (signs with the data) and its planes */
-    const uint32_t fs = s_sc[3], nib_sign = fs ? 0u : 1u;
+    const uint32_t fs = FS ? s_sc[3] : 0u;
     for (uint32_t qi = next_seg(&s_next[0], lane); qi < nseg; qi = next_seg(&s_next[0], lane)) {
         const uint32_t sidx = s_ord[qi];
-        const jxs_seg_t sg = segs[sidx];
-        const jxs_bline_t B = bls[sg.bl];
-        const UkLine L = ln[sg.bl];
-        const UkPk P = pk[L.pk];
-        const uint32_t gend = min(sg.g0 + SG, B.gcli_w);
-        uint32_t cw = s_base[sidx], dsum = 0;
-        for (uint32_t base = sg.g0; base < gend; base += 128) {
-            const uint32_t g0 = base + 4 * lane;
-            const uint32_t nv = g0 < gend ? min(4u, gend - g0) : 0u;
-            uint32_t v4 = 0;
-            bool coded = false;
-            if (nv) {
-                if (L.raw) {
-                    /* 4 raw 4-bit GCLIs, group g0 in the top nibble */
-                    const uint32_t w = bits32_at(pbuf, L.sig_pos + 4 * g0);
-                    v4 = __byte_perm(((w >> 28) & 15u) | (((w >> 24) & 15u) << 8), ((w >> 20) & 15u) | (((w >> 16) & 15u) << 8),
-                                     0x5410);
-                } else {
-                    const uint32_t sp = L.sig_pos + (g0 >> 3);
-                    coded = !(L.meth && ((pbuf[sp >> 3] >> (7 - (sp & 7))) & 1));
-                    /* predicted lines keep the codeword value (0xff: no
-                     * codeword) until the line above is known */
-                    if (!coded) v4 = L.vp ? 0xffffffffu : L.t * 0x01010101u;
-                }
-            }
-            const uint32_t bal = __ballot_sync(FULL, coded);
-            if (coded) {
-                /* codeword c + q ends at the (c + q)-th zero bit: its value
-                 * is the distance to the zero before, less one; the four
-                 * distances as 16-bit pairs */
-                const uint32_t c = cw + 4 * __popc(bal & lt_mask);
-                const uint32_t zr = P.zbase + c;
-                const uint32_t zm = c ? zend[zr - 1] : 0xffffu; /* -1 */
-                uint32_t z[4];
-#pragma unroll
-                for (int q = 0; q < 4; q++) z[q] = q < (int)nv ? zend[zr + q] : 0u;
-                const uint32_t r01 = __vsub2(__vsub2(z[0] | (z[1] << 16), zm | (z[0] << 16)), 0x00010001u);
-                const uint32_t r23 = __vsub2(__vsub2(z[2] | (z[3] << 16), z[1] | (z[2] << 16)), 0x00010001u);
-                /* GCLI = base + r, at most 15 (31 for a predicted line's
-                 * codeword value) */
-                const uint32_t base = L.vp ? 0u : L.t, room = (L.vp ? 31u : 15u) - base;
-                const uint32_t room2 = room * 0x00010001u, base2 = base * 0x00010001u;
-                const uint32_t keep = nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
-                if (__byte_perm(__vcmpgtu2(r01, room2), __vcmpgtu2(r23, room2), 0x6420) & keep) bad = 1;
-                v4 = __byte_perm(__vadd2(__vminu2(r01, room2), base2), __vadd2(__vminu2(r23, room2), base2), 0x6420) & keep;
-            }
-            uint8_t* gdst = gcl + B.gbase + g0;
-            if (nv == 4) {
-                *(uint32_t*)gdst = v4;
+        const UkSeg D = s_desc[sidx];
+        const uint32_t n = D.info & 0xffffu, t = (D.info >> 16) & 15u;
+        const bool raw = (D.info >> 21) & 1u, sig = (D.info >> 20) & 1u, vp = VP && ((D.info >> 22) & 1u);
+        uint32_t cw = D.vpos, dsum = 0;
+        for (uint32_t base = 0; base < n; base += 128) {
+            const uint32_t g = base + 4 * lane;
+            const uint32_t nv = g < n ? min(4u, n - g) : 0u;
+            const uint32_t keep = nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u, t4 = t * 0x01010101u;
+            uint32_t v4;
+            if (raw) {
+                /* 4 raw 4-bit GCLIs, the first in the top nibble */
+                const uint32_t w = nv ? bits32_at(pbuf, D.vpos + 4 * g) : 0u;
+                v4 = (w >> 28) | ((w >> 16) & 0x00000f00u) | ((w >> 4) & 0x000f0000u) | ((w << 8) & 0x0f000000u);
             } else {
-                for (uint32_t q = 0; q < nv; q++) gdst[q] = (uint8_t)(v4 >> (8 * q));
+                /* the groups of 8 in lanes 2i, 2i + 1 share flag i */
+                bool coded = nv != 0;
+                if (sig) coded = coded && !((bits32_at(pbuf, D.sig + (base >> 3)) >> (31 - (lane >> 1))) & 1u);
+                const uint32_t bal = __ballot_sync(FULL, coded);
+                /* predicted lines keep the codeword value (0xff: no
+                 * codeword) until the line above is known */
+                v4 = vp ? 0xffffffffu : t4;
+                if (coded) {
+                    const uint32_t c = cw + 4 * __popc(bal & lt_mask);
+                    const uint32_t* zw = (const uint32_t*)(zval + (c & ~3u));
+                    const uint32_t r4 = __funnelshift_r(zw[0], zw[1], 8 * (c & 3u)) & keep;
+                    /* GCLI = gtli + value, at most 15 (31 for a predicted
+                     * line's codeword value; values are below 128) */
+                    const uint32_t room = vp ? 31u : 15u - t;
+                    v4 = vp ? r4 : r4 + t4;
+                    if ((r4 + (127u - room) * 0x01010101u) & 0x80808080u) {
+                        bad = 1;
+                        v4 = t4;
+                    }
+                }
+                if (base + 128 < n) cw += 4 * __popc(bal);
             }
-            cw += __reduce_add_sync(FULL, coded ? nv : 0u);
-            if (!L.vp) {
+            if (nv) *(uint32_t*)(gcl + D.z + g) = v4; /* lines are padded to a multiple of 4 */
+            if (!vp) {
                 /* data bits: 4 (v - t + 1) per group above gtli (4 (v - t)
                  * with separate signs) */
-                const uint32_t t4 = L.t * 0x01010101u;
-                const uint32_t vm = v4 & (nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u);
-                dsum += 4 * (__vsadu4(__vsubus4(vm, t4), 0u) + nib_sign * __popc(__vcmpgtu4(vm, t4) & 0x01010101u));
+                const uint32_t y = ((v4 & keep) | 0x80808080u) - (t + 1) * 0x01010101u;
+                const uint32_t above = sign_bytes(y), one = above & 0x01010101u;
+                dsum += __dp4a((y & above & 0x7f7f7f7fu) + (fs ? one : 2u * one), 0x01010101u, 0u);
             }
         }
         dsum = __reduce_add_sync(FULL, dsum);
-        if (lane == 0) s_cnt[sidx] = dsum;
+        if (lane == 0) s_cnt[sidx] = 4 * dsum;
     }
     __syncthreads();
-    if (s_hasvp) {
+    if (VP && s_hasvp) {
         /* vertical prediction (unpack_verical_pred_gclis_*, Packing.c:267-431):
          * GCLI = the predictor max(top, max(gtli_top, gtli)) moved by the
          * codeword value; without a codeword (insignificant group) the
@@ -748,24 +793,22 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         const uint32_t rm = s_sc[8];
         for (uint32_t lvl = 0; lvl < 4; lvl++) {
             for (uint32_t sidx = warp; sidx < nseg; sidx += UK_WARPS) {
-                const jxs_seg_t sg = segs[sidx];
-                const jxs_bline_t B = bls[sg.bl];
-                const UkLine L = ln[sg.bl];
-                if (!L.vp || B.line != lvl) continue;
-                const uint32_t tb = s_topbl[sg.bl];
-                const int from_prev = s_topprev[sg.bl];
-                const uint8_t* src = (from_prev ? top_gcl : gcl) + s_topg[sg.bl];
-                const uint32_t tt = max(from_prev ? (uint32_t)top_t[tb] : (uint32_t)ln[tb].t, (uint32_t)L.t);
-                const uint32_t gend = min(sg.g0 + SG, B.gcli_w);
+                const UkSeg D = s_desc[sidx];
+                const uint32_t bl = D.info >> 24, n = D.info & 0xffffu, lt = (D.info >> 16) & 15u;
+                if (!((D.info >> 22) & 1u) || bls[bl].line != lvl) continue;
+                const uint32_t tb = s_topbl[bl];
+                const int from_prev = s_topprev[bl];
+                const uint8_t* src = (from_prev ? top_gcl : gcl) + s_topg[bl] + (D.z - bls[bl].gbase);
+                const uint32_t tt = max(from_prev ? (uint32_t)top_t[tb] : (uint32_t)ln[tb].t, lt);
                 uint32_t dsum = 0;
-                for (uint32_t g = sg.g0 + lane; g < gend; g += 32) {
-                    const uint32_t x = gcl[B.gbase + g];
+                for (uint32_t g = lane; g < n; g += 32) {
+                    const uint32_t x = gcl[D.z + g];
                     const uint32_t mt = max((uint32_t)src[g], tt);
                     uint32_t v;
                     if (x == 0xffu) {
-                        v = rm ? L.t : mt;
+                        v = rm ? lt : mt;
                     } else {
-                        const uint32_t thr = mt > L.t ? mt - L.t : 0u;
+                        const uint32_t thr = mt > lt ? mt - lt : 0u;
                         int d = 0;
                         if (x > 2 * thr) d = (int)(x - thr);
                         else if (x > 0) d = (x & 1) ? -(int)((x + 1) >> 1) : (int)(x >> 1);
@@ -775,8 +818,8 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
                         bad = 1;
                         v = 15;
                     }
-                    gcl[B.gbase + g] = (uint8_t)v;
-                    if (v > L.t) dsum += 4 * (v - L.t + nib_sign);
+                    gcl[D.z + g] = (uint8_t)v;
+                    if (v > lt) dsum += 4 * (v - lt + (fs ? 0u : 1u));
                 }
                 dsum = __reduce_add_sync(FULL, dsum);
                 if (lane == 0) s_cnt[sidx] = dsum;
@@ -785,9 +828,11 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         }
     }
     {
-        /* data base of every segment inside its packet */
-        const uint32_t dbits = seg_bases(threadIdx.x < nseg ? s_cnt[threadIdx.x] : 0u, nseg, npk, segs, bls, s_pkbl0, s_pknbl,
-                                         s_ex, s_base, ws);
+        /* data position of every segment */
+        uint32_t dbits;
+        const uint32_t b = seg_bases(threadIdx.x < nseg ? s_cnt[threadIdx.x] : 0u, myseg.bl, nseg, npk, bls, s_pkbl0, s_pknbl, s_ex, ws,
+                                     &dbits);
+        if (threadIdx.x < nseg) s_base[threadIdx.x] = pk[bls[myseg.bl].pk].dpos + b;
         const int bad_pk = threadIdx.x < npk && pk[threadIdx.x].present && dbits > pk[threadIdx.x].dbits;
         if (__syncthreads_or(bad_pk)) {
             if (threadIdx.x == 0) JXS_STATUS_SET(status, JXS_E_DEC_BITSTREAM);
@@ -797,7 +842,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
 
     /* pass 3: data */
     const uint32_t uniform = cfg->qpih;
-    if (fs) {
+    if (FS && fs) {
         /* separate signs (unpack_sign, Packing.c:221-247): a sign bit for
          * every non-zero magnitude, band lines of the packet in order and each
          * line in coefficient order (the last group's padding coefficients
@@ -805,16 +850,13 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
          * bit in the packet's sign sub-packet, then decode with the signs. */
         for (uint32_t qi = next_seg(&s_next[1], lane); qi < nseg; qi = next_seg(&s_next[1], lane)) {
             const uint32_t sidx = s_ord[qi];
-            const jxs_seg_t sg = segs[sidx];
-            const jxs_bline_t B = bls[sg.bl];
-            const UkLine L = ln[sg.bl];
-            const UkPk P = pk[L.pk];
-            const uint32_t gend = min(sg.g0 + SG, B.gcli_w);
-            uint32_t dpos = P.dpos + s_base[sidx], nzs = 0;
-            for (uint32_t base = sg.g0; base < gend; base += 32) {
+            const UkSeg D = s_desc[sidx];
+            const uint32_t n = D.info & 0xffffu, t = (D.info >> 16) & 15u;
+            uint32_t dpos = s_base[sidx], nzs = 0;
+            for (uint32_t base = 0; base < n; base += 32) {
                 const uint32_t g = base + lane;
-                const uint32_t v = g < gend ? gcl[B.gbase + g] : 0u;
-                const uint32_t np = v > L.t ? v - L.t : 0u;
+                const uint32_t v = g < n ? gcl[D.z + g] : 0u;
+                const uint32_t np = v > t ? v - t : 0u;
                 const uint32_t len = 4 * np;
                 uint32_t tot;
                 const uint32_t ex = warp_excl_scan(len, &tot);
@@ -822,17 +864,19 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
                     const uint32_t pos = dpos + ex;
                     const uint64_t win = ((uint64_t)bits32_at(pbuf, pos) << 32) | bits32_at(pbuf, pos + 32);
                     uint32_t A, B2;
-                    nzs += __popc(group_mags(win >> (64 - len), np, L.t, v, uniform, &A, &B2));
+                    nzs += __popc(group_mags(win >> (64 - len), np, t, v, uniform, &A, &B2));
                 }
                 dpos += tot;
             }
             nzs = __reduce_add_sync(FULL, nzs);
-            if (lane == 0) s_nz[sidx] = nzs;
+            if (lane == 0) s_cnt[sidx] = nzs;
         }
         __syncthreads();
-        /* first sign bit of every segment inside its packet */
-        const uint32_t sbits = seg_bases(threadIdx.x < nseg ? s_nz[threadIdx.x] : 0u, nseg, npk, segs, bls, s_pkbl0, s_pknbl,
-                                         s_ex, s_sgb, ws);
+        /* first sign bit of every segment */
+        uint32_t sbits;
+        const uint32_t b = seg_bases(threadIdx.x < nseg ? s_cnt[threadIdx.x] : 0u, myseg.bl, nseg, npk, bls, s_pkbl0, s_pknbl, s_ex, ws,
+                                     &sbits);
+        if (threadIdx.x < nseg) s_sgb[threadIdx.x] = pk[bls[myseg.bl].pk].sgpos + b;
         const int bad_pk = threadIdx.x < npk && pk[threadIdx.x].present && sbits > pk[threadIdx.x].sgbits;
         if (threadIdx.x == 0) s_next[1] = 0;
         if (__syncthreads_or(bad_pk)) {
@@ -842,37 +886,31 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
     }
     for (uint32_t qi = next_seg(&s_next[1], lane); qi < nseg; qi = next_seg(&s_next[1], lane)) {
         const uint32_t sidx = s_ord[qi];
-        const jxs_seg_t sg = segs[sidx];
-        const jxs_bline_t B = bls[sg.bl];
-        const UkLine L = ln[sg.bl];
-        const UkPk P = pk[L.pk];
-        int16_t* crow = coef + s_crow[sg.bl];
-        const uint32_t gend = min(sg.g0 + SG, B.gcli_w);
-        uint32_t dpos = P.dpos + s_base[sidx];
-        if (!fs) {
+        const UkSeg D = s_desc[sidx];
+        const uint32_t n = D.info & 0xffffu, t = (D.info >> 16) & 15u, bl = D.info >> 24;
+        int16_t* crow = coef + (s_crow[bl] + 4 * (uint64_t)D.z);
+        const int wend = (int)(s_wend[bl] - 4 * D.z); /* coefficients of the line from the segment on */
+        uint32_t dpos = s_base[sidx];
+        if (!FS || !fs) {
             /* signs with the data: each lane 4 consecutive groups.  The lane
              * writes zeros for its groups, then the warp lists the groups
-             * with data (bit offset in the warp's data, group, GCLI) and each
-             * lane decodes one listed group at a time, so that the decode
+             * with data (nibble offset in the warp's data, group, GCLI) and
+             * each lane decodes one listed group at a time, so that the decode
              * work follows the groups that have data */
-            uint32_t* list = (uint32_t*)(dsm + UL.zend) + 128 * warp;
-            const uint32_t t = L.t;
-            for (uint32_t base = sg.g0; base < gend; base += 128) {
+            uint32_t* list = (uint32_t*)zval + 128 * warp;
+            for (uint32_t base = 0; base < n; base += 128) {
                 const uint32_t g = base + 4 * lane;
-                const uint32_t nv = g < gend ? min(4u, gend - g) : 0u;
-                uint32_t v4 = 0;
-                if (nv == 4) {
-                    v4 = *(const uint32_t*)(gcl + B.gbase + g);
-                } else {
-                    for (uint32_t q = 0; q < nv; q++) v4 |= (uint32_t)gcl[B.gbase + g + q] << (8 * q);
-                }
-                /* per byte: v > t, and the data of such a group: 4 (v - t + 1)
-                 * bits; one scan for the data bits / 4 and the listed groups */
-                const uint32_t t4 = t * 0x01010101u;
-                const uint32_t s4 = __vcmpgtu4(v4, t4), nsig = __popc(s4 & 0x01010101u);
-                uint32_t tot;
-                const uint32_t ex = warp_excl_scan((__vsadu4(__vsubus4(v4, t4), 0u) + nsig) | (nsig << 24), &tot);
-                const uint32_t o = (ex & 0xffffffu) << 2;
+                const uint32_t nv = g < n ? min(4u, n - g) : 0u;
+                const uint32_t keep = nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
+                const uint32_t v4 = nv ? *(const uint32_t*)(gcl + D.z + g) & keep : 0u;
+                /* per byte: v > t, and the data nibbles of such a group (v - t
+                 * + 1); running sums over the lane's bytes, then one scan for
+                 * the nibbles and the listed groups */
+                const uint32_t y = (v4 | 0x80808080u) - (t + 1) * 0x01010101u;
+                const uint32_t above = sign_bytes(y), one = above & 0x01010101u;
+                const uint32_t nibs = ((y & above & 0x7f7f7f7fu) + 2u * one) * 0x01010101u;
+                const uint32_t own = (nibs >> 24) | ((uint32_t)__popc(one) << 24);
+                const uint32_t inc = warp_incl_scan(own), ex = inc - own, tot = __shfl_sync(FULL, inc, 31), cnt = tot >> 24;
                 /* zeros for the lane's groups (those with data are written
                  * again below, after the warp barrier) */
                 if (one_col) {
@@ -885,35 +923,31 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
                 } else {
                     /* a column starts anywhere in the row and ends where the
                      * next begins: the groups' coefficients inside it only */
-                    const int wl = (int)B.w - 4 * (int)g;
-                    for (int c = 0; c < 4 * (int)nv && c < wl; c++)
-                        if (!((s4 >> (8 * (c >> 2))) & 1u)) crow[4 * g + c] = 0;
+                    for (int c = 0; c < 4 * (int)nv && c < wend - 4 * (int)g; c++)
+                        if (!((one >> (8 * (c >> 2))) & 1u)) crow[4 * g + c] = 0;
                 }
-                const uint32_t cnt = tot >> 24;
                 {
-                    /* per byte: 1 for a listed group, and its data nibbles
-                     * v - t + 1; their exclusive prefix sums over the lane's
-                     * bytes give each entry's slot and offset */
-                    const uint32_t one = s4 & 0x01010101u, dd = __vsubus4(v4, t4) + one;
-                    const uint32_t po = dd * 0x01010100u, pi = one * 0x01010100u;
-                    const uint32_t e0 = (o << 11) | ((uint32_t)lane << 6), i0 = ex >> 24;
-#pragma unroll
-                    for (int q = 0; q < 4; q++)
-                        if ((one >> (8 * q)) & 1u)
-                            list[i0 + ((pi >> (8 * q)) & 255u)] =
-                                e0 + (((po >> (8 * q)) & 255u) << 13) + ((uint32_t)q << 4) + ((v4 >> (8 * q)) & 15u);
+                    const uint32_t po = nibs << 8, pi = one * 0x01010100u; /* before each byte's group */
+                    const uint32_t e0 = ((ex & 0xffffu) << 16) | ((uint32_t)lane << 6);
+                    uint32_t* slot = list + (ex >> 24);
+                    if (one & 0x00000001u) slot[0] = e0 + (v4 & 255u);
+                    if (one & 0x00000100u) slot[(pi >> 8) & 255u] = e0 + 0x10u + __byte_perm(v4, po, 0x4541);
+                    if (one & 0x00010000u) slot[(pi >> 16) & 255u] = e0 + 0x20u + __byte_perm(v4, po, 0x4642);
+                    if (one & 0x01000000u) slot[pi >> 24] = e0 + 0x30u + __byte_perm(v4, po, 0x4743);
                 }
                 __syncwarp();
                 for (uint32_t r = lane; r < cnt; r += 32) {
                     const uint32_t e = list[r];
-                    const uint32_t gi = base + ((e >> 4) & 127u), v = e & 15u, np = v - t, ln = 4 * (np + 1);
-                    const uint32_t pos = dpos + (e >> 11);
-                    const uint32_t wi = pos >> 5, sh = pos & 31;
-                    const uint32_t w0 = be_word(pbuf, wi), w1 = be_word(pbuf, wi + 1), w2 = be_word(pbuf, wi + 2);
-                    const uint64_t win = ((uint64_t)__funnelshift_l(w1, w0, sh) << 32) | __funnelshift_l(w2, w1, sh);
-                    const int wl = (int)B.w - 4 * (int)gi;
-                    const uint2 ov = uniform ? decode_group(win >> (64 - ln), np, t, v, uniform, wl)
-                                             : decode_group_dz(win >> (64 - ln), np, t, wl);
+                    const uint32_t gi = base + ((e >> 4) & 127u), v = e & 15u, np = v - t, pos = dpos + 4 * (e >> 16);
+                    const int wl = wend - 4 * (int)gi;
+                    const uint32_t win = bits32_at(pbuf, pos);
+                    uint2 ov;
+                    if (np < 8 && !uniform) {
+                        ov = decode_group_dz(win >> (28 - 4 * np), np, t, wl);
+                    } else {
+                        const uint64_t w2 = (((uint64_t)win << 32) | bits32_at(pbuf, pos + 32)) >> (60 - 4 * np);
+                        ov = uniform ? decode_group(w2, np, t, v, uniform, wl) : decode_group_dz(w2, np, t, wl);
+                    }
                     if (one_col) {
                         *(uint2*)(crow + 4 * gi) = ov;
                     } else {
@@ -924,16 +958,16 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
                     }
                 }
                 __syncwarp();
-                dpos += (tot & 0xffffffu) << 2;
+                dpos += 4 * (tot & 0xffffu);
             }
             continue;
         }
-        uint32_t spos = P.sgpos + s_sgb[sidx];
-        for (uint32_t base = sg.g0; base < gend; base += 32) {
+        uint32_t spos = s_sgb[sidx];
+        for (uint32_t base = 0; base < n; base += 32) {
             const uint32_t g = base + lane;
-            const bool valid = g < gend;
-            const uint32_t v = valid ? gcl[B.gbase + g] : 0u;
-            const uint32_t np = v > L.t ? v - L.t : 0u;
+            const bool valid = g < n;
+            const uint32_t v = valid ? gcl[D.z + g] : 0u;
+            const uint32_t np = v > t ? v - t : 0u;
             const uint32_t len = 4 * np; /* separate signs: planes only */
             uint32_t tot;
             const uint32_t ex = warp_excl_scan(len, &tot);
@@ -943,7 +977,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
                 if (len) {
                     const uint32_t pos = dpos + ex;
                     const uint64_t win = ((uint64_t)bits32_at(pbuf, pos) << 32) | bits32_at(pbuf, pos + 32);
-                    nz = group_mags(win >> (64 - len), np, L.t, v, uniform, &A, &B2);
+                    nz = group_mags(win >> (64 - len), np, t, v, uniform, &A, &B2);
                 }
                 /* this group's sign bits follow those of the lanes before it */
                 uint32_t stot;
@@ -960,7 +994,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
                         }
                     }
                 }
-                if (len) o = group_finish(A, B2, sgn, uniform && L.t != 0, (int)B.w - 4 * (int)g);
+                if (len) o = group_finish(A, B2, sgn, uniform && t != 0, wend - 4 * (int)g);
                 spos += stot;
             }
             if (valid) {
@@ -969,7 +1003,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
                 } else {
                     /* a column starts anywhere in the row and ends where the
                      * next begins: the group's coefficients inside it only */
-                    const int wl = (int)B.w - 4 * (int)g;
+                    const int wl = wend - 4 * (int)g;
                     crow[4 * g] = (int16_t)(o.x & 0xffffu);
                     if (wl > 1) crow[4 * g + 1] = (int16_t)(o.x >> 16);
                     if (wl > 2) crow[4 * g + 2] = (int16_t)(o.y & 0xffffu);
@@ -980,7 +1014,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         }
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) JXS_STATUS_SET(status, JXS_E_DEC_BITSTREAM);
-    if (top_gcl) {
+    if (VP) {
         /* slice-ordered decoding: this row is the next one's row above */
         for (uint32_t i = threadIdx.x; i < (cap_groups >> 2); i += blockDim.x) ((uint32_t*)top_gcl)[i] = ((const uint32_t*)gcl)[i];
         for (uint32_t x = threadIdx.x; x < nbl; x += blockDim.x) top_t[x] = ln[x].t;
@@ -1073,20 +1107,23 @@ DEV void walk_sequential(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __res
 /* ------------------------------------------------------------------------ */
 /* 4 blocks of 512 threads per SM where the shared memory allows it (32
  * registers) */
+template <bool FS>
 __global__ void __launch_bounds__(UK_THREADS, 4) unpack_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs,
                                                                uint32_t bs_size, const uint32_t* __restrict__ prec_off,
                                                                int16_t* __restrict__ coef, uint32_t cap_bytes, uint32_t cap_groups,
                                                                uint32_t cap_seg, int* status) {
-    unpack_body(cfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status, (int)blockIdx.x, nullptr, nullptr, 0);
+    unpack_body<FS, false>(cfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status, (int)blockIdx.x, nullptr, nullptr,
+                           0);
 }
 
 /* cap_bytes / cap_groups / cap_seg: the largest of the batch's frames
  * (shared-memory layout of the launch) */
+template <bool FS>
 __global__ void __launch_bounds__(UK_THREADS, 4) unpack_batch_kernel(const __grid_constant__ DecPrecLaunch L, uint32_t cap_bytes,
                                                                      uint32_t cap_groups, uint32_t cap_seg) {
     const DecPrecFrame& F = L.job[find_job<JXS_BATCH_FRAMES>(L.job, L.nframes, (int)blockIdx.x)];
-    unpack_body(F.cfg, F.bs, F.bs_size, F.prec_off, F.coef, cap_bytes, cap_groups, cap_seg, F.status,
-                (int)blockIdx.x - F.first_block, nullptr, nullptr, 0);
+    unpack_body<FS, false>(F.cfg, F.bs, F.bs_size, F.prec_off, F.coef, cap_bytes, cap_groups, cap_seg, F.status,
+                           (int)blockIdx.x - F.first_block, nullptr, nullptr, 0);
 }
 
 /* Streams with vertical prediction: one block per slice, its precinct rows
@@ -1104,8 +1141,8 @@ __global__ void __launch_bounds__(UK_THREADS) unpack_vpred_kernel(const jxs_cfg_
     const uint32_t first = s * cfg->pps, end = min(cfg->np, first + cfg->pps);
     for (uint32_t col = 0; col < ncol; col++) {
         for (uint32_t row = first; row < end; row++) {
-            unpack_body(cfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status, (int)(row * ncol + col), top_gcl,
-                        top_t, row != first);
+            unpack_body<true, true>(cfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status, (int)(row * ncol + col),
+                                    top_gcl, top_t, row != first);
             __syncthreads();
             if (*(volatile int*)status) return;
         }
@@ -1154,17 +1191,23 @@ extern "C" cudaError_t jxs_launch_walk(const jxs_cfg_t* dcfg, uint32_t nslices, 
     return cudaGetLastError();
 }
 
-extern "C" cudaError_t jxs_launch_unpack(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t bs_size, const uint32_t* prec_off,
-                                         int16_t* coef, uint32_t np, uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg,
-                                         int* status, cudaStream_t st) {
+template <bool FS>
+static cudaError_t unpack_one(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t bs_size, const uint32_t* prec_off, int16_t* coef,
+                              uint32_t np, uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg, int* status, cudaStream_t st) {
     const size_t smem = uk_layout(cap_bytes, cap_groups, cap_seg).end;
     static std::atomic<int> attr[JXS_MAX_DEV];
-    cudaError_t e = jxs_smem_attr(unpack_kernel, (int)smem, attr);
+    cudaError_t e = jxs_smem_attr(unpack_kernel<FS>, (int)smem, attr);
     if (e != cudaSuccess) return e;
-    unpack_kernel<<<np, UK_THREADS, smem, st>>>(dcfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status);
+    unpack_kernel<FS><<<np, UK_THREADS, smem, st>>>(dcfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status);
     return cudaGetLastError();
 }
-
+/* fs: the frame has separate sign sub-packets (batch: some frame has) */
+extern "C" cudaError_t jxs_launch_unpack(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t bs_size, const uint32_t* prec_off,
+                                         int16_t* coef, uint32_t np, uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg,
+                                         int fs, int* status, cudaStream_t st) {
+    if (fs) return unpack_one<true>(dcfg, bs, bs_size, prec_off, coef, np, cap_bytes, cap_groups, cap_seg, status, st);
+    return unpack_one<false>(dcfg, bs, bs_size, prec_off, coef, np, cap_bytes, cap_groups, cap_seg, status, st);
+}
 
 extern "C" cudaError_t jxs_launch_walk_batch(const DecPrecLaunch* L, cudaStream_t st) {
     if (L->nframes <= 0) return cudaSuccess;
@@ -1173,15 +1216,20 @@ extern "C" cudaError_t jxs_launch_walk_batch(const DecPrecLaunch* L, cudaStream_
     return cudaGetLastError();
 }
 
-extern "C" cudaError_t jxs_launch_unpack_batch(const DecPrecLaunch* L, uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg,
-                                               cudaStream_t st) {
+template <bool FS>
+static cudaError_t unpack_batch_one(const DecPrecLaunch* L, uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg, cudaStream_t st) {
     const size_t smem = uk_layout(cap_bytes, cap_groups, cap_seg).end;
     static std::atomic<int> attr[JXS_MAX_DEV];
-    cudaError_t e = jxs_smem_attr(unpack_batch_kernel, (int)smem, attr);
+    cudaError_t e = jxs_smem_attr(unpack_batch_kernel<FS>, (int)smem, attr);
     if (e != cudaSuccess) return e;
     if (L->nblocks <= 0) return cudaSuccess;
-    unpack_batch_kernel<<<L->nblocks, UK_THREADS, smem, st>>>(*L, cap_bytes, cap_groups, cap_seg);
+    unpack_batch_kernel<FS><<<L->nblocks, UK_THREADS, smem, st>>>(*L, cap_bytes, cap_groups, cap_seg);
     return cudaGetLastError();
+}
+extern "C" cudaError_t jxs_launch_unpack_batch(const DecPrecLaunch* L, uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg,
+                                               int fs, cudaStream_t st) {
+    return fs ? unpack_batch_one<true>(L, cap_bytes, cap_groups, cap_seg, st)
+              : unpack_batch_one<false>(L, cap_bytes, cap_groups, cap_seg, st);
 }
 
 extern "C" cudaError_t jxs_launch_unpack_vpred(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t bs_size, const uint32_t* prec_off,

@@ -757,7 +757,7 @@ extern "C" jxs_gpu_dec_t* jxs_gpu_dec_create(const jxs_cfg_t* cfg, int nslots, i
     uint64_t cap = (uint64_t)cfg->lcod / (cfg->nslices ? cfg->nslices : 1);
     cap = cfg->max_slice_budget ? cfg->max_slice_budget + 64ull : cap + cap / 4 + 4096;
     if (cap > cfg->lcod + 64ull) cap = cfg->lcod + 64ull;
-    const size_t fixed = uk_layout(0, d->cap_groups, d->cap_seg).top_end;
+    const size_t fixed = uk_reserved(d->cap_groups, d->cap_seg, 1);
     const size_t room = kSmemMax - UK_STATIC_SMEM;
     if (cap + fixed > room) cap = room > fixed + 4096 ? room - fixed : 4096;
     d->cap_bytes = (uint32_t)(cap + 15) & ~15u;
@@ -838,8 +838,8 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
         CK(jxs_launch_unpack_vpred(d->dcfg, dbs, size, doff, s->coef, c->nslices, d->cap_bytes, d->cap_groups, d->cap_seg,
                                    s->status, st));
     else
-        CK(jxs_launch_unpack(d->dcfg, dbs, size, doff, s->coef, c->nprec, d->cap_bytes, d->cap_groups, d->cap_seg, s->status,
-                             st));
+        CK(jxs_launch_unpack(d->dcfg, dbs, size, doff, s->coef, c->nprec, d->cap_bytes, d->cap_groups, d->cap_seg, (int)c->fs,
+                             s->status, st));
     KMARK();
     TMARK(2);
 

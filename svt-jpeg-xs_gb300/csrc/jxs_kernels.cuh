@@ -236,37 +236,36 @@ struct DecPrecLaunch {
 
 /* Dynamic shared memory of the unpacking kernels (jxs_dec_kernels.cu), laid
  * out for the largest frame of a launch: the precinct's bytes (cap_bytes +
- * 32), a GCLI per group (cap_groups), the zero-bit table (a 16-bit offset per
- * zero: one per codeword plus up to 7 padding bits per packet), then the
- * per-segment arrays (cap_seg segments): the segment table, its work order,
- * counts, bases, block-wide sums and, for separate signs, sign counts and
- * first sign bits.  `end` is the size of one precinct's area; slice-ordered
- * decoding keeps the row above's GCLIs after it (top, cap_groups bytes). */
+ * 32), a GCLI per group (cap_groups), a byte per codeword (its value; one per
+ * zero bit of the unary codes: one per codeword plus up to 7 padding bits per
+ * packet), then the per-segment arrays (cap_seg segments): records, bases,
+ * block-wide sums, work order and, for separate signs, first sign bits.
+ * `end` is the size of one precinct's area; slice-ordered decoding keeps the
+ * row above's GCLIs after it (top, cap_groups bytes). */
 #define UK_ZCAP(cap_groups) ((cap_groups) + 8 * JXS_MAXPK + 32)
 /* 128 list entries per warp of a 512-thread unpacking block */
 #define UK_LIST_BYTES (4 * 128 * 16)
 struct UkLayout {
-    uint32_t gcl, zend, seg, cnt, base, ex, nz, sgb, ord, end, top, top_end;
+    uint32_t gcl, zval, desc, cnt, base, ex, sgb, ord, end, top, top_end;
 };
 static inline __host__ __device__ UkLayout uk_layout(uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg) {
     UkLayout L;
     uint32_t o = cap_bytes + 32;
     L.gcl = o;
     o = (o + cap_groups + 15) & ~15u;
-    L.zend = o;
-    /* the zero-bit table; in the data pass the same area holds each warp's
-     * list of groups with data (UK_LIST_BYTES) */
-    o = (o + (2 * UK_ZCAP(cap_groups) > UK_LIST_BYTES ? 2 * UK_ZCAP(cap_groups) : UK_LIST_BYTES) + 15) & ~15u;
-    L.seg = o;
-    o += 8 * cap_seg;
+    L.zval = o;
+    /* the codeword values (read 8 bytes at a time from any multiple of 4);
+     * in the data pass the same area holds each warp's list of groups with
+     * data (UK_LIST_BYTES) */
+    o = (o + (UK_ZCAP(cap_groups) + 8 > UK_LIST_BYTES ? UK_ZCAP(cap_groups) + 8 : UK_LIST_BYTES) + 15) & ~15u;
+    L.desc = o;
+    o += 16 * cap_seg;
     L.cnt = o;
     o += 4 * cap_seg;
     L.base = o;
     o += 4 * cap_seg;
     L.ex = o;
     o += 4 * (cap_seg + 1);
-    L.nz = o;
-    o += 4 * cap_seg;
     L.sgb = o;
     o += 4 * cap_seg;
     L.ord = o;
@@ -275,6 +274,18 @@ static inline __host__ __device__ UkLayout uk_layout(uint32_t cap_bytes, uint32_
     L.top = o;
     L.top_end = (o + cap_groups + 15) & ~15u;
     return L;
+}
+/* Shared memory set aside besides the precinct's bytes when a decoder fixes
+ * how long a precinct it takes (larger ones are invalid streams): at least
+ * that of the layout above, `ordered` with the row above's GCLIs. */
+static inline uint32_t uk_reserved(uint32_t cap_groups, uint32_t cap_seg, int ordered) {
+    uint32_t o = (32 + cap_groups + 15) & ~15u;
+    o = (o + (2 * UK_ZCAP(cap_groups) > UK_LIST_BYTES ? 2 * UK_ZCAP(cap_groups) : UK_LIST_BYTES) + 15) & ~15u;
+    o = (o + 30 * cap_seg + 4 + 15) & ~15u;
+    if (ordered) o = (o + cap_groups + 15) & ~15u;
+    const UkLayout L = uk_layout(0, cap_groups, cap_seg);
+    const uint32_t need = ordered ? L.top_end : L.end;
+    return o > need ? o : need;
 }
 /* Static shared memory of the unpacking kernels at most (the launchers size
  * the dynamic part against what is left of an SM's shared memory). */

@@ -34,9 +34,9 @@ extern "C" cudaError_t jxs_launch_pack(const jxs_cfg_t* dcfg, uint32_t np, const
 extern "C" cudaError_t jxs_launch_pack_batch(const EncPrecLaunch* L, uint32_t cap_words, int modes, cudaStream_t st);
 extern "C" cudaError_t jxs_launch_unpack(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t bs_size, const uint32_t* prec_off,
                                          int16_t* coef, uint32_t np, uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg,
-                                         int* status, cudaStream_t st);
+                                         int fs, int* status, cudaStream_t st);
 extern "C" cudaError_t jxs_launch_unpack_batch(const DecPrecLaunch* L, uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg,
-                                               cudaStream_t st);
+                                               int fs, cudaStream_t st);
 extern "C" cudaError_t jxs_launch_unpack_vpred(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t bs_size, const uint32_t* prec_off,
                                                int16_t* coef, uint32_t nslices, uint32_t cap_bytes, uint32_t cap_groups,
                                                uint32_t cap_seg, int* status, cudaStream_t st);
