@@ -255,35 +255,19 @@ DEV uint2 decode_group(uint64_t chunk, uint32_t np, uint32_t t, uint32_t gv, uin
     return group_finish(A, B, sgn, uniform && t != 0, wl);
 }
 
-/* The same under deadzone quantization, for a group inside its band line or
- * at its end (`wl` remaining coefficients): the sign nibble is transposed
- * with the planes, as the plane above the np magnitude planes, so that the
- * signs arrive as bit np of each coefficient. */
-DEV uint2 decode_group_dz(uint64_t chunk, uint32_t np, uint32_t t, int wl) {
-    const uint32_t tl = planes_to_coefs((uint32_t)chunk);
-    uint32_t P01 = __byte_perm(tl, 0u, 0x4243), P23 = __byte_perm(tl, 0u, 0x4041);
-    if (np >= 8) {
-        const uint32_t th = planes_to_coefs((uint32_t)(chunk >> 32));
-        P01 |= __byte_perm(th, 0u, 0x4243) << 8;
-        P23 |= __byte_perm(th, 0u, 0x4041) << 8;
-    }
-    /* signs to all-ones halves; magnitudes without them */
-    const uint32_t s01 = (P01 >> np) & 0x00010001u, s23 = (P23 >> np) & 0x00010001u;
-    const uint32_t n01 = s01 * 0xffffu, n23 = s23 * 0xffffu;
-    uint32_t a = (P01 ^ (s01 << np)) << t, b = (P23 ^ (s23 << np)) << t;
-    if (t > 0) {
-        /* deadzone reconstruction (Dequant.c:9-21): half a step on non-zero magnitudes */
-        const uint32_t half = (1u << (t - 1)) * 0x00010001u;
-        a |= __vcmpne2(a, 0u) & half;
-        b |= __vcmpne2(b, 0u) & half;
-    }
-    /* two's complement of the negative ones, two per word */
-    a = __vsub2(a ^ n01, n01);
-    b = __vsub2(b ^ n23, n23);
-    const uint32_t keepA = (wl > 1 ? 0xffff0000u : 0u) | 0xffffu, keepB = (wl > 2 ? 0xffffu : 0u) | (wl > 3 ? 0xffff0000u : 0u);
-    return make_uint2(a & keepA, b & keepB);
+/* Two coefficients of a group under deadzone quantization from their plane
+ * bits P (16-bit halves, the sign as bit np above the magnitude), without a
+ * comparison: `mag` has the np magnitude bits of both halves, `half` half a
+ * step, 2^(t-1) (0 for t = 0), in both.  Magnitudes stay below 2^15, so that
+ * adding 0x7fff sets bit 15 of the non-zero ones; a sign counts for those
+ * only. */
+DEV uint32_t dequant_pair(uint32_t P, uint32_t np, uint32_t t, uint32_t mag, uint32_t half) {
+    uint32_t a = (P & mag) << t;
+    const uint32_t u = a + 0x7fff7fffu;
+    a |= (u >> (16 - t)) & half; /* deadzone reconstruction (Dequant.c:9-21) */
+    const uint32_t neg = (P >> np) & (u >> 15) & 0x00010001u;
+    return (a ^ (neg * 0xffffu)) + neg; /* two's complement (Precinct.c:9-14) */
 }
-
 /* unpack_precinct (Packing.c:513-868) for one precinct.  FS: the launch may
  * hold frames with separate sign sub-packets; VP: slice-ordered decoding,
  * which resolves vertical prediction (otherwise a precinct with predicted
@@ -671,13 +655,15 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
             uint32_t z = ~bits32_at(pbuf, at);
             if (valid < 32) z &= ~(0xffffffffu >> valid);
             const uint32_t tail = z ? (uint32_t)__ffs((int)z) - 1 : min(ones + 32u, 64u);
-            while (z) {
+            const uint32_t nz = __popc(z);
+            uint8_t* o = zval + z0;
+            for (uint32_t k2 = z0 < zcap ? min(nz, zcap - z0) : 0u; k2; k2--) {
                 const uint32_t run = __clz((int)z);
-                if (z0 < zcap) zval[z0] = (uint8_t)(ones + run);
-                z0++;
+                *o++ = (uint8_t)(ones + run);
                 ones = 0;
                 z = shl_or_0(z, run + 1);
             }
+            z0 += nz;
             ones = tail;
         }
     }
@@ -942,11 +928,32 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
                     const int wl = wend - 4 * (int)gi;
                     const uint32_t win = bits32_at(pbuf, pos);
                     uint2 ov;
-                    if (np < 8 && !uniform) {
-                        ov = decode_group_dz(win >> (28 - 4 * np), np, t, wl);
-                    } else {
+                    if (uniform) {
                         const uint64_t w2 = (((uint64_t)win << 32) | bits32_at(pbuf, pos + 32)) >> (60 - 4 * np);
-                        ov = uniform ? decode_group(w2, np, t, v, uniform, wl) : decode_group_dz(w2, np, t, wl);
+                        ov = decode_group(w2, np, t, v, uniform, wl);
+                    } else {
+                        /* the sign nibble is transposed with the planes, as the
+                         * plane above the np magnitude planes, 8 at a time; the
+                         * upper ones only where the warp has a group with more
+                         * than 7 planes.  Coefficients past the band width come
+                         * out as the stream has them: they go to the row's
+                         * padding, or nowhere */
+                        const uint32_t more = np >= 8 ? 4 * np - 28 : 0u; /* bits past the first 32 */
+                        uint32_t low = np >= 8 ? win : win >> ((28 - 4 * np) & 31), high = 0u;
+                        const bool any8 = __any_sync(__activemask(), np >= 8);
+                        if (any8) {
+                            low = __funnelshift_lc(bits32_at(pbuf, pos + 32), low, more);
+                            high = more ? win >> (32 - more) : 0u;
+                        }
+                        const uint32_t tl = planes_to_coefs(low);
+                        uint32_t P01 = __byte_perm(tl, 0u, 0x4243), P23 = __byte_perm(tl, 0u, 0x4041);
+                        if (any8) {
+                            const uint32_t th = planes_to_coefs(high);
+                            P01 |= __byte_perm(th, 0u, 0x2434);
+                            P23 |= __byte_perm(th, 0u, 0x0414);
+                        }
+                        const uint32_t mag = ((1u << np) - 1u) * 0x00010001u, half = ((1u << t) >> 1) * 0x00010001u;
+                        ov = make_uint2(dequant_pair(P01, np, t, mag, half), dequant_pair(P23, np, t, mag, half));
                     }
                     if (one_col) {
                         *(uint2*)(crow + 4 * gi) = ov;

@@ -1707,10 +1707,27 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
                     const uint2 raw4 = *(const uint2*)(crow + 4 * gi);
                     uint32_t P01, P23;
                     quantize_signed(raw4, e & 15u, t, uq, P01, P23);
+                    /* up to 8 planes with the sign's in one word, left-aligned;
+                     * the upper ones only where the warp has a group with more */
                     const uint32_t low = coefs_to_planes(__byte_perm(P01, P23, 0x0246));
-                    if (np < 8) put_left32(buf, pos, low << (28 - 4 * np));
-                    else
-                        put_bits(buf, words, pos, (uint64_t)coefs_to_planes(__byte_perm(P01, P23, 0x1357)) << 32 | low, 4 * (np + 1), ovf);
+                    const uint32_t w = pos >> 5, sh = pos & 31;
+                    uint32_t hi = low << ((28 - 4 * np) & 31);
+                    if (__any_sync(__activemask(), np >= 8)) {
+                        const uint32_t high = coefs_to_planes(__byte_perm(P01, P23, 0x1357));
+                        uint32_t lo = 0u;
+                        if (np >= 8) {
+                            hi = __funnelshift_l(low, high, 60 - 4 * np); /* 4 (np + 1) bits of high : low */
+                            lo = low << (60 - 4 * np);
+                        }
+                        const uint32_t w2 = __funnelshift_r(0u, lo, sh);
+                        if (w2) atomicOr(&buf[w + 2], w2);
+                        const uint32_t w1 = __funnelshift_r(lo, hi, sh);
+                        if (w1) atomicOr(&buf[w + 1], w1);
+                    } else {
+                        const uint32_t w1 = __funnelshift_r(0u, hi, sh);
+                        if (w1) atomicOr(&buf[w + 1], w1);
+                    }
+                    atomicOr(&buf[w], hi >> sh);
                 }
                 __syncwarp();
                 vpos += tot_v;
