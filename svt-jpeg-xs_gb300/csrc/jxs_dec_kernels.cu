@@ -271,7 +271,8 @@ DEV uint32_t dequant_pair(uint32_t P, uint32_t np, uint32_t t, uint32_t mag, uin
 /* unpack_precinct (Packing.c:513-868) for one precinct.  FS: the launch may
  * hold frames with separate sign sub-packets; VP: slice-ordered decoding,
  * which resolves vertical prediction (otherwise a precinct with predicted
- * bands reports JXS_E_DEC_VPRED); both compiled out otherwise.
+ * bands reports JXS_E_DEC_VPRED); both compiled out otherwise.  BATCH: a
+ * launch of many frames.
  *
  * Dynamic shared memory: see uk_layout.
  *
@@ -293,7 +294,7 @@ DEV uint32_t dequant_pair(uint32_t P, uint32_t np, uint32_t t, uint32_t mag, uin
  * each, instead of by every warp that takes one; codeword values are read 4
  * at a time instead of 5 zero positions; bytes are swapped once.  8 4K 4:2:2
  * 10-bit frames: 263 us before, UNPACK_US us now. */
-template <bool FS, bool VP>
+template <bool FS, bool VP, bool BATCH>
 __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t bs_size,
                                             const uint32_t* __restrict__ prec_off, int16_t* __restrict__ coef,
                                             uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg, int* status, const int p,
@@ -339,17 +340,39 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
     const uint32_t prow = (uint32_t)p / cfg->ncol, pcol = (uint32_t)p - prow * cfg->ncol;
     const int one_col = cfg->ncol == 1;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    /* thread 0: the frame's status and the precinct's length field; every
-     * thread meanwhile stages this precinct kind's tables and the scalars
-     * the parse needs, so that no single-warp phase waits on device memory */
+    /* the frame's status and the precinct's length field, by a warp that has
+     * little to stage */
+    auto begin = [&]() {
+        if (threadIdx.x == UK_THREADS - 32) {
+            /* the precinct's offset and length field are read in bounds before
+             * the frame status, so that the three loads do not wait in turn */
+            const uint32_t off = prec_off[p], phb = cfg->prec_hdr_bytes;
+            s_off = off; /* read once: the offsets may be in host memory */
+            const bool inb = (uint64_t)off + phb <= bs_size;
+            const uint32_t lprc = inb ? ((uint32_t)bs[off] << 16) | ((uint32_t)bs[off + 1] << 8) | bs[off + 2] : 0u;
+            int err = *(volatile int*)status; /* set: the precinct offsets could not be found */
+            if (!err) {
+                if (!inb) {
+                    err = JXS_E_DEC_SHORT;
+                } else {
+                    s_total = phb + lprc;
+                    s_lead = (uint32_t)((uintptr_t)(bs + off) & 15);
+                    if (lprc > JXS_PREC_MAX_BYTES || s_total + 48 > cap_bytes) err = JXS_E_DEC_BITSTREAM;
+                    else if ((uint64_t)off + s_total > bs_size) err = JXS_E_DEC_SHORT;
+                }
+                if (err) JXS_STATUS_SET(status, err);
+            } else {
+                err = -1; /* already reported */
+            }
+            s_err = err;
+        }
+    };
+    /* BATCH: an ordinary launch, these first; else the tables first, which need
+     * not wait for the kernel before */
+    if (BATCH) begin();
+    /* every thread stages this precinct kind's tables and the scalars the
+     * parse needs, so that no single-warp phase waits on device memory */
     if (threadIdx.x == 0) {
-        /* the precinct's offset and length field are read in bounds before
-         * the frame status, so that the three loads do not wait in turn */
-        const uint32_t off = prec_off[p], phb = cfg->prec_hdr_bytes;
-        s_off = off; /* read once: the offsets may be in host memory */
-        const bool inb = (uint64_t)off + phb <= bs_size;
-        const uint32_t lprc = inb ? ((uint32_t)bs[off] << 16) | ((uint32_t)bs[off + 1] << 8) | bs[off + 2] : 0u;
-        int err = *(volatile int*)status; /* set: the precinct offsets could not be found */
         s_sc[0] = cfg->nbands_all;
         s_sc[1] = cfg->npk;
         s_sc[2] = cfg->lh || !cfg->short_hdr;
@@ -360,20 +383,6 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         s_sc[7] = cfg->seg_groups;
         s_sc[8] = cfg->rm;
         s_hasvp = 0;
-        if (!err) {
-            if (!inb) {
-                err = JXS_E_DEC_SHORT;
-            } else {
-                s_total = phb + lprc;
-                s_lead = (uint32_t)((uintptr_t)(bs + off) & 15);
-                if (lprc > JXS_PREC_MAX_BYTES || s_total + 48 > cap_bytes) err = JXS_E_DEC_BITSTREAM;
-                else if ((uint64_t)off + s_total > bs_size) err = JXS_E_DEC_SHORT;
-            }
-            if (err) JXS_STATUS_SET(status, err);
-        } else {
-            err = -1; /* already reported */
-        }
-        s_err = err;
     }
     if (threadIdx.x < 2) s_next[threadIdx.x] = 0;
     jxs_seg_t myseg; /* thread i: segment i */
@@ -404,6 +413,11 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
             s_pknbl[k] = cfg->pk_nbl[last][k];
         }
         for (uint32_t gb = threadIdx.x; gb < cfg->nbands_all; gb += blockDim.x) s_g2f[gb] = cfg->g2f[gb];
+    }
+    /* up to here configuration only */
+    if (!BATCH) {
+        dep_wait();
+        begin();
     }
     __syncthreads();
     if (s_err) return;
@@ -1119,7 +1133,7 @@ __global__ void __launch_bounds__(UK_THREADS, 4) unpack_kernel(const jxs_cfg_t* 
                                                                uint32_t bs_size, const uint32_t* __restrict__ prec_off,
                                                                int16_t* __restrict__ coef, uint32_t cap_bytes, uint32_t cap_groups,
                                                                uint32_t cap_seg, int* status) {
-    unpack_body<FS, false>(cfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status, (int)blockIdx.x, nullptr, nullptr,
+    unpack_body<FS, false, false>(cfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status, (int)blockIdx.x, nullptr, nullptr,
                            0);
 }
 
@@ -1129,7 +1143,7 @@ template <bool FS>
 __global__ void __launch_bounds__(UK_THREADS, 4) unpack_batch_kernel(const __grid_constant__ DecPrecLaunch L, uint32_t cap_bytes,
                                                                      uint32_t cap_groups, uint32_t cap_seg) {
     const DecPrecFrame& F = L.job[find_job<JXS_BATCH_FRAMES>(L.job, L.nframes, (int)blockIdx.x)];
-    unpack_body<FS, false>(F.cfg, F.bs, F.bs_size, F.prec_off, F.coef, cap_bytes, cap_groups, cap_seg, F.status,
+    unpack_body<FS, false, true>(F.cfg, F.bs, F.bs_size, F.prec_off, F.coef, cap_bytes, cap_groups, cap_seg, F.status,
                            (int)blockIdx.x - F.first_block, nullptr, nullptr, 0);
 }
 
@@ -1148,7 +1162,7 @@ __global__ void __launch_bounds__(UK_THREADS) unpack_vpred_kernel(const jxs_cfg_
     const uint32_t first = s * cfg->pps, end = min(cfg->np, first + cfg->pps);
     for (uint32_t col = 0; col < ncol; col++) {
         for (uint32_t row = first; row < end; row++) {
-            unpack_body<true, true>(cfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status, (int)(row * ncol + col),
+            unpack_body<true, true, false>(cfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status, (int)(row * ncol + col),
                                     top_gcl, top_t, row != first);
             __syncthreads();
             if (*(volatile int*)status) return;
@@ -1158,11 +1172,13 @@ __global__ void __launch_bounds__(UK_THREADS) unpack_vpred_kernel(const jxs_cfg_
 
 __global__ void walk_slices_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size,
                                    uint32_t* __restrict__ prec_off, int* walk_bad) {
+    dep_wait();
     walk_slice(cfg, bs, size, prec_off, walk_bad, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 __global__ void walk_sequential_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size,
                                        uint32_t* __restrict__ prec_off, const int* walk_bad, int* status) {
+    dep_wait();
     walk_sequential(cfg, bs, size, prec_off, walk_bad, status);
 }
 
@@ -1193,9 +1209,9 @@ __global__ void walk_sequential_batch_kernel(const __grid_constant__ DecPrecLaun
 /* ------------------------------------------------------------------------ */
 extern "C" cudaError_t jxs_launch_walk(const jxs_cfg_t* dcfg, uint32_t nslices, const uint8_t* bs, uint32_t size, uint32_t* prec_off,
                                        int* walk_bad, int* status, cudaStream_t st) {
-    walk_slices_kernel<<<(nslices + 127) / 128, 128, 0, st>>>(dcfg, bs, size, prec_off, walk_bad);
-    walk_sequential_kernel<<<1, 1, 0, st>>>(dcfg, bs, size, prec_off, walk_bad, status);
-    return cudaGetLastError();
+    const cudaError_t e = jxs_launch(walk_slices_kernel, dim3((nslices + 127) / 128), 128, 0, st, dcfg, bs, size, prec_off, walk_bad);
+    if (e != cudaSuccess) return e;
+    return jxs_launch(walk_sequential_kernel, dim3(1), 1, 0, st, dcfg, bs, size, prec_off, walk_bad, status);
 }
 
 template <bool FS>
@@ -1205,8 +1221,8 @@ static cudaError_t unpack_one(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t
     static std::atomic<int> attr[JXS_MAX_DEV];
     cudaError_t e = jxs_smem_attr(unpack_kernel<FS>, (int)smem, attr);
     if (e != cudaSuccess) return e;
-    unpack_kernel<FS><<<np, UK_THREADS, smem, st>>>(dcfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status);
-    return cudaGetLastError();
+    return jxs_launch(unpack_kernel<FS>, dim3(np), UK_THREADS, smem, st, dcfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups,
+                      cap_seg, status);
 }
 /* fs: the frame has separate sign sub-packets (batch: some frame has) */
 extern "C" cudaError_t jxs_launch_unpack(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t bs_size, const uint32_t* prec_off,
@@ -1246,7 +1262,6 @@ extern "C" cudaError_t jxs_launch_unpack_vpred(const jxs_cfg_t* dcfg, const uint
     static std::atomic<int> attr[JXS_MAX_DEV];
     cudaError_t e = jxs_smem_attr(unpack_vpred_kernel, (int)smem, attr);
     if (e != cudaSuccess) return e;
-    unpack_vpred_kernel<<<nslices, UK_THREADS, smem, st>>>(dcfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg,
+    return jxs_launch(unpack_vpred_kernel, dim3((unsigned)nslices), UK_THREADS, smem, st, dcfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg,
                                                            status);
-    return cudaGetLastError();
 }

@@ -720,6 +720,7 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
         const jxs_band_t& bd = cfg->band[B.fb];
         s_grow[x] = bd.gcli_off + (uint64_t)(p * bd.lines + B.line) * bd.gpitch;
     }
+    dep_wait(); /* up to here configuration only */
     __syncthreads();
 
     /* histograms: each lane 4 consecutive groups (one 4-byte load) in 4-bit
@@ -1170,14 +1171,14 @@ struct PkSeg {
  *           gtli listed per warp, each lane then packing one listed group's
  *           data bits; everything OR-ed into the buffer.
  * SIGNS: the launch may hold frames with sign handling; VPRED: with vertical
- * prediction (both compiled out otherwise).  With vertical prediction a
+ * prediction (both compiled out otherwise); BATCH: a launch of many frames.  With vertical prediction a
  * precinct row below another of its slice also sums, per segment, the
  * codes of its GCLIs predicted from the line above at its gtli (line 0:
  * from the row above, with that row's gtli) and the groups that need no
  * code; the layout chooses among the four codings per band like the rate
  * control (RateControl.c:526-676), and pass B writes the prediction codes
  * (pack_bitplane_count_vpred_*, PackPrecinct.c:47-74). */
-template <bool SIGNS, bool VPRED>
+template <bool SIGNS, bool VPRED, bool BATCH>
 __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, const uint16_t* __restrict__ coef,
                                           const uint8_t* __restrict__ gcli, const PrecRC* __restrict__ rc,
                                           const uint32_t* __restrict__ cost, uint8_t* __restrict__ out, uint32_t cap_words,
@@ -1211,6 +1212,7 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
     __shared__ uint64_t s_grow[JXS_MAXBLINES], s_crow[JXS_MAXBLINES]; /* per line: GCLI / coefficient row offsets */
     __shared__ uint32_t s_sigp[JXS_MAXBLINES];                         /* per line: bit position of its significance flags */
     __shared__ uint8_t s_lt[JXS_MAXBLINES];                            /* per line: gtli */
+    __shared__ uint16_t s_lgp[BATCH ? 1 : JXS_MAXBLINES];              /* per line: band gain | priority << 8 */
     __shared__ uint8_t s_pkbl0[JXS_MAXPK], s_pknbl[JXS_MAXPK];
     __shared__ uint32_t s_praw[JXS_MAXPK];
     __shared__ uint8_t s_g2f[JXS_MAXBL];                               /* global band -> flat band */
@@ -1221,54 +1223,60 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
     __shared__ int s_ok;
 
     const int last = (p + 1 >= (int)cfg->np);
-    const PrecRC R = rc[p];
-    /* nothing to pack once the rate control failed somewhere in the frame;
-     * the flag is read once so that the whole block takes the same branch */
-    if (threadIdx.x == 0) s_ok = *(volatile int*)status == 0;
-    __syncthreads();
-    if (!s_ok) return;
-    const uint32_t total = R.total_bytes;
-    const uint32_t lead = (uint32_t)((uintptr_t)(out + R.offset) & 15);
-    const uint32_t words = ((lead + total + 15) >> 4) << 2;
-    if (words > cap_words) {
-        if (threadIdx.x == 0) {
-            printf("jxs pack: precinct %d needs %u words, buffer holds %u\n", p, words, cap_words);
-            JXS_STATUS_SET(status, JXS_E_ENC_FRAME);
-        }
-        return;
-    }
-    int ovf = 0;
-    for (uint32_t i = threadIdx.x; i < words >> 2; i += blockDim.x) ((uint4*)buf)[i] = make_uint4(0u, 0u, 0u, 0u);
-    for (uint32_t fb = threadIdx.x; fb < cfg->nbands; fb += blockDim.x) {
-        s_cn[fb] = 0;
-        s_cs[fb] = 0;
-        if (VPRED) {
-            s_cv[fb] = 0;
-            s_cvs[fb] = 0;
-        }
-    }
-    /* vertical prediction applies below the first row of a slice */
-    const int vp = VPRED && cfg->vpred && !R.first_in_slice;
+    const uint32_t nbl = cfg->nbline[last];
+    PrecRC R;
+    uint32_t total = 0, lead = 0, words = 0;
+    int ovf = 0, vp = 0;
     const int rmode = VPRED ? (int)cfg->rm : 0;
+    /* the precinct's record and the buffer's size; false: nothing to pack */
+    auto begin = [&]() {
+        R = rc[p];
+        /* nothing to pack once the rate control failed somewhere in the
+         * frame; the flag is read once so that the whole block takes the same
+         * branch */
+        if (threadIdx.x == 0) s_ok = *(volatile int*)status == 0;
+        __syncthreads();
+        if (!s_ok) return false;
+        total = R.total_bytes;
+        lead = (uint32_t)((uintptr_t)(out + R.offset) & 15);
+        words = ((lead + total + 15) >> 4) << 2;
+        if (words > cap_words) {
+            if (threadIdx.x == 0) {
+                printf("jxs pack: precinct %d needs %u words, buffer holds %u\n", p, words, cap_words);
+                JXS_STATUS_SET(status, JXS_E_ENC_FRAME);
+            }
+            return false;
+        }
+        for (uint32_t i = threadIdx.x; i < words >> 2; i += blockDim.x) ((uint4*)buf)[i] = make_uint4(0u, 0u, 0u, 0u);
+        /* vertical prediction applies below the first row of a slice */
+        vp = VPRED && cfg->vpred && !R.first_in_slice;
+        return true;
+    };
+    /* a line's gtli, and that of the line above where it is in the row above */
+    auto line_gtli = [&](uint32_t x, uint8_t gain, uint8_t prio, uint32_t line) {
+        s_lt[x] = jxs_truncation(gain, prio, R.q, R.r);
+        if (VPRED) s_gtt[x] = (int8_t)(vp && line == 0 ? jxs_truncation(gain, prio, rc[p - 1].q, rc[p - 1].r) : -1);
+    };
+    /* BATCH: an ordinary launch, the record first; else the tables first, and
+     * the record once the rate control is done */
+    if (BATCH && !begin()) return;
     {
-        const uint32_t ns = cfg->nseg[last], nl = cfg->nbline[last];
+        const uint32_t ns = cfg->nseg[last];
         for (uint32_t i = threadIdx.x; i < ns * (sizeof(jxs_seg_t) / 4); i += blockDim.x)
             ((uint32_t*)s_seg)[i] = ((const uint32_t*)cfg->seg[last])[i];
-        for (uint32_t i = threadIdx.x; i < nl * (sizeof(jxs_bline_t) / 4); i += blockDim.x)
+        for (uint32_t i = threadIdx.x; i < nbl * (sizeof(jxs_bline_t) / 4); i += blockDim.x)
             ((uint32_t*)s_bl)[i] = ((const uint32_t*)cfg->bline[last])[i];
         for (uint32_t i = threadIdx.x; i < ns; i += blockDim.x) s_ord[i] = cfg->seg_ord[last][i];
         if (threadIdx.x < 2) s_q[threadIdx.x] = 0;
-        for (uint32_t x = threadIdx.x; x < nl; x += blockDim.x) {
+        for (uint32_t x = threadIdx.x; x < nbl; x += blockDim.x) {
             const jxs_bline_t& B = cfg->bline[last][x];
             const jxs_band_t& bd = cfg->band[B.fb];
             const uint64_t row = (uint64_t)(p * bd.lines + B.line);
             s_grow[x] = bd.gcli_off + row * bd.gpitch;
             s_crow[x] = bd.coef_off + row * bd.pitch;
-            s_lt[x] = jxs_truncation(bd.gain, bd.prio, R.q, R.r);
-            if (VPRED) {
-                s_gp[x] = bd.gpitch;
-                s_gtt[x] = (int8_t)(vp && B.line == 0 ? jxs_truncation(bd.gain, bd.prio, rc[p - 1].q, rc[p - 1].r) : -1);
-            }
+            if (BATCH) line_gtli(x, bd.gain, bd.prio, B.line);
+            else s_lgp[x] = (uint16_t)(bd.gain | (bd.prio << 8));
+            if (VPRED) s_gp[x] = bd.gpitch;
         }
         for (uint32_t k = threadIdx.x; k < cfg->npk; k += blockDim.x) {
             s_pkbl0[k] = cfg->pk_bl0[last][k];
@@ -1276,8 +1284,15 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
             s_praw[k] = cfg->raw_bytes[last][k];
         }
         for (uint32_t gb = threadIdx.x; gb < cfg->nbands_all; gb += blockDim.x) s_g2f[gb] = cfg->g2f[gb];
-        for (uint32_t fb = threadIdx.x; fb < cfg->nbands; fb += blockDim.x)
+        for (uint32_t fb = threadIdx.x; fb < cfg->nbands; fb += blockDim.x) {
             s_blines[fb] = (uint8_t)(last ? cfg->band[fb].last_lines : cfg->band[fb].lines);
+            s_cn[fb] = 0;
+            s_cs[fb] = 0;
+            if (VPRED) {
+                s_cv[fb] = 0;
+                s_cvs[fb] = 0;
+            }
+        }
     }
     if (threadIdx.x == 0) {
         s_nbands = cfg->nbands;
@@ -1287,7 +1302,13 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
         s_short = cfg->short_hdr;
         s_phb = cfg->prec_hdr_bytes;
         s_hdrs = cfg->hdrs_bytes[last];
-        s_nbl = cfg->nbline[last];
+        s_nbl = nbl;
+    }
+    if (!BATCH) {
+        dep_wait(); /* up to here configuration only */
+        if (!begin()) return;
+        for (uint32_t x = threadIdx.x; x < nbl; x += blockDim.x)
+            line_gtli(x, (uint8_t)(s_lgp[x] & 255u), (uint8_t)(s_lgp[x] >> 8), s_bl[x].line);
     }
     __syncthreads();
 
@@ -2010,13 +2031,13 @@ __global__ void __launch_bounds__(PK_THREADS, 4) pack_kernel(const jxs_cfg_t* __
                                                           const uint8_t* __restrict__ gcli, const PrecRC* __restrict__ rc,
                                                           const uint32_t* __restrict__ cost, uint8_t* __restrict__ out,
                                                           uint32_t cap_words, int* status) {
-    pack_body<SIGNS, VPRED>(cfg, coef, gcli, rc, cost, out, cap_words, status, (int)blockIdx.x);
+    pack_body<SIGNS, VPRED, false>(cfg, coef, gcli, rc, cost, out, cap_words, status, (int)blockIdx.x);
 }
 
 template <bool SIGNS, bool VPRED>
 __global__ void __launch_bounds__(PK_THREADS, 4) pack_batch_kernel(const __grid_constant__ EncPrecLaunch L, uint32_t cap_words) {
     const EncPrecFrame& F = L.job[find_job<JXS_BATCH_FRAMES>(L.job, L.nframes, (int)blockIdx.x)];
-    pack_body<SIGNS, VPRED>(F.cfg, F.coef, F.gcli, F.rc, F.cost, F.out, cap_words, F.status, (int)blockIdx.x - F.first_block);
+    pack_body<SIGNS, VPRED, true>(F.cfg, F.coef, F.gcli, F.rc, F.cost, F.out, cap_words, F.status, (int)blockIdx.x - F.first_block);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -2034,8 +2055,7 @@ static cudaError_t rc_one(const jxs_cfg_t* dcfg, uint32_t np, const uint8_t* gcl
         cudaError_t e = jxs_smem_attr(rc_cost_kernel<S, V>, RC_VP_SMEM, attr);
         if (e != cudaSuccess) return e;
     }
-    rc_cost_kernel<S, V><<<np, RC_THREADS, V ? RC_VP_SMEM : 0, st>>>(dcfg, gcli, coef, cost, slice_done, rc, status);
-    return cudaGetLastError();
+    return jxs_launch(rc_cost_kernel<S, V>, dim3(np), RC_THREADS, V ? RC_VP_SMEM : 0, st, dcfg, gcli, coef, cost, slice_done, rc, status);
 }
 template <bool S, bool V>
 static cudaError_t rc_batch_one(const EncPrecLaunch* L, cudaStream_t st) {
@@ -2067,8 +2087,7 @@ static cudaError_t pack_one(const jxs_cfg_t* dcfg, uint32_t np, const uint16_t* 
     static std::atomic<int> attr[JXS_MAX_DEV];
     cudaError_t e = jxs_smem_attr(pack_kernel<S, V>, (int)smem, attr);
     if (e != cudaSuccess) return e;
-    pack_kernel<S, V><<<np, PK_THREADS, smem, st>>>(dcfg, coef, gcli, rc, cost, out, cap_words, status);
-    return cudaGetLastError();
+    return jxs_launch(pack_kernel<S, V>, dim3(np), PK_THREADS, smem, st, dcfg, coef, gcli, rc, cost, out, cap_words, status);
 }
 
 /* `modes` as for the rate control */

@@ -559,6 +559,7 @@ DEV void fv_strip(const FwdVJob& J, int r0, int rend, int c0) {
 
 template <int SRC, int NJ>
 __global__ void __launch_bounds__(32, SRC == SRC_I32 ? 28 : 32) fwd_v_kernel(const __grid_constant__ FwdVLaunchN<NJ> L) {
+    if (NJ <= JXS_MAXC) dep_wait();
     const FwdVJob& J = L.job[find_job<NJ>(L.job, L.njobs, (int)blockIdx.x)];
     const int u = blockIdx.x - J.first_block;
     const int ty = u / J.col_tiles, tx = u - ty * J.col_tiles;
@@ -687,6 +688,7 @@ DEV void fh_chunk(const FwdHJob& J, int row, int c0, bool out_lane) {
 
 template <int SRC, int NJ>
 __global__ void __launch_bounds__(FH_MAX_WARPS * 32) fwd_h_kernel(const __grid_constant__ FwdHLaunchN<NJ> L) {
+    if (NJ <= JXS_MAXC) dep_wait();
     const FwdHJob& J = L.job[find_job<NJ>(L.job, L.njobs, (int)blockIdx.x)];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int unit = (blockIdx.x - J.first_block) * L.rows_per_block + warp;
@@ -710,8 +712,11 @@ template <int SRC, int NJ>
 static cudaError_t launch_v(const FwdVLaunchN<NJ>* L, int grid_per_sm, cudaStream_t st) {
     (void)grid_per_sm; /* one block per tile */
     if (L->ntiles <= 0) return cudaSuccess;
-    fwd_v_kernel<SRC, NJ><<<L->ntiles, 32, 0, st>>>(*L);
-    return cudaGetLastError();
+    if (NJ > JXS_MAXC) {
+        fwd_v_kernel<SRC, NJ><<<L->ntiles, 32, 0, st>>>(*L);
+        return cudaGetLastError();
+    }
+    return jxs_launch(fwd_v_kernel<SRC, NJ>, dim3((unsigned)L->ntiles), (unsigned)(32), 0, st, *L);
 }
 
 template <int NJ>
@@ -735,8 +740,11 @@ extern "C" cudaError_t jxs_launch_fwd_v_batch(const FwdVLaunchB* L, int src_kind
 template <int SRC, int NJ>
 static cudaError_t launch_h(const FwdHLaunchN<NJ>* L, int nblocks, cudaStream_t st) {
     if (nblocks <= 0) return cudaSuccess;
-    fwd_h_kernel<SRC, NJ><<<nblocks, L->rows_per_block * 32, 0, st>>>(*L);
-    return cudaGetLastError();
+    if (NJ > JXS_MAXC) {
+        fwd_h_kernel<SRC, NJ><<<nblocks, L->rows_per_block * 32, 0, st>>>(*L);
+        return cudaGetLastError();
+    }
+    return jxs_launch(fwd_h_kernel<SRC, NJ>, dim3((unsigned)nblocks), (unsigned)(L->rows_per_block * 32), 0, st, *L);
 }
 
 template <int NJ>

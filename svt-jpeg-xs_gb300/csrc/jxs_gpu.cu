@@ -74,6 +74,7 @@ extern "C" int jxs_gpu_is_page_locked(const void* p) {
  * after the frame's last compute kernel: no 4-byte copy waits in the copy
  * engines' queues between the frames' large transfers. */
 __global__ void publish_status_kernel(int* __restrict__ host, const int* __restrict__ status) {
+    dep_wait();
     if (threadIdx.x == 0) *(volatile int*)host = *(const volatile int*)status;
 }
 
@@ -475,8 +476,7 @@ static int32_t enc_run(jxs_gpu_enc_t* e, EncSlot* s, void* const planes[4], cons
     CK(jxs_launch_pack(e->dcfg, c->np, s->coef, s->gcli, s->rc, s->cost, dst, e->cap_words, s->status,
                        (c->fs ? 1 : 0) | (c->vpred ? 2 : 0), st));
     KMARK();
-    publish_status_kernel<<<1, 32, 0, st>>>(s->status_hd, s->status);
-    CK(cudaGetLastError());
+    CK(jxs_launch(publish_status_kernel, dim3(1), 32, 0, st, s->status_hd, s->status));
     TMARK(4);
     s->ndefer = 0;
     if (!out_dev) {
@@ -923,8 +923,7 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
         nlt_out_params(c, tin, out, &P);
         CK(jxs_launch_nlt_out(&P, st));
     }
-    publish_status_kernel<<<1, 32, 0, st>>>(s->status_hd, s->status);
-    CK(cudaGetLastError());
+    CK(jxs_launch(publish_status_kernel, dim3(1), 32, 0, st, s->status_hd, s->status));
     TMARK(3);
     s->ndefer = 0;
     for (uint32_t k = 0; k < c->nc; k++) {

@@ -247,6 +247,7 @@ DEV void ih_chunk(const InvHJob& J, int row, int c0, bool out_lane, const OutSca
 
 template <int OUT, int NJ>
 __global__ void __launch_bounds__(IH_MAX_WARPS * 32) inv_h_kernel(const __grid_constant__ InvHLaunchN<NJ> L) {
+    if (NJ <= JXS_MAXC) dep_wait();
     const InvHJob& J = L.job[find_job<NJ>(L.job, L.njobs, (int)blockIdx.x)];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int unit = (blockIdx.x - J.first_block) * L.rows_per_block + warp;
@@ -570,6 +571,7 @@ DEV void iv_strip_any(const InvVJob& J, int r0, int rend, int c0) {
 
 template <int OUT, int NJ>
 __global__ void __launch_bounds__(32, 24) inv_v_kernel(const __grid_constant__ InvVLaunchN<NJ> L) {
+    if (NJ <= JXS_MAXC) dep_wait();
     const InvVJob& J = L.job[find_job<NJ>(L.job, L.njobs, (int)blockIdx.x)];
     const int t = blockIdx.x - J.first_block;
     const int ty = t / J.col_tiles, tx = t - ty * J.col_tiles;
@@ -604,8 +606,11 @@ extern "C" int jxs_inv_h_chunk_cols(int nh) { return ih_net_cols(nh); }
 template <int OUT, int NJ>
 static cudaError_t launch_iv(const InvVLaunchN<NJ>* L, int nblocks, cudaStream_t st) {
     if (nblocks <= 0) return cudaSuccess;
-    inv_v_kernel<OUT, NJ><<<nblocks, 32, 0, st>>>(*L);
-    return cudaGetLastError();
+    if (NJ > JXS_MAXC) {
+        inv_v_kernel<OUT, NJ><<<nblocks, 32, 0, st>>>(*L);
+        return cudaGetLastError();
+    }
+    return jxs_launch(inv_v_kernel<OUT, NJ>, dim3((unsigned)nblocks), (unsigned)(32), 0, st, *L);
 }
 
 extern "C" cudaError_t jxs_launch_inv_v(const InvVLaunch* L, int out_kind, int nblocks, cudaStream_t st) {
@@ -622,8 +627,11 @@ extern "C" cudaError_t jxs_launch_inv_v_batch(const InvVLaunchB* L, int out_kind
 template <int OUT, int NJ>
 static cudaError_t launch_ih(const InvHLaunchN<NJ>* L, int nblocks, cudaStream_t st) {
     if (nblocks <= 0) return cudaSuccess;
-    inv_h_kernel<OUT, NJ><<<nblocks, L->rows_per_block * 32, 0, st>>>(*L);
-    return cudaGetLastError();
+    if (NJ > JXS_MAXC) {
+        inv_h_kernel<OUT, NJ><<<nblocks, L->rows_per_block * 32, 0, st>>>(*L);
+        return cudaGetLastError();
+    }
+    return jxs_launch(inv_h_kernel<OUT, NJ>, dim3((unsigned)nblocks), (unsigned)(L->rows_per_block * 32), 0, st, *L);
 }
 
 extern "C" cudaError_t jxs_launch_inv_h(const InvHLaunch* L, int out_kind, int nblocks, cudaStream_t st) {
@@ -675,6 +683,7 @@ DEV int32_t nlt_sample(const NltOut& P, int64_t v) {
 }
 
 __global__ void __launch_bounds__(256) nlt_out_kernel(const __grid_constant__ NltOut P) {
+    dep_wait();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     int32_t v[JXS_MAXC];
 #pragma unroll
@@ -702,8 +711,7 @@ extern "C" cudaError_t jxs_launch_nlt_out(const NltOut* P, cudaStream_t st) {
         wmax = max(wmax, P->w[k]);
         hmax = max(hmax, P->h[k]);
     }
-    nlt_out_kernel<<<dim3((unsigned)((wmax + 255) / 256), (unsigned)hmax), 256, 0, st>>>(*P);
-    return cudaGetLastError();
+    return jxs_launch(nlt_out_kernel, dim3((unsigned)((wmax + 255) / 256), (unsigned)hmax), 256, 0, st, *P);
 }
 
 /* Inverse Star-Tetrix (Cpih = 3; ISO/IEC 21122-1 Annex F, Mct.c:14-136) on
@@ -733,6 +741,7 @@ DEV int32_t st_access(const StParams& P, int c, int x, int y, int rx, int ry) {
 DEV int32_t st_mul(int32_t k, int32_t v) { return (int32_t)((uint32_t)k * (uint32_t)v); }
 
 __global__ void __launch_bounds__(256) star_tetrix_kernel(const __grid_constant__ StParams P, int step) {
+    dep_wait();
     const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
     if (x >= P.w || y >= P.h) return;
     const long long i = (long long)y * P.pitch + x;
@@ -755,8 +764,7 @@ __global__ void __launch_bounds__(256) star_tetrix_kernel(const __grid_constant_
 extern "C" cudaError_t jxs_launch_star_tetrix(const StParams* P, cudaStream_t st) {
     const dim3 grid((unsigned)((P->w + 255) / 256), (unsigned)P->h);
     for (int step = 0; step < 4; step++) {
-        star_tetrix_kernel<<<grid, 256, 0, st>>>(*P, step);
-        cudaError_t e = cudaGetLastError();
+        const cudaError_t e = jxs_launch(star_tetrix_kernel, grid, 256, 0, st, *P, step);
         if (e != cudaSuccess) return e;
     }
     return cudaSuccess;

@@ -7,8 +7,10 @@
 
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <atomic>
+#include <utility>
 
 #include "jxs_core.h"
 
@@ -309,6 +311,41 @@ static inline cudaError_t jxs_smem_attr(K kern, int bytes, std::atomic<int>* cac
     }
     return e;
 }
+
+/* The kernels of a frame follow one another by programmatic dependent
+ * launch: the next kernel's launch is prepared while the one before runs, and
+ * its blocks read their configuration tables before they wait for it.  Every
+ * block of every such kernel calls dep_wait() before it reads or writes
+ * anything another kernel of the stream touches (it returns when the kernel
+ * before has completed, and with it, since that one waited too, all earlier
+ * ones).  Behind a copy, a memset or an event the launch is an ordinary one,
+ * and dep_wait() returns at once in a kernel that was launched the ordinary
+ * way.  A 4K frame encodes in 114 us instead of 125 and decodes in 107
+ * instead of 118; a 256x64 one takes 119 us there and back instead of 145.
+ * Starting the next kernel's blocks earlier still (a trigger at the top of
+ * each kernel) gained nothing there, and their waiting blocks cost batches up
+ * to 8 %.  The launches of many frames at once, where a launch is a small
+ * part, are ordinary ones. */
+#ifdef __CUDACC__
+__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... P, typename... A>
+static inline cudaError_t jxs_launch(void (*kern)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
+    cudaLaunchAttribute at;
+    memset(&at, 0, sizeof(at));
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c;
+    memset(&c, 0, sizeof(c));
+    c.gridDim = grid;
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &at;
+    c.numAttrs = 1;
+    return cudaLaunchKernelEx(&c, kern, std::forward<A>(args)...);
+}
+#endif
 
 #define JXS_STATUS_SET(ptr, code) atomicCAS((int*)(ptr), 0, (int)(code))
 
