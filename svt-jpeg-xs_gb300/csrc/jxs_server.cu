@@ -141,6 +141,7 @@ static int lane_poll(jxs_server_t* s, SrvLane& L) {
 /* Working sets of frames that are batched whenever several wait: up to about
  * 0.3 Mpixel. */
 static const uint64_t kSmallWork = 4ull << 20;
+static const int64_t kSmallWaitNs = 30000;
 
 /* Takes the oldest waiting requests of the lane's kind and launches them as
  * one batch.  Returns 1 if anything was launched. */
@@ -149,8 +150,11 @@ static int lane_launch(jxs_server_t* s, SrvLane& L) {
         /* batch only what the idle lanes cannot take one by one: with as
          * many idle lanes of this kind as waiting requests, each lane takes
          * one (a lone request runs as soon as a lane is free) */
-        int idle = 0;
-        for (const SrvLane& o : s->lanes) idle += o.kind == L.kind && !o.busy;
+        int idle = 0, lanes = 0;
+        for (const SrvLane& o : s->lanes) {
+            idle += o.kind == L.kind && !o.busy;
+            lanes += o.kind == L.kind;
+        }
         std::lock_guard<std::mutex> g(s->mu);
         std::deque<SrvReq>& q = s->queue[L.kind];
         const int waiting = (int)q.size();
@@ -158,9 +162,13 @@ static int lane_launch(jxs_server_t* s, SrvLane& L) {
         /* small frames that wait together run together, whatever is idle: one
          * alone leaves most of the device empty and takes its launches' time
          * (256x64: 60 us encoding), so that a lane's launches serve them all
-         * and the other lanes stay free for the next arrivals */
+         * and the other lanes stay free for the next arrivals.  While another
+         * lane of its kind runs, a small frame alone waits for company, about
+         * half the time that the running one takes at the least: requests
+         * that come in a burst are otherwise started one by one. */
         int small = 0;
         while (small < std::min(s->max_batch, waiting) && s->streams[q[small].io.stream].work_bytes <= kSmallWork) small++;
+        if (small == 1 && waiting == 1 && idle < lanes && now_ns() - q.front().t_arrive < kSmallWaitNs) return 0;
         take = std::max(take, small);
         while (!q.empty() && (int)L.reqs.size() < take) {
             L.reqs.push_back(q.front());
