@@ -88,15 +88,29 @@ __global__ void publish_status_kernel(int* __restrict__ host, const int* __restr
  * enc_run).  The caller's buffers are the library's until the frame is
  * returned, as with the reference (EncHandle.c:1006 keeps only the input
  * structure, and its workers read the planes later). */
-__global__ void __launch_bounds__(256) host_copy16_kernel(uint8_t* dst, size_t dpitch, const uint8_t* src, size_t spitch,
-                                                          uint32_t chunks) {
-    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x < chunks) *(uint4*)(dst + y * dpitch + 16 * (size_t)x) = *(const uint4*)(src + y * spitch + 16 * (size_t)x);
-}
-__global__ void __launch_bounds__(256) host_copy1_kernel(uint8_t* dst, size_t dpitch, const uint8_t* src, size_t spitch,
-                                                         uint32_t width) {
-    const uint32_t x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
-    if (x < width) dst[y * dpitch + x] = src[y * spitch + x];
+struct HostCopy {
+    uint8_t* dst;
+    const uint8_t* src;
+    size_t dpitch, spitch;
+    uint32_t items;     /* 16-byte chunks (or bytes) per row */
+    uint32_t total;     /* in all rows */
+    int v16;
+    uint32_t first_block;
+};
+struct HostCopies {
+    int n;
+    uint32_t nblocks;
+    HostCopy c[JXS_MAXC];
+};
+__global__ void __launch_bounds__(256) host_copy_kernel_n(const __grid_constant__ HostCopies L) {
+    int k = 0;
+    while (k + 1 < L.n && blockIdx.x >= L.c[k + 1].first_block) k++;
+    const HostCopy& C = L.c[k];
+    const uint32_t i = (blockIdx.x - C.first_block) * blockDim.x + threadIdx.x;
+    if (i >= C.total) return;
+    const uint32_t y = i / C.items, x = i - y * C.items;
+    if (C.v16) *(uint4*)(C.dst + y * C.dpitch + 16 * (size_t)x) = *(const uint4*)(C.src + y * C.spitch + 16 * (size_t)x);
+    else C.dst[y * C.dpitch + x] = C.src[y * C.spitch + x];
 }
 
 /* 1: kernels may access this device's pageable host memory through the
@@ -138,24 +152,45 @@ static int host_resident(const void* p, size_t bytes) {
     return 1;
 }
 
-/* A 2-D copy with one side in host memory (`host`, pageable or page-locked)
- * by a copy kernel, when the device reaches pageable memory directly and the
- * host side's pages are resident; returns 0 otherwise (the caller then
- * copies another way). */
-static int host_copy_kernel(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t rows, cudaStream_t st,
-                            cudaError_t* err, const void* host, size_t host_pitch) {
-    *err = cudaSuccess;
+/* Adds a 2-D copy with one side in host memory (`host`, pageable or
+ * page-locked) to the copies of one launch, when the device reaches pageable
+ * memory directly and the host side's pages are resident; returns 0 otherwise
+ * (the caller then copies another way). */
+static int host_copy_add(HostCopies* L, void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t rows,
+                         const void* host, size_t host_pitch) {
     if (!pageable_direct()) return 0;
     if (!width || !rows) return 1;
     if (!host_resident(host, (rows - 1) * host_pitch + width)) return 0;
-    if (rows > 65535 || width > 0xffffffffull) return 0;
-    /* a thread per 16-byte chunk (or byte), a grid row per row */
     const int v16 = (((uintptr_t)dst | (uintptr_t)src | dpitch | spitch | width) & 15) == 0;
-    const size_t items = v16 ? width / 16 : width;
-    const dim3 grid((unsigned)((items + 255) / 256), (unsigned)rows);
-    if (v16) host_copy16_kernel<<<grid, 256, 0, st>>>((uint8_t*)dst, dpitch, (const uint8_t*)src, spitch, (uint32_t)items);
-    else host_copy1_kernel<<<grid, 256, 0, st>>>((uint8_t*)dst, dpitch, (const uint8_t*)src, spitch, (uint32_t)items);
-    *err = cudaGetLastError();
+    const uint64_t items = v16 ? width / 16 : width, total = items * rows;
+    if (rows > 65535 || width > 0xffffffffull || total > 0x7fffffffull || L->n >= JXS_MAXC) return 0;
+    HostCopy& c = L->c[L->n++];
+    c.dst = (uint8_t*)dst;
+    c.src = (const uint8_t*)src;
+    c.dpitch = dpitch;
+    c.spitch = spitch;
+    c.items = (uint32_t)items;
+    c.total = (uint32_t)total;
+    c.v16 = v16;
+    c.first_block = L->nblocks;
+    L->nblocks += (uint32_t)((total + 255) / 256);
+    return 1;
+}
+/* All of them in one launch: the three planes of a 1080p 4:2:2 8-bit frame
+ * cross the link one after another without a launch between them. */
+static cudaError_t host_copy_launch(const HostCopies& L, cudaStream_t st) {
+    if (!L.nblocks) return cudaSuccess;
+    host_copy_kernel_n<<<L.nblocks, 256, 0, st>>>(L);
+    return cudaGetLastError();
+}
+static int host_copy_kernel(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t rows, cudaStream_t st,
+                            cudaError_t* err, const void* host, size_t host_pitch) {
+    HostCopies L;
+    L.n = 0;
+    L.nblocks = 0;
+    *err = cudaSuccess;
+    if (!host_copy_add(&L, dst, dpitch, src, spitch, width, rows, host, host_pitch)) return 0;
+    *err = host_copy_launch(L, st);
     return 1;
 }
 
@@ -404,6 +439,9 @@ static int32_t enc_run(jxs_gpu_enc_t* e, EncSlot* s, void* const planes[4], cons
     const void* src[JXS_MAXC];
     long long pitch[JXS_MAXC];
     const int nplanes = packed ? 1 : (int)c->nc;
+    HostCopies copies;
+    copies.n = 0;
+    copies.nblocks = 0;
     for (int k = 0; k < nplanes; k++) {
         const uint32_t w = packed ? c->W * 3 : c->comp[k].w, h = packed ? c->H : c->comp[k].h;
         if (jxs_gpu_is_device_ptr(planes[k])) {
@@ -412,18 +450,16 @@ static int32_t enc_run(jxs_gpu_enc_t* e, EncSlot* s, void* const planes[4], cons
         } else {
             uint8_t* d = s->in_stage + s->in_off[k];
             const uint32_t sp = stage_pitch(w, bps);
-            cudaError_t ce = cudaSuccess;
-            if (!jxs_gpu_is_page_locked(planes[k]) &&
-                host_copy_kernel(d, (size_t)sp * bps, planes[k], (size_t)strides[k] * bps, (size_t)w * bps, h, st, &ce, planes[k],
-                                 (size_t)strides[k] * bps))
-                CK(ce);
-            else
+            if (jxs_gpu_is_page_locked(planes[k]) ||
+                !host_copy_add(&copies, d, (size_t)sp * bps, planes[k], (size_t)strides[k] * bps, (size_t)w * bps, h, planes[k],
+                               (size_t)strides[k] * bps))
                 CK(cudaMemcpy2DAsync(d, (size_t)sp * bps, planes[k], (size_t)strides[k] * bps, (size_t)w * bps, h,
                                      cudaMemcpyHostToDevice, st));
             src[k] = d;
             pitch[k] = sp;
         }
     }
+    CK(host_copy_launch(copies, st));
     TMARK(1);
     s->nkev = 0;
     KMARK();
