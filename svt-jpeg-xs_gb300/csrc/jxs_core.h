@@ -47,6 +47,10 @@ extern "C" {
  * which the per-precinct unpacking cannot resolve; the frame is decoded
  * again slice by slice */
 #define JXS_E_DEC_VPRED ((int32_t)0x800030ff)
+/* internal as well: a device codestream's slices are not where its
+ * constant-bit-rate split puts them; the frame is decoded again with its
+ * precincts located first */
+#define JXS_E_DEC_WALK ((int32_t)0x800030fe)
 
 typedef struct jxs_band {
     uint32_t w, h;              /* band size over the whole component */

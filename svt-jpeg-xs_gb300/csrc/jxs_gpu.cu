@@ -72,10 +72,18 @@ extern "C" int jxs_gpu_is_page_locked(const void* p) {
 
 /* A frame's final status into page-locked host memory, written by the GPU
  * after the frame's last compute kernel: no 4-byte copy waits in the copy
- * engines' queues between the frames' large transfers. */
-__global__ void publish_status_kernel(int* __restrict__ host, const int* __restrict__ status) {
+ * engines' queues between the frames' large transfers.  Leaves the status at
+ * zero for the slot's next frame, which so needs no memset.  `hdr`: header of
+ * a device codestream, for the host to check. */
+__global__ void publish_status_kernel(int* __restrict__ host, int* __restrict__ status, uint8_t* __restrict__ hdr_h,
+                                      const uint8_t* __restrict__ hdr, uint32_t hdr_len) {
     dep_wait();
-    if (threadIdx.x == 0) *(volatile int*)host = *(const volatile int*)status;
+    for (uint32_t i = threadIdx.x; i < hdr_len; i += blockDim.x) hdr_h[i] = hdr[i];
+    if (threadIdx.x == 0) {
+        *(volatile int*)host = status[1] ? JXS_E_DEC_WALK : status[0];
+        status[0] = 0;
+        status[1] = 0;
+    }
 }
 
 /* Copies from host memory by a kernel.  On a GB300 behind NVLink-C2C with
@@ -340,6 +348,7 @@ static int32_t enc_slot_alloc(jxs_gpu_enc_t* e, EncSlot* s) {
     CK(cudaMemset(s->slice_done, 0, (size_t)c->nslices * sizeof(uint32_t)));
     CK(cudaMalloc(&s->rc, (size_t)c->np * sizeof(PrecRC)));
     CK(cudaMalloc(&s->status, 64));
+    CK(cudaMemset(s->status, 0, 64));
     CK(cudaMalloc(&s->out_stage, c->lcod + 64));
     CK(cudaMallocHost(&s->status_h, 64));
     *s->status_h = 0;
@@ -433,7 +442,6 @@ static int32_t enc_run(jxs_gpu_enc_t* e, EncSlot* s, void* const planes[4], cons
 #define TMARK(i) \
     if (s->timed) CK(cudaEventRecord(s->tev[i], st))
     TMARK(0);
-    CK(cudaMemsetAsync(s->status, 0, sizeof(int), st));
     /* sources of the first level: caller device planes read in place, host
      * planes staged with one 2-D copy each */
     const void* src[JXS_MAXC];
@@ -512,7 +520,7 @@ static int32_t enc_run(jxs_gpu_enc_t* e, EncSlot* s, void* const planes[4], cons
     CK(jxs_launch_pack(e->dcfg, c->np, s->coef, s->gcli, s->rc, s->cost, dst, e->cap_words, s->status,
                        (c->fs ? 1 : 0) | (c->vpred ? 2 : 0), st));
     KMARK();
-    CK(jxs_launch(publish_status_kernel, dim3(1), 32, 0, st, s->status_hd, s->status));
+    CK(jxs_launch(publish_status_kernel, dim3(1), 32, 0, st, s->status_hd, s->status, (uint8_t*)nullptr, (const uint8_t*)nullptr, 0u));
     TMARK(4);
     s->ndefer = 0;
     if (!out_dev) {
@@ -644,6 +652,7 @@ struct DecSlot {
     uint32_t* prec_off_h;
     const uint32_t* prec_off_hd; /* prec_off_h as the device addresses it */
     uint8_t* hdr_h;       /* header of a device-resident codestream, checked at completion */
+    uint8_t* hdr_hd;      /* hdr_h as the device addresses it */
     int hdr_check;
     /* the frame's arguments, for a second decode slice by slice when it
      * turns out to use vertical prediction */
@@ -677,6 +686,7 @@ struct jxs_gpu_dec {
     uint64_t timed_frames;
     uint64_t serial;
     int vpred;                   /* decode slice by slice: the stream uses vertical prediction */
+    int walk;                    /* locate a device codestream's precincts first: its slices are not where predicted */
     std::mutex mu;
 };
 
@@ -696,6 +706,7 @@ static int32_t dec_slot_alloc(jxs_gpu_dec_t* d, DecSlot* s) {
     CK(cudaMallocHost(&s->prec_off_h, (size_t)c->nprec * sizeof(uint32_t)));
     CK(cudaHostGetDevicePointer((void**)&s->prec_off_hd, s->prec_off_h, 0));
     CK(cudaMallocHost(&s->hdr_h, sizeof(c->hdr)));
+    CK(cudaHostGetDevicePointer((void**)&s->hdr_hd, s->hdr_h, 0));
     CK(cudaMalloc(&s->coef, c->coef_total * sizeof(int16_t) + 64));
     for (uint32_t k = 0; k < c->nc; k++) {
         for (uint32_t v = 0; v < c->comp[k].dv && v < 2; v++) {
@@ -722,6 +733,7 @@ static int32_t dec_slot_alloc(jxs_gpu_dec_t* d, DecSlot* s) {
         CK(cudaMalloc(&s->mct, mb * sizeof(int32_t)));
     }
     CK(cudaMalloc(&s->status, 64));
+    CK(cudaMemset(s->status, 0, 64));
     CK(cudaMallocHost(&s->status_h, 64));
     *s->status_h = 0;
     CK(cudaHostGetDevicePointer((void**)&s->status_hd, s->status_h, 0));
@@ -816,29 +828,39 @@ extern "C" jxs_gpu_dec_t* jxs_gpu_dec_create(const jxs_cfg_t* cfg, int nslots, i
     return d;
 }
 
+/* Precincts per slice up to which the unpacking blocks of a device codestream
+ * find their own precinct.  Each step to it is a dependent load, so the gain
+ * over two launches that locate all precincts first shrinks with them: 3840x2160
+ * 4:2:2 with 4 / 16 / 32 precincts per slice 100 -> 89, 147 -> 136 and
+ * 160 -> 148 us, 1280x720 with 64 precincts 78 -> 64 us.  Slices of more
+ * precincts than measured keep the launches. */
+static const uint32_t kSelfSteps = 64;
 static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t size, const uint32_t* prec_off,
                        void* const planes[4], const uint32_t strides[4]) {
     s->ndefer = 0;
     const jxs_cfg_t* c = &d->cfg;
     const uint32_t bps = bytes_per_sample(c);
     const cudaStream_t st = dec_stream(d, s);
+    const int walk = !prec_off && (d->walk || d->vpred || c->max_slice_budget == 0 || c->pps * c->ncol > kSelfSteps);
     s->timed = d->timing;
 #define TMARK(i) \
     if (s->timed) CK(cudaEventRecord(s->tev[i], st))
     TMARK(0);
-    CK(cudaMemsetAsync(s->status, 0, sizeof(int), st));
     const uint8_t* dbs = bs;
     s->hdr_check = 0;
     s->nkev = 0;
     if (!prec_off) {
         /* device-resident codestream: header compared at completion, precinct
-         * offsets found on the GPU */
+         * offsets found on the GPU, by each unpacking block where its slice
+         * can be predicted */
         if (!jxs_gpu_is_device_ptr(bs) || size < c->hdr_len) return JXS_E_DEC_PTR;
-        CK(cudaMemcpyAsync(s->hdr_h, bs, c->hdr_len, cudaMemcpyDeviceToHost, st));
         s->hdr_check = 1;
-        CK(cudaMemsetAsync(s->status + 1, 0, sizeof(int), st));
         KMARK();
-        CK(jxs_launch_walk(d->dcfg, c->nslices, bs, size, s->prec_off, s->status + 1, s->status, st));
+        if (walk) {
+            /* the walk's own flag of a failed prediction, which it deals with */
+            CK(jxs_launch_walk(d->dcfg, c->nslices, bs, size, s->prec_off, s->status + 2, s->status, st));
+            CK(cudaMemsetAsync(s->status + 2, 0, sizeof(int), st));
+        }
     } else if (!jxs_gpu_is_device_ptr(bs)) {
         if (size > s->bs_cap) {
             CK(cudaStreamSynchronize(st));
@@ -860,7 +882,7 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
     }
     /* host-walked offsets are read by the unpacking blocks straight from the
      * page-locked buffer (one word per block), not copied */
-    const uint32_t* doff = prec_off ? s->prec_off_hd : s->prec_off;
+    const uint32_t* doff = prec_off ? s->prec_off_hd : walk ? s->prec_off : NULL;
     s->arg_bs = dbs;
     s->arg_size = size;
     s->arg_walked = prec_off != NULL;
@@ -916,7 +938,10 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
         L.njobs = plan_inv_h(c, d->dcfg, fb, lout, pass, L.job);
         if (!L.njobs) continue;
         const int blocks = inv_h_layout(L, jxs_inv_h_max_rows_per_block());
-        if (blocks < 0) return JXS_E_BAD_PARAM;
+        if (blocks < 0) {
+            CK(cudaMemsetAsync(s->status, 0, 64, st)); /* this frame's status is not published */
+            return JXS_E_BAD_PARAM;
+        }
         CK(jxs_launch_inv_h(&L, pass == 0 ? 0 : sample_kind, blocks, st));
         KMARK();
     }
@@ -959,7 +984,8 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
         nlt_out_params(c, tin, out, &P);
         CK(jxs_launch_nlt_out(&P, st));
     }
-    CK(jxs_launch(publish_status_kernel, dim3(1), 32, 0, st, s->status_hd, s->status));
+    CK(jxs_launch(publish_status_kernel, dim3(1), s->hdr_check ? 128u : 32u, 0, st, s->status_hd, s->status, s->hdr_hd, dbs,
+                  s->hdr_check ? c->hdr_len : 0u));
     TMARK(3);
     s->ndefer = 0;
     for (uint32_t k = 0; k < c->nc; k++) {
@@ -992,10 +1018,21 @@ extern "C" int32_t jxs_gpu_dec_wait(jxs_gpu_dec_t* d, int slot) {
         s->ndefer = 0;
         return JXS_E_DEC_INTERNAL;
     }
-    if (*s->status_h == JXS_E_DEC_VPRED) {
+    /* every header byte of a device codestream but Lcod (12..15) must match
+     * the stream's */
+    const jxs_cfg_t* c = &d->cfg;
+    const int other_hdr =
+        s->hdr_check && (memcmp(s->hdr_h, c->hdr, 12) != 0 || memcmp(s->hdr_h + 16, c->hdr + 16, c->hdr_len - 16) != 0);
+    int again = 0;
+    while (!other_hdr && (*s->status_h == JXS_E_DEC_VPRED || *s->status_h == JXS_E_DEC_WALK) && again < 2) {
         /* the frame uses vertical prediction: decode it again slice by slice,
-         * and the stream's later frames that way from the start */
-        d->vpred = 1;
+         * and the stream's later frames that way from the start; or its
+         * slices are not at the constant-bit-rate split: decode it again with
+         * its precincts located first, and later frames too if that helps */
+        const int vpred = *s->status_h == JXS_E_DEC_VPRED, before = d->walk;
+        if (vpred) d->vpred = 1;
+        else d->walk = 1;
+        again++;
         const int32_t r = dec_run(d, s, s->arg_bs, s->arg_size, s->arg_walked ? s->prec_off_h : NULL, s->arg_planes,
                                   s->arg_strides);
         if (r != JXS_OK) return r;
@@ -1004,6 +1041,7 @@ extern "C" int32_t jxs_gpu_dec_wait(jxs_gpu_dec_t* d, int slot) {
             s->ndefer = 0;
             return JXS_E_DEC_INTERNAL;
         }
+        if (!vpred && *s->status_h != 0 && *s->status_h != JXS_E_DEC_VPRED) d->walk = before;
     }
     if (!run_deferred(s->defer, &s->ndefer, s->st)) {
         fprintf(stderr, "jxs: copying the decoded planes to host memory failed\n");
@@ -1025,13 +1063,8 @@ extern "C" int32_t jxs_gpu_dec_wait(jxs_gpu_dec_t* d, int slot) {
         d->timed_frames++;
         s->timed = 0;
     }
-    if (s->hdr_check) {
-        /* every header byte but Lcod (12..15) must match the stream's */
-        s->hdr_check = 0;
-        const jxs_cfg_t* c = &d->cfg;
-        if (memcmp(s->hdr_h, c->hdr, 12) != 0 || memcmp(s->hdr_h + 16, c->hdr + 16, c->hdr_len - 16) != 0)
-            return JXS_E_DEC_CONFIG;
-    }
+    s->hdr_check = 0;
+    if (other_hdr) return JXS_E_DEC_CONFIG;
     return *s->status_h;
 }
 
