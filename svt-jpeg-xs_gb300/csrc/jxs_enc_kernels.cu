@@ -399,8 +399,15 @@ DEV uint32_t vlc_vp_bits(int x, int r, int t) {
  *            cheaper;
  *   costs    as in the parallel pass, with those methods and exact signs
  *            for the full strategy;
- *   search   thread 0: quantization on the plain table, then the scan and
- *            refinement on the prediction table (:909-1083). */
+ *   search   warp 0: quantization on the plain table, then the scan and
+ *            refinement on the prediction table (:909-1083).
+ * A chain of a slice's precincts with few blocks at work, bound by the vpred
+ * part.  Two GCLIs to an instruction and two gtli values to a warp, with the
+ * coding choice as minima and maxima, take it from 65,000 to 18,000 cycles
+ * per precinct (1279x717 4:4:4), the costs by a warp per packet from 13,000
+ * to 5,500; the kernel 231 -> 102 us, of which the sign counts above
+ * 30 us.  Two blocks per SM: with registers for three (40) the loop spills
+ * (114 us). */
 template <typename Stage>
 DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint8_t* __restrict__ gcli,
                             const uint32_t* __restrict__ cost, uint32_t* area, PrecRC* __restrict__ rc,
@@ -409,9 +416,9 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
                             const jxs_seg_t* segs, const uint8_t* s_pkbl0, const uint8_t* s_pknbl, const uint8_t* s_order) {
     __shared__ int s_err;
     __shared__ uint8_t s_gtop[JXS_MAXBL], s_bl0[JXS_MAXBL], s_bl1[JXS_MAXBL];
-    __shared__ uint32_t s_methv[JXS_MAXBL]; /* per band: 2 bits per t */
     uint32_t(*vtfs)[16] = (uint32_t(*)[16])area;
-    uint32_t(*dV)[32] = (uint32_t(*)[32])(area + RC_LT_REGION);
+    uint32_t(*dV)[33] = (uint32_t(*)[33])(area + RC_LT_REGION);
+    static_assert(32 * 33 <= RC_LT_REGION, "rows of 33 words: a lane per Q adds at one R");
     uint32_t(*vtdat)[16] = (uint32_t(*)[16])(area + 2 * RC_LT_REGION);
     uint32_t(*vtnos)[16] = (uint32_t(*)[16])(area + 3 * RC_LT_REGION);
     uint32_t(*vtsig)[16] = (uint32_t(*)[16])(area + 4 * RC_LT_REGION);
@@ -420,7 +427,7 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
     uint32_t(*vred)[16] = (uint32_t(*)[16])(area + 7 * RC_LT_REGION);
     uint32_t* Ts = area + 8 * RC_LT_REGION;
     uint32_t* Fs = area + 9 * RC_LT_REGION;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = lane >> 4;
     const RcParams P = rc_params(cfg);
     const SliceSplit sp = slice_split(cfg, s);
     uint32_t carry = 0, run = cfg->slice_begin[s] + 6; /* of warp 0 */
@@ -429,6 +436,7 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
     const uint32_t np_all = cfg->np, signs = cfg->signs, fs = cfg->fs, SG = cfg->seg_groups, npk = cfg->npk;
     const uint32_t nbands = cfg->nbands, sig = cfg->sig;
     const int rm = cfg->rm;
+    uint32_t(*vtz)[16] = signs == 2 ? vtnz : vtfs; /* sign bits */
     __syncthreads();
     if (P.rc_mode >= 2 && slice_common(P, s, sp, cost, Ts, rc, status)) return;
     int kind_staged = -1;
@@ -447,7 +455,6 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
         for (uint32_t fb = threadIdx.x; fb < nbands; fb += blockDim.x) {
             s_bl0[fb] = 0xff;
             s_bl1[fb] = 0xff;
-            s_methv[fb] = 0;
         }
         __syncthreads();
         for (uint32_t x = threadIdx.x; x < nbl; x += blockDim.x) {
@@ -473,7 +480,7 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
             Ts[e] = __ldcg(cost + (uint64_t)p * 1024 + q * 32 + r);
             if (fs) Fs[e] = __ldcg(cost + ((uint64_t)np_all + p) * 1024 + q * 32 + r);
         }
-        for (int e = threadIdx.x; e < nq * 32; e += blockDim.x) dV[e >> 5][e & 31] = 0;
+        for (int e = threadIdx.x; e < nq * 33; e += blockDim.x) (&dV[0][0])[e] = 0;
         __syncthreads();
         /* vertical prediction costs of every line, for every t */
         if (i > 0) {
@@ -486,33 +493,56 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
                 const uint8_t* top = cur - bd.gpitch; /* the row above: the previous line, for line 0 in the row above */
                 const int gtt = B.line ? -1 : (int)s_gtop[B.fb];
                 const uint32_t gend = min(sg.g0 + SG, B.gcli_w);
+                uint32_t acc = 0; /* lane t: bits at t; lane 16 + t: those that significance groups save */
                 for (uint32_t base = sg.g0; base < gend; base += 128) {
-                    const uint32_t g = base + 4 * lane;
-                    const uint32_t nv = g < gend ? min(4u, gend - g) : 0u;
-                    const uint32_t wc = nv ? *(const uint32_t*)(cur + g) : 0u, wt = nv ? *(const uint32_t*)(top + g) : 0u;
-                    for (int t = 0; t < 16; t++) {
-                        const int gmax = max(t, gtt);
-                        uint32_t sum = 0, flag = 1;
+                    /* a significance group of 8 GCLIs per lane, in both
+                     * halves of the warp; pairs of GCLIs in 16-bit halves */
+                    const uint32_t g = base + 8 * (lane & 15);
+                    const uint32_t nv = g < gend ? min(8u, gend - g) : 0u;
+                    const uint32_t E = 0x00ff00ffu, ONE = 0x00010001u, K = 0x20002000u;
+                    uint32_t wc[2] = {0, 0}, wt[2] = {0, 0}, c[4], tp[4], pv[4], kc = 0;
+                    if (nv) {
+                        wc[0] = *(const uint32_t*)(cur + g);
+                        wt[0] = *(const uint32_t*)(top + g);
+                    }
+                    if (nv > 4) {
+                        wc[1] = *(const uint32_t*)(cur + g + 4);
+                        wt[1] = *(const uint32_t*)(top + g + 4);
+                    }
+#pragma unroll
+                    for (int k = 0; k < 4; k++) {
+                        const int n = min(max((int)nv - 4 * (k >> 1), 0), 4), sh = 8 * (k & 1);
+                        const uint32_t vm = n == 4 ? 0xffffffffu : (1u << (8 * n)) - 1u;
+                        pv[k] = ((vm >> sh) & E) * 0x101u;
+                        c[k] = (wc[k >> 1] >> sh) & E & pv[k];
+                        tp[k] = (wt[k >> 1] >> sh) & E;
+                        kc += (K - ONE) & pv[k];
+                    }
+                    uint32_t m8 = __vmaxu2(__vmaxu2(c[0], c[1]), __vmaxu2(c[2], c[3]));
+                    m8 = max(m8 & 0xffffu, m8 >> 16);
+#pragma unroll 2
+                    for (int it = 0; it < 8; it++) {
+                        const int t = 2 * it + half;
+                        const uint32_t t2 = t * ONE, G2 = max(t, gtt) * ONE;
+                        uint32_t sum = 0, off = 0;
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
-                            if (k < (int)nv) {
-                                const int c = (int)((wc >> (8 * k)) & 255u), tp = (int)((wt >> (8 * k)) & 255u);
-                                const int mt = max(tp, gmax), gv = max(c, t);
-                                sum += vlc_vp_bits(gv - mt, mt, t) + 1;
-                                flag &= rm ? (uint32_t)(c <= t) : (uint32_t)(mt == gv);
-                            }
+                            /* with d the GCLI less its prediction mt, neither
+                             * below t: d < 0 takes -2 d - 1 ones, else 2 d
+                             * or, past mt - t, d + mt - t; all plus K */
+                            const uint32_t mt = __vmaxu2(tp[k], G2), gv = __vmaxu2(c[k], t2);
+                            const uint32_t X = 2u * (gv - mt) + K;
+                            sum += __vmaxu2(__vminu2(X, gv + (K - t2)), (2u * K - ONE) - X) & pv[k];
+                            off |= (X ^ K) & pv[k];
                         }
-                        /* significance group of 8 GCLIs: lanes 2j, 2j + 1 */
-                        const uint32_t f2 = flag & __shfl_xor_sync(FULL, flag, 1);
-                        const uint32_t s2 = sum + __shfl_xor_sync(FULL, sum, 1);
-                        const uint32_t red = (!(lane & 1) && f2) ? s2 : 0u;
-                        const uint32_t tot = __reduce_add_sync(FULL, sum), rtot = __reduce_add_sync(FULL, red);
-                        if (lane == 0) {
-                            if (tot) atomicAdd(&vnos[x][t], tot);
-                            if (rtot) atomicAdd(&vred[x][t], rtot);
-                        }
+                        sum -= kc; /* and the code's closing zero */
+                        sum = (sum & 0xffffu) + (sum >> 16);
+                        const uint32_t red = (rm ? m8 <= (uint32_t)t : off == 0) ? sum : 0u;
+                        const uint32_t a = __reduce_add_sync(FULL, sum << (16 * half)), b = __reduce_add_sync(FULL, red << (16 * half));
+                        if (((lane & 15) >> 1) == it) acc += ((lane < 16 ? a : b) >> (16 * (lane & 1))) & 0xffffu;
                     }
                 }
+                if (acc) atomicAdd(lane < 16 ? &vnos[x][lane] : &vred[x][lane - 16], acc);
             }
         }
         __syncthreads();
@@ -521,8 +551,9 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
             const uint32_t fb = e >> 4, t = e & 15;
             const uint32_t x0 = s_bl0[fb], x1 = s_bl1[fb];
             if (x0 == 0xff) continue;
+            const bool two = x1 != 0xff;
             uint32_t cnv = vtnos[x0][t], csv = vtsig[x0][t] + lsig[x0], vn = vnos[x0][t], vs = vnos[x0][t] - vred[x0][t] + lsig[x0];
-            if (x1 != 0xff) {
+            if (two) {
                 cnv += vtnos[x1][t];
                 csv += vtsig[x1][t] + lsig[x1];
                 vn += vnos[x1][t];
@@ -540,59 +571,59 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
                 }
                 if (sig && best > vs) m = 3;
             }
-            atomicOr(&s_methv[fb], m << (2 * t));
+            /* vtnos becomes the GCLI bits of the method chosen, vtsig its
+             * significance flags */
+            for (uint32_t x = x0, k = 0; k < (two ? 2u : 1u); x = x1, k++) {
+                if (m) vtnos[x][t] = m == 2 ? vtsig[x][t] : vnos[x][t] - (m == 3 ? vred[x][t] : 0u);
+                vtsig[x][t] = m & 2u ? lsig[x] : 0u;
+            }
         }
         __syncthreads();
-        /* costs with those methods, per (Q, packet) as in the parallel pass */
-        auto gbits = [&](uint32_t x, uint32_t m, int t) -> uint32_t {
-            return m == 0 ? vtnos[x][t] : m == 2 ? vtsig[x][t] : m == 1 ? vnos[x][t] : vnos[x][t] - vred[x][t];
-        };
-        auto nbits = [&](uint32_t x, int t) -> uint32_t { return signs == 2 ? vtnz[x][t] : signs == 1 ? vtfs[x][t] : 0u; };
-        for (uint32_t e = threadIdx.x; e < (uint32_t)nq * npk; e += blockDim.x) {
-            const int q = (int)(e / npk);
-            const uint32_t k = e - (uint32_t)q * npk;
-            const uint32_t b0 = s_pkbl0[k], nb = s_pknbl[k];
-            if (!nb) continue;
+        /* costs with those methods, a warp per packet and a lane per Q, as in
+         * the parallel pass */
+        for (uint32_t k = warp; k < npk; k += RC_WARPS) {
+            const int q = lane;
+            const uint32_t b0 = s_pkbl0[k], nb = s_pknbl[k], raw = lraw[k];
+            if (!nb || q >= nq) continue;
             uint32_t db = 0, gb = 0, sb = 0, zb = 0;
             for (uint32_t x = b0; x < b0 + nb; x++) {
-                const int g = lgain[x];
-                const int t = q < g ? 0 : min(q - g, 15);
-                const uint32_t m = (s_methv[lfb[x]] >> (2 * t)) & 3u;
+                const int t = min(max(q - (int)lgain[x], 0), 15);
                 db += vtdat[x][t];
-                gb += gbits(x, m, t);
-                sb += (m & 2u) ? lsig[x] : 0u;
-                zb += nbits(x, t);
+                gb += vtnos[x][t];
+                sb += vtsig[x][t];
+                if (signs) zb += vtz[x][t];
             }
-            uint32_t c = ((db + 7) >> 3) + min(lraw[k], ((sb + 7) >> 3) + ((gb + 7) >> 3)) + ((zb + 7) >> 3);
+            uint32_t c = ((db + 7) >> 3) + min(raw, ((sb + 7) >> 3) + ((gb + 7) >> 3)) + ((zb + 7) >> 3);
             atomicAdd(&dV[q][0], c);
             for (uint32_t j = 0; j < nb; j++) {
                 const uint32_t x = s_order[b0 + j];
                 const int rf = lprio[x] + 1;
                 if (rf >= nr) break;
                 const int g = lgain[x];
-                const int t0 = q < g ? 0 : min(q - g, 15), t1 = q < g + 1 ? 0 : min(q - g - 1, 15);
-                const uint32_t m0 = (s_methv[lfb[x]] >> (2 * t0)) & 3u, m1 = (s_methv[lfb[x]] >> (2 * t1)) & 3u;
+                const int t0 = min(max(q - g, 0), 15), t1 = min(max(q - g - 1, 0), 15);
                 db += vtdat[x][t1] - vtdat[x][t0];
-                gb += gbits(x, m1, t1) - gbits(x, m0, t0);
-                sb += ((m1 & 2u) ? lsig[x] : 0u) - ((m0 & 2u) ? lsig[x] : 0u);
-                zb += nbits(x, t1) - nbits(x, t0);
-                const uint32_t c1 = ((db + 7) >> 3) + min(lraw[k], ((sb + 7) >> 3) + ((gb + 7) >> 3)) + ((zb + 7) >> 3);
+                gb += vtnos[x][t1] - vtnos[x][t0];
+                sb += vtsig[x][t1] - vtsig[x][t0];
+                if (signs) zb += vtz[x][t1] - vtz[x][t0];
+                const uint32_t c1 = ((db + 7) >> 3) + min(raw, ((sb + 7) >> 3) + ((gb + 7) >> 3)) + ((zb + 7) >> 3);
                 atomicAdd(&dV[q][rf], c1 - c);
                 c = c1;
             }
         }
         __syncthreads();
-        for (int q = threadIdx.x; q < nq; q += blockDim.x) {
-            uint32_t run = 0;
-            for (int r = 0; r < nr; r++) {
-                run += dV[q][r];
-                dV[q][r] = run;
+        for (int q = warp; q < nq; q += RC_WARPS) {
+            uint32_t c = dV[q][lane];
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, c, o);
+                if (lane >= o) c += y;
             }
+            dV[q][lane] = c;
         }
         __syncthreads();
         if (warp == 0) {
             int q, r;
-            const int err = prec_select(P, s, i, sp, Ts, fs ? Fs : Ts, nr, &dV[0][0], 32, 1, carry, run, q, r, rc, status);
+            const int err = prec_select(P, s, i, sp, Ts, fs ? Fs : Ts, nr, &dV[0][0], 33, 1, carry, run, q, r, rc, status);
             if (err) {
                 if (lane == 0) s_err = err;
             } else {
@@ -609,13 +640,11 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
  * rate_control_sign_coding_get_sum_nonzero_coeff_c, :366-455): the bits of
  * m for deadzone quantization; for uniform quantization the value
  * ((m << (g - t + 1)) - m + 2^g) >> (g + 1) falls as t grows and is non-zero
- * while m (2^(g-t+1) - 1) >= 2^g. */
+ * while m (2^(g-t+1) - 1) >= 2^g, which for m of b <= g bits holds at
+ * t = b - 1, never at t = b + 1. */
 DEV uint32_t nz_levels(uint32_t m, uint32_t g, uint32_t uniform) {
-    if (!m) return 0;
-    if (!uniform) return 32 - __clz(m);
-    uint32_t n = 0;
-    while (n < g && m * ((2u << (g - n)) - 1u) >= (1u << g)) n++;
-    return n;
+    const uint32_t b = 32u - __clz(m);
+    return b + (uniform && (m << (g - b + 1u)) - m >= (1u << g));
 }
 
 /* Byte cost of every (quantization, refinement) candidate of one precinct
@@ -791,31 +820,45 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
             if (fs) {
                 /* sign handling: the lane's 16 coefficients (inside the band
                  * width) by the number of gtli values at which they stay
-                 * non-zero; 16-bit counters two to a register */
+                 * non-zero, counted like the GCLIs, 8 coefficients to 4-bit
+                 * counters and 16 to 8-bit ones */
                 uint4 c0 = make_uint4(0, 0, 0, 0), c1 = c0;
                 if (nv) {
                     c0 = *(const uint4*)(crow + 4 * g);
                     c1 = *(const uint4*)(crow + 4 * g + 8);
                 }
-                const uint32_t cw[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
-                const int wleft = (int)bls[x].w - 4 * (int)g;
-                uint32_t zc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+                uint32_t cw[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+                const int left16 = min((int)bls[x].w - 4 * (int)g, 4 * (int)nv);
+                if (left16 < 16) {
 #pragma unroll
-                for (int i = 0; i < 16; i++) {
-                    const uint32_t m = (cw[i >> 1] >> (16 * (i & 1))) & 0x7fffu;
-                    const uint32_t v = (w4 >> (8 * (i >> 2))) & 255u;
-                    const uint32_t n = i < wleft && (i >> 2) < (int)nv ? nz_levels(m, v, uniform) : 0u;
-#pragma unroll
-                    for (int r = 0; r < 8; r++) zc[r] += (n >> 1) == (uint32_t)r ? 1u << (16 * (n & 1)) : 0u;
+                    for (int i = 0; i < 8; i++) cw[i] &= 2 * i + 1 < left16 ? 0xffffffffu : 2 * i < left16 ? 0xffffu : 0u;
                 }
+                const bool large = __any_sync(FULL, w4 & 0x08080808u);
+                uint32_t za[4] = {0, 0, 0, 0}; /* levels 0, 2, 4, 6; 1, 3, 5, 7; the same of 8..15 */
 #pragma unroll
-                for (int r = 0; r < 8; r++) {
-                    const uint32_t zs = __reduce_add_sync(FULL, zc[r]);
-                    if (lane < 2) {
-                        const uint32_t c = (zs >> (16 * lane)) & 0xffffu;
-                        if (c) atomicAdd(&nzh[x][2 * r + lane], c);
+                for (int i0 = 0; i0 < 16; i0 += 8) {
+                    uint32_t zl = 0, zg = 0;
+#pragma unroll
+                    for (int i = i0; i < i0 + 8; i++) {
+                        const uint32_t n = nz_levels(cw[i >> 1] >> (16 * (i & 1)) & 0x7fffu, (w4 >> (8 * (i >> 2))) & 255u, uniform);
+                        zl += shl_or_0(1u, 4 * n);
+                        if (large) zg += shl_or_0(1u, 4 * n - 32u);
                     }
+                    za[0] += zl & M;
+                    za[1] += (zl >> 4) & M;
+                    za[2] += zg & M;
+                    za[3] += (zg >> 4) & M;
                 }
+                const uint32_t M2 = 0x00ff00ffu;
+                uint32_t zw = 0; /* of lane b < 16: levels b & 11 and (b & 11) + 4 in its halves */
+#pragma unroll
+                for (int i = 0; i < 4; i++) {
+                    if (i >= 2 && !large) break;
+                    const uint32_t e = __reduce_add_sync(FULL, za[i] & M2), o = __reduce_add_sync(FULL, (za[i] >> 8) & M2);
+                    if ((lane >> 3) == (i >> 1) && (lane & 1) == (i & 1)) zw = lane & 2 ? o : e;
+                }
+                const uint32_t zn = (zw >> (16 * ((lane >> 2) & 1))) & 0xffffu;
+                if (lane < 16 && zn) atomicAdd(&nzh[x][lane], zn);
             }
         }
     }
@@ -2013,7 +2056,7 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
 /* kernels: one frame, or a batch of frames (block -> frame by its first block) */
 /* ------------------------------------------------------------------------ */
 template <bool SIGNS, bool VPRED>
-__global__ void __launch_bounds__(RC_THREADS, (SIGNS || VPRED) ? 3 : 4) rc_cost_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ gcli,
+__global__ void __launch_bounds__(RC_THREADS, VPRED ? 2 : SIGNS ? 3 : 4) rc_cost_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ gcli,
                                                            const uint16_t* __restrict__ coef, uint32_t* __restrict__ cost,
                                                            uint32_t* __restrict__ slice_done, PrecRC* __restrict__ rc,
                                                            int* __restrict__ status) {
@@ -2021,7 +2064,7 @@ __global__ void __launch_bounds__(RC_THREADS, (SIGNS || VPRED) ? 3 : 4) rc_cost_
 }
 
 template <bool SIGNS, bool VPRED>
-__global__ void __launch_bounds__(RC_THREADS, (SIGNS || VPRED) ? 3 : 4) rc_cost_batch_kernel(const __grid_constant__ EncPrecLaunch L) {
+__global__ void __launch_bounds__(RC_THREADS, VPRED ? 2 : SIGNS ? 3 : 4) rc_cost_batch_kernel(const __grid_constant__ EncPrecLaunch L) {
     const EncPrecFrame& F = L.job[find_job<JXS_BATCH_FRAMES>(L.job, L.nframes, (int)blockIdx.x)];
     rc_cost_body<SIGNS, VPRED>(F.cfg, F.gcli, F.coef, F.cost, F.slice_done, F.rc, F.status, (int)blockIdx.x - F.first_block);
 }
