@@ -29,6 +29,8 @@
 #define RC_WARPS (RC_THREADS / 32)
 /* shared area of the rate control: 5 tables of 16 words per band line, 6
  * with sign handling */
+#define RC_NOS 24
+#define RC_SIG 46
 #define RC_AREA_WORDS(signs) (((signs) ? 6 : 5) * JXS_MAXBLINES * 16)
 
 /* binary_search_init / binary_search_next_step (BinarySearch.c:9-78) */
@@ -706,6 +708,8 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
     __shared__ jxs_bline_t s_bl[JXS_MAXBLINES];
     __shared__ uint64_t s_grow[JXS_MAXBLINES];
     __shared__ uint8_t s_pkbl0[JXS_MAXPK], s_pknbl[JXS_MAXPK], s_order[JXS_MAXBLINES];
+    __shared__ uint32_t s_opk[JXS_MAXBLINES + 1]; /* the order's lines: number | gain << 8 | first R that lowers its gtli << 16 */
+    uint64_t(*tw)[16] = (uint64_t(*)[16])(s_area + (SIGNS ? 2 : 0) * JXS_MAXBLINES * 16); /* in place of hist and shist, or tdat and tnos */
 
     const int last = (p + 1 >= (int)cfg->np);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -923,15 +927,32 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
         }
     }
     /* coding method per band and t: significance only if strictly cheaper
-     * (RateControl.c:528-575); tnos becomes the GCLI bits of the method
-     * chosen, tsig its significance flags */
+     * (RateControl.c:528-575).  Per line and t one word: data bits, from bit
+     * RC_NOS the GCLI bits of the method chosen, from bit RC_SIG its
+     * significance flags; a packet's sums stay within these fields, at most
+     * 4 * 16384 groups of 64 data and 16 GCLI bits */
     const int nq = cfg->max_q + 1, nr = cfg->max_r + 1;
     const uint32_t sig = cfg->sig;
-    for (uint32_t i = threadIdx.x; i < nbl * 16; i += blockDim.x) {
-        const uint32_t x = i >> 4, t = i & 15, fb = lfb[x];
-        const bool m = sig && cn[fb][t] > cs[fb][t];
-        if (m) tnos[x][t] = tsig[x][t];
-        tsig[x][t] = m ? lsig[x] : 0u;
+    static_assert(JXS_MAXBLINES * 16 <= 3 * RC_THREADS, "three words per thread");
+    uint64_t word[3] = {0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const uint32_t i = threadIdx.x + k * RC_THREADS, x = i >> 4, t = i & 15;
+        if (i < nbl * 16) {
+            const uint32_t fb = lfb[x];
+            const bool m = sig && cn[fb][t] > cs[fb][t];
+            word[k] = tdat[x][t] | (uint64_t)(m ? tsig[x][t] : tnos[x][t]) << RC_NOS | (uint64_t)(m ? lsig[x] : 0u) << RC_SIG;
+        }
+    }
+    if (SIGNS) __syncthreads(); /* the words take the place of tdat and tnos */
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        const uint32_t i = threadIdx.x + k * RC_THREADS;
+        if (i < nbl * 16) tw[i >> 4][i & 15] = word[k];
+    }
+    for (uint32_t x = threadIdx.x; x < nbl; x += blockDim.x) {
+        const uint32_t y = s_order[x];
+        s_opk[x] = y | (uint32_t)lgain[y] << 8 | (lprio[y] + 1u) << 16;
     }
     /* costs: band priorities are distinct, so raising R by one lowers the
      * gtli of one band only; each (Q, packet) thread adds its packet's cost
@@ -952,37 +973,42 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
         const int q = lane;
         const uint32_t b0 = s_pkbl0[k], nb = s_pknbl[k], raw = lraw[k];
         if (!nb || q >= nq) continue;
-        uint32_t db = 0, gb = 0, sb = 0, fb = 0, zb = 0;
-        for (uint32_t x = b0; x < b0 + nb; x++) {
-            const int t = min(max(q - (int)lgain[x], 0), 15);
-            db += tdat[x][t];
-            gb += tnos[x][t];
-            sb += tsig[x][t];
+        /* sums of the words plus 7 in each field; bytes of the fields */
+        uint64_t S = 7u | (uint64_t)7u << RC_NOS | (uint64_t)7u << RC_SIG;
+        auto bytes = [&](uint64_t v) {
+            return ((uint32_t)v << (32 - RC_NOS) >> (35 - RC_NOS)) +
+                   min(raw, (uint32_t)(v >> (RC_SIG + 3)) + ((uint32_t)(v >> (RC_NOS + 3)) & ((1u << (RC_SIG - RC_NOS - 3)) - 1u)));
+        };
+        uint32_t fb = 7, zb = 7;
+#pragma unroll 4
+        for (uint32_t i = b0; i < b0 + nb; i++) {
+            const uint32_t w = s_opk[i], x = w & 255u;
+            const int t = min(max(q - (int)((w >> 8) & 255u), 0), 15);
+            S += tw[x][t];
             if (fs) {
                 fb += tfs[x][t];
                 zb += tnz[x][t];
             }
         }
-        const uint32_t base = ((db + 7) >> 3) + min(raw, ((sb + 7) >> 3) + ((gb + 7) >> 3));
-        uint32_t c = base + (fs ? (fb + 7) >> 3 : 0u), cf = base + ((zb + 7) >> 3);
+        const uint32_t base = bytes(S);
+        uint32_t c = base + (fs ? fb >> 3 : 0u), cf = base + (zb >> 3);
         atomicAdd(&dC[q][0], c);
         if (fs) atomicAdd(&dF[q][0], cf);
-        for (uint32_t i = 0; i < nb; i++) {
-            const uint32_t x = s_order[b0 + i];
-            const int rf = lprio[x] + 1; /* the line's gtli drops by one for R >= priority + 1 */
-            if (rf >= nr) break;
-            const int g = lgain[x];
-            const int t0 = min(max(q - g, 0), 15), t1 = min(max(q - g - 1, 0), 15);
-            db += tdat[x][t1] - tdat[x][t0];
-            gb += tnos[x][t1] - tnos[x][t0];
-            sb += tsig[x][t1] - tsig[x][t0];
-            const uint32_t base1 = ((db + 7) >> 3) + min(raw, ((sb + 7) >> 3) + ((gb + 7) >> 3));
+        uint32_t w = s_opk[b0];
+        for (uint32_t i = b0; i < b0 + nb; i++) {
+            const uint32_t x = w & 255u, rf = w >> 16; /* the line's gtli drops by one for R >= priority + 1 */
+            if (rf >= (uint32_t)nr) break;
+            const int d = q - (int)((w >> 8) & 255u);
+            const int t0 = min(max(d, 0), 15), t1 = min(max(d - 1, 0), 15);
+            S += tw[x][t1] - tw[x][t0];
+            w = s_opk[i + 1]; /* the next line's before its turn */
+            const uint32_t base1 = bytes(S);
             uint32_t c1 = base1;
             if (fs) {
                 fb += tfs[x][t1] - tfs[x][t0];
                 zb += tnz[x][t1] - tnz[x][t0];
-                c1 += (fb + 7) >> 3;
-                const uint32_t cf1 = base1 + ((zb + 7) >> 3);
+                c1 += fb >> 3;
+                const uint32_t cf1 = base1 + (zb >> 3);
                 atomicAdd(&dF[q][rf], cf1 - cf);
                 cf = cf1;
             }
@@ -1013,15 +1039,17 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
     /* the block that completes a slice runs the slice's selection: tables
      * published with a fence, blocks counted per slice */
     __shared__ int s_last;
-    __threadfence();
     __syncthreads();
     const uint32_t s = (uint32_t)p / cfg->pps;
     const uint32_t first_p = cfg->pps * s;
     const uint32_t nprec = (s + 1 == cfg->nslices) ? cfg->np - first_p : cfg->pps;
-    if (threadIdx.x == 0) s_last = atomicAdd(&slice_done[s], 1u) + 1 == nprec;
+    if (threadIdx.x == 0) {
+        __threadfence(); /* the block's writes, ordered before by the barrier */
+        s_last = atomicAdd(&slice_done[s], 1u) + 1 == nprec;
+        __threadfence();
+    }
     __syncthreads();
     if (!s_last) return;
-    __threadfence();
     if constexpr (VPRED) {
         if (cfg->vpred) select_slice_vpred(cfg, (int)s, gcli, cost, s_area, rc, status, stage_kind, lgain, lprio, lfb, lsig,
                                            lraw, s_bl, s_seg, s_pkbl0, s_pknbl, s_order);
