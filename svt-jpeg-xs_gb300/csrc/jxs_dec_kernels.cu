@@ -38,6 +38,7 @@ struct UkPk {
     uint32_t wbase, nwords;     /* its 32-bit words in the concatenated GCLI word list (VLC packets) */
     uint32_t zbase, nzero;      /* rank of its first zero bit among all VLC zeros; zeros in its range */
     uint32_t ncoded;            /* unary codewords */
+    uint32_t rbase;             /* codewords with ones among all VLC zeros before it */
     uint32_t raw, present;
 };
 /* A segment as the warp passes read it: rank of its first codeword's zero
@@ -142,6 +143,49 @@ DEV uint32_t seg_bases(uint32_t cnt, uint32_t bl, uint32_t nseg, uint32_t npk, c
         *sum = ex[bls[lb].seg0 + bls[lb].nseg] - ex[bls[b0].seg0];
     }
     return i < nseg ? e - ex[bls[pkbl0[bls[bl].pk]].seg0] : 0u;
+}
+
+/* Data nibbles of a VLC packet's first n codewords (signs with the data): a
+ * codeword of r > 0 ones stands for a group of r planes and its signs, so
+ * they are the ones before the n-th zero bit and the codewords among them
+ * that have ones (a zero bit after a one).  zpre / rpre: zeros and codewords
+ * with ones before each thread's `per` words of the zeros pass. */
+DEV uint32_t vlc_nibbles(const uint32_t* b, const UkPk& P, uint32_t n, const uint32_t* zpre, const uint32_t* rpre, uint32_t per) {
+    if (!n) return 0;
+    const uint32_t Z = P.zbase + n; /* the zero bits of all packets up to the n-th */
+    uint32_t T = 0;
+#pragma unroll 1
+    for (uint32_t step = UK_THREADS / 2; step; step >>= 1)
+        if (zpre[T + step] < Z) T += step;
+    uint32_t i = 0, zeros = P.zbase, runs = P.rbase;
+    if (T * per > P.wbase) {
+        i = T * per - P.wbase;
+        zeros = zpre[T];
+        runs = rpre[T];
+    }
+    uint32_t z, before;
+    for (;; i++) {
+        const uint32_t at = P.gpos + 32 * i;
+        z = ~bits32_at(b, at);
+        before = i ? bits32_at(b, at - 1) : ~z >> 1; /* the bit before each */
+        const uint32_t nz = __popc(z);
+        if (zeros + nz >= Z || i + 1 >= P.nwords) break;
+        zeros += nz;
+        runs += __popc(z & before);
+    }
+    /* place of the last one in the word, by halves */
+    uint32_t left = Z - zeros, y = z, pos = 0;
+#pragma unroll
+    for (int s = 16; s; s >>= 1) {
+        const uint32_t c = __popc(y >> (32 - s));
+        if (left > c) {
+            left -= c;
+            pos += s;
+            y <<= s;
+        }
+    }
+    runs += __popc(z & before & ~(0x7fffffffu >> pos));
+    return 32 * i + pos + 1 - n + (runs - P.rbase);
 }
 
 /* Packet header fields (get_packet_header, ParseHeader.c:20-44): raw flag,
@@ -319,24 +363,34 @@ DEV bool slice_ends(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict
  *           at the c-th zero bit of its sub-packet (unpack_pred_zero_gclis_*,
  *           Packing.c:435-511); its value, the ones before that bit, goes to
  *           byte c of a table;
- *   pass 2  warp per segment: GCLI = gtli + codeword value, or raw; data bits;
- *   pass 3  warp per segment: data bits at warp-scanned offsets, decoded and
- *           written as int16 coefficients (8 bytes per lane, coalesced).
+ *   bases   signs with the data, no prediction: thread per segment, the data
+ *           nibbles before it by a search in the unary codes' bits;
+ *   pass 2  otherwise, warp per segment: GCLI = gtli + codeword value, or raw;
+ *           prediction; data bits; running sums of these;
+ *   pass 3  warp per segment: GCLIs (bases), data bits at warp-scanned
+ *           offsets, decoded and written as int16 coefficients (8 bytes per
+ *           lane, coalesced).
  *
  * Bound by instruction issue.  Segments are described once, a 16-byte record
  * each, instead of by every warp that takes one; codeword values are read 4
  * at a time instead of 5 zero positions; bytes are swapped once.  8 4K 4:2:2
- * 10-bit frames: 263 us before, 223 us now. */
+ * 10-bit frames: 263 us before, 223 us so; 203 us with the segments' data
+ * positions from the codes' bits instead of from a pass over all GCLIs. */
 template <bool FS, bool VP, bool BATCH>
 __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t bs_size,
                                             const uint32_t* __restrict__ prec_off, int16_t* __restrict__ coef,
                                             uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg, int* status, const int p,
                                             uint8_t* top_gcl, uint8_t* top_t, const int vp_ok) {
     extern __shared__ __align__(16) uint8_t dsm[];
-    const UkLayout UL = uk_layout(cap_bytes, cap_groups, cap_seg);
+    /* signs with the data, no prediction: the segments' data positions come
+     * from the unary codes' bits and the GCLIs are read in the data pass */
+    constexpr bool LEAN = !FS && !VP;
+    const UkLayout UL = uk_layout(cap_bytes, cap_groups, cap_seg, LEAN);
     uint32_t* pbuf = (uint32_t*)dsm;
     uint8_t* gcl = dsm + UL.gcl;
     uint8_t* zval = dsm + UL.zval;
+    uint32_t* zpre = (uint32_t*)(dsm + UL.list); /* LEAN, until the data pass: see vlc_nibbles */
+    uint32_t* rpre = zpre + UK_THREADS;
     /* zero bits: one per codeword plus up to 7 padding bits per packet */
     const uint32_t zcap = UK_ZCAP(cap_groups);
     __shared__ UkLine ln[JXS_MAXBLINES];
@@ -347,7 +401,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
     /* per segment (dynamic: sized for the launch's largest segment count) */
     uint16_t* s_ord = (uint16_t*)(dsm + UL.ord);
     UkSeg* s_desc = (UkSeg*)(dsm + UL.desc);
-    uint32_t* s_cnt = (uint32_t*)(dsm + UL.cnt);   /* data bits; separate signs: then signs */
+    uint32_t* s_cnt = (uint32_t*)(dsm + UL.cnt);   /* data bits (LEAN: of raw packets); separate signs: then signs */
     uint32_t* s_base = (uint32_t*)(dsm + UL.base); /* bit position of the data */
     uint32_t* s_ex = (uint32_t*)(dsm + UL.ex);
     uint32_t* s_sgb = (uint32_t*)(dsm + UL.sgb);   /* separate signs: bit position of the signs */
@@ -357,7 +411,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
     __shared__ uint32_t s_wend[JXS_MAXBLINES]; /* per line: coefficients, plus 4 times the line's first group */
     __shared__ uint32_t s_lsx[JXS_MAXBLINES + 1], s_lrx[JXS_MAXBLINES + 1]; /* per line: significance / raw GCLI bits before it */
     __shared__ uint8_t s_pkbl0[JXS_MAXPK], s_pknbl[JXS_MAXPK];
-    __shared__ uint32_t ws[UK_WARPS];
+    __shared__ uint32_t ws[UK_WARPS], ws2[UK_WARPS];
     __shared__ int s_err;
     __shared__ uint32_t s_total, s_lead, s_tw, s_off;
     __shared__ uint8_t s_g2f[JXS_MAXBL];          /* global band -> flat band */
@@ -366,7 +420,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
                                                       band lines, segments, groups per segment, run mode */
     __shared__ uint8_t s_topbl[VP ? JXS_MAXBLINES : 1], s_topprev[VP ? JXS_MAXBLINES : 1]; /* vertical prediction: the line above */
     __shared__ uint32_t s_topg[VP ? JXS_MAXBLINES : 1];
-    __shared__ int s_hasvp;
+    __shared__ int s_hasvp, s_hasraw;
 
     /* the precinct kind's tables (last row / last of several columns) */
     const int last = jxs_pkind(cfg, (uint32_t)p);
@@ -611,6 +665,10 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
             }
             if (lane == 0) s_tw = tw;
         }
+        if (LEAN) {
+            const bool any_raw = __any_sync(FULL, lane < (int)npk && pk[min(lane, JXS_MAXPK - 1)].raw);
+            if (lane == 0) s_hasraw = any_raw;
+        }
         err = __reduce_or_sync(FULL, (uint32_t)err) ? JXS_E_DEC_BITSTREAM : 0;
         if (!err && __any_sync(FULL, vp_seen)) {
             if (!VP) err = JXS_E_DEC_VPRED;
@@ -680,7 +738,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         }
         k0 = lo;
     }
-    uint32_t zc = 0;
+    uint32_t zc = 0, nc = 0; /* zeros; of them after a one */
     {
         uint32_t k = k0;
         for (uint32_t wi = wa; wi < we; wi++) {
@@ -688,12 +746,20 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
             const uint32_t i = wi - pk[k].wbase;
             const uint32_t valid = min(32u, pk[k].gbits - 32 * i);
             uint32_t z = ~bits32_at(pbuf, pk[k].gpos + 32 * i);
+            const uint32_t before = !LEAN ? 0u : i ? bits32_at(pbuf, pk[k].gpos + 32 * i - 1) : ~z >> 1;
             if (valid < 32) z &= ~(0xffffffffu >> valid);
+            if (LEAN && i == 0) pk[k].rbase = nc;
             zc += __popc(z);
+            nc += __popc(z & before);
         }
     }
-    uint32_t z0;
+    uint32_t z0, r0 = 0;
     const uint32_t ztotal = block_scan1(zc, &z0, ws);
+    if (LEAN) {
+        (void)block_scan1(nc, &r0, ws2);
+        zpre[threadIdx.x] = z0;
+        rpre[threadIdx.x] = r0;
+    }
     {
         uint32_t k = k0, ones = 0; /* ones since the last zero bit */
         for (uint32_t wi = wa; wi < we; wi++) {
@@ -701,6 +767,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
             const uint32_t i = wi - pk[k].wbase, at = pk[k].gpos + 32 * i;
             if (i == 0) {
                 pk[k].zbase = z0;
+                if (LEAN) pk[k].rbase += r0;
                 ones = 0;
             } else if (wi == wa) {
                 /* the end of the word before (32 ones: no valid codeword is
@@ -766,16 +833,57 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
                  (VP ? (uint32_t)L.vp << 22 : 0u) | ((uint32_t)myseg.bl << 24);
         s_desc[threadIdx.x] = D;
     }
+    int bad = 0;
+    if constexpr (LEAN) {
+        /* data position of every segment, then of every packet's end */
+        bool bad_pk = false;
+        for (uint32_t j = threadIdx.x; j < nseg + npk; j += UK_THREADS) {
+            const uint32_t k = j < nseg ? bls[myseg.bl].pk : j - nseg;
+            const UkPk& P = pk[k];
+            const bool vlc = P.present && !P.raw;
+            const uint32_t bits = vlc ? 4 * vlc_nibbles(pbuf, P, j < nseg ? cwbase : P.ncoded, zpre, rpre, per) : 0u;
+            if (j < nseg) s_base[j] = P.dpos + bits;
+            else bad_pk |= vlc && bits > P.dbits;
+        }
+        if (__syncthreads_or(bad_pk)) {
+            if (threadIdx.x == 0) JXS_STATUS_SET(status, JXS_E_DEC_BITSTREAM);
+            return;
+        }
+        if (s_hasraw) {
+            /* raw packets: from their GCLIs, a warp per segment */
+            for (uint32_t sidx = warp; sidx < nseg; sidx += UK_WARPS) {
+                const UkSeg D = s_desc[sidx];
+                const uint32_t n = D.info & 0xffffu, t = (D.info >> 16) & 15u;
+                uint32_t nib = 0;
+                if ((D.info >> 21) & 1u)
+                    for (uint32_t g = lane; g < n; g += 32) {
+                        const uint32_t v = bits32_at(pbuf, D.vpos + 4 * g) >> 28;
+                        nib += v > t ? v - t + 1 : 0u;
+                    }
+                nib = __reduce_add_sync(FULL, nib);
+                if (lane == 0) s_cnt[sidx] = 4 * nib;
+            }
+            __syncthreads();
+            uint32_t dbits;
+            const uint32_t b = seg_bases(threadIdx.x < nseg ? s_cnt[threadIdx.x] : 0u, myseg.bl, nseg, npk, bls, s_pkbl0, s_pknbl, s_ex,
+                                         ws, &dbits);
+            if (threadIdx.x < nseg && pk[bls[myseg.bl].pk].raw) s_base[threadIdx.x] = pk[bls[myseg.bl].pk].dpos + b;
+            if (__syncthreads_or(threadIdx.x < npk && pk[threadIdx.x].present && pk[threadIdx.x].raw && dbits > pk[threadIdx.x].dbits)) {
+                if (threadIdx.x == 0) JXS_STATUS_SET(status, JXS_E_DEC_BITSTREAM);
+                return;
+            }
+        }
+    }
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    /* a group's data: its sign nibble (signs with the data) and its planes */
+    const uint32_t fs = FS ? s_sc[3] : 0u;
+    if constexpr (!LEAN) {
     __syncthreads();
 
     /* pass 2: GCLIs from codeword values; data bits per segment.  Each lane
      * takes 4 consecutive groups: they share one significance flag, so
      * either all of them carry a codeword or none (only the segment's last
      * lane may hold fewer than 4 groups, and no lane after it holds any). */
-    int bad = 0;
-    const uint32_t lt_mask = (1u << lane) - 1u;
-    /* a group's data: its sign nibble (signs with the data) and its planes */
-    const uint32_t fs = FS ? s_sc[3] : 0u;
     for (uint32_t qi = next_seg(&s_next[0], lane); qi < nseg; qi = next_seg(&s_next[0], lane)) {
         const uint32_t sidx = s_ord[qi];
         const UkSeg D = s_desc[sidx];
@@ -883,6 +991,8 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         }
     }
 
+    } /* !LEAN */
+
     /* pass 3: data */
     const uint32_t uniform = cfg->qpih;
     if (FS && fs) {
@@ -940,12 +1050,40 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
              * with data (nibble offset in the warp's data, group, GCLI) and
              * each lane decodes one listed group at a time, so that the decode
              * work follows the groups that have data */
-            uint32_t* list = (uint32_t*)zval + 128 * warp;
+            uint32_t* list = (uint32_t*)(dsm + UL.list) + 128 * warp;
+            uint32_t cw = D.vpos;
             for (uint32_t base = 0; base < n; base += 128) {
                 const uint32_t g = base + 4 * lane;
                 const uint32_t nv = g < n ? min(4u, n - g) : 0u;
                 const uint32_t keep = nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
-                const uint32_t v4 = nv ? *(const uint32_t*)(gcl + D.z + g) & keep : 0u;
+                uint32_t v4;
+                if constexpr (LEAN) {
+                    if ((D.info >> 21) & 1u) {
+                        /* 4 raw 4-bit GCLIs, the first in the top nibble */
+                        const uint32_t w = nv ? bits32_at(pbuf, D.vpos + 4 * g) : 0u;
+                        v4 = (w >> 28) | ((w >> 16) & 0x00000f00u) | ((w >> 4) & 0x000f0000u) | ((w << 8) & 0x0f000000u);
+                    } else {
+                        /* the groups of 8 in lanes 2i, 2i + 1 share flag i, so
+                         * that a lane's groups all carry a codeword or none
+                         * (only the segment's last lane may hold fewer than 4) */
+                        bool coded = nv != 0;
+                        if ((D.info >> 20) & 1u) coded = coded && !((bits32_at(pbuf, D.sig + (base >> 3)) >> (31 - (lane >> 1))) & 1u);
+                        const uint32_t bal = __ballot_sync(FULL, coded);
+                        v4 = t * 0x01010101u;
+                        if (coded) {
+                            const uint32_t c = cw + 4 * __popc(bal & lt_mask);
+                            const uint32_t* zw = (const uint32_t*)(zval + (c & ~3u));
+                            const uint32_t r4 = __funnelshift_r(zw[0], zw[1], 8 * (c & 3u)) & keep;
+                            /* GCLI = gtli + value, at most 15 (values are below 128) */
+                            if ((r4 + (112u + t) * 0x01010101u) & 0x80808080u) bad = 1;
+                            else v4 += r4;
+                        }
+                        cw += 4 * __popc(bal);
+                    }
+                    v4 &= keep;
+                } else {
+                    v4 = nv ? *(const uint32_t*)(gcl + D.z + g) & keep : 0u;
+                }
                 /* per byte: v > t, and the data nibbles of such a group (v - t
                  * + 1); running sums over the lane's bytes, then one scan for
                  * the nibbles and the listed groups */
@@ -1198,7 +1336,7 @@ __global__ void __launch_bounds__(UK_THREADS) unpack_vpred_kernel(const jxs_cfg_
                                                                   uint32_t cap_groups, uint32_t cap_seg, int* status) {
     extern __shared__ __align__(16) uint8_t dsm[];
     __shared__ uint8_t top_t[JXS_MAXBLINES];
-    uint8_t* top_gcl = dsm + uk_layout(cap_bytes, cap_groups, cap_seg).top;
+    uint8_t* top_gcl = dsm + uk_layout(cap_bytes, cap_groups, cap_seg, false).top;
     const uint32_t s = blockIdx.x, ncol = cfg->ncol;
     const uint32_t first = s * cfg->pps, end = min(cfg->np, first + cfg->pps);
     for (uint32_t col = 0; col < ncol; col++) {
@@ -1258,7 +1396,7 @@ extern "C" cudaError_t jxs_launch_walk(const jxs_cfg_t* dcfg, uint32_t nslices, 
 template <bool FS>
 static cudaError_t unpack_one(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t bs_size, const uint32_t* prec_off, int16_t* coef,
                               uint32_t np, uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg, int* status, cudaStream_t st) {
-    const size_t smem = uk_layout(cap_bytes, cap_groups, cap_seg).end;
+    const size_t smem = uk_layout(cap_bytes, cap_groups, cap_seg, !FS).end;
     static std::atomic<int> attr[JXS_MAX_DEV];
     cudaError_t e = jxs_smem_attr(unpack_kernel<FS>, (int)smem, attr);
     if (e != cudaSuccess) return e;
@@ -1286,7 +1424,7 @@ extern "C" cudaError_t jxs_launch_walk_batch(const DecPrecLaunch* L, cudaStream_
 
 template <bool FS>
 static cudaError_t unpack_batch_one(const DecPrecLaunch* L, uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg, cudaStream_t st) {
-    const size_t smem = uk_layout(cap_bytes, cap_groups, cap_seg).end;
+    const size_t smem = uk_layout(cap_bytes, cap_groups, cap_seg, !FS).end;
     static std::atomic<int> attr[JXS_MAX_DEV];
     cudaError_t e = jxs_smem_attr(unpack_batch_kernel<FS>, (int)smem, attr);
     if (e != cudaSuccess) return e;
@@ -1303,7 +1441,7 @@ extern "C" cudaError_t jxs_launch_unpack_batch(const DecPrecLaunch* L, uint32_t 
 extern "C" cudaError_t jxs_launch_unpack_vpred(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t bs_size, const uint32_t* prec_off,
                                                int16_t* coef, uint32_t nslices, uint32_t cap_bytes, uint32_t cap_groups,
                                                uint32_t cap_seg, int* status, cudaStream_t st) {
-    const size_t smem = uk_layout(cap_bytes, cap_groups, cap_seg).top_end;
+    const size_t smem = uk_layout(cap_bytes, cap_groups, cap_seg, false).top_end;
     static std::atomic<int> attr[JXS_MAX_DEV];
     cudaError_t e = jxs_smem_attr(unpack_vpred_kernel, (int)smem, attr);
     if (e != cudaSuccess) return e;

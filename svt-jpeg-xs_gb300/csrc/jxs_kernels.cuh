@@ -248,18 +248,21 @@ struct DecPrecLaunch {
 /* 128 list entries per warp of a 512-thread unpacking block */
 #define UK_LIST_BYTES (4 * 128 * 16)
 struct UkLayout {
-    uint32_t gcl, zval, desc, cnt, base, ex, sgb, ord, end, top, top_end;
+    uint32_t gcl, zval, list, desc, cnt, base, ex, sgb, ord, end, top, top_end;
 };
-static inline __host__ __device__ UkLayout uk_layout(uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg) {
+static inline __host__ __device__ UkLayout uk_layout(uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg, bool lean) {
     UkLayout L;
     uint32_t o = cap_bytes + 32;
     L.gcl = o;
-    o = (o + cap_groups + 15) & ~15u;
+    if (!lean) o = (o + cap_groups + 15) & ~15u;
+    /* each warp's list of groups with data in the data pass (UK_LIST_BYTES):
+     * in the place of the codeword values where those are done with */
+    L.list = o;
+    if (lean) o = (o + UK_LIST_BYTES + 15) & ~15u;
     L.zval = o;
-    /* the codeword values (read 8 bytes at a time from any multiple of 4);
-     * in the data pass the same area holds each warp's list of groups with
-     * data (UK_LIST_BYTES) */
-    o = (o + (UK_ZCAP(cap_groups) + 8 > UK_LIST_BYTES ? UK_ZCAP(cap_groups) + 8 : UK_LIST_BYTES) + 15) & ~15u;
+    /* the codeword values, read 8 bytes at a time from any multiple of 4 */
+    const uint32_t z = UK_ZCAP(cap_groups) + 8;
+    o = (o + (lean || z > UK_LIST_BYTES ? z : UK_LIST_BYTES) + 15) & ~15u;
     L.desc = o;
     o += 16 * cap_seg;
     L.cnt = o;
@@ -285,7 +288,7 @@ static inline uint32_t uk_reserved(uint32_t cap_groups, uint32_t cap_seg, int or
     o = (o + (2 * UK_ZCAP(cap_groups) > UK_LIST_BYTES ? 2 * UK_ZCAP(cap_groups) : UK_LIST_BYTES) + 15) & ~15u;
     o = (o + 30 * cap_seg + 4 + 15) & ~15u;
     if (ordered) o = (o + cap_groups + 15) & ~15u;
-    const UkLayout L = uk_layout(0, cap_groups, cap_seg);
+    const UkLayout L = uk_layout(0, cap_groups, cap_seg, false);
     const uint32_t need = ordered ? L.top_end : L.end;
     return o > need ? o : need;
 }
