@@ -11,6 +11,7 @@
  *  walk_*_kernel   precinct offsets of a device-resident codestream.
  * The inverse transform is in jxs_inv_dwt.cu.
  */
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -380,7 +381,8 @@ template <bool FS, bool VP, bool BATCH>
 __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t bs_size,
                                             const uint32_t* __restrict__ prec_off, int16_t* __restrict__ coef,
                                             uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg, int* status, const int p,
-                                            uint8_t* top_gcl, uint8_t* top_t, const int vp_ok) {
+                                            uint8_t* top_gcl, uint8_t* top_t, const int vp_ok, const int rank = 0,
+                                            const int turns = 0) {
     extern __shared__ __align__(16) uint8_t dsm[];
     /* signs with the data, no prediction: the segments' data positions come
      * from the unary codes' bits and the GCLIs are read in the data pass */
@@ -517,7 +519,15 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         begin();
     }
     __syncthreads();
-    if (s_err) return;
+    /* VP: a row that fails before its turn leaves it, and the others', in step */
+    auto leave = [&]() {
+        if constexpr (VP)
+            for (int i = 0; i < turns; i++) cooperative_groups::this_cluster().sync();
+    };
+    if (s_err) {
+        leave();
+        return;
+    }
     const uint32_t off = s_off;
     const uint32_t total = s_total, lead = s_lead;
     {
@@ -688,6 +698,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
     __syncthreads();
     if (s_err) {
         if (threadIdx.x == 0) JXS_STATUS_SET(status, s_err);
+        leave();
         return;
     }
 
@@ -818,6 +829,7 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
     __syncthreads();
     if (s_err) {
         if (threadIdx.x == 0) JXS_STATUS_SET(status, s_err);
+        leave();
         return;
     }
     /* the segments' records */
@@ -935,47 +947,69 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         if (lane == 0) s_cnt[sidx] = 4 * dsum;
     }
     __syncthreads();
-    if (VP && s_hasvp) {
-        /* vertical prediction (unpack_verical_pred_gclis_*, Packing.c:267-431):
-         * GCLI = the predictor max(top, max(gtli_top, gtli)) moved by the
-         * codeword value; without a codeword (insignificant group) the
-         * predictor, or gtli in run mode.  Line levels in order: line l reads
-         * line l - 1 of its band (line 0: the row above, top_gcl). */
-        const uint32_t rm = s_sc[8];
-        for (uint32_t lvl = 0; lvl < 4; lvl++) {
-            for (uint32_t sidx = warp; sidx < nseg; sidx += UK_WARPS) {
-                const UkSeg D = s_desc[sidx];
-                const uint32_t bl = D.info >> 24, n = D.info & 0xffffu, lt = (D.info >> 16) & 15u;
-                if (!((D.info >> 22) & 1u) || bls[bl].line != lvl) continue;
-                const uint32_t tb = s_topbl[bl];
-                const int from_prev = s_topprev[bl];
-                const uint8_t* src = (from_prev ? top_gcl : gcl) + s_topg[bl] + (D.z - bls[bl].gbase);
-                const uint32_t tt = max(from_prev ? (uint32_t)top_t[tb] : (uint32_t)ln[tb].t, lt);
-                uint32_t dsum = 0;
-                for (uint32_t g = lane; g < n; g += 32) {
-                    const uint32_t x = gcl[D.z + g];
-                    const uint32_t mt = max((uint32_t)src[g], tt);
-                    uint32_t v;
-                    if (x == 0xffu) {
-                        v = rm ? lt : mt;
-                    } else {
-                        const uint32_t thr = mt > lt ? mt - lt : 0u;
-                        int d = 0;
-                        if (x > 2 * thr) d = (int)(x - thr);
-                        else if (x > 0) d = (x & 1) ? -(int)((x + 1) >> 1) : (int)(x >> 1);
-                        v = (uint32_t)((int)mt + d);
+    if constexpr (VP) {
+        /* the slice's rows in their order: each resolves its own and hands its
+         * GCLIs and gtlis to the block of the next */
+        cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+        for (int turn = 0; turn < turns; turn++) {
+            if (turn == rank) {
+                if (s_hasvp) {
+                /* vertical prediction (unpack_verical_pred_gclis_*, Packing.c:267-431):
+                 * GCLI = the predictor max(top, max(gtli_top, gtli)) moved by the
+                 * codeword value; without a codeword (insignificant group) the
+                 * predictor, or gtli in run mode.  Line levels in order: line l reads
+                 * line l - 1 of its band (line 0: the row above, top_gcl). */
+                    const uint32_t rm = s_sc[8];
+                    for (uint32_t lvl = 0;; lvl++) {
+                        bool more = false; /* lines below this level */
+                        for (uint32_t sidx = warp; sidx < nseg; sidx += UK_WARPS) {
+                            const UkSeg D = s_desc[sidx];
+                            const uint32_t bl = D.info >> 24, n = D.info & 0xffffu, lt = (D.info >> 16) & 15u;
+                            if (!((D.info >> 22) & 1u)) continue;
+                            more |= bls[bl].line > lvl;
+                            if (bls[bl].line != lvl) continue;
+                            const uint32_t tb = s_topbl[bl];
+                            const int from_prev = s_topprev[bl];
+                            /* in both rows a line starts at a multiple of 4 */
+                            const uint8_t* src = (from_prev ? top_gcl : gcl) + s_topg[bl] + (D.z - bls[bl].gbase);
+                            const uint32_t tt = max(from_prev ? (uint32_t)top_t[tb] : (uint32_t)ln[tb].t, lt);
+                            uint32_t dsum = 0;
+                            for (uint32_t g = 4 * lane; g < n; g += 128) {
+                                const uint32_t x4 = *(const uint32_t*)(gcl + D.z + g), m4 = *(const uint32_t*)(src + g);
+                                uint32_t v4 = 0;
+#pragma unroll
+                                for (int k = 0; k < 2; k++) {
+                                    /* two GCLIs in 16-bit halves: x > 2 thr moves the
+                                     * predictor by x - thr, a smaller odd x by -(x + 1)
+                                     * / 2, an even one by x / 2 */
+                                    const uint32_t x = (x4 >> (8 * k)) & 0x00ff00ffu;
+                                    const uint32_t mt = __vmaxu2((m4 >> (8 * k)) & 0x00ff00ffu, tt * 0x00010001u);
+                                    const uint32_t up = __vcmpgtu2(x, 2u * (mt - lt * 0x00010001u)), none = __vcmpeq2(x, 0x00ff00ffu);
+                                    const uint32_t odd = (x & 0x00010001u) * 0xffffu, half = (x >> 1) & 0x007f007fu;
+                                    const uint32_t moved = __vadd2(mt, half ^ odd), far = x + lt * 0x00010001u;
+                                    const uint32_t v = (none & (rm ? lt * 0x00010001u : mt)) | (~none & ((up & far) | (~up & moved)));
+                                    bad |= (__vcmpgtu2(v, 0x000f000fu) & (g + k + 2 < n ? 0xffffffffu : g + k < n ? 0xffffu : 0u)) != 0u;
+                                    v4 |= __vminu2(v, 0x000f000fu) << (8 * k);
+                                }
+                                const uint32_t nv = min(4u, n - g), keep = nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
+                                *(uint32_t*)(gcl + D.z + g) = v4;
+                                const uint32_t y = ((v4 & keep) | 0x80808080u) - (lt + 1) * 0x01010101u;
+                                const uint32_t above = sign_bytes(y), one = above & 0x01010101u;
+                                dsum += __dp4a((y & above & 0x7f7f7f7fu) + (fs ? one : 2u * one), 0x01010101u, 0u);
+                            }
+                            dsum = __reduce_add_sync(FULL, dsum);
+                            if (lane == 0) s_cnt[sidx] = 4 * dsum;
+                        }
+                        if (!__syncthreads_or(more)) break;
                     }
-                    if (v > 15) {
-                        bad = 1;
-                        v = 15;
-                    }
-                    gcl[D.z + g] = (uint8_t)v;
-                    if (v > lt) dsum += 4 * (v - lt + (fs ? 0u : 1u));
                 }
-                dsum = __reduce_add_sync(FULL, dsum);
-                if (lane == 0) s_cnt[sidx] = dsum;
+                const int next = rank + 1 == turns ? 0 : rank + 1;
+                uint32_t* to = cl.map_shared_rank((uint32_t*)top_gcl, next);
+                uint8_t* tot = cl.map_shared_rank(top_t, next);
+                for (uint32_t i = threadIdx.x; i < (cap_groups >> 2); i += blockDim.x) to[i] = ((const uint32_t*)gcl)[i];
+                for (uint32_t x = threadIdx.x; x < nbl; x += blockDim.x) tot[x] = ln[x].t;
             }
-            __syncthreads();
+            cl.sync();
         }
     }
     {
@@ -1216,11 +1250,6 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
         }
     }
     if (__syncthreads_or(bad) && threadIdx.x == 0) JXS_STATUS_SET(status, JXS_E_DEC_BITSTREAM);
-    if (VP) {
-        /* slice-ordered decoding: this row is the next one's row above */
-        for (uint32_t i = threadIdx.x; i < (cap_groups >> 2); i += blockDim.x) ((uint32_t*)top_gcl)[i] = ((const uint32_t*)gcl)[i];
-        for (uint32_t x = threadIdx.x; x < nbl; x += blockDim.x) top_t[x] = ln[x].t;
-    }
 }
 
 /* ------------------------------------------------------------------------ */
@@ -1326,10 +1355,17 @@ __global__ void __launch_bounds__(UK_THREADS, 4) unpack_batch_kernel(const __gri
                            (int)blockIdx.x - F.first_block, nullptr, nullptr, 0);
 }
 
-/* Streams with vertical prediction: one block per slice, its precinct rows
- * in order, each predicting from the row above (kept in shared memory after
- * the zero-bit table: cap_groups bytes); with several precinct columns,
- * column after column (the precinct above is in the same column). */
+/* Streams with vertical prediction: a cluster of blocks per slice, a
+ * precinct row each (more rows than blocks: in rounds).  Only the GCLIs
+ * depend on the row above; parsing, codeword values and coefficients of the
+ * slice's rows run side by side, the GCLIs in turns with a cluster barrier
+ * after each, handed on through the next block's shared memory (after the
+ * codeword values: cap_groups bytes).  With several precinct columns, column
+ * after column (the precinct above is in the same column).  Every block takes
+ * the same number of barriers, failed rows and rows past the slice's end
+ * included.  Bound by the latency of one precinct and the turns, which take
+ * two GCLIs to an instruction: 1279x717 4:4:4 with slices of 4 rows 116 us
+ * with a block per slice and a GCLI per lane, 48 us now. */
 __global__ void __launch_bounds__(UK_THREADS) unpack_vpred_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs,
                                                                   uint32_t bs_size, const uint32_t* __restrict__ prec_off,
                                                                   int16_t* __restrict__ coef, uint32_t cap_bytes,
@@ -1337,16 +1373,24 @@ __global__ void __launch_bounds__(UK_THREADS) unpack_vpred_kernel(const jxs_cfg_
     extern __shared__ __align__(16) uint8_t dsm[];
     __shared__ uint8_t top_t[JXS_MAXBLINES];
     uint8_t* top_gcl = dsm + uk_layout(cap_bytes, cap_groups, cap_seg, false).top;
-    const uint32_t s = blockIdx.x, ncol = cfg->ncol;
+    cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+    const uint32_t turns = cl.num_blocks(), rank = cl.block_rank();
+    const uint32_t s = blockIdx.x / turns, ncol = cfg->ncol;
     const uint32_t first = s * cfg->pps, end = min(cfg->np, first + cfg->pps);
+    cl.sync(); /* every block runs before another writes to it */
     for (uint32_t col = 0; col < ncol; col++) {
-        for (uint32_t row = first; row < end; row++) {
-            unpack_body<true, true, false>(cfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status, (int)(row * ncol + col),
-                                    top_gcl, top_t, row != first);
-            __syncthreads();
-            if (*(volatile int*)status) return;
+        for (uint32_t row0 = first; row0 < end; row0 += turns) {
+            const uint32_t row = row0 + rank;
+            if (row < end) {
+                unpack_body<true, true, false>(cfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status,
+                                               (int)(row * ncol + col), top_gcl, top_t, row != first, (int)rank, (int)turns);
+                __syncthreads();
+            } else {
+                for (uint32_t i = 0; i < turns; i++) cl.sync();
+            }
         }
     }
+    cl.sync(); /* and until none does any more */
 }
 
 __global__ void walk_slices_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size,
@@ -1439,12 +1483,22 @@ extern "C" cudaError_t jxs_launch_unpack_batch(const DecPrecLaunch* L, uint32_t 
 }
 
 extern "C" cudaError_t jxs_launch_unpack_vpred(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t bs_size, const uint32_t* prec_off,
-                                               int16_t* coef, uint32_t nslices, uint32_t cap_bytes, uint32_t cap_groups,
-                                               uint32_t cap_seg, int* status, cudaStream_t st) {
+                                               int16_t* coef, uint32_t nslices, uint32_t pps, uint32_t cap_bytes,
+                                               uint32_t cap_groups, uint32_t cap_seg, int* status, cudaStream_t st) {
     const size_t smem = uk_layout(cap_bytes, cap_groups, cap_seg, false).top_end;
     static std::atomic<int> attr[JXS_MAX_DEV];
     cudaError_t e = jxs_smem_attr(unpack_vpred_kernel, (int)smem, attr);
     if (e != cudaSuccess) return e;
-    return jxs_launch(unpack_vpred_kernel, dim3((unsigned)nslices), UK_THREADS, smem, st, dcfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg,
-                                                           status);
+    /* a block per row of a slice, up to the 8 that every device takes, while
+     * the blocks are all resident (2 to an SM by their registers, fewer by
+     * their shared memory): beyond that they wait in place of others' work.
+     * 1, 2, 4, 8 blocks: 1279x717 in 45 slices of 4 rows 123, 92, 83 us,
+     * 3840x2160 in 135 158, 131, 146 us, in 34 of 16 rows 419, 283, 211,
+     * 359 us, 7680x4320 in 270 of 4 rows 283, 302, 337 us */
+    const unsigned resident = 152 * (2 * (smem + UK_STATIC_SMEM) <= 228 * 1024 ? 2 : 1);
+    unsigned cluster = 8;
+    while (cluster > 1 && nslices * (cluster < pps ? cluster : pps) > resident) cluster >>= 1;
+    if (cluster > pps) cluster = pps;
+    return jxs_launch_cluster(unpack_vpred_kernel, dim3((unsigned)nslices), cluster, UK_THREADS, smem, st, dcfg, bs, bs_size, prec_off,
+                              coef, cap_bytes, cap_groups, cap_seg, status);
 }

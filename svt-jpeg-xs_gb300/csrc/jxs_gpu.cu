@@ -893,7 +893,7 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
     TMARK(1);
     KMARK();
     if (d->vpred)
-        CK(jxs_launch_unpack_vpred(d->dcfg, dbs, size, doff, s->coef, c->nslices, d->cap_bytes, d->cap_groups, d->cap_seg,
+        CK(jxs_launch_unpack_vpred(d->dcfg, dbs, size, doff, s->coef, c->nslices, c->pps, d->cap_bytes, d->cap_groups, d->cap_seg,
                                    s->status, st));
     else
         CK(jxs_launch_unpack(d->dcfg, dbs, size, doff, s->coef, c->nprec, d->cap_bytes, d->cap_groups, d->cap_seg, (int)c->fs,

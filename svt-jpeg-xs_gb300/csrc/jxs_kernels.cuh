@@ -332,6 +332,28 @@ static inline cudaError_t jxs_smem_attr(K kern, int bytes, std::atomic<int>* cac
 #ifdef __CUDACC__
 __device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+/* grid.x clusters of `cluster` blocks each */
+template <typename... P, typename... A>
+static inline cudaError_t jxs_launch_cluster(void (*kern)(P...), dim3 grid, unsigned cluster, unsigned block, size_t smem, cudaStream_t st,
+                                             A&&... args) {
+    cudaLaunchAttribute at[2];
+    memset(at, 0, sizeof(at));
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    at[1].id = cudaLaunchAttributeClusterDimension;
+    at[1].val.clusterDim.x = cluster;
+    at[1].val.clusterDim.y = 1;
+    at[1].val.clusterDim.z = 1;
+    cudaLaunchConfig_t c;
+    memset(&c, 0, sizeof(c));
+    c.gridDim = dim3(grid.x * cluster, grid.y, grid.z);
+    c.blockDim = dim3(block);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = at;
+    c.numAttrs = 2;
+    return cudaLaunchKernelEx(&c, kern, std::forward<A>(args)...);
+}
 template <typename... P, typename... A>
 static inline cudaError_t jxs_launch(void (*kern)(P...), dim3 grid, unsigned block, size_t smem, cudaStream_t st, A&&... args) {
     cudaLaunchAttribute at;
