@@ -1137,53 +1137,10 @@ DEV uint32_t coefs_to_planes(uint32_t x) {
     return dswap(x, 14, 0x0000ccccu);
 }
 
-/* Data bits of one 4-coefficient group with GCLI v > gtli t
- * (pack_data_c, PackPrecinct.c:128-198): bit-planes v-1 .. t, each a
- * nibble (coefficient 0 in the most significant bit).  Quantization
- * (Quant.c:9-45) is skipped for t == 0 like the reference
- * (QuantStageProcess.c:18-31).  `signs` receives the sign nibble, which has
- * a bit only for a non-zero quantized magnitude, and `nzm` the non-zero
- * magnitudes, both with coefficient 0 in bit 3.  Without sign handling the
- * sign nibble leads the group's data; with it the signs of the non-zero
- * magnitudes go to the packet's sign sub-packet (pack_sign_c, :200-233). */
-DEV uint64_t data_chunk(uint2 raw4, int wleft, uint32_t v, uint32_t t, uint32_t uniform, uint32_t& signs, uint32_t& nzm) {
-    /* coefficients past the band width are zero */
-    uint32_t c01 = raw4.x & ((wleft > 1 ? 0xffff0000u : 0u) | 0xffffu);
-    uint32_t c23 = raw4.y & ((wleft > 2 ? 0xffffu : 0u) | (wleft > 3 ? 0xffff0000u : 0u));
-    uint32_t P01, P23;
-    if (t == 0) {
-        P01 = c01 & 0x7fff7fffu;
-        P23 = c23 & 0x7fff7fffu;
-    } else if (!uniform) {
-        /* deadzone: magnitude >> t, two coefficients per word */
-        const uint32_t keep = (0x7fffu >> t) * 0x00010001u;
-        P01 = ((c01 & 0x7fff7fffu) >> t) & keep;
-        P23 = ((c23 & 0x7fff7fffu) >> t) & keep;
-    } else {
-        uint32_t q[4];
-        const uint32_t c[4] = {c01 & 0xffffu, c01 >> 16, c23 & 0xffffu, c23 >> 16};
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const uint32_t m = c[k] & 0x7fffu;
-            /* computed in int like the reference, truncated to 16 bits */
-            const uint32_t u = (((m << (v - t + 1)) - m + (1u << v)) >> (v + 1)) & 0xffffu;
-            q[k] = ((u << t) & 0xffffu) >> t;
-        }
-        P01 = q[0] | (q[1] << 16);
-        P23 = q[2] | (q[3] << 16);
-    }
-    const uint32_t n01 = __vcmpne2(P01, 0u), n23 = __vcmpne2(P23, 0u);
-    nzm = ((n01 << 3) & 8u) | ((n01 >> 14) & 4u) | ((n23 << 1) & 2u) | (n23 >> 31);
-    const uint32_t s01 = n01 & c01 & 0x80008000u, s23 = n23 & c23 & 0x80008000u;
-    signs = ((s01 >> 12) & 8u) | ((s01 >> 29) & 4u) | ((s23 >> 14) & 2u) | (s23 >> 31);
-    /* byte 3 - c of the word = low 8 plane bits of coefficient c */
-    uint64_t planes = coefs_to_planes(__byte_perm(P01, P23, 0x0246));
-    if (v - t > 8) planes |= (uint64_t)coefs_to_planes(__byte_perm(P01, P23, 0x1357)) << 32;
-    return planes;
-}
-
-/* A group's quantized magnitudes as 16-bit pairs (coefficients 0 | 1 << 16
- * and 2 | 3 << 16) with the sign of every coefficient that stays non-zero as
+/* A group's (pack_data_c, PackPrecinct.c:128-198; quantization, Quant.c:9-45,
+ * is skipped for t = 0 like the reference, QuantStageProcess.c:18-31)
+ * quantized magnitudes as 16-bit pairs (coefficients 0 | 1 << 16 and 2 | 3 <<
+ * 16) with the sign of every coefficient that stays non-zero as
  * plane v - t, above the magnitude: one transpose then gives the sign nibble
  * and the planes.  For signs with the data and a group whose coefficients
  * past the band width are stored as zero; uq: uniform quantization, t > 0
@@ -1210,6 +1167,15 @@ DEV void quantize_signed(uint2 raw4, uint32_t v, uint32_t t, bool uq, uint32_t& 
      * ones; the sign moves to bit np (<= 15) */
     P01 |= ((P01 + 0x7fff7fffu) & c01 & 0x80008000u) >> (15 - np);
     P23 |= ((P23 + 0x7fff7fffu) & c23 & 0x80008000u) >> (15 - np);
+}
+
+/* Bits 15 and 31 where the quantized magnitudes of two coefficients are not
+ * zero: under deadzone quantization m >= 2^t, under uniform quantization
+ * m (2^(v-t+1) - 1) >= 2^v. */
+DEV uint32_t nonzero_flags(uint32_t c, uint32_t v, uint32_t t, bool uq) {
+    if (!uq) return (((c >> t) & (0x7fffu >> t) * 0x00010001u) + 0x7fff7fffu) & 0x80008000u;
+    const uint32_t k = (2u << (v - t)) - 1u, least = 1u << v;
+    return ((c & 0x7fffu) * k >= least ? 0x8000u : 0u) | (((c >> 16) & 0x7fffu) * k >= least ? 0x80000000u : 0u);
 }
 
 /* A segment as pass B reads it: bit positions of its first GCLI code and
@@ -1427,7 +1393,6 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
         const uint32_t t = s_lt[sg.bl];
         const uint8_t* grow = gcli + s_grow[sg.bl];
         const uint16_t* crow = coef + s_crow[sg.bl];
-        const int bw = (int)bls[sg.bl].w;
         const uint32_t gend = min(sg.g0 + SG, bls[sg.bl].gcli_w);
         uint32_t dsum = 0, vsum = 0, zsum = 0, nsum = 0, pnsum = 0, prsum = 0;
         for (uint32_t base = sg.g0; base < gend; base += 128) {
@@ -1468,15 +1433,11 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
             }
             if (fs && m > t) {
                 const uint4 c0 = *(const uint4*)(crow + 4 * g), c1 = *(const uint4*)(crow + 4 * g + 8);
-                const uint2 cw[4] = {make_uint2(c0.x, c0.y), make_uint2(c0.z, c0.w), make_uint2(c1.x, c1.y), make_uint2(c1.z, c1.w)};
+                const uint32_t cw[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
 #pragma unroll
                 for (int k = 0; k < 4; k++) {
                     const uint32_t v = (w4 >> (8 * k)) & 255u;
-                    if (k < (int)nv && v > t) {
-                        uint32_t sgn, nzm;
-                        (void)data_chunk(cw[k], bw - 4 * (int)(g + k), v, t, uniform, sgn, nzm);
-                        nsum += __popc(nzm);
-                    }
+                    if (k < (int)nv && v > t) nsum += __popc(nonzero_flags(cw[2 * k], v, t, uniform && t) | nonzero_flags(cw[2 * k + 1], v, t, uniform && t) >> 1);
                 }
             }
         }
@@ -1829,8 +1790,7 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
     } else {
         /* pass B with signs in a sub-packet of their own or predicted codes:
          * each lane 4 consecutive groups; its unary codes are joined into one
-         * write, its data chunks into writes of up to 64 bits, its signs into
-         * one write */
+         * write, then a listed group's data and signs into one each */
         for (uint32_t qi = queue_next(&s_q[1], lane); qi < nseg; qi = queue_next(&s_q[1], lane)) {
             const uint32_t sidx = s_ord[qi];
             const jxs_seg_t sg = segs[sidx];
@@ -1847,11 +1807,6 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
                 /* the lane's GCLIs, one per byte (0 past the line's end) */
                 uint32_t w4 = nv ? *(const uint32_t*)(grow + g) : 0u;
                 w4 &= nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
-                uint4 c0 = make_uint4(0, 0, 0, 0), c1 = c0;
-                if (nv && fs) {
-                    c0 = *(const uint4*)(crow + 4 * g);
-                    c1 = *(const uint4*)(crow + 4 * g + 8);
-                }
                 /* per byte: planes above gtli d = max(v - t, 0), and v > t */
                 const uint32_t t4 = t * 0x01010101u;
                 const uint32_t d4 = __vsubus4(w4, t4), s4 = __vcmpgtu4(w4, t4);
@@ -1959,86 +1914,60 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
                         put_bits(buf, words, vpos + ex_v, vacc, vl, ovf);
                     }
                 }
-                uint32_t sbits = 0, sn = 0;
-                if (!fs) {
-                    /* signs with the data: the warp lists its groups with GCLI
-                     * > gtli (bit offset in the warp's data, group, GCLI), then
-                     * each lane packs one listed group at a time, its sign
-                     * nibble and planes in one write of at most 64 bits; the
-                     * coefficients of the other groups are never read */
-                    uint32_t* list = &s_segw[0][0] + 128 * warp;
-                    const uint32_t cnt = __reduce_add_sync(FULL, nsig);
-                    {
-                        /* per byte: 1 for a listed group, and its data nibbles
-                         * v - t + 1; their exclusive prefix sums over the
-                         * lane's bytes give each entry's slot and offset */
-                        const uint32_t one = s4 & 0x01010101u, dd = d4 + one;
-                        const uint32_t po = dd * 0x01010100u, pi = one * 0x01010100u;
-                        const uint32_t e0 = (ex_d << 11) | ((uint32_t)lane << 6), i0 = ex >> 25;
+                /* the warp lists its groups above gtli (bit offset in the warp's
+                 * data, group, GCLI), then each lane packs one listed group at a
+                 * time; the coefficients of the other groups are never read */
+                uint32_t* list = &s_segw[0][0] + 128 * warp;
+                const uint32_t cnt = __reduce_add_sync(FULL, nsig);
+                {
+                    /* per byte: 1 for a listed group, and its data nibbles v -
+                     * t + 1 (v - t with separate signs); their exclusive prefix
+                     * sums over the lane's bytes give each entry's slot and
+                     * offset */
+                    const uint32_t one = s4 & 0x01010101u, dd = fs ? d4 : d4 + one;
+                    const uint32_t po = dd * 0x01010100u, pi = one * 0x01010100u;
+                    const uint32_t e0 = (ex_d << 11) | ((uint32_t)lane << 6), i0 = ex >> 25;
 #pragma unroll
-                        for (int k = 0; k < 4; k++)
-                            if ((one >> (8 * k)) & 1u)
-                                list[i0 + ((pi >> (8 * k)) & 255u)] = e0 + (((po >> (8 * k)) & 255u) << 13) + ((uint32_t)k << 4) + v[k];
-                    }
-                    __syncwarp();
-                    for (uint32_t r = lane; r < cnt; r += 32) {
-                        const uint32_t e = list[r];
+                    for (int k = 0; k < 4; k++)
+                        if ((one >> (8 * k)) & 1u)
+                            list[i0 + ((pi >> (8 * k)) & 255u)] = e0 + (((po >> (8 * k)) & 255u) << 13) + ((uint32_t)k << 4) + v[k];
+                }
+                __syncwarp();
+                for (uint32_t r0 = 0; r0 < cnt; r0 += 32) {
+                    const bool have = r0 + lane < cnt;
+                    uint32_t sbits = 0, sn = 0;
+                    if (have) {
+                        const uint32_t e = list[r0 + lane];
                         const uint32_t gi = base + ((e >> 4) & 127u), vv = e & 15u, np = vv - t;
                         /* the coefficients past the band width are stored as zero */
                         const uint2 raw4 = *(const uint2*)(crow + 4 * gi);
                         uint32_t P01, P23;
-                        quantize_signed(raw4, vv, t, uniform && t, P01, P23);
+                        quantize_signed(fs ? make_uint2(raw4.x & 0x7fff7fffu, raw4.y & 0x7fff7fffu) : raw4, vv, t, uniform && t, P01, P23);
                         uint64_t planes = coefs_to_planes(__byte_perm(P01, P23, 0x0246));
                         if (np >= 8) planes |= (uint64_t)coefs_to_planes(__byte_perm(P01, P23, 0x1357)) << 32;
-                        put_bits(buf, words, dpos + (e >> 11), planes, 4 * (np + 1), ovf);
-                    }
-                    __syncwarp();
-                } else if (dl4) {
-                    /* data bits of the groups with gcli > gtli (pack_data_c,
-                     * PackPrecinct.c:128-198), joined while they fit 64 bits */
-                    uint32_t pos = dpos + ex_d;
-                    uint64_t acc = 0;
-                    uint32_t an = 0;
-                    const uint2 cw[4] = {make_uint2(c0.x, c0.y), make_uint2(c0.z, c0.w), make_uint2(c1.x, c1.y), make_uint2(c1.z, c1.w)};
+                        put_bits(buf, words, dpos + (e >> 11), planes, 4 * (np + 1 - fs), ovf);
+                        if (fs) {
+                            /* the signs of the non-zero magnitudes (pack_sign_c,
+                             * PackPrecinct.c:200-233), coefficient 0 first */
+                            const uint32_t z01 = (P01 + 0x7fff7fffu) & 0x80008000u, z23 = (P23 + 0x7fff7fffu) & 0x80008000u;
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        if (k < (int)nv && v[k] > t) {
-                            const uint32_t np = v[k] - t, n = 4 * (np + 1 - fs);
-                            uint32_t sgn, nzm;
-                            uint64_t ch = data_chunk(cw[k], (int)B.w - 4 * (int)(g + k), v[k], t, uniform, sgn, nzm);
-                            if (fs) {
-                                /* the signs of the non-zero magnitudes, coefficient 0 first */
-#pragma unroll
-                                for (int j = 3; j >= 0; j--) {
-                                    if ((nzm >> j) & 1u) {
-                                        sbits = (sbits << 1) | ((sgn >> j) & 1u);
-                                        sn++;
-                                    }
-                                }
-                            } else {
-                                ch |= (uint64_t)sgn << (4 * np);
+                            for (int j = 0; j < 4; j++) {
+                                const uint32_t at = 15 + 16 * (j & 1), on = ((j < 2 ? z01 : z23) >> at) & 1u;
+                                sbits = (sbits << on) | (on & ((j < 2 ? raw4.x : raw4.y) >> at));
+                                sn += on;
                             }
-                            if (an + n > 64) {
-                                put_bits(buf, words, pos, acc, an, ovf);
-                                pos += an;
-                                acc = 0;
-                                an = 0;
-                            }
-                            acc = n == 64 ? ch : (acc << n) | ch;
-                            an += n;
                         }
                     }
-                    if (an) put_bits(buf, words, pos, acc, an, ovf);
+                    if (fs) {
+                        uint32_t stot;
+                        const uint32_t sx = warp_excl_scan(sn, &stot);
+                        if (sn) put_bits(buf, words, npos + sx, sbits, sn, ovf);
+                        npos += stot;
+                    }
                 }
+                __syncwarp();
                 vpos += tot_v;
                 dpos += tot_d;
-                if (fs) {
-                    /* sign sub-packet (pack_sign_c, PackPrecinct.c:200-233) */
-                    uint32_t stot;
-                    const uint32_t sx = warp_excl_scan(sn, &stot);
-                    if (sn) put_bits(buf, words, npos + sx, sbits, sn, ovf);
-                    npos += stot;
-                }
             }
         }
     }
@@ -2098,7 +2027,7 @@ __global__ void __launch_bounds__(RC_THREADS, VPRED ? 2 : SIGNS ? 3 : 4) rc_cost
 }
 
 template <bool SIGNS, bool VPRED>
-__global__ void __launch_bounds__(PK_THREADS, 4) pack_kernel(const jxs_cfg_t* __restrict__ cfg, const uint16_t* __restrict__ coef,
+__global__ void __launch_bounds__(PK_THREADS, VPRED ? 3 : 4) pack_kernel(const jxs_cfg_t* __restrict__ cfg, const uint16_t* __restrict__ coef,
                                                           const uint8_t* __restrict__ gcli, const PrecRC* __restrict__ rc,
                                                           const uint32_t* __restrict__ cost, uint8_t* __restrict__ out,
                                                           uint32_t cap_words, int* status) {
@@ -2106,7 +2035,7 @@ __global__ void __launch_bounds__(PK_THREADS, 4) pack_kernel(const jxs_cfg_t* __
 }
 
 template <bool SIGNS, bool VPRED>
-__global__ void __launch_bounds__(PK_THREADS, 4) pack_batch_kernel(const __grid_constant__ EncPrecLaunch L, uint32_t cap_words) {
+__global__ void __launch_bounds__(PK_THREADS, VPRED ? 3 : 4) pack_batch_kernel(const __grid_constant__ EncPrecLaunch L, uint32_t cap_words) {
     const EncPrecFrame& F = L.job[find_job<JXS_BATCH_FRAMES>(L.job, L.nframes, (int)blockIdx.x)];
     pack_body<SIGNS, VPRED, true>(F.cfg, F.coef, F.gcli, F.rc, F.cost, F.out, cap_words, F.status, (int)blockIdx.x - F.first_block);
 }
