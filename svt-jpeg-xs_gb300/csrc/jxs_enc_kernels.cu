@@ -1197,7 +1197,7 @@ struct PkSeg {
  *           per segment), or, with sign handling, vertical prediction or
  *           segments of more than 128 groups, from the GCLIs (warp per
  *           segment);
- *   layout  band totals (thread per segment); warp 0: coding method per band
+ *   layout  band totals (thread per segment); coding method per band
  *           (significance only if strictly cheaper), running sums over the
  *           segments and lines in packet order, packet headers, raw
  *           fallback, packet positions; then each segment's positions
@@ -1238,6 +1238,7 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
     __shared__ uint32_t s_cv[VPRED ? JXS_MAXBL : 1], s_cvs[VPRED ? JXS_MAXBL : 1];   /* per band: prediction totals */
     __shared__ int8_t s_gtt[VPRED ? JXS_MAXBLINES : 1];                            /* per line: gtli of the line above (-1: this row's) */
     __shared__ uint32_t s_gp[VPRED ? JXS_MAXBLINES : 1];                           /* per line: GCLI row pitch */
+    __shared__ uint32_t s_part[SIGNS ? 3 : 2][JXS_MAXSEG / 32 + 1]; /* per 32 segments: data, GCLI, sign bits, then those before */
     __shared__ uint32_t s_lsx[JXS_MAXBLINES + 1], s_lrx[JXS_MAXBLINES + 1]; /* per line: significance / raw GCLI bits before it */
     __shared__ uint32_t s_pks[JXS_MAXPK], s_pkg[JXS_MAXPK], s_pkd[JXS_MAXPK], s_pkn[JXS_MAXPK]; /* per packet: sub-packet starts less the running sums there */
     __shared__ uint8_t s_pkr[JXS_MAXPK];
@@ -1474,82 +1475,121 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
         }
     }
     __syncthreads();
-    if (warp == 0) {
-        const uint32_t nbl = s_nbl;
-        /* coding method per band, D[p,b] (bit 1 significance, bit 0
-         * prediction): a later one only if strictly cheaper
-         * (RateControl.c:526-676) */
-        for (uint32_t fb = lane; fb < s_nbands; fb += 32) {
-            uint32_t m = 0, best = s_cn[fb];
-            if (s_sig && best > s_cs[fb]) {
-                m = 2;
-                best = s_cs[fb];
+    /* coding method of a band, D[p,b] (bit 1 significance, bit 0 prediction):
+     * a later one only if strictly cheaper (RateControl.c:526-676) */
+    auto data_at = [&](uint32_t i) { return s_data[i] + s_part[0][i >> 5]; };
+    auto vlc_at = [&](uint32_t i) { return s_vlc[i] + s_part[1][i >> 5]; };
+    auto nz_at = [&](uint32_t i) { return s_nz[i] + s_part[SIGNS ? 2 : 0][i >> 5]; };
+    auto method = [&](uint32_t fb) {
+        uint32_t m = 0, best = s_cn[fb];
+        if (s_sig && best > s_cs[fb]) {
+            m = 2;
+            best = s_cs[fb];
+        }
+        if (VPRED && vp) {
+            if (best > s_cv[fb]) {
+                m = 1;
+                best = s_cv[fb];
             }
-            if (VPRED && vp) {
-                if (best > s_cv[fb]) {
-                    m = 1;
-                    best = s_cv[fb];
-                }
-                if (s_sig && best > s_cvs[fb]) m = 3;
-            }
-            s_meth[fb] = (uint8_t)m;
+            if (s_sig && best > s_cvs[fb]) m = 3;
+        }
+        return m;
+    };
+    if (warp == PK_WARPS - 1) {
+        /* significance flags and raw GCLI bits before every line, each lane a
+         * run of them */
+        const uint32_t nbl = s_nbl, per = (nbl + 31) >> 5, x0 = min(nbl, per * lane), x1 = min(nbl, x0 + per);
+        uint32_t sg = 0, rw = 0;
+        for (uint32_t x = x0; x < x1; x++) {
+            sg += (method(bls[x].fb) & 2) ? bls[x].sig_w : 0u;
+            rw += 4 * bls[x].gcli_w;
+        }
+        uint32_t tsg, trw;
+        sg = warp_excl_scan(sg, &tsg);
+        rw = warp_excl_scan(rw, &trw);
+        for (uint32_t x = x0; x < x1; x++) {
+            s_lsx[x] = sg;
+            s_lrx[x] = rw;
+            sg += (method(bls[x].fb) & 2) ? bls[x].sig_w : 0u;
+            rw += 4 * bls[x].gcli_w;
+        }
+        if (lane == 0) {
+            s_lsx[nbl] = tsg;
+            s_lrx[nbl] = trw;
+        }
+    } else if (warp == PK_WARPS - 2) {
+        for (uint32_t fb = lane; fb < s_nbands; fb += 32) s_meth[fb] = (uint8_t)method(fb);
+        /* precinct header: Lprc, Q, R as bytes first, then the 2-bit band
+         * coding modes D[p,b] of every existing band */
+        if (lane == 0) {
+            const uint32_t lprc = total - s_phb;
+            byte_at(buf, lead) = (uint8_t)(lprc >> 16);
+            byte_at(buf, lead + 1) = (uint8_t)(lprc >> 8);
+            byte_at(buf, lead + 2) = (uint8_t)lprc;
+            byte_at(buf, lead + 3) = R.q;
+            byte_at(buf, lead + 4) = R.r;
         }
         __syncwarp();
-        /* data, GCLI and sign bits before every segment (into s_data, s_vlc,
-         * s_nz), each lane a run of them */
-        {
-            const uint32_t per = (nseg + 31) >> 5, i0 = min(nseg, per * lane), i1 = min(nseg, i0 + per);
-            uint32_t d = 0, g = 0, n = 0;
-            for (uint32_t i = i0; i < i1; i++) {
-                const uint32_t m = s_meth[bls[segs[i].bl].fb];
-                const uint32_t gi = m == 0 ? s_vlc[i] : m == 2 ? s_vlc[i] - s_zero[i] : m == 1 ? s_vn[VPRED ? i : 0] : s_vn[VPRED ? i : 0] - s_vr[VPRED ? i : 0];
-                s_zero[i] = gi;
-                d += s_data[i];
-                g += gi;
-                if (SIGNS) n += s_nz[i];
-            }
-            uint32_t td, tg, tn = 0;
-            d = warp_excl_scan(d, &td);
-            g = warp_excl_scan(g, &tg);
-            if (SIGNS) n = warp_excl_scan(n, &tn);
-            for (uint32_t i = i0; i < i1; i++) {
-                const uint32_t di = s_data[i], gi = s_zero[i];
-                s_data[i] = d;
-                s_vlc[i] = g;
-                d += di;
-                g += gi;
-                if (SIGNS) {
-                    const uint32_t ni = s_nz[i];
-                    s_nz[i] = n;
-                    n += ni;
-                }
-            }
-            if (lane == 0) {
-                s_data[nseg] = td;
-                s_vlc[nseg] = tg;
-                if (SIGNS) s_nz[nseg] = tn;
-            }
+        uint32_t idx0 = 0;
+        for (uint32_t gb0 = 0; gb0 < s_nbands_all; gb0 += 32) {
+            const uint32_t gb = gb0 + lane;
+            const int fb = gb < s_nbands_all ? s_g2f[gb] : JXS_NOBAND;
+            const bool ex = fb != JXS_NOBAND;
+            const uint32_t bal = __ballot_sync(FULL, ex);
+            if (ex && s_blines[fb] > 0 && s_meth[fb])
+                put_bits(buf, words, lead * 8 + 40 + 2 * (idx0 + __popc(bal & ((1u << lane) - 1))), s_meth[fb], 2, ovf);
+            idx0 += __popc(bal);
         }
-        /* significance flags and raw GCLI bits before every line */
+    }
+    /* data, GCLI and sign bits before every segment, in its warp's part of 32
+     * (into s_data, s_vlc, s_nz), and those of the parts; the warps from the
+     * first on hold the segments, the lines are the last's in a precinct of
+     * few */
+    for (uint32_t i0 = 32 * warp; i0 < nseg; i0 += 32 * PK_WARPS) {
+        const uint32_t i = i0 + lane;
+        uint32_t d = 0, g = 0, n = 0;
+        if (i < nseg) {
+            const uint32_t m = method(bls[segs[i].bl].fb);
+            d = s_data[i];
+            g = m == 0 ? s_vlc[i] : m == 2 ? s_vlc[i] - s_zero[i] : m == 1 ? s_vn[VPRED ? i : 0] : s_vn[VPRED ? i : 0] - s_vr[VPRED ? i : 0];
+            if (SIGNS) n = s_nz[i];
+        }
+        uint32_t td, tg, tn = 0;
+        d = warp_excl_scan(d, &td);
+        g = warp_excl_scan(g, &tg);
+        if (SIGNS) n = warp_excl_scan(n, &tn);
+        if (i < nseg) {
+            s_data[i] = d;
+            s_vlc[i] = g;
+            if (SIGNS) s_nz[i] = n;
+        }
+        if (lane == 0) {
+            s_part[0][i0 >> 5] = td;
+            s_part[1][i0 >> 5] = tg;
+            if (SIGNS) s_part[2][i0 >> 5] = tn;
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        /* the parts' running sums: bits before segment i are its own in
+         * s_data[i] and those of the parts before, s_part[0][i >> 5] */
+        static_assert(JXS_MAXSEG / 32 < 32, "a lane per part, and the end");
         {
-            const uint32_t per = (nbl + 31) >> 5, x0 = min(nbl, per * lane), x1 = min(nbl, x0 + per);
-            uint32_t sg = 0, rw = 0;
-            for (uint32_t x = x0; x < x1; x++) {
-                sg += (s_meth[bls[x].fb] & 2) ? bls[x].sig_w : 0u;
-                rw += 4 * bls[x].gcli_w;
+            const uint32_t parts = (nseg + 31) >> 5;
+            uint32_t td, tg, tn = 0;
+            const uint32_t d = warp_excl_scan(lane < parts ? s_part[0][lane] : 0u, &td);
+            const uint32_t g = warp_excl_scan(lane < parts ? s_part[1][lane] : 0u, &tg);
+            const uint32_t n = SIGNS ? warp_excl_scan(lane < parts ? s_part[2][lane] : 0u, &tn) : 0u;
+            if (lane <= parts) {
+                s_part[0][lane] = d;
+                s_part[1][lane] = g;
+                if (SIGNS) s_part[2][lane] = n;
             }
-            uint32_t tsg, trw;
-            sg = warp_excl_scan(sg, &tsg);
-            rw = warp_excl_scan(rw, &trw);
-            for (uint32_t x = x0; x < x1; x++) {
-                s_lsx[x] = sg;
-                s_lrx[x] = rw;
-                sg += (s_meth[bls[x].fb] & 2) ? bls[x].sig_w : 0u;
-                rw += 4 * bls[x].gcli_w;
-            }
-            if (lane == 0) {
-                s_lsx[nbl] = tsg;
-                s_lrx[nbl] = trw;
+            /* the end, in the last part or the first place of the next */
+            if (lane == (nseg >> 5)) {
+                s_data[nseg] = td - d;
+                s_vlc[nseg] = tg - g;
+                if (SIGNS) s_nz[nseg] = tn - n;
             }
         }
         __syncwarp();
@@ -1560,10 +1600,10 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
         if (nb) {
             i0 = bls[b0].seg0;
             const uint32_t i1 = bls[b0 + nb - 1].seg0 + bls[b0 + nb - 1].nseg;
-            db = s_data[i1] - s_data[i0];
-            gbits = s_vlc[i1] - s_vlc[i0];
+            db = data_at(i1) - data_at(i0);
+            gbits = vlc_at(i1) - vlc_at(i0);
             sbits = s_lsx[b0 + nb] - s_lsx[b0];
-            if (SIGNS) nbits = s_nz[i1] - s_nz[i0];
+            if (SIGNS) nbits = nz_at(i1) - nz_at(i0);
         }
         const uint32_t dB = (db + 7) >> 3, gB = (gbits + 7) >> 3, sB = (sbits + 7) >> 3, nB = (nbits + 7) >> 3;
         const uint32_t rawB = nb ? s_praw[k] : 0u;
@@ -1596,31 +1636,10 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
              * running sums at the packet's first segment or line */
             const uint32_t p0 = (start + hb) * 8, pd = p0 + (raw ? rawB : sB + gB) * 8;
             s_pks[k] = p0 - s_lsx[b0];
-            s_pkg[k] = raw ? p0 - s_lrx[b0] : p0 + sB * 8 - s_vlc[i0];
-            s_pkd[k] = pd - s_data[i0];
-            if (SIGNS) s_pkn[k] = pd + dB * 8 - s_nz[i0];
+            s_pkg[k] = raw ? p0 - s_lrx[b0] : p0 + sB * 8 - vlc_at(i0);
+            s_pkd[k] = pd - data_at(i0);
+            if (SIGNS) s_pkn[k] = pd + dB * 8 - nz_at(i0);
             s_pkr[k] = (uint8_t)raw;
-        }
-        /* precinct header: Lprc, Q, R as bytes first, then the 2-bit band
-         * coding modes D[p,b] of every existing band */
-        if (lane == 0) {
-            const uint32_t lprc = total - hdr;
-            byte_at(buf, lead) = (uint8_t)(lprc >> 16);
-            byte_at(buf, lead + 1) = (uint8_t)(lprc >> 8);
-            byte_at(buf, lead + 2) = (uint8_t)lprc;
-            byte_at(buf, lead + 3) = R.q;
-            byte_at(buf, lead + 4) = R.r;
-        }
-        __syncwarp();
-        uint32_t idx0 = 0;
-        for (uint32_t gb0 = 0; gb0 < s_nbands_all; gb0 += 32) {
-            const uint32_t gb = gb0 + lane;
-            const int fb = gb < s_nbands_all ? s_g2f[gb] : JXS_NOBAND;
-            const bool ex = fb != JXS_NOBAND;
-            const uint32_t bal = __ballot_sync(FULL, ex);
-            if (ex && s_blines[fb] > 0 && s_meth[fb])
-                put_bits(buf, words, lead * 8 + 40 + 2 * (idx0 + __popc(bal & ((1u << lane) - 1))), s_meth[fb], 2, ovf);
-            idx0 += __popc(bal);
         }
         /* the packed size must be what the rate control paid for */
         const int all_fit = __all_sync(FULL, fits || !nb);
@@ -1642,12 +1661,12 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
         const jxs_bline_t& B = bls[sg.bl];
         const uint32_t m = s_meth[B.fb], raw = s_pkr[B.pk];
         PkSeg D;
-        D.vpos = s_pkg[B.pk] + (raw ? s_lrx[sg.bl] + 4 * sg.g0 : s_vlc[i]);
-        D.dpos = s_pkd[B.pk] + s_data[i];
+        D.vpos = s_pkg[B.pk] + (raw ? s_lrx[sg.bl] + 4 * sg.g0 : vlc_at(i));
+        D.dpos = s_pkd[B.pk] + data_at(i);
         D.g0n = sg.g0 | (min(SG, B.gcli_w - sg.g0) << 16);
         D.info = s_lt[sg.bl] | (m << 4) | (raw << 6) | ((uint32_t)sg.bl << 8);
         s_desc[i] = D;
-        if (SIGNS) s_nst[i] = s_pkn[B.pk] + s_nz[i];
+        if (SIGNS) s_nst[i] = s_pkn[B.pk] + nz_at(i);
     }
     for (uint32_t x = threadIdx.x; x < s_nbl; x += blockDim.x) s_sigp[x] = s_pks[bls[x].pk] + s_lsx[x];
     __syncthreads();
