@@ -497,8 +497,8 @@ static int32_t plan_decode_chain(const std::vector<DecItem>& it, const std::vect
         auto flush = [&]() {
             if (L->nframes) {
                 if (op == 0) {
-                    if (L->nframes > 1) P->add(OP_WALK, 0, chain, L->nslices, 0, 0, L, sizeof(*L));
-                    else P->add(OP_WALK1, 0, chain, L->nslices, 0, 0, &L->job[0], sizeof(L->job[0]));
+                    if (L->nframes > 1) P->add(OP_WALK, 0, chain, L->nframes, 0, 0, L, sizeof(*L));
+                    else P->add(OP_WALK1, 0, chain, 1, 0, 0, &L->job[0], sizeof(L->job[0]));
                 } else {
                     /* one shared-memory layout for the launch: the largest
                      * precinct buffer that leaves room for the rest */
@@ -527,9 +527,7 @@ static int32_t plan_decode_chain(const std::vector<DecItem>& it, const std::vect
             F.coef = (int16_t*)d.w->fb.coef;
             F.status = d.status;
             F.first_block = L->nblocks;
-            F.first_slice = L->nslices;
             L->nblocks += (int)d.c->nprec;
-            L->nslices += (int)d.c->nslices;
             cb = std::max(cb, d.cap_bytes);
             cg = std::max(cg, d.cap_groups);
             cs = std::max(cs, d.cap_seg);
@@ -665,7 +663,7 @@ static int32_t issue(jxs_gpu_batch_t* b, const Plan& P, cudaStream_t st) {
         }
         case OP_WALK1: {
             const DecPrecFrame* F = (const DecPrecFrame*)d;
-            e = jxs_launch_walk(F->cfg, (uint32_t)o.nblocks, F->bs, F->bs_size, F->prec_off, F->status + 1, F->status, s);
+            e = jxs_launch_walk(F->cfg, F->bs, F->bs_size, F->prec_off, F->status, s);
             break;
         }
         case OP_UNPACK1: {

@@ -1258,47 +1258,33 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
 /* One thread per slice: the slice is expected where the constant-bit-rate
  * split of Lcod puts it (EncHandle.c:760-809); its precincts are found by
  * following the 24-bit precinct lengths, and the walk must end exactly at
- * the next slice (or at EOC).  Any mismatch raises *walk_bad. */
-DEV void walk_slice(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size,
-                    uint32_t* __restrict__ prec_off, int* walk_bad, const uint32_t s) {
-    if (s >= cfg->nslices) return;
-    if (cfg->max_slice_budget == 0) {
-        *walk_bad = 1;
-        return;
-    }
+ * the next slice (or at EOC).  False if anything is not so. */
+DEV bool walk_slice(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size,
+                    uint32_t* __restrict__ prec_off, const uint32_t s) {
+    if (cfg->max_slice_budget == 0) return false;
     uint64_t off = cfg->slice_begin[s];
     if (off + 6 > size || bs[off] != 0xff || bs[off + 1] != 0x20 || bs[off + 2] != 0 || bs[off + 3] != 4 ||
-        (((uint32_t)bs[off + 4] << 8) | bs[off + 5]) != s) {
-        atomicExch(walk_bad, 1);
-        return;
-    }
+        (((uint32_t)bs[off + 4] << 8) | bs[off + 5]) != s) return false;
     off += 6;
     /* the slice's precincts: rows x columns, row after row */
     const uint32_t first = s * cfg->pps * cfg->ncol,
                    n = ((s + 1 == cfg->nslices) ? cfg->np - s * cfg->pps : cfg->pps) * cfg->ncol;
     for (uint32_t i = 0; i < n; i++) {
-        if (off + cfg->prec_hdr_bytes > size) {
-            atomicExch(walk_bad, 1);
-            return;
-        }
+        if (off + cfg->prec_hdr_bytes > size) return false;
         const uint32_t lprc = be24(bs + off);
-        if (lprc > JXS_PREC_MAX_BYTES) {
-            atomicExch(walk_bad, 1);
-            return;
-        }
+        if (lprc > JXS_PREC_MAX_BYTES) return false;
         prec_off[first + i] = (uint32_t)off;
         off += cfg->prec_hdr_bytes + lprc;
     }
     const int ok = (s + 1 < cfg->nslices) ? off == cfg->slice_begin[s + 1]
                                           : (off + 2 <= size && bs[off] == 0xff && bs[off + 1] == 0x11);
-    if (!ok) atomicExch(walk_bad, 1);
+    return ok;
 }
 
 /* Fallback when the prediction failed: one thread walks the whole codestream
  * from the header (get_slice_size, DecThreadInit.c:35-131). */
 DEV void walk_sequential(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size,
-                         uint32_t* __restrict__ prec_off, const int* walk_bad, int* status) {
-    if (!*walk_bad) return;
+                         uint32_t* __restrict__ prec_off, int* status) {
     uint64_t off = cfg->hdr_len;
     for (uint32_t s = 0; s < cfg->nslices; s++) {
         if (off + 6 > size) {
@@ -1329,6 +1315,18 @@ DEV void walk_sequential(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __res
     }
     if (off + 2 > size) JXS_STATUS_SET(status, JXS_E_DEC_SHORT);
     else if (bs[off] != 0xff || bs[off + 1] != 0x11) JXS_STATUS_SET(status, JXS_E_DEC_BITSTREAM);
+}
+
+/* A frame's precincts, by one block: a thread per slice (or more slices),
+ * then one thread in order if any slice is not where it is expected.  Bound by
+ * the latency of a handful of loads that wait for one another; the second step
+ * as a launch of its own cost 5 us, taken or not. */
+#define WALK_THREADS 512
+DEV void walk_frame(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size, uint32_t* __restrict__ prec_off,
+                    int* status) {
+    bool lost = false;
+    for (uint32_t s = threadIdx.x; s < cfg->nslices; s += blockDim.x) lost |= !walk_slice(cfg, bs, size, prec_off, s);
+    if (__syncthreads_or(lost) && threadIdx.x == 0) walk_sequential(cfg, bs, size, prec_off, status);
 }
 
 /* ------------------------------------------------------------------------ */
@@ -1393,48 +1391,24 @@ __global__ void __launch_bounds__(UK_THREADS) unpack_vpred_kernel(const jxs_cfg_
     cl.sync(); /* and until none does any more */
 }
 
-__global__ void walk_slices_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size,
-                                   uint32_t* __restrict__ prec_off, int* walk_bad) {
+__global__ void __launch_bounds__(WALK_THREADS) walk_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs,
+                                                            uint32_t size, uint32_t* __restrict__ prec_off, int* status) {
     dep_wait();
-    walk_slice(cfg, bs, size, prec_off, walk_bad, blockIdx.x * blockDim.x + threadIdx.x);
+    walk_frame(cfg, bs, size, prec_off, status);
 }
 
-__global__ void walk_sequential_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size,
-                                       uint32_t* __restrict__ prec_off, const int* walk_bad, int* status) {
-    dep_wait();
-    walk_sequential(cfg, bs, size, prec_off, walk_bad, status);
-}
-
-/* one thread per slice of every frame of the batch */
-__global__ void walk_slices_batch_kernel(const __grid_constant__ DecPrecLaunch L) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= L.nslices) return;
-    int lo = 0, hi = L.nframes - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (g >= L.job[mid].first_slice) lo = mid;
-        else hi = mid - 1;
-    }
-    const DecPrecFrame& F = L.job[lo];
-    walk_slice(F.cfg, F.bs, F.bs_size, F.prec_off, F.status + 1, (uint32_t)(g - F.first_slice));
-}
-
-/* one thread per frame of the batch */
-__global__ void walk_sequential_batch_kernel(const __grid_constant__ DecPrecLaunch L) {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= L.nframes) return;
-    const DecPrecFrame& F = L.job[f];
-    walk_sequential(F.cfg, F.bs, F.bs_size, F.prec_off, F.status + 1, F.status);
+/* one block per frame of the batch */
+__global__ void __launch_bounds__(WALK_THREADS) walk_batch_kernel(const __grid_constant__ DecPrecLaunch L) {
+    const DecPrecFrame& F = L.job[blockIdx.x];
+    walk_frame(F.cfg, F.bs, F.bs_size, F.prec_off, F.status);
 }
 
 /* ------------------------------------------------------------------------ */
 /* host-side launchers                                                       */
 /* ------------------------------------------------------------------------ */
-extern "C" cudaError_t jxs_launch_walk(const jxs_cfg_t* dcfg, uint32_t nslices, const uint8_t* bs, uint32_t size, uint32_t* prec_off,
-                                       int* walk_bad, int* status, cudaStream_t st) {
-    const cudaError_t e = jxs_launch(walk_slices_kernel, dim3((nslices + 127) / 128), 128, 0, st, dcfg, bs, size, prec_off, walk_bad);
-    if (e != cudaSuccess) return e;
-    return jxs_launch(walk_sequential_kernel, dim3(1), 1, 0, st, dcfg, bs, size, prec_off, walk_bad, status);
+extern "C" cudaError_t jxs_launch_walk(const jxs_cfg_t* dcfg, const uint8_t* bs, uint32_t size, uint32_t* prec_off, int* status,
+                                       cudaStream_t st) {
+    return jxs_launch(walk_kernel, dim3(1), WALK_THREADS, 0, st, dcfg, bs, size, prec_off, status);
 }
 
 template <bool FS>
@@ -1461,8 +1435,7 @@ extern "C" cudaError_t jxs_launch_unpack(const jxs_cfg_t* dcfg, const uint8_t* b
 
 extern "C" cudaError_t jxs_launch_walk_batch(const DecPrecLaunch* L, cudaStream_t st) {
     if (L->nframes <= 0) return cudaSuccess;
-    walk_slices_batch_kernel<<<(L->nslices + 127) / 128, 128, 0, st>>>(*L);
-    walk_sequential_batch_kernel<<<(L->nframes + 31) / 32, 32, 0, st>>>(*L);
+    walk_batch_kernel<<<L->nframes, WALK_THREADS, 0, st>>>(*L);
     return cudaGetLastError();
 }
 

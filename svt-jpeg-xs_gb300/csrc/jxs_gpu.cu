@@ -897,11 +897,7 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
         if (!jxs_gpu_is_device_ptr(bs) || size < c->hdr_len) return JXS_E_DEC_PTR;
         s->hdr_check = 1;
         KMARK();
-        if (walk) {
-            /* the walk's own flag of a failed prediction, which it deals with */
-            CK(jxs_launch_walk(d->dcfg, c->nslices, bs, size, s->prec_off, s->status + 2, s->status, st));
-            CK(cudaMemsetAsync(s->status + 2, 0, sizeof(int), st));
-        }
+        if (walk) CK(jxs_launch_walk(d->dcfg, bs, size, s->prec_off, s->status, st));
     } else if (!jxs_gpu_is_device_ptr(bs)) {
         if (size > s->bs_cap) {
             CK(cudaStreamSynchronize(st));

@@ -226,13 +226,12 @@ struct DecPrecFrame {
     uint32_t bs_size;
     uint32_t* prec_off;     /* precinct byte offsets */
     int16_t* coef;
-    int* status;            /* status[0]: frame status; status[1]: the slice walk found a mismatch */
+    int* status;            /* frame status */
     int first_block;        /* unpacking: first precinct block */
-    int first_slice;        /* walk: first slice thread */
 };
 struct DecPrecLaunch {
     int nframes;
-    int nblocks, nslices;
+    int nblocks;
     DecPrecFrame job[JXS_BATCH_FRAMES];
 };
 

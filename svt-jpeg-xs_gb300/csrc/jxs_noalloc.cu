@@ -7,8 +7,8 @@
  * (header through EOC) and the byte offset of every precinct, using the
  * decoder handle's configuration.
  *
- * The decoder's own path walks the same structure (walk_slices_kernel /
- * walk_sequential_kernel in jxs_dec_kernels.cu) with scratch that belongs
+ * The decoder's own path walks the same structure (walk_kernel in
+ * jxs_dec_kernels.cu) with scratch that belongs
  * to a frame slot, allocated when the decoder was created.  This variant
  * allocates nothing: no cudaMalloc, no cudaFree, no host heap or pinned
  * memory (the header and the results come back into stack variables and
