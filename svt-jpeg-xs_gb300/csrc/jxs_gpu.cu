@@ -882,7 +882,7 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
     const jxs_cfg_t* c = &d->cfg;
     const uint32_t bps = bytes_per_sample(c);
     const cudaStream_t st = dec_stream(d, s);
-    const int walk = !prec_off && (d->walk || d->vpred || c->max_slice_budget == 0 || c->pps * c->ncol > kSelfSteps);
+    const int walk = !prec_off && (d->walk || c->max_slice_budget == 0 || c->pps * c->ncol > kSelfSteps);
     s->timed = d->timing;
 #define TMARK(i) \
     if (s->timed) CK(cudaEventRecord(s->tev[i], st))
