@@ -522,8 +522,19 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
                     }
                     uint32_t m8 = __vmaxu2(__vmaxu2(c[0], c[1]), __vmaxu2(c[2], c[3]));
                     m8 = max(m8 & 0xffffu, m8 >> 16);
+                    /* from the largest GCLI of both rows on, every GCLI is at t
+                     * and its prediction at max(t, gtt): without the loop */
+                    uint32_t top8 = __vmaxu2(__vmaxu2(tp[0] & pv[0], tp[1] & pv[1]), __vmaxu2(tp[2] & pv[2], tp[3] & pv[3]));
+                    top8 = max(m8, max(top8 & 0xffffu, top8 >> 16));
+                    const int its = (int)min((__reduce_max_sync(FULL, top8) + 1) >> 1, 8u);
+                    {
+                        const int t = lane & 15, G = max(t, gtt);
+                        const uint32_t n = min(128u, gend - base);
+                        const uint32_t bits = G == t ? n : 2u * (uint32_t)(G - t) * n;
+                        if (t >= 2 * its) acc += lane < 16 || rm ? bits : G == t ? n : 0u;
+                    }
 #pragma unroll 2
-                    for (int it = 0; it < 8; it++) {
+                    for (int it = 0; it < its; it++) {
                         const int t = 2 * it + half;
                         const uint32_t t2 = t * ONE, G2 = max(t, gtt) * ONE;
                         uint32_t sum = 0, off = 0;
