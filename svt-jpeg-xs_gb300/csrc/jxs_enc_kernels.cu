@@ -374,7 +374,7 @@ DEV void select_slice(const jxs_cfg_t* __restrict__ cfg, int s, const uint32_t* 
  * that selection */
 #define RC_LT_REGION (JXS_MAXBLINES * 16)
 #define RC_LT_WORDS (5 * RC_LT_REGION) /* data, GCLI bits, GCLI bits with significance, fast / full sign bits */
-#define RC_VP_REGIONS 10
+#define RC_VP_REGIONS 12
 
 /* vlc_encode_get_bits (PackPrecinct.h:86-104): ones of the unary code of a
  * GCLI difference x for the vertical prediction range (r, t). */
@@ -383,6 +383,89 @@ DEV uint32_t vlc_vp_bits(int x, int r, int t) {
     if (x > mx) return (uint32_t)(x + mx);
     x *= 2;
     return (uint32_t)(x < 0 ? -x - 1 : x);
+}
+
+/* Byte costs of a packet at quantization q for the refinements that lower the
+ * gtli of its lines `chunk` of four (in the order of their priorities), as
+ * changes at those refinements; the first chunk also the cost at R = 0.
+ * tw: a line's word per gtli (fields at 0, RC_NOS and RC_SIG); ta, tb: sign
+ * bits per line and gtli, each rounded on its own (SB tables: SB = 1 adds ta
+ * to da, SB = 2 also keeps a second cost with tb in db, RateControl.c:745-756).
+ * A chain of one line after another: by whole packets the first one, with most
+ * of the lines, kept all warps waiting (a 256x64 block's costs 4,100 cycles,
+ * 2,800 by four lines). */
+template <int SB>
+DEV void packet_costs(int q, uint32_t chunk, uint32_t b0, uint32_t nb, uint32_t raw, uint32_t nr, const uint32_t* opk,
+                      const uint64_t (*tw)[16], const uint32_t (*ta)[16], const uint32_t (*tb)[16], uint32_t (*da)[33],
+                      uint32_t (*db)[33]) {
+    /* sums of the words plus 7 in each field; bytes of the fields */
+    uint64_t S = 7u | (uint64_t)7u << RC_NOS | (uint64_t)7u << RC_SIG;
+    auto bytes = [&](uint64_t v) {
+        return ((uint32_t)v << (32 - RC_NOS) >> (35 - RC_NOS)) +
+               min(raw, (uint32_t)(v >> (RC_SIG + 3)) + ((uint32_t)(v >> (RC_NOS + 3)) & ((1u << (RC_SIG - RC_NOS - 3)) - 1u)));
+    };
+    uint32_t fb = 7, zb = 7;
+#pragma unroll 4
+    for (uint32_t i = b0; i < b0 + nb; i++) {
+        const uint32_t w = opk[i], x = w & 255u;
+        const int t = min(max(q - (int)((w >> 8) & 255u), 0), 15);
+        S += tw[x][t];
+        if (SB > 0) fb += ta[x][t];
+        if (SB > 1) zb += tb[x][t];
+    }
+    auto lower = [&](uint32_t w) { /* the line's gtli drops by one */
+        const uint32_t x = w & 255u;
+        const int d = q - (int)((w >> 8) & 255u);
+        const int t0 = min(max(d, 0), 15), t1 = min(max(d - 1, 0), 15);
+        S += tw[x][t1] - tw[x][t0];
+        if (SB > 0) fb += ta[x][t1] - ta[x][t0];
+        if (SB > 1) zb += tb[x][t1] - tb[x][t0];
+    };
+    const uint32_t i0 = b0 + 4 * chunk, i1 = min(b0 + nb, i0 + 4);
+    for (uint32_t i = b0; i < i0; i++) {
+        const uint32_t w = opk[i];
+        if ((w >> 16) >= nr) return;
+        lower(w);
+    }
+    const uint32_t base = bytes(S);
+    uint32_t c = base + (SB > 0 ? fb >> 3 : 0u), cf = base + (zb >> 3);
+    if (chunk == 0) {
+        atomicAdd(&da[q][0], c);
+        if (SB > 1) atomicAdd(&db[q][0], cf);
+    }
+    uint32_t w = opk[i0];
+    for (uint32_t i = i0; i < i1; i++) {
+        const uint32_t rf = w >> 16; /* the first R at which it has dropped */
+        if (rf >= nr) break;
+        lower(w);
+        w = opk[i + 1]; /* the next line's before its turn */
+        const uint32_t base1 = bytes(S), c1 = base1 + (SB > 0 ? fb >> 3 : 0u), cf1 = base1 + (zb >> 3);
+        atomicAdd(&da[q][rf], c1 - c);
+        if (SB > 1) atomicAdd(&db[q][rf], cf1 - cf);
+        c = c1;
+        cf = cf1;
+    }
+}
+/* What packet_costs reads of the precinct kind's tables: the order's lines, and
+ * the packets' chunks (packet | chunk << 8, their number last).  By a block. */
+#define RC_MAXITEM (JXS_MAXBLINES / 4 + JXS_MAXPK)
+DEV void cost_items(uint32_t nbl, uint32_t npk, const uint8_t* order, const uint8_t* gain, const uint8_t* prio, const uint8_t* pknbl,
+                    uint32_t* opk, uint16_t* items) {
+    for (uint32_t x = threadIdx.x; x < nbl; x += blockDim.x) {
+        const uint32_t y = order[x];
+        opk[x] = y | (uint32_t)gain[y] << 8 | (prio[y] + 1u) << 16;
+    }
+    if ((threadIdx.x >> 5) == RC_WARPS - 1) {
+        const uint32_t lane = threadIdx.x & 31, n = lane < npk ? (pknbl[lane] + 3u) >> 2 : 0u;
+        uint32_t e = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(FULL, e, o);
+            if (lane >= (uint32_t)o) e += y;
+        }
+        for (uint32_t c = 0; c < n; c++) items[e - n + c] = (uint16_t)(lane | c << 8);
+        if (lane == 31) items[RC_MAXITEM] = (uint16_t)e;
+    }
 }
 
 /* One slice's selection with vertical prediction, precinct after precinct
@@ -415,7 +498,8 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
                             const uint32_t* __restrict__ cost, uint32_t* area, PrecRC* __restrict__ rc,
                             int* __restrict__ status, Stage& stage_kind, const uint8_t* lgain, const uint8_t* lprio,
                             const uint8_t* lfb, const uint32_t* lsig, const uint32_t* lraw, const jxs_bline_t* bls,
-                            const jxs_seg_t* segs, const uint8_t* s_pkbl0, const uint8_t* s_pknbl, const uint8_t* s_order) {
+                            const jxs_seg_t* segs, const uint8_t* s_pkbl0, const uint8_t* s_pknbl, const uint8_t* s_order, uint32_t* opk,
+                            uint16_t* items) {
     __shared__ int s_err;
     __shared__ uint8_t s_gtop[JXS_MAXBL], s_bl0[JXS_MAXBL], s_bl1[JXS_MAXBL];
     uint32_t(*vtfs)[16] = (uint32_t(*)[16])area;
@@ -429,6 +513,7 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
     uint32_t(*vred)[16] = (uint32_t(*)[16])(area + 7 * RC_LT_REGION);
     uint32_t* Ts = area + 8 * RC_LT_REGION;
     uint32_t* Fs = area + 9 * RC_LT_REGION;
+    uint64_t(*tw)[16] = (uint64_t(*)[16])(area + 10 * RC_LT_REGION);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, half = lane >> 4;
     const RcParams P = rc_params(cfg);
     const SliceSplit sp = slice_split(cfg, s);
@@ -483,6 +568,7 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
             if (fs) Fs[e] = __ldcg(cost + ((uint64_t)np_all + p) * 1024 + q * 32 + r);
         }
         for (int e = threadIdx.x; e < nq * 33; e += blockDim.x) (&dV[0][0])[e] = 0;
+        cost_items(nbl, npk, s_order, lgain, lprio, s_pknbl, opk, items);
         __syncthreads();
         /* vertical prediction costs of every line, for every t */
         if (i > 0) {
@@ -584,44 +670,18 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, int s, const uint
                 }
                 if (sig && best > vs) m = 3;
             }
-            /* vtnos becomes the GCLI bits of the method chosen, vtsig its
-             * significance flags */
             for (uint32_t x = x0, k = 0; k < (two ? 2u : 1u); x = x1, k++) {
-                if (m) vtnos[x][t] = m == 2 ? vtsig[x][t] : vnos[x][t] - (m == 3 ? vred[x][t] : 0u);
-                vtsig[x][t] = m & 2u ? lsig[x] : 0u;
+                const uint32_t bits = m == 0 ? vtnos[x][t] : m == 2 ? vtsig[x][t] : vnos[x][t] - (m == 3 ? vred[x][t] : 0u);
+                tw[x][t] = vtdat[x][t] | (uint64_t)bits << RC_NOS | (uint64_t)(m & 2u ? lsig[x] : 0u) << RC_SIG;
             }
         }
         __syncthreads();
-        /* costs with those methods, a warp per packet and a lane per Q, as in
-         * the parallel pass */
-        for (uint32_t k = warp; k < npk; k += RC_WARPS) {
-            const int q = lane;
-            const uint32_t b0 = s_pkbl0[k], nb = s_pknbl[k], raw = lraw[k];
-            if (!nb || q >= nq) continue;
-            uint32_t db = 0, gb = 0, sb = 0, zb = 0;
-            for (uint32_t x = b0; x < b0 + nb; x++) {
-                const int t = min(max(q - (int)lgain[x], 0), 15);
-                db += vtdat[x][t];
-                gb += vtnos[x][t];
-                sb += vtsig[x][t];
-                if (signs) zb += vtz[x][t];
-            }
-            uint32_t c = ((db + 7) >> 3) + min(raw, ((sb + 7) >> 3) + ((gb + 7) >> 3)) + ((zb + 7) >> 3);
-            atomicAdd(&dV[q][0], c);
-            for (uint32_t j = 0; j < nb; j++) {
-                const uint32_t x = s_order[b0 + j];
-                const int rf = lprio[x] + 1;
-                if (rf >= nr) break;
-                const int g = lgain[x];
-                const int t0 = min(max(q - g, 0), 15), t1 = min(max(q - g - 1, 0), 15);
-                db += vtdat[x][t1] - vtdat[x][t0];
-                gb += vtnos[x][t1] - vtnos[x][t0];
-                sb += vtsig[x][t1] - vtsig[x][t0];
-                if (signs) zb += vtz[x][t1] - vtz[x][t0];
-                const uint32_t c1 = ((db + 7) >> 3) + min(raw, ((sb + 7) >> 3) + ((gb + 7) >> 3)) + ((zb + 7) >> 3);
-                atomicAdd(&dV[q][rf], c1 - c);
-                c = c1;
-            }
+        /* costs with those methods, as in the parallel pass */
+        for (uint32_t it = warp; it < items[RC_MAXITEM]; it += RC_WARPS) {
+            const uint32_t e = items[it], k = e & 255u;
+            if (lane >= nq) continue;
+            if (signs) packet_costs<1>(lane, e >> 8, s_pkbl0[k], s_pknbl[k], lraw[k], nr, opk, tw, vtz, nullptr, dV, nullptr);
+            else packet_costs<0>(lane, e >> 8, s_pkbl0[k], s_pknbl[k], lraw[k], nr, opk, tw, nullptr, nullptr, dV, nullptr);
         }
         __syncthreads();
         for (int q = warp; q < nq; q += RC_WARPS) {
@@ -720,6 +780,7 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
     __shared__ uint64_t s_grow[JXS_MAXBLINES];
     __shared__ uint8_t s_pkbl0[JXS_MAXPK], s_pknbl[JXS_MAXPK], s_order[JXS_MAXBLINES];
     __shared__ uint32_t s_opk[JXS_MAXBLINES + 1]; /* the order's lines: number | gain << 8 | first R that lowers its gtli << 16 */
+    __shared__ uint16_t s_item[RC_MAXITEM + 1];
     uint64_t(*tw)[16] = (uint64_t(*)[16])(s_area + (SIGNS ? 2 : 0) * JXS_MAXBLINES * 16); /* in place of hist and shist, or tdat and tnos */
 
     const int last = (p + 1 >= (int)cfg->np);
@@ -961,10 +1022,7 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
         const uint32_t i = threadIdx.x + k * RC_THREADS;
         if (i < nbl * 16) tw[i >> 4][i & 15] = word[k];
     }
-    for (uint32_t x = threadIdx.x; x < nbl; x += blockDim.x) {
-        const uint32_t y = s_order[x];
-        s_opk[x] = y | (uint32_t)lgain[y] << 8 | (lprio[y] + 1u) << 16;
-    }
+    cost_items(nbl, cfg->npk, s_order, lgain, lprio, s_pknbl, s_opk, s_item);
     /* costs: band priorities are distinct, so raising R by one lowers the
      * gtli of one band only; each (Q, packet) thread adds its packet's cost
      * at R = 0 and its change at every R where one of its band lines drops,
@@ -977,55 +1035,12 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
     __syncthreads();
     /* with sign handling each packet adds its sign sub-packet, rounded on
      * its own: fast signs in dC, full signs in dF (RateControl.c:745-756) */
-    const uint32_t npk = cfg->npk;
-    /* a warp per packet, a lane per Q (at most 32): the packet's band lines
-     * are the same for the whole warp */
-    for (uint32_t k = warp; k < npk; k += RC_WARPS) {
-        const int q = lane;
-        const uint32_t b0 = s_pkbl0[k], nb = s_pknbl[k], raw = lraw[k];
-        if (!nb || q >= nq) continue;
-        /* sums of the words plus 7 in each field; bytes of the fields */
-        uint64_t S = 7u | (uint64_t)7u << RC_NOS | (uint64_t)7u << RC_SIG;
-        auto bytes = [&](uint64_t v) {
-            return ((uint32_t)v << (32 - RC_NOS) >> (35 - RC_NOS)) +
-                   min(raw, (uint32_t)(v >> (RC_SIG + 3)) + ((uint32_t)(v >> (RC_NOS + 3)) & ((1u << (RC_SIG - RC_NOS - 3)) - 1u)));
-        };
-        uint32_t fb = 7, zb = 7;
-#pragma unroll 4
-        for (uint32_t i = b0; i < b0 + nb; i++) {
-            const uint32_t w = s_opk[i], x = w & 255u;
-            const int t = min(max(q - (int)((w >> 8) & 255u), 0), 15);
-            S += tw[x][t];
-            if (fs) {
-                fb += tfs[x][t];
-                zb += tnz[x][t];
-            }
-        }
-        const uint32_t base = bytes(S);
-        uint32_t c = base + (fs ? fb >> 3 : 0u), cf = base + (zb >> 3);
-        atomicAdd(&dC[q][0], c);
-        if (fs) atomicAdd(&dF[q][0], cf);
-        uint32_t w = s_opk[b0];
-        for (uint32_t i = b0; i < b0 + nb; i++) {
-            const uint32_t x = w & 255u, rf = w >> 16; /* the line's gtli drops by one for R >= priority + 1 */
-            if (rf >= (uint32_t)nr) break;
-            const int d = q - (int)((w >> 8) & 255u);
-            const int t0 = min(max(d, 0), 15), t1 = min(max(d - 1, 0), 15);
-            S += tw[x][t1] - tw[x][t0];
-            w = s_opk[i + 1]; /* the next line's before its turn */
-            const uint32_t base1 = bytes(S);
-            uint32_t c1 = base1;
-            if (fs) {
-                fb += tfs[x][t1] - tfs[x][t0];
-                zb += tnz[x][t1] - tnz[x][t0];
-                c1 += fb >> 3;
-                const uint32_t cf1 = base1 + (zb >> 3);
-                atomicAdd(&dF[q][rf], cf1 - cf);
-                cf = cf1;
-            }
-            atomicAdd(&dC[q][rf], c1 - c);
-            c = c1;
-        }
+    /* a warp per packet's chunk, a lane per Q (at most 32) */
+    for (uint32_t it = warp; it < s_item[RC_MAXITEM]; it += RC_WARPS) {
+        const uint32_t e = s_item[it], k = e & 255u;
+        if (lane >= nq) continue;
+        if (SIGNS && fs) packet_costs<2>(lane, e >> 8, s_pkbl0[k], s_pknbl[k], lraw[k], nr, s_opk, tw, tfs, tnz, dC, dF);
+        else packet_costs<0>(lane, e >> 8, s_pkbl0[k], s_pknbl[k], lraw[k], nr, s_opk, tw, nullptr, nullptr, dC, nullptr);
     }
     __syncthreads();
     /* a warp per Q, a lane per R */
@@ -1063,7 +1078,7 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
     if (!s_last) return;
     if constexpr (VPRED) {
         if (cfg->vpred) select_slice_vpred(cfg, (int)s, gcli, cost, s_area, rc, status, stage_kind, lgain, lprio, lfb, lsig,
-                                           lraw, s_bl, s_seg, s_pkbl0, s_pknbl, s_order);
+                                           lraw, s_bl, s_seg, s_pkbl0, s_pknbl, s_order, s_opk, s_item);
         else select_slice(cfg, (int)s, cost, s_area, RC_VP_REGIONS * RC_LT_REGION, rc, status);
     } else {
         select_slice(cfg, (int)s, cost, s_area, RC_AREA_WORDS(SIGNS), rc, status);
