@@ -402,7 +402,7 @@ static int32_t plan_encode_chain(const std::vector<EncItem>& it, const std::vect
             uint32_t warps = 0;
             for (int f : fr)
                 if (v > 0 || enc_level0_kind(it[f].c) == kind) warps += v_warps(it[f].c, v, (uint32_t)jxs_fwd_v_tile_cols());
-            const int rp = v_rowpairs(warps);
+            const int rp = v_rowpairs(warps, v > 0);
             for (int f : fr) {
                 const EncItem& e = it[f];
                 if (v == 0 && enc_level0_kind(e.c) != kind) continue;
@@ -593,7 +593,7 @@ static int32_t plan_decode_chain(const std::vector<DecItem>& it, const std::vect
             for (int f : fr)
                 if ((v > (int)it[f].c->proxy ? 0 : dec_sample_kind(it[f].c)) == ok)
                     warps += v_warps(it[f].c, v, (uint32_t)jxs_inv_v_tile_cols());
-            const int rp = v_rowpairs(warps);
+            const int rp = v_rowpairs(warps, ok == 0);
             for (int f : fr) {
                 const DecItem& d = it[f];
                 if ((v > (int)d.c->proxy ? 0 : dec_sample_kind(d.c)) != ok) continue;

@@ -524,7 +524,7 @@ static int32_t enc_run(jxs_gpu_enc_t* e, EncSlot* s, void* const planes[4], cons
         FwdVLaunch L;
         memset(&L, 0, sizeof(L));
         int tiles[JXS_MAXC];
-        L.njobs = plan_fwd_v(c, e->dcfg, fb, in, v, v_rowpairs(v_warps(c, v, (uint32_t)jxs_fwd_v_tile_cols())), L.job, tiles);
+        L.njobs = plan_fwd_v(c, e->dcfg, fb, in, v, v_rowpairs(v_warps(c, v, (uint32_t)jxs_fwd_v_tile_cols()), v > 0), L.job, tiles);
         for (int i = 0; i < L.njobs; i++) {
             L.job[i].first_block = L.ntiles;
             L.ntiles += tiles[i];
@@ -988,7 +988,7 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
         InvVLaunch L;
         memset(&L, 0, sizeof(L));
         int tiles[JXS_MAXC], blocks = 0;
-        L.njobs = plan_inv_v(c, d->dcfg, fb, lout, v, v_rowpairs(v_warps(c, v, (uint32_t)jxs_inv_v_tile_cols())), L.job, tiles);
+        L.njobs = plan_inv_v(c, d->dcfg, fb, lout, v, v_rowpairs(v_warps(c, v, (uint32_t)jxs_inv_v_tile_cols()), v > (int)c->proxy), L.job, tiles);
         for (int i = 0; i < L.njobs; i++) {
             L.job[i].first_block = blocks;
             blocks += tiles[i];

@@ -225,10 +225,13 @@ static inline uint32_t v_warps(const jxs_cfg_t* c, int v, uint32_t cols) {
  * for smaller launches, down to one, where a warp's chain of steps is what
  * takes the time.  Fewer cost rows read twice (3 per warp): at 8 / 4 / 2 row
  * pairs 8 4K frames encode in 642 / 645 / 700 us and one frame in 155 / 147 /
- * 150 us, a 256x64 frame there and back takes 174 us at 8 and 157 at 1. */
-static inline int v_rowpairs(uint32_t warps) {
+ * 150 us, a 256x64 frame there and back takes 174 us at 8 and 157 at 1.
+ * The levels with int32 low bands on their other side (`deep`) read twice as
+ * much per row again, and 8 warps on each SM do for them: level 1 of a 4K frame
+ * at 4 / 1 row pairs takes 10.9 / 11.9 us forward and 10.4 / 12.3 inverse. */
+static inline int v_rowpairs(uint32_t warps, int deep) {
     int rp = JXS_V_ROWPAIRS;
-    while (rp > 1 && warps < 152 * 32) {
+    while (rp > 1 && warps < 152 * (deep ? 8u : 32u)) {
         rp >>= 1;
         warps <<= 1;
     }
