@@ -102,6 +102,7 @@ struct HostCopy {
     size_t dpitch, spitch;
     uint32_t items;     /* 16-byte chunks (or bytes) per row */
     uint32_t total;     /* in all rows */
+    uint32_t width;     /* bytes per row */
     int v16;
     uint32_t first_block;
 };
@@ -119,6 +120,31 @@ __global__ void __launch_bounds__(256) host_copy_kernel_n(const __grid_constant_
     const uint32_t y = i / C.items, x = i - y * C.items;
     if (C.v16) *(uint4*)(C.dst + y * C.dpitch + 16 * (size_t)x) = *(const uint4*)(C.src + y * C.spitch + 16 * (size_t)x);
     else C.dst[y * C.dpitch + x] = C.src[y * C.spitch + x];
+}
+
+/* Staged rows (starting on 16-byte boundaries, whole 16-byte words readable)
+ * to host memory at any address and pitch: a thread per 16-byte word of the
+ * destination, written whole where it lies inside a row (single bytes cross the
+ * link slowly), the source shifted to fit. */
+__global__ void __launch_bounds__(256) host_store_kernel_n(const __grid_constant__ HostCopies L) {
+    int k = 0;
+    while (k + 1 < L.n && blockIdx.x >= L.c[k + 1].first_block) k++;
+    const HostCopy& C = L.c[k];
+    const uint32_t i = (blockIdx.x - C.first_block) * blockDim.x + threadIdx.x;
+    if (i >= C.total) return;
+    const uint32_t y = i / C.items, x = i - y * C.items;
+    uint8_t* row = C.dst + y * C.dpitch;
+    const uint8_t* src = C.src + y * C.spitch;
+    const int width = (int)C.width, o = 16 * (int)x - (int)((uintptr_t)row & 15); /* the word's first byte in the row */
+    if (o >= width) return;
+    if (o >= 0 && o + 16 <= width) {
+        const uint32_t* w = (const uint32_t*)(src + (o & ~3));
+        const uint32_t sh = 8u * ((uint32_t)o & 3u), last = sh ? w[4] : 0u;
+        *(uint4*)(row + o) = make_uint4(__funnelshift_r(w[0], w[1], sh), __funnelshift_r(w[1], w[2], sh),
+                                        __funnelshift_r(w[2], w[3], sh), __funnelshift_r(w[3], last, sh));
+    } else {
+        for (int b = max(o, 0); b < min(o + 16, width); b++) row[b] = src[b];
+    }
 }
 
 /* 1: kernels may access this device's pageable host memory through the
@@ -183,9 +209,10 @@ struct HandleLoad {
 };
 
 /* 1: kernels may write `rows` rows of `width` bytes in pageable memory in
- * place, in whole 16-byte words for `aligned` (single samples cross the link
- * slowly: 1278x716 4:2:0 10 bit, rows not a multiple of 16 bytes, 209 us
- * instead of 116). */
+ * place, in whole 16-byte words for `aligned`: single samples cross the link
+ * slowly (1278x716 4:2:0 10 bit, rows not a multiple of 16 bytes, decodes in
+ * 209 us with the last level writing them, 116 with copies on completion, 88
+ * with host_store_kernel_n). */
 static int host_in_place(const void* p, size_t pitch, size_t width, size_t rows, int aligned) {
     return (!aligned || (((uintptr_t)p | pitch) & 15) == 0) && width && rows && pageable_direct() && !jxs_gpu_is_page_locked(p) &&
            host_resident(p, (rows - 1) * pitch + width);
@@ -210,6 +237,7 @@ static int host_copy_add(HostCopies* L, void* dst, size_t dpitch, const void* sr
     c.spitch = spitch;
     c.items = (uint32_t)items;
     c.total = (uint32_t)total;
+    c.width = (uint32_t)width;
     c.v16 = v16;
     c.first_block = L->nblocks;
     L->nblocks += (uint32_t)((total + 255) / 256);
@@ -221,6 +249,24 @@ static cudaError_t host_copy_launch(const HostCopies& L, cudaStream_t st) {
     if (!L.nblocks) return cudaSuccess;
     host_copy_kernel_n<<<L.nblocks, 256, 0, st>>>(L);
     return cudaGetLastError();
+}
+/* The same for rows to be stored at any address (host_store_kernel_n). */
+static int host_store_add(HostCopies* L, void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t rows) {
+    const uint64_t items = (width + 30) / 16, total = items * rows;
+    if (total > 0x7fffffffull || width > 0x3fffffffull || L->n >= JXS_MAXC) return 0;
+    if (!host_in_place(dst, dpitch, width, rows, 0)) return 0;
+    HostCopy& c = L->c[L->n++];
+    c.dst = (uint8_t*)dst;
+    c.src = (const uint8_t*)src;
+    c.dpitch = dpitch;
+    c.spitch = spitch;
+    c.items = (uint32_t)items;
+    c.total = (uint32_t)total;
+    c.width = (uint32_t)width;
+    c.v16 = 0;
+    c.first_block = L->nblocks;
+    L->nblocks += (uint32_t)((total + 255) / 256);
+    return 1;
 }
 static int host_copy_kernel(void* dst, size_t dpitch, const void* src, size_t spitch, size_t width, size_t rows, cudaStream_t st,
                             cudaError_t* err, const void* host, size_t host_pitch) {
@@ -1026,17 +1072,26 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
     CK(jxs_launch(publish_status_kernel, dim3(1), s->hdr_check ? 128u : 32u, 0, st, s->status_hd, s->status, s->hdr_hd, dbs,
                   s->hdr_check ? c->hdr_len : 0u));
     TMARK(3);
+    HostCopies stores;
+    stores.n = 0;
+    stores.nblocks = 0;
     s->ndefer = 0;
     for (uint32_t k = 0; k < c->nc; k++) {
         if (out_dev[k]) continue;
         const uint32_t ow = jxs_out_w(c, k), oh = jxs_out_h(c, k);
         const DeferredCopy cp{planes[k], (size_t)strides[k] * bps, s->out_stage + s->out_off[k], (size_t)stage_pitch(ow, bps) * bps,
                               (size_t)ow * bps, oh};
-        /* pageable planes are left to the completion thread */
+        /* pageable planes are left to the completion thread, or with one frame
+         * in flight stored by a kernel */
+        if (alone && host_store_add(&stores, cp.dst, cp.dpitch, cp.src, cp.spitch, cp.width, cp.height)) continue;
         if (jxs_gpu_is_page_locked(planes[k]))
             CK(cudaMemcpy2DAsync(cp.dst, cp.dpitch, cp.src, cp.spitch, cp.width, cp.height, cudaMemcpyDeviceToHost, st));
         else
             s->defer[s->ndefer++] = cp;
+    }
+    if (stores.nblocks) {
+        host_store_kernel_n<<<stores.nblocks, 256, 0, st>>>(stores);
+        CK(cudaGetLastError());
     }
     TMARK(4);
 #undef TMARK
