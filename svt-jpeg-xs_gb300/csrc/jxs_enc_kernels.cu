@@ -395,13 +395,18 @@ DEV void select_slice(const SliceInfo& I, int s, const uint32_t* __restrict__ co
 #define RC_LT_WORDS (5 * RC_LT_REGION) /* data, GCLI bits, GCLI bits with significance, fast / full sign bits */
 #define RC_VP_REGIONS 12
 
-/* vlc_encode_get_bits (PackPrecinct.h:86-104): ones of the unary code of a
- * GCLI difference x for the vertical prediction range (r, t). */
-DEV uint32_t vlc_vp_bits(int x, int r, int t) {
-    const int mx = max(r - t, 0);
-    if (x > mx) return (uint32_t)(x + mx);
-    x *= 2;
-    return (uint32_t)(x < 0 ? -x - 1 : x);
+/* Code lengths of two GCLIs c (16-bit halves) predicted from those above, tp,
+ * as ones of the unary code (vlc_encode_get_bits, PackPrecinct.h:86-104) plus
+ * K - VP_ONE: with d the GCLI less its prediction mt, neither below t (t2: t in
+ * both halves, G2: max(t, gtli above)), d < 0 takes -2 d - 1 ones, else 2 d or,
+ * past mt - t, d + mt - t.  *off: zero where d is 0. */
+#define VP_ONE 0x00010001u
+#define VP_K 0x20002000u
+DEV uint32_t vp_codes(uint32_t c, uint32_t tp, uint32_t t2, uint32_t G2, uint32_t* off) {
+    const uint32_t mt = __vmaxu2(tp, G2), gv = __vmaxu2(c, t2);
+    const uint32_t X = 2u * (gv - mt) + VP_K;
+    *off = X ^ VP_K;
+    return __vmaxu2(__vminu2(X, gv + (VP_K - t2)), (2u * VP_K - VP_ONE) - X);
 }
 
 /* Byte costs of a packet at quantization q for the refinements that lower the
@@ -607,7 +612,7 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, const SliceInfo& 
                      * halves of the warp; pairs of GCLIs in 16-bit halves */
                     const uint32_t g = base + 8 * (lane & 15);
                     const uint32_t nv = g < gend ? min(8u, gend - g) : 0u;
-                    const uint32_t E = 0x00ff00ffu, ONE = 0x00010001u, K = 0x20002000u;
+                    const uint32_t E = 0x00ff00ffu;
                     uint32_t wc[2] = {0, 0}, wt[2] = {0, 0}, c[4], tp[4], pv[4], kc = 0;
                     if (nv) {
                         wc[0] = *(const uint32_t*)(cur + g);
@@ -624,7 +629,7 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, const SliceInfo& 
                         pv[k] = ((vm >> sh) & E) * 0x101u;
                         c[k] = (wc[k >> 1] >> sh) & E & pv[k];
                         tp[k] = (wt[k >> 1] >> sh) & E;
-                        kc += (K - ONE) & pv[k];
+                        kc += (VP_K - VP_ONE) & pv[k];
                     }
                     uint32_t m8 = __vmaxu2(__vmaxu2(c[0], c[1]), __vmaxu2(c[2], c[3]));
                     m8 = max(m8 & 0xffffu, m8 >> 16);
@@ -642,17 +647,13 @@ DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, const SliceInfo& 
 #pragma unroll 2
                     for (int it = 0; it < its; it++) {
                         const int t = 2 * it + half;
-                        const uint32_t t2 = t * ONE, G2 = max(t, gtt) * ONE;
+                        const uint32_t t2 = t * VP_ONE, G2 = max(t, gtt) * VP_ONE;
                         uint32_t sum = 0, off = 0;
 #pragma unroll
                         for (int k = 0; k < 4; k++) {
-                            /* with d the GCLI less its prediction mt, neither
-                             * below t: d < 0 takes -2 d - 1 ones, else 2 d
-                             * or, past mt - t, d + mt - t; all plus K */
-                            const uint32_t mt = __vmaxu2(tp[k], G2), gv = __vmaxu2(c[k], t2);
-                            const uint32_t X = 2u * (gv - mt) + K;
-                            sum += __vmaxu2(__vminu2(X, gv + (K - t2)), (2u * K - ONE) - X) & pv[k];
-                            off |= (X ^ K) & pv[k];
+                            uint32_t x;
+                            sum += vp_codes(c[k], tp[k], t2, G2, &x) & pv[k];
+                            off |= x & pv[k];
                         }
                         sum -= kc; /* and the code's closing zero */
                         sum = (sum & 0xffffu) + (sum >> 16);
@@ -1445,40 +1446,36 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
         for (uint32_t base = sg.g0; base < gend; base += 128) {
             const uint32_t g = base + 4 * lane;
             const uint32_t nv = g < gend ? min(4u, gend - g) : 0u;
-            const uint32_t w4 = nv ? *(const uint32_t*)(grow + g) : 0u;
+            const uint32_t keep = nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
+            const uint32_t w4 = nv ? *(const uint32_t*)(grow + g) & keep : 0u;
             if (VPRED && vp) {
                 /* GCLIs predicted from the line above: code bits, and the
                  * groups of 8 that need none (lanes 2j, 2j + 1) */
                 const uint32_t wt = nv ? *(const uint32_t*)(grow - s_gp[sg.bl] + g) : 0u;
-                const int gmax = max((int)t, (int)s_gtt[sg.bl]);
-                uint32_t sum = 0, flag = 1;
+                const uint32_t t2 = t * VP_ONE, G2 = (uint32_t)max((int)t, (int)s_gtt[sg.bl]) * VP_ONE;
+                uint32_t two = 0, off = 0;
 #pragma unroll
-                for (int k = 0; k < 4; k++) {
-                    if (k < (int)nv) {
-                        const int c = (int)((w4 >> (8 * k)) & 255u), tp = (int)((wt >> (8 * k)) & 255u);
-                        const int mt = max(tp, gmax), gv = max(c, (int)t);
-                        sum += vlc_vp_bits(gv - mt, mt, (int)t) + 1;
-                        flag &= rmode ? (uint32_t)(c <= (int)t) : (uint32_t)(mt == gv);
-                    }
+                for (int k = 0; k < 2; k++) {
+                    const uint32_t pv = ((keep >> (8 * k)) & 0x00ff00ffu) * 0x101u;
+                    uint32_t x;
+                    two += (vp_codes((w4 >> (8 * k)) & 0x00ff00ffu, (wt >> (8 * k)) & 0x00ff00ffu, t2, G2, &x) - (VP_K - VP_ONE)) & pv;
+                    off |= x & pv;
                 }
+                const uint32_t sum = (two & 0xffffu) + (two >> 16);
+                const uint32_t flag = rmode ? (((w4 | 0x80808080u) - (t + 1) * 0x01010101u) & 0x80808080u) == 0u : off == 0u;
                 const uint32_t f2 = flag & __shfl_xor_sync(FULL, flag, 1), s2 = sum + __shfl_xor_sync(FULL, sum, 1);
                 pnsum += sum;
                 prsum += (!(lane & 1) && f2) ? s2 : 0u;
             }
-            uint32_t m = 0;
-#pragma unroll
-            for (int k = 0; k < 4; k++) m = max(m, k < (int)nv ? (w4 >> (8 * k)) & 255u : 0u);
-            const uint32_t mx = max(m, __shfl_xor_sync(FULL, m, 1)); /* significance group: 2 lanes */
-#pragma unroll
-            for (int k = 0; k < 4; k++) {
-                if (k < (int)nv) {
-                    const uint32_t v = (w4 >> (8 * k)) & 255u;
-                    dsum += v > t ? 4 * (v - t + 1 - fs) : 0u;
-                    vsum += v > t ? v - t + 1 : 1u;
-                    zsum += mx <= t;
-                }
-            }
-            if (fs && m > t) {
+            /* per byte: all ones for a group above gtli t, and its v - t - 1 */
+            const uint32_t y = (w4 | 0x80808080u) - (t + 1) * 0x01010101u;
+            const uint32_t above = sign_bytes(y), na = __popc(above & 0x01010101u);
+            const uint32_t dd = __dp4a(y & above & 0x7f7f7f7fu, 0x01010101u, 0u);
+            const uint32_t some = above | __shfl_xor_sync(FULL, above, 1); /* significance group: 2 lanes */
+            dsum += 4 * (dd + (2 - fs) * na);
+            vsum += dd + na + nv;
+            zsum += some ? 0u : nv;
+            if (fs && above) {
                 const uint4 c0 = *(const uint4*)(crow + 4 * g), c1 = *(const uint4*)(crow + 4 * g + 8);
                 const uint32_t cw[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
 #pragma unroll
@@ -1872,18 +1869,18 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
                 /* the lane's GCLIs, one per byte (0 past the line's end) */
                 uint32_t w4 = nv ? *(const uint32_t*)(grow + g) : 0u;
                 w4 &= nv >= 4 ? 0xffffffffu : (1u << (8 * nv)) - 1u;
-                /* per byte: planes above gtli d = max(v - t, 0), and v > t */
-                const uint32_t t4 = t * 0x01010101u;
-                const uint32_t d4 = __vsubus4(w4, t4), s4 = __vcmpgtu4(w4, t4);
-                const uint32_t dsum = __vsadu4(d4, 0u), nsig = __popc(s4 & 0x01010101u);
+                /* per byte: all ones for a group above gtli, and its planes
+                 * above gtli */
+                const uint32_t y = (w4 | 0x80808080u) - (t + 1) * 0x01010101u;
+                const uint32_t s4 = sign_bytes(y), d4 = (y & s4 & 0x7f7f7f7fu) + (s4 & 0x01010101u);
+                const uint32_t dsum = __dp4a(d4, 0x01010101u, 0u), nsig = __popc(s4 & 0x01010101u);
                 uint32_t v[4];
 #pragma unroll
                 for (int k = 0; k < 4; k++) v[k] = (w4 >> (8 * k)) & 255u;
-                const uint32_t m2 = __vmaxu4(w4, w4 >> 16), m = max(m2 & 255u, (m2 >> 8) & 255u);
-                const uint32_t mx = max(m, __shfl_xor_sync(FULL, m, 1));
+                const uint32_t some = s4 | __shfl_xor_sync(FULL, s4, 1);
                 /* a significance group without codes: all GCLIs <= gtli, or with
                  * prediction the group's flag */
-                bool insig = mx <= t;
+                bool insig = !some;
                 uint32_t n4[4] = {0, 0, 0, 0}; /* prediction: each GCLI's code length */
                 uint64_t vacc = 0;             /* otherwise: the lane's codes joined */
                 uint32_t vl = 0;
@@ -1891,17 +1888,18 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
                     /* codes predicted from the line above (vlc_encode,
                      * PackPrecinct.h:41-65) */
                     const uint32_t wt = nv ? *(const uint32_t*)(grow - s_gp[VPRED ? sg.bl : 0] + g) : 0u;
-                    const int gmax = max((int)t, (int)s_gtt[VPRED ? sg.bl : 0]);
-                    uint32_t flag = 1;
+                    const uint32_t t2 = t * VP_ONE, G2 = (uint32_t)max((int)t, (int)s_gtt[VPRED ? sg.bl : 0]) * VP_ONE;
+                    uint32_t off = 0;
 #pragma unroll
-                    for (int k = 0; k < 4; k++) {
-                        if (k < (int)nv) {
-                            const int c = (int)v[k], tp = (int)((wt >> (8 * k)) & 255u);
-                            const int mt = max(tp, gmax), gv = max(c, (int)t);
-                            n4[k] = vlc_vp_bits(gv - mt, mt, (int)t) + 1;
-                            flag &= rmode ? (uint32_t)(c <= (int)t) : (uint32_t)(mt == gv);
-                        }
+                    for (int k = 0; k < 2; k++) {
+                        const uint32_t pv = (k < (int)nv ? 0xffffu : 0u) | (k + 2 < (int)nv ? 0xffff0000u : 0u);
+                        uint32_t x;
+                        const uint32_t two = (vp_codes((w4 >> (8 * k)) & 0x00ff00ffu, (wt >> (8 * k)) & 0x00ff00ffu, t2, G2, &x) - (VP_K - VP_ONE)) & pv;
+                        off |= x & pv;
+                        n4[k] = two & 0xffffu;
+                        n4[k + 2] = two >> 16;
                     }
+                    const uint32_t flag = rmode ? s4 == 0u : off == 0u;
                     insig = (flag & __shfl_xor_sync(FULL, flag, 1)) != 0;
                 }
                 if (raw) {
