@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <type_traits>
 
 #include "jxs_core.h"
 #include "jxs_kernels.cuh"
@@ -920,7 +921,8 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
                 /* sign handling: the lane's 16 coefficients (inside the band
                  * width) by the number of gtli values at which they stay
                  * non-zero, counted like the GCLIs, 8 coefficients to 4-bit
-                 * counters and 16 to 8-bit ones */
+                 * counters and 16 to 8-bit ones, by a loop per quantizer
+                 * (8 4K frames with signs: 0.096 -> 0.094 ms each) */
                 uint4 c0 = make_uint4(0, 0, 0, 0), c1 = c0;
                 if (nv) {
                     c0 = *(const uint4*)(crow + 4 * g);
@@ -934,20 +936,25 @@ __device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, 
                 }
                 const bool large = __any_sync(FULL, w4 & 0x08080808u);
                 uint32_t za[4] = {0, 0, 0, 0}; /* levels 0, 2, 4, 6; 1, 3, 5, 7; the same of 8..15 */
+                auto count = [&](auto uq) {
 #pragma unroll
-                for (int i0 = 0; i0 < 16; i0 += 8) {
-                    uint32_t zl = 0, zg = 0;
+                    for (int i0 = 0; i0 < 16; i0 += 8) {
+                        uint32_t zl = 0, zg = 0;
 #pragma unroll
-                    for (int i = i0; i < i0 + 8; i++) {
-                        const uint32_t n = nz_levels(cw[i >> 1] >> (16 * (i & 1)) & 0x7fffu, (w4 >> (8 * (i >> 2))) & 255u, uniform);
-                        zl += shl_or_0(1u, 4 * n);
-                        if (large) zg += shl_or_0(1u, 4 * n - 32u);
+                        for (int i = i0; i < i0 + 8; i++) {
+                            const uint32_t m = cw[i >> 1] >> (16 * (i & 1)) & 0x7fffu;
+                            const uint32_t n = nz_levels(m, (w4 >> (8 * (i >> 2))) & 255u, decltype(uq)::value);
+                            zl += shl_or_0(1u, 4 * n);
+                            if (large) zg += shl_or_0(1u, 4 * n - 32u);
+                        }
+                        za[0] += zl & M;
+                        za[1] += (zl >> 4) & M;
+                        za[2] += zg & M;
+                        za[3] += (zg >> 4) & M;
                     }
-                    za[0] += zl & M;
-                    za[1] += (zl >> 4) & M;
-                    za[2] += zg & M;
-                    za[3] += (zg >> 4) & M;
-                }
+                };
+                if (uniform) count(std::true_type());
+                else count(std::false_type());
                 const uint32_t M2 = 0x00ff00ffu;
                 uint32_t zw = 0; /* of lane b < 16: levels b & 11 and (b & 11) + 4 in its halves */
 #pragma unroll
