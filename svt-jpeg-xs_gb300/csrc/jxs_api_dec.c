@@ -290,19 +290,23 @@ static int32_t submit_picture_locked(dec_prv_t* p, int slot, const uint8_t* bs, 
         uint32_t strides[4] = {f->image.stride[0], f->image.stride[1], f->image.stride[2], f->image.stride[3]};
         return jxs_gpu_dec_submit(p->gpu, slot, bs, size, NULL, planes, strides);
     }
+    /* the codestream crosses the link meanwhile */
+    const int staged = jxs_gpu_dec_stage(p->gpu, slot, bs, size);
     jxs_hdr_info_t info;
     int32_t r = jxs_cfg_decoder(p->tmp_cfg, bs, size, &info);
-    if (r) return r;
     /* every header byte but Lcod (bytes 12..15) must match the stream's */
-    if (info.hdr_len != p->info.hdr_len || memcmp(bs, p->cfg->hdr, 12) != 0 ||
-        memcmp(bs + 16, p->cfg->hdr + 16, info.hdr_len - 16) != 0)
-        return JXS_E_DEC_CONFIG;
-    int32_t err = 0;
-    jxs_frame_bytes_walk(p->cfg, bs, size, info.hdr_len, p->prec_off, &err);
-    if (err) return err;
+    if (!r && (info.hdr_len != p->info.hdr_len || memcmp(bs, p->cfg->hdr, 12) != 0 ||
+               memcmp(bs + 16, p->cfg->hdr + 16, info.hdr_len - 16) != 0))
+        r = JXS_E_DEC_CONFIG;
+    if (!r) jxs_frame_bytes_walk(p->cfg, bs, size, info.hdr_len, p->prec_off, &r);
+    if (r) {
+        /* the caller has its buffer back */
+        if (staged) jxs_gpu_dec_unstage(p->gpu, slot);
+        return r;
+    }
     void* planes[4] = {f->image.data_yuv[0], f->image.data_yuv[1], f->image.data_yuv[2], f->image.data_yuv[3]};
     uint32_t strides[4] = {f->image.stride[0], f->image.stride[1], f->image.stride[2], f->image.stride[3]};
-    return jxs_gpu_dec_submit(p->gpu, slot, bs, size, p->prec_off, planes, strides);
+    return jxs_gpu_dec_submit_staged(p->gpu, slot, bs, size, p->prec_off, planes, strides, staged);
 }
 
 static int32_t submit_picture(dec_prv_t* p, int slot, const uint8_t* bs, uint32_t size, svt_jpeg_xs_frame_t* f) {

@@ -398,7 +398,7 @@ DEV void select_slice(const SliceInfo& I, int s, const uint32_t* __restrict__ co
 
 /* Code lengths of two GCLIs c (16-bit halves) predicted from those above, tp,
  * as ones of the unary code (vlc_encode_get_bits, PackPrecinct.h:86-104) plus
- * K - VP_ONE: with d the GCLI less its prediction mt, neither below t (t2: t in
+ * VP_K - VP_ONE: with d the GCLI less its prediction mt, neither below t (t2: t in
  * both halves, G2: max(t, gtli above)), d < 0 takes -2 d - 1 ones, else 2 d or,
  * past mt - t, d + mt - t.  *off: zero where d is 0. */
 #define VP_ONE 0x00010001u

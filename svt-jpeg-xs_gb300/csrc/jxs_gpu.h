@@ -41,6 +41,11 @@ void jxs_gpu_dec_destroy(jxs_gpu_dec_t* d);
  * and its header is compared with the stream's when the frame completes. */
 int32_t jxs_gpu_dec_submit(jxs_gpu_dec_t* d, int slot, const uint8_t* bs, uint32_t size, const uint32_t* prec_off,
                            void* const planes[4], const uint32_t strides[4]);
+/* A host codestream's copy started before its precincts are known (jxs_gpu.cu). */
+int jxs_gpu_dec_stage(jxs_gpu_dec_t* d, int slot, const uint8_t* bs, uint32_t size);
+void jxs_gpu_dec_unstage(jxs_gpu_dec_t* d, int slot);
+int32_t jxs_gpu_dec_submit_staged(jxs_gpu_dec_t* d, int slot, const uint8_t* bs, uint32_t size, const uint32_t* prec_off,
+                                  void* const planes[4], const uint32_t strides[4], int staged);
 int32_t jxs_gpu_dec_wait(jxs_gpu_dec_t* d, int slot);
 int jxs_gpu_dec_ready(jxs_gpu_dec_t* d, int slot);
 

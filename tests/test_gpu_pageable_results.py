@@ -52,3 +52,26 @@ def test_results_in_pageable_memory(gpu, oracle, w, h, fmt, d, pad, offset):
                         assert (whole == 0xA5).all()
     enc.close()
     dec.close()
+
+
+def test_refused_codestreams_between_good_ones(gpu, oracle):
+    """A host codestream whose precincts or header are found wrong is refused
+    by the host, with its copy to the device already under way."""
+    w, h, fmt, d = 640, 64, S.FMT_YUV422, 8
+    p = oracle.make_params(w, h, d, fmt, 6, 1, 2, 5)
+    err, bs = oracle.oracle_encode(p, S.frame(w, h, d, fmt, seed=5))[:2]
+    assert err == 0
+    err, want = oracle.oracle_decode(bs)
+    assert err == 0
+    slice1 = bs.tobytes().index(b"\xff\x20\x00\x04\x00\x01")
+    dec = gpu.Decoder(bs)
+    for at in (None, None, slice1 + 5, None, slice1 + 6, None, 20, None):
+        sent = bs.copy()
+        if at is not None:
+            sent[at] ^= 0xff
+        outs = [np.zeros(x.shape, x.dtype) for x in want]
+        r = dec.send(sent, outs)
+        r = r or dec.get()[0]
+        assert (r != 0) == (at is not None)
+        assert r or all(np.array_equal(a, b) for a, b in zip(outs, want))
+    dec.close()
