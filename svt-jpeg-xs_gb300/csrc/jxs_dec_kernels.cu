@@ -319,14 +319,17 @@ DEV uint32_t be24(const uint8_t* p) { return ((uint32_t)p[0] << 16) | ((uint32_t
  * the constant-bit-rate split of Lcod puts it (EncHandle.c:760-809), and the
  * 24-bit precinct lengths lead from there to p, three steps at most in slices
  * of 16 lines with two vertical levels.  False if the slice is not there. */
-DEV bool find_precinct(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size, uint32_t phb, uint32_t p,
+DEV bool find_precinct(const jxs_cfg_t* __restrict__ cfg, const uint8_t* bs, uint32_t size, uint32_t phb, uint32_t p,
                        uint32_t* out) {
     const uint32_t per = cfg->pps * cfg->ncol, s = p / per;
     uint64_t off = cfg->slice_begin[s];
     *out = 0;
-    if (off + 6 > size || bs[off] != 0xff || bs[off + 1] != 0x20 || bs[off + 2] != 0 || bs[off + 3] != 4 ||
-        (((uint32_t)bs[off + 4] << 8) | bs[off + 5]) != s)
-        return false;
+    if (off + 6 > size) return false;
+    /* its six bytes at once: byte after byte, each load would wait for the
+     * comparison before it (2 % of a 3840x2160 frame's time) */
+    const uint8_t* h = bs + off;
+    const uint32_t at = ((uint32_t)h[0] << 24) | ((uint32_t)h[1] << 16) | ((uint32_t)h[2] << 8) | h[3], num = ((uint32_t)h[4] << 8) | h[5];
+    if (at != 0xff200004u || num != s) return false;
     off += 6;
     for (uint32_t i = s * per; i < p; i++) {
         if (off + phb > size) return false;
@@ -340,9 +343,9 @@ DEV bool find_precinct(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restr
 }
 /* The same for the end of a slice's last precinct p: the next slice, or the
  * end of the codestream (true for the other precincts). */
-DEV bool slice_ends(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size, uint32_t p, uint64_t end) {
+DEV bool slice_ends(const jxs_cfg_t* __restrict__ cfg, const uint8_t* bs, uint32_t size, uint32_t p, uint64_t end) {
     const uint32_t per = cfg->pps * cfg->ncol, s = p / per;
-    if (p + 1 == cfg->nprec) return end + 2 <= size && bs[end] == 0xff && bs[end + 1] == 0x11;
+    if (p + 1 == cfg->nprec) return end + 2 <= size && (((uint32_t)bs[end] << 8) | bs[end + 1]) == 0xff11u;
     return p + 1 != (s + 1) * per || end == cfg->slice_begin[s + 1];
 }
 
@@ -378,8 +381,8 @@ DEV bool slice_ends(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict
  * 10-bit frames: 263 us before, 223 us so; 203 us with the segments' data
  * positions from the codes' bits instead of from a pass over all GCLIs. */
 template <bool FS, bool VP, bool BATCH>
-__device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t bs_size,
-                                            const uint32_t* __restrict__ prec_off, int16_t* __restrict__ coef,
+__device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, const uint8_t* bs, uint32_t bs_size,
+                                            const uint32_t* prec_off, int16_t* coef,
                                             uint32_t cap_bytes, uint32_t cap_groups, uint32_t cap_seg, int* status, const int p,
                                             uint8_t* top_gcl, uint8_t* top_t, const int vp_ok, const int rank = 0,
                                             const int turns = 0) {
@@ -1259,8 +1262,8 @@ __device__ __forceinline__ void unpack_body(const jxs_cfg_t* __restrict__ cfg, c
  * split of Lcod puts it (EncHandle.c:760-809); its precincts are found by
  * following the 24-bit precinct lengths, and the walk must end exactly at
  * the next slice (or at EOC).  False if anything is not so. */
-DEV bool walk_slice(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size,
-                    uint32_t* __restrict__ prec_off, const uint32_t s) {
+DEV bool walk_slice(const jxs_cfg_t* __restrict__ cfg, const uint8_t* bs, uint32_t size,
+                    uint32_t* prec_off, const uint32_t s) {
     if (cfg->max_slice_budget == 0) return false;
     uint64_t off = cfg->slice_begin[s];
     if (off + 6 > size || bs[off] != 0xff || bs[off + 1] != 0x20 || bs[off + 2] != 0 || bs[off + 3] != 4 ||
@@ -1283,8 +1286,8 @@ DEV bool walk_slice(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict
 
 /* Fallback when the prediction failed: one thread walks the whole codestream
  * from the header (get_slice_size, DecThreadInit.c:35-131). */
-DEV void walk_sequential(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size,
-                         uint32_t* __restrict__ prec_off, int* status) {
+DEV void walk_sequential(const jxs_cfg_t* __restrict__ cfg, const uint8_t* bs, uint32_t size,
+                         uint32_t* prec_off, int* status) {
     uint64_t off = cfg->hdr_len;
     for (uint32_t s = 0; s < cfg->nslices; s++) {
         if (off + 6 > size) {
@@ -1322,7 +1325,7 @@ DEV void walk_sequential(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __res
  * the latency of a handful of loads that wait for one another; the second step
  * as a launch of its own cost 5 us, taken or not. */
 #define WALK_THREADS 512
-DEV void walk_frame(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs, uint32_t size, uint32_t* __restrict__ prec_off,
+DEV void walk_frame(const jxs_cfg_t* __restrict__ cfg, const uint8_t* bs, uint32_t size, uint32_t* prec_off,
                     int* status) {
     bool lost = false;
     for (uint32_t s = threadIdx.x; s < cfg->nslices; s += blockDim.x) lost |= !walk_slice(cfg, bs, size, prec_off, s);
@@ -1335,9 +1338,9 @@ DEV void walk_frame(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict
 /* 4 blocks of 512 threads per SM where the shared memory allows it (32
  * registers) */
 template <bool FS>
-__global__ void __launch_bounds__(UK_THREADS, 4) unpack_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs,
-                                                               uint32_t bs_size, const uint32_t* __restrict__ prec_off,
-                                                               int16_t* __restrict__ coef, uint32_t cap_bytes, uint32_t cap_groups,
+__global__ void __launch_bounds__(UK_THREADS, 4) unpack_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* bs,
+                                                               uint32_t bs_size, const uint32_t* prec_off,
+                                                               int16_t* coef, uint32_t cap_bytes, uint32_t cap_groups,
                                                                uint32_t cap_seg, int* status) {
     unpack_body<FS, false, false>(cfg, bs, bs_size, prec_off, coef, cap_bytes, cap_groups, cap_seg, status, (int)blockIdx.x, nullptr, nullptr,
                            0);
@@ -1364,9 +1367,9 @@ __global__ void __launch_bounds__(UK_THREADS, 4) unpack_batch_kernel(const __gri
  * included.  Bound by the latency of one precinct and the turns, which take
  * two GCLIs to an instruction: 1279x717 4:4:4 with slices of 4 rows 116 us
  * with a block per slice and a GCLI per lane, 48 us now. */
-__global__ void __launch_bounds__(UK_THREADS) unpack_vpred_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs,
-                                                                  uint32_t bs_size, const uint32_t* __restrict__ prec_off,
-                                                                  int16_t* __restrict__ coef, uint32_t cap_bytes,
+__global__ void __launch_bounds__(UK_THREADS) unpack_vpred_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* bs,
+                                                                  uint32_t bs_size, const uint32_t* prec_off,
+                                                                  int16_t* coef, uint32_t cap_bytes,
                                                                   uint32_t cap_groups, uint32_t cap_seg, int* status) {
     extern __shared__ __align__(16) uint8_t dsm[];
     __shared__ uint8_t top_t[JXS_MAXBLINES];
@@ -1391,8 +1394,8 @@ __global__ void __launch_bounds__(UK_THREADS) unpack_vpred_kernel(const jxs_cfg_
     cl.sync(); /* and until none does any more */
 }
 
-__global__ void __launch_bounds__(WALK_THREADS) walk_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ bs,
-                                                            uint32_t size, uint32_t* __restrict__ prec_off, int* status) {
+__global__ void __launch_bounds__(WALK_THREADS) walk_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* bs,
+                                                            uint32_t size, uint32_t* prec_off, int* status) {
     dep_wait();
     walk_frame(cfg, bs, size, prec_off, status);
 }

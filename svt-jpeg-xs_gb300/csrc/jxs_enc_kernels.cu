@@ -198,8 +198,8 @@ DEV int prec_search(const RcParams& P, const uint32_t* T, int ldt, const uint32_
  * into `area`, one (Q, R) for the slice by the precinct searches, then the
  * budget of each precinct, kept in rc[p].total_bytes.  Run by a whole
  * block; returns the error (every thread). */
-DEV int slice_common(const RcParams& P, int s, const SliceSplit& sp, const uint32_t* __restrict__ cost, uint32_t* area,
-                     PrecRC* __restrict__ rc, int* __restrict__ status) {
+DEV int slice_common(const RcParams& P, int s, const SliceSplit& sp, const uint32_t* cost, uint32_t* area,
+                     PrecRC* rc, int* status) {
     __shared__ int s_cerr;
     const int nr = P.nr, nt = (P.max_q + 1) * nr, rc_mode = P.rc_mode;
     const uint32_t np_all = P.np, hdrs0 = P.hdrs0, hdrs1 = P.hdrs1;
@@ -297,8 +297,8 @@ DEV int slice_common(const RcParams& P, int s, const SliceSplit& sp, const uint3
  * PackPrecinct.c:513-536).  Returns an error code; that, the carry, the
  * running offset and q, r are the same in every lane. */
 DEV int prec_select(const RcParams& P, int s, uint32_t i, const SliceSplit& sp, const uint32_t* T, const uint32_t* F, int ldt,
-                    const uint32_t* TS, int ld, int scan, uint32_t& carry, uint32_t& run, int& q, int& r, PrecRC* __restrict__ rc,
-                    int* __restrict__ status) {
+                    const uint32_t* TS, int ld, int scan, uint32_t& carry, uint32_t& run, int& q, int& r, PrecRC* rc,
+                    int* status) {
     const uint32_t p = sp.first_p + i;
     const uint32_t budget = (P.rc_mode >= 2 ? rc[p].total_bytes : (i == 0 ? sp.first_b : sp.min_b) + (i < sp.left ? 1 : 0)) + carry;
     const uint32_t hdr = p + 1 >= P.np ? P.hdrs1 : P.hdrs0;
@@ -354,8 +354,8 @@ DEV int prec_select(const RcParams& P, int s, uint32_t i, const SliceSplit& sp, 
  * A chain of one search after another, 4 per slice of 16 lines: by one
  * thread, step by step, 24,000 cycles of the slice's last block, alone on
  * the critical path of a single frame; now 5,000. */
-DEV void select_slice(const SliceInfo& I, int s, const uint32_t* __restrict__ cost, uint32_t* area, uint32_t area_words,
-                      PrecRC* __restrict__ rc, int* __restrict__ status) {
+DEV void select_slice(const SliceInfo& I, int s, const uint32_t* cost, uint32_t* area, uint32_t area_words,
+                      PrecRC* rc, int* status) {
     __shared__ int s_err;
     RcParams P = I.P;
     P.empty = I.empty[threadIdx.x & 31];
@@ -519,9 +519,9 @@ DEV void cost_items(uint32_t nbl, uint32_t npk, const uint8_t* order, const uint
  * 30 us.  Two blocks per SM: with registers for three (40) the loop spills
  * (114 us). */
 template <typename Stage>
-DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, const SliceInfo& I, int s, const uint8_t* __restrict__ gcli,
-                            const uint32_t* __restrict__ cost, uint32_t* area, PrecRC* __restrict__ rc,
-                            int* __restrict__ status, Stage& stage_kind, const uint8_t* lgain, const uint8_t* lprio,
+DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, const SliceInfo& I, int s, const uint8_t* gcli,
+                            const uint32_t* cost, uint32_t* area, PrecRC* rc,
+                            int* status, Stage& stage_kind, const uint8_t* lgain, const uint8_t* lprio,
                             const uint8_t* lfb, const uint32_t* lsig, const uint32_t* lraw, const jxs_bline_t* bls,
                             const jxs_seg_t* segs, const uint8_t* s_pkbl0, const uint8_t* s_pknbl, const uint8_t* s_order, uint32_t* opk,
                             uint16_t* items) {
@@ -766,10 +766,10 @@ DEV uint32_t shl_or_0(uint32_t a, uint32_t n) {
 }
 
 template <bool SIGNS, bool VPRED>
-__device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ gcli,
-                                             const uint16_t* __restrict__ coef, uint32_t* __restrict__ cost,
-                                             uint32_t* __restrict__ slice_done, PrecRC* __restrict__ rc,
-                                             int* __restrict__ status, const int p) {
+__device__ __forceinline__ void rc_cost_body(const jxs_cfg_t* __restrict__ cfg, const uint8_t* gcli,
+                                             const uint16_t* coef, uint32_t* cost,
+                                             uint32_t* slice_done, PrecRC* rc,
+                                             int* status, const int p) {
     /* per band line: GCLI and significance-maximum histograms (with sign
      * handling also the coefficients by non-zero levels), then per gtli data
      * / GCLI bits without and with significance and the sign bits; the area
@@ -1270,9 +1270,9 @@ struct PkSeg {
  * control (RateControl.c:526-676), and pass B writes the prediction codes
  * (pack_bitplane_count_vpred_*, PackPrecinct.c:47-74). */
 template <bool SIGNS, bool VPRED, bool BATCH>
-__device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, const uint16_t* __restrict__ coef,
-                                          const uint8_t* __restrict__ gcli, const PrecRC* __restrict__ rc,
-                                          const uint32_t* __restrict__ cost, uint8_t* __restrict__ out, uint32_t cap_words,
+__device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, const uint16_t* coef,
+                                          const uint8_t* gcli, const PrecRC* rc,
+                                          const uint32_t* cost, uint8_t* out, uint32_t cap_words,
                                           int* status, const int p) {
     extern __shared__ __align__(16) uint32_t buf[];
     /* per segment: data bits, VLC bits, groups without codes, signs, then
@@ -2083,10 +2083,10 @@ __device__ __forceinline__ void pack_body(const jxs_cfg_t* __restrict__ cfg, con
 /* kernels: one frame, or a batch of frames (block -> frame by its first block) */
 /* ------------------------------------------------------------------------ */
 template <bool SIGNS, bool VPRED>
-__global__ void __launch_bounds__(RC_THREADS, VPRED ? 2 : SIGNS ? 3 : 4) rc_cost_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* __restrict__ gcli,
-                                                           const uint16_t* __restrict__ coef, uint32_t* __restrict__ cost,
-                                                           uint32_t* __restrict__ slice_done, PrecRC* __restrict__ rc,
-                                                           int* __restrict__ status) {
+__global__ void __launch_bounds__(RC_THREADS, VPRED ? 2 : SIGNS ? 3 : 4) rc_cost_kernel(const jxs_cfg_t* __restrict__ cfg, const uint8_t* gcli,
+                                                           const uint16_t* coef, uint32_t* cost,
+                                                           uint32_t* slice_done, PrecRC* rc,
+                                                           int* status) {
     rc_cost_body<SIGNS, VPRED>(cfg, gcli, coef, cost, slice_done, rc, status, (int)blockIdx.x);
 }
 
@@ -2097,9 +2097,9 @@ __global__ void __launch_bounds__(RC_THREADS, VPRED ? 2 : SIGNS ? 3 : 4) rc_cost
 }
 
 template <bool SIGNS, bool VPRED>
-__global__ void __launch_bounds__(PK_THREADS, VPRED ? 3 : 4) pack_kernel(const jxs_cfg_t* __restrict__ cfg, const uint16_t* __restrict__ coef,
-                                                          const uint8_t* __restrict__ gcli, const PrecRC* __restrict__ rc,
-                                                          const uint32_t* __restrict__ cost, uint8_t* __restrict__ out,
+__global__ void __launch_bounds__(PK_THREADS, VPRED ? 3 : 4) pack_kernel(const jxs_cfg_t* __restrict__ cfg, const uint16_t* coef,
+                                                          const uint8_t* gcli, const PrecRC* rc,
+                                                          const uint32_t* cost, uint8_t* out,
                                                           uint32_t cap_words, int* status) {
     pack_body<SIGNS, VPRED, false>(cfg, coef, gcli, rc, cost, out, cap_words, status, (int)blockIdx.x);
 }

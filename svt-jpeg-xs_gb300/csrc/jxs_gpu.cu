@@ -75,8 +75,8 @@ extern "C" int jxs_gpu_is_page_locked(const void* p) {
  * engines' queues between the frames' large transfers.  Leaves the status at
  * zero for the slot's next frame, which so needs no memset.  `hdr`: header of
  * a device codestream, for the host to check. */
-__global__ void publish_status_kernel(int* __restrict__ host, int* __restrict__ status, uint8_t* __restrict__ hdr_h,
-                                      const uint8_t* __restrict__ hdr, uint32_t hdr_len) {
+__global__ void publish_status_kernel(int* host, int* status, uint8_t* hdr_h,
+                                      const uint8_t* hdr, uint32_t hdr_len) {
     dep_wait();
     for (uint32_t i = threadIdx.x; i < hdr_len; i += blockDim.x) hdr_h[i] = hdr[i];
     if (threadIdx.x == 0) {

@@ -320,9 +320,12 @@ static inline cudaError_t jxs_smem_attr(K kern, int bytes, std::atomic<int>* cac
  * block of every such kernel calls dep_wait() before it reads or writes
  * anything another kernel of the stream touches (it returns when the kernel
  * before has completed, and with it, since that one waited too, all earlier
- * ones).  Behind a copy, a memset or an event the launch is an ordinary one,
- * and dep_wait() returns at once in a kernel that was launched the ordinary
- * way.  A 4K frame encodes in 114 us instead of 125 and decodes in 107
+ * ones).  Pointers to such data carry no __restrict__, here and in what
+ * these kernels call: it would promise that nothing else writes the data while
+ * the kernel runs, which before the wait is not so, and let their loads move
+ * above it.  Only the handle's configuration is constant that long.  Behind a
+ * copy, a memset or an event the launch is an ordinary one, and dep_wait()
+ * returns at once in a kernel that was launched the ordinary way.  A 4K frame encodes in 114 us instead of 125 and decodes in 107
  * instead of 118; a 256x64 one takes 119 us there and back instead of 145.
  * Starting the next kernel's blocks earlier still (a trigger at the top of
  * each kernel) gained nothing there, and their waiting blocks cost batches up
