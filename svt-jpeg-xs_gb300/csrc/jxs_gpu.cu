@@ -510,6 +510,18 @@ extern "C" jxs_gpu_enc_t* jxs_gpu_enc_create(const jxs_cfg_t* cfg, int nslots, i
     return e;
 }
 
+/* After a submission that failed half way: waits for what it had queued,
+ * which reads and writes the caller's buffers, and leaves the frame status at
+ * zero, as a frame's last launch does otherwise.  The CUDA call's error is
+ * reported already and must not turn up behind the next frame's launches. */
+template <class Slot> static int32_t abandon(Slot* s, cudaStream_t st, int32_t r) {
+    s->ndefer = 0;
+    cudaMemsetAsync(s->status, 0, 64, st);
+    cudaStreamSynchronize(st);
+    cudaGetLastError();
+    return r;
+}
+
 static int32_t enc_run(jxs_gpu_enc_t* e, EncSlot* s, void* const planes[4], const uint32_t strides[4], uint8_t* out, int alone) {
     s->ndefer = 0;
     const jxs_cfg_t* c = &e->cfg;
@@ -624,7 +636,9 @@ extern "C" int32_t jxs_gpu_enc_submit(jxs_gpu_enc_t* e, int slot, void* const pl
     EncSlot* s = &e->slot[slot];
     s->busy = 1;
     const int32_t r = enc_run(e, s, planes, strides, out, e->load.submit());
-    if (r != JXS_OK) e->load.done();
+    if (r == JXS_OK) return r;
+    abandon(s, enc_stream(e, s), r);
+    e->load.done();
     return r;
 }
 
@@ -1032,10 +1046,7 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
         L.njobs = plan_inv_h(c, d->dcfg, fb, lout, pass, L.job);
         if (!L.njobs) continue;
         const int blocks = inv_h_layout(L, jxs_inv_h_max_rows_per_block());
-        if (blocks < 0) {
-            CK(cudaMemsetAsync(s->status, 0, 64, st)); /* this frame's status is not published */
-            return JXS_E_BAD_PARAM;
-        }
+        if (blocks < 0) return JXS_E_BAD_PARAM;
         CK(jxs_launch_inv_h(&L, pass == 0 ? 0 : sample_kind, blocks, st));
         KMARK();
     }
@@ -1130,8 +1141,11 @@ extern "C" int32_t jxs_gpu_dec_submit(jxs_gpu_dec_t* d, int slot, const uint8_t*
 extern "C" int32_t jxs_gpu_dec_submit_staged(jxs_gpu_dec_t* d, int slot, const uint8_t* bs, uint32_t size, const uint32_t* prec_off,
                                              void* const planes[4], const uint32_t strides[4], int staged) {
     if (!d || slot < 0 || slot >= d->nslots) return JXS_E_BAD_PARAM;
-    const int32_t r = dec_run(d, &d->slot[slot], bs, size, prec_off, planes, strides, d->load.submit(), staged);
-    if (r != JXS_OK) d->load.done();
+    DecSlot* s = &d->slot[slot];
+    const int32_t r = dec_run(d, s, bs, size, prec_off, planes, strides, d->load.submit(), staged);
+    if (r == JXS_OK) return r;
+    abandon(s, dec_stream(d, s), r);
+    d->load.done();
     return r;
 }
 
@@ -1159,7 +1173,7 @@ static int32_t dec_wait(jxs_gpu_dec_t* d, int slot) {
         again++;
         const int32_t r = dec_run(d, s, s->arg_bs, s->arg_size, s->arg_walked ? s->prec_off_h : NULL, s->arg_planes,
                                   s->arg_strides, 0, 0);
-        if (r != JXS_OK) return r;
+        if (r != JXS_OK) return abandon(s, dec_stream(d, s), r);
         if (cudaEventSynchronize(s->done) != cudaSuccess) {
             fprintf(stderr, "jxs: decode failed: %s\n", cudaGetErrorString(cudaGetLastError()));
             s->ndefer = 0;
