@@ -29,6 +29,7 @@
 #include "SvtJpegxs.h"
 #include "jxs_batch.h"
 #include "jxs_gpu.h"
+#include "jxs_handle.h"
 #include "jxs_kernels.cuh"
 #include "jxs_plan.cuh"
 
@@ -185,28 +186,6 @@ static int host_resident(const void* p, size_t bytes) {
         if (!(vec[i] & 1)) return 0;
     return 1;
 }
-
-/* A handle's frames in flight (submitted and not yet waited for).  One frame
- * at a time, a result for pageable memory is best written there by the
- * kernel that makes it, when the device reaches that memory directly: no
- * staging, no copy after the host has seen the frame done (1920x1080 4:2:2
- * 8 bit decodes in 121 us instead of 157).  With more in flight the copy
- * engines carry it beside the next frames' kernels, which otherwise wait on
- * the link (a pipeline of 4K frames from and to pageable memory: 18.5 instead
- * of 20.2 Gpix/s).  A pipeline is at times down to no frame, so that the
- * first way takes more than kAlone such submissions in a row. */
-struct HandleLoad {
-    static const int kAlone = 4;
-    std::atomic<int> in_flight{0}, alone{0};
-    int submit() { /* 1: write results in place */
-        if (in_flight.fetch_add(1) != 0) {
-            alone.store(0);
-            return 0;
-        }
-        return alone.fetch_add(1) >= kAlone;
-    }
-    void done() { in_flight.fetch_sub(1); }
-};
 
 /* 1: kernels may write `rows` rows of `width` bytes in pageable memory in
  * place, in whole 16-byte words for `aligned`: single samples cross the link
