@@ -738,6 +738,7 @@ struct DecSlot {
     const uint8_t* arg_bs;  /* device codestream (the caller's or the slot's copy) */
     uint32_t arg_size;
     int arg_walked;         /* precinct offsets in prec_off_h */
+    int arg_vpred, arg_locate;
     void* arg_planes[4];
     uint32_t arg_strides[4];
     DeferredCopy defer[JXS_MAXC]; /* output planes in pageable memory */
@@ -764,8 +765,7 @@ struct jxs_gpu_dec {
     int nkern;
     uint64_t timed_frames;
     uint64_t serial;
-    int vpred;                   /* decode slice by slice: the stream uses vertical prediction */
-    int walk;                    /* locate a device codestream's precincts first: its slices are not where predicted */
+    DecHints hints;
     HandleLoad load;
     std::mutex mu;
 };
@@ -927,12 +927,12 @@ static int32_t dec_bs_room(DecSlot* s, uint32_t size, cudaStream_t st) {
     return JXS_OK;
 }
 static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t size, const uint32_t* prec_off,
-                       void* const planes[4], const uint32_t strides[4], int alone, int staged) {
+                       void* const planes[4], const uint32_t strides[4], int alone, int staged, int vpred, int locate) {
     s->ndefer = 0;
     const jxs_cfg_t* c = &d->cfg;
     const uint32_t bps = bytes_per_sample(c);
     const cudaStream_t st = dec_stream(d, s);
-    const int walk = !prec_off && (d->walk || c->max_slice_budget == 0 || c->pps * c->ncol > kSelfSteps);
+    const int walk = !prec_off && (locate || c->max_slice_budget == 0 || c->pps * c->ncol > kSelfSteps);
     s->timed = d->timing;
 #define TMARK(i) \
     if (s->timed) CK(cudaEventRecord(s->tev[i], st))
@@ -971,13 +971,15 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
     s->arg_bs = dbs;
     s->arg_size = size;
     s->arg_walked = prec_off != NULL;
+    s->arg_vpred = vpred;
+    s->arg_locate = locate;
     for (int k = 0; k < 4; k++) {
         s->arg_planes[k] = planes[k];
         s->arg_strides[k] = strides[k];
     }
     TMARK(1);
     KMARK();
-    if (d->vpred)
+    if (vpred)
         CK(jxs_launch_unpack_vpred(d->dcfg, dbs, size, doff, s->coef, c->nslices, c->pps, d->cap_bytes, d->cap_groups, d->cap_seg,
                                    s->status, st));
     else
@@ -1121,7 +1123,8 @@ extern "C" int32_t jxs_gpu_dec_submit_staged(jxs_gpu_dec_t* d, int slot, const u
                                              void* const planes[4], const uint32_t strides[4], int staged) {
     if (!d || slot < 0 || slot >= d->nslots) return JXS_E_BAD_PARAM;
     DecSlot* s = &d->slot[slot];
-    const int32_t r = dec_run(d, s, bs, size, prec_off, planes, strides, d->load.submit(), staged);
+    const int32_t r = dec_run(d, s, bs, size, prec_off, planes, strides, d->load.submit(), staged, d->hints.vpred.load(),
+                              prec_off ? 0 : d->hints.locate());
     if (r == JXS_OK) return r;
     abandon(s, dec_stream(d, s), r);
     d->load.done();
@@ -1140,25 +1143,26 @@ static int32_t dec_wait(jxs_gpu_dec_t* d, int slot) {
     const jxs_cfg_t* c = &d->cfg;
     const int other_hdr =
         s->hdr_check && (memcmp(s->hdr_h, c->hdr, 12) != 0 || memcmp(s->hdr_h + 16, c->hdr + 16, c->hdr_len - 16) != 0);
-    int again = 0;
-    while (!other_hdr && (*s->status_h == JXS_E_DEC_VPRED || *s->status_h == JXS_E_DEC_WALK) && again < 2) {
-        /* the frame uses vertical prediction: decode it again slice by slice,
-         * and the stream's later frames that way from the start; or its
-         * slices are not at the constant-bit-rate split: decode it again with
-         * its precincts located first, and later frames too if that helps */
-        const int vpred = *s->status_h == JXS_E_DEC_VPRED, before = d->walk;
-        if (vpred) d->vpred = 1;
-        else d->walk = 1;
-        again++;
+    const int vpred0 = s->arg_vpred, locate0 = s->arg_locate;
+    for (int again = 0; !other_hdr && (*s->status_h == JXS_E_DEC_VPRED || *s->status_h == JXS_E_DEC_WALK) && again < 2; again++) {
+        /* the frame uses vertical prediction: decode it again slice by
+         * slice; or its slices are not at the constant-bit-rate split: decode
+         * it again with its precincts located first */
+        const int vpred = s->arg_vpred || *s->status_h == JXS_E_DEC_VPRED;
+        const int locate = s->arg_locate || *s->status_h == JXS_E_DEC_WALK;
         const int32_t r = dec_run(d, s, s->arg_bs, s->arg_size, s->arg_walked ? s->prec_off_h : NULL, s->arg_planes,
-                                  s->arg_strides, 0, 0);
+                                  s->arg_strides, 0, 0, vpred, locate);
         if (r != JXS_OK) return abandon(s, dec_stream(d, s), r);
         if (cudaEventSynchronize(s->done) != cudaSuccess) {
             fprintf(stderr, "jxs: decode failed: %s\n", cudaGetErrorString(cudaGetLastError()));
             s->ndefer = 0;
             return JXS_E_DEC_INTERNAL;
         }
-        if (!vpred && *s->status_h != 0 && *s->status_h != JXS_E_DEC_VPRED) d->walk = before;
+    }
+    if (*s->status_h == 0) {
+        /* that helped: later frames so from the start */
+        if (s->arg_vpred && !vpred0) d->hints.vpred.store(1);
+        if (s->arg_locate && !locate0) d->hints.elsewhere();
     }
     if (!run_deferred(s->defer, &s->ndefer, s->st)) {
         fprintf(stderr, "jxs: copying the decoded planes to host memory failed\n");

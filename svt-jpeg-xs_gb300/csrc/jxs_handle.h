@@ -24,4 +24,27 @@ struct HandleLoad {
     void done() { in_flight.fetch_sub(1); }
 };
 
+/* What a decoder's frames told about its stream, for the frames after them:
+ * set by the completion thread, read by the submitting ones. */
+struct DecHints {
+    /* the stream uses vertical prediction (decoded slice by slice) */
+    std::atomic<int> vpred{0};
+    /* Device codestreams whose slices are not at the constant-bit-rate split:
+     * the precincts of this many frames to come are located first, which
+     * costs a 4K frame 11 us, where finding that out costs a decode.  Each
+     * time the split fails again after that, twice as many. */
+    static constexpr int kFirst = 16, kMost = 4096;
+    std::atomic<int> left{0}, next{kFirst};
+    int locate() { /* 1: locate this frame's precincts first */
+        int n = left.load();
+        while (n > 0 && !left.compare_exchange_weak(n, n - 1)) {}
+        return n > 0;
+    }
+    void elsewhere() { /* a frame not at the split was decoded after all */
+        int none = 0;
+        const int n = next.load();
+        if (left.compare_exchange_strong(none, n)) next.store(n < kMost ? 2 * n : kMost);
+    }
+};
+
 #endif
