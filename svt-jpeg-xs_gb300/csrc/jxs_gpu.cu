@@ -738,7 +738,7 @@ struct DecSlot {
     const uint8_t* arg_bs;  /* device codestream (the caller's or the slot's copy) */
     uint32_t arg_size;
     int arg_walked;         /* precinct offsets in prec_off_h */
-    int arg_vpred, arg_locate;
+    int arg_vpred, arg_locate; /* arg_locate 2: prec_off already has this frame's precincts */
     void* arg_planes[4];
     uint32_t arg_strides[4];
     DeferredCopy defer[JXS_MAXC]; /* output planes in pageable memory */
@@ -947,7 +947,7 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
         if (!jxs_gpu_is_device_ptr(bs) || size < c->hdr_len) return JXS_E_DEC_PTR;
         s->hdr_check = 1;
         KMARK();
-        if (walk) CK(jxs_launch_walk(d->dcfg, bs, size, s->prec_off, s->status, st));
+        if (walk && locate != 2) CK(jxs_launch_walk(d->dcfg, bs, size, s->prec_off, s->status, st));
     } else if (!jxs_gpu_is_device_ptr(bs)) {
         if (!staged) {
             const int32_t r = dec_bs_room(s, size, st);
@@ -1131,13 +1131,30 @@ extern "C" int32_t jxs_gpu_dec_submit_staged(jxs_gpu_dec_t* d, int slot, const u
     return r;
 }
 
+/* Locates the precincts of the slot's device codestream, and nothing else:
+ * most frames that are not at the split are damaged, and end here instead of
+ * after a second decode. */
+static int32_t dec_locate(jxs_gpu_dec_t* d, DecSlot* s) {
+    const cudaStream_t st = dec_stream(d, s);
+    CK(jxs_launch_walk(d->dcfg, s->arg_bs, s->arg_size, s->prec_off, s->status, st));
+    CK(jxs_launch(publish_status_kernel, dim3(1), 32u, 0, st, s->status_hd, s->status, (uint8_t*)nullptr, (const uint8_t*)nullptr, 0u));
+    CK(cudaEventRecord(s->done, st));
+    return JXS_OK;
+}
+
+/* Waits for the slot's work, submitted with result r. */
+static int32_t dec_finish(jxs_gpu_dec_t* d, DecSlot* s, int32_t r) {
+    if (r != JXS_OK) return abandon(s, dec_stream(d, s), r);
+    if (cudaEventSynchronize(s->done) == cudaSuccess) return JXS_OK;
+    fprintf(stderr, "jxs: decode failed: %s\n", cudaGetErrorString(cudaGetLastError()));
+    s->ndefer = 0;
+    return JXS_E_DEC_INTERNAL;
+}
+
 static int32_t dec_wait(jxs_gpu_dec_t* d, int slot) {
     DecSlot* s = &d->slot[slot];
-    if (cudaEventSynchronize(s->done) != cudaSuccess) {
-        fprintf(stderr, "jxs: decode failed: %s\n", cudaGetErrorString(cudaGetLastError()));
-        s->ndefer = 0;
-        return JXS_E_DEC_INTERNAL;
-    }
+    int32_t r = dec_finish(d, s, JXS_OK);
+    if (r != JXS_OK) return r;
     /* every header byte of a device codestream but Lcod (12..15) must match
      * the stream's */
     const jxs_cfg_t* c = &d->cfg;
@@ -1146,18 +1163,18 @@ static int32_t dec_wait(jxs_gpu_dec_t* d, int slot) {
     const int vpred0 = s->arg_vpred, locate0 = s->arg_locate;
     for (int again = 0; !other_hdr && (*s->status_h == JXS_E_DEC_VPRED || *s->status_h == JXS_E_DEC_WALK) && again < 2; again++) {
         /* the frame uses vertical prediction: decode it again slice by
-         * slice; or its slices are not at the constant-bit-rate split: decode
-         * it again with its precincts located first */
+         * slice; or its slices are not at the constant-bit-rate split: locate
+         * its precincts, and decode it again if they are there */
         const int vpred = s->arg_vpred || *s->status_h == JXS_E_DEC_VPRED;
-        const int locate = s->arg_locate || *s->status_h == JXS_E_DEC_WALK;
-        const int32_t r = dec_run(d, s, s->arg_bs, s->arg_size, s->arg_walked ? s->prec_off_h : NULL, s->arg_planes,
-                                  s->arg_strides, 0, 0, vpred, locate);
-        if (r != JXS_OK) return abandon(s, dec_stream(d, s), r);
-        if (cudaEventSynchronize(s->done) != cudaSuccess) {
-            fprintf(stderr, "jxs: decode failed: %s\n", cudaGetErrorString(cudaGetLastError()));
-            s->ndefer = 0;
-            return JXS_E_DEC_INTERNAL;
+        int locate = s->arg_locate;
+        if (*s->status_h == JXS_E_DEC_WALK) {
+            if ((r = dec_finish(d, s, dec_locate(d, s))) != JXS_OK) return r;
+            if (*s->status_h != 0) break;
+            locate = 2;
         }
+        r = dec_finish(d, s, dec_run(d, s, s->arg_bs, s->arg_size, s->arg_walked ? s->prec_off_h : NULL, s->arg_planes, s->arg_strides,
+                                     0, 0, vpred, locate));
+        if (r != JXS_OK) return r;
     }
     if (*s->status_h == 0) {
         /* that helped: later frames so from the start */
