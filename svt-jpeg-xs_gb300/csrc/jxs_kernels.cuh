@@ -281,7 +281,12 @@ static inline __host__ __device__ UkLayout uk_layout(uint32_t cap_bytes, uint32_
 }
 /* Shared memory set aside besides the precinct's bytes when a decoder fixes
  * how long a precinct it takes (larger ones are invalid streams): at least
- * that of the layout above, `ordered` with the row above's GCLIs. */
+ * that of the full layout above, `ordered` with the row above's GCLIs.  The
+ * lean one takes up to UK_LEAN_MORE bytes more (its list is not in the place
+ * of the codeword values, which matters for fewer than 5,000 groups); how
+ * long a precinct may be does not depend on that, the memory left over does
+ * (jxs_plan.cuh). */
+#define UK_LEAN_MORE 288
 static inline uint32_t uk_reserved(uint32_t cap_groups, uint32_t cap_seg, int ordered) {
     uint32_t o = (32 + cap_groups + 15) & ~15u;
     o = (o + (2 * UK_ZCAP(cap_groups) > UK_LIST_BYTES ? 2 * UK_ZCAP(cap_groups) : UK_LIST_BYTES) + 15) & ~15u;

@@ -53,7 +53,10 @@ extern "C" int jxs_inv_v_tile_cols(void);
 extern "C" int jxs_inv_h_max_rows_per_block(void);
 extern "C" int jxs_inv_h_chunk_cols(int nh);
 
+/* Shared memory that a block's buffers are planned within, its static part
+ * included; the device gives a block 227 KB. */
 static const size_t kSmemMax = 220 * 1024;
+static_assert(kSmemMax + UK_LEAN_MORE <= 227 * 1024, "the lean unpacking layout fits where the full one does");
 
 /* Rate-control tables of a frame: per precinct row the byte cost of every
  * (Q, R); with sign handling a second set with exact sign counts; with
