@@ -926,6 +926,19 @@ static int32_t dec_bs_room(DecSlot* s, uint32_t size, cudaStream_t st) {
     s->bs_cap = size + 4096;
     return JXS_OK;
 }
+/* 0: component k's rows cross the link faster staged and stored by
+ * host_store_kernel_n than written by the last inverse level.  A vertical level
+ * writes the strips at either end of a row sample by sample unless the row is
+ * a multiple of 8 samples; 16-bit ones cost it more than the staging
+ * (3838x2160 4:2:2 10 bit in aligned rows 404 us in place, 337 staged).  8-bit
+ * ones do not (3836x2160 4:2:0 183 and 195 us), nor rows without vertical
+ * levels, where only the end is written so (3832x2160 4:2:2 338 and 342), nor
+ * those of a non-linear output, a thread per sample (1910x1080 4:4:4 154 and
+ * 176). */
+static int writes_in_place(const jxs_cfg_t* c, uint32_t k) {
+    return jxs_out_w(c, k) % 8 == 0 || bytes_per_sample(c) == 1 || c->comp[k].dv <= c->proxy || dec_needs_nlt_pass(c);
+}
+
 static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t size, const uint32_t* prec_off,
                        void* const planes[4], const uint32_t strides[4], int alone, int staged, int vpred, int locate) {
     s->ndefer = 0;
@@ -989,9 +1002,12 @@ static int32_t dec_run(jxs_gpu_dec_t* d, DecSlot* s, const uint8_t* bs, uint32_t
     TMARK(2);
 
     int out_dev[JXS_MAXC];
-    for (uint32_t k = 0; k < c->nc; k++)
+    for (uint32_t k = 0; k < c->nc; k++) {
+        const uint32_t ow = jxs_out_w(c, k);
         out_dev[k] = jxs_gpu_is_device_ptr(planes[k]) ||
-                     (alone && host_in_place(planes[k], (size_t)strides[k] * bps, (size_t)jxs_out_w(c, k) * bps, jxs_out_h(c, k), 1));
+                     (alone && writes_in_place(c, k) &&
+                      host_in_place(planes[k], (size_t)strides[k] * bps, (size_t)ow * bps, jxs_out_h(c, k), 1));
+    }
     /* horizontal-only levels of every component (into the int32 low band of
      * its last vertical level, or straight to the output plane), then the
      * vertical levels from the deepest up */
