@@ -402,16 +402,19 @@ static int32_t enc_slot_alloc(jxs_gpu_enc_t* e, EncSlot* s) {
     }
         CK(cudaMalloc(&s->cost, jxs_cost_bytes(c)));
     CK(cudaMalloc(&s->slice_done, (size_t)c->nslices * sizeof(uint32_t)));
-    CK(cudaMemset(s->slice_done, 0, (size_t)c->nslices * sizeof(uint32_t)));
+    CK(cudaMemsetAsync(s->slice_done, 0, (size_t)c->nslices * sizeof(uint32_t), s->st));
     CK(cudaMalloc(&s->rc, (size_t)c->np * sizeof(PrecRC)));
     CK(cudaMalloc(&s->status, 64));
-    CK(cudaMemset(s->status, 0, 64));
+    CK(cudaMemsetAsync(s->status, 0, 64, s->st));
     CK(cudaMalloc(&s->out_stage, c->lcod + 64));
     CK(cudaMallocHost(&s->status_h, 64));
     *s->status_h = 0;
     CK(cudaHostGetDevicePointer((void**)&s->status_hd, s->status_h, 0));
     for (int i = 0; i < 6; i++) CK(cudaEventCreate(&s->tev[i]));
     for (int i = 0; i < JXS_KEV; i++) CK(cudaEventCreate(&s->kev[i]));
+    /* kept at zero by the kernels from here on: there before the first frame,
+     * whatever stream that takes and whatever holds the default one */
+    CK(cudaStreamSynchronize(s->st));
     return JXS_OK;
 }
 
@@ -813,12 +816,13 @@ static int32_t dec_slot_alloc(jxs_gpu_dec_t* d, DecSlot* s) {
         CK(cudaMalloc(&s->mct, mb * sizeof(int32_t)));
     }
     CK(cudaMalloc(&s->status, 64));
-    CK(cudaMemset(s->status, 0, 64));
+    CK(cudaMemsetAsync(s->status, 0, 64, s->st));
     CK(cudaMallocHost(&s->status_h, 64));
     *s->status_h = 0;
     CK(cudaHostGetDevicePointer((void**)&s->status_hd, s->status_h, 0));
     for (int i = 0; i < 5; i++) CK(cudaEventCreate(&s->tev[i]));
     for (int i = 0; i < JXS_KEV; i++) CK(cudaEventCreate(&s->kev[i]));
+    CK(cudaStreamSynchronize(s->st)); /* the status is zero before the first frame, as for the encoder */
     return JXS_OK;
 }
 
