@@ -696,7 +696,9 @@ __global__ void __launch_bounds__(FH_MAX_WARPS * 32) fwd_h_kernel(const __grid_c
     if (row >= J.h) return; /* the whole warp */
     const int halo = fh_halo_lanes(J.nh), first = ch * fh_net_cols(J.nh) - FH_COLS * halo;
     const int c0 = first + FH_COLS * lane;
-    const bool out_lane = lane >= halo && lane < 32 - halo && c0 < J.w;
+    /* lanes past the row's end too: the last group of a deeper band, which
+     * several lanes share, ends in theirs with zeros */
+    const bool out_lane = lane >= halo && lane < 32 - halo;
     if (first >= 0 && first + 32 * FH_COLS <= J.w) fh_chunk<SRC, false>(J, row, c0, out_lane);
     else fh_chunk<SRC, true>(J, row, c0, out_lane);
 }
