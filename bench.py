@@ -850,8 +850,8 @@ def run_ours(args, rank, world, local):
             cpu, cpu_port = cpu_port, None
 
     # per frame: 2 vertical + 1 horizontal transform, rate control, pack;
-    # unpack, 1 horizontal + 2 vertical inverse
-    launches_per_frame = 5 + 4
+    # unpack, 1 horizontal + 2 vertical inverse; the status of each direction
+    launches_per_frame = 5 + 4 + 2
     head_ms = bat["dev_ms"] if head_batched else dev_ms
     head_clk = clk_b if head_batched else clk
     line = {

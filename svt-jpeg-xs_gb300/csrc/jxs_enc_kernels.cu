@@ -515,9 +515,10 @@ DEV void cost_items(uint32_t nbl, uint32_t npk, const uint8_t* order, const uint
  * part.  Two GCLIs to an instruction and two gtli values to a warp, with the
  * coding choice as minima and maxima, take it from 65,000 to 18,000 cycles
  * per precinct (1279x717 4:4:4), the costs by a warp per packet from 13,000
- * to 5,500; the kernel 231 -> 102 us, of which the sign counts above
- * 30 us.  Two blocks per SM: with registers for three (40) the loop spills
- * (114 us). */
+ * to 5,500; the kernel from 231 to 102 us, 88 us with what came after (gtli
+ * values above every GCLI without the loop, costs by chunks of lines).  Two
+ * blocks per SM: with registers for three (40) the loop spilled (114 us
+ * against 102). */
 template <typename Stage>
 DEV void select_slice_vpred(const jxs_cfg_t* __restrict__ cfg, const SliceInfo& I, int s, const uint8_t* gcli,
                             const uint32_t* cost, uint32_t* area, PrecRC* rc,

@@ -596,8 +596,8 @@ __global__ void __launch_bounds__(32, SRC == SRC_I32 ? 28 : 32) fwd_v_kernel(con
  * Bound by memory: 4 bytes read and 2 1/4 written per column.  The form
  * before kept whole rows in shared memory, one warp per row, which left 8
  * warps on an SM for the 3840-column rows of an 8K frame with one vertical
- * level: 8 such frames took 650 us, now 250 (1.24 GB; encode 3308 -> 2907
- * us). */
+ * level: 8 such frames took 650 us, now 283 (1.24 GB; that step took their
+ * encode from 3308 to 2907 us). */
 #define FH_MAX_WARPS 4
 #define FH_COLS 16
 

@@ -81,7 +81,8 @@ DEV CoefRow coef_row(const jxs_band_t& bd, int r, const int16_t* coef) {
  * Bound by memory: 2 bytes read and 4 written per column.  The form before
  * kept whole rows in shared memory, one warp per row, which left few warps
  * on an SM for wide rows: 8 8K frames with one vertical level (3840-column
- * rows) took 1050 us, now 220 (1.2 GB; decode 3081 -> 2249 us). */
+ * rows) took 1050 us, now 225 (1.2 GB; that step took their decode from 3081
+ * to 2249 us). */
 #define IH_MAX_WARPS 4
 #define IH_COLS 16
 

@@ -330,8 +330,9 @@ static inline cudaError_t jxs_smem_attr(K kern, int bytes, std::atomic<int>* cac
  * the kernel runs, which before the wait is not so, and let their loads move
  * above it.  Only the handle's configuration is constant that long.  Behind a
  * copy, a memset or an event the launch is an ordinary one, and dep_wait()
- * returns at once in a kernel that was launched the ordinary way.  A 4K frame encodes in 114 us instead of 125 and decodes in 107
- * instead of 118; a 256x64 one takes 119 us there and back instead of 145.
+ * returns at once in a kernel that was launched the ordinary way.  A 4K frame
+ * encodes in 113 us instead of 122 and decodes in 90 instead of 99; a 256x64 one
+ * takes 104 us there and back instead of 127.
  * Starting the next kernel's blocks earlier still (a trigger at the top of
  * each kernel) gained nothing there, and their waiting blocks cost batches up
  * to 8 %.  The launches of many frames at once, where a launch is a small

@@ -226,9 +226,10 @@ static inline uint32_t v_warps(const jxs_cfg_t* c, int v, uint32_t cols) {
 /* Row pairs per warp of a vertical level's launch with `warps` warps at 8
  * each: 8 where that fills the device (32 warps on each of 152 SMs), fewer
  * for smaller launches, down to one, where a warp's chain of steps is what
- * takes the time.  Fewer cost rows read twice (3 per warp): at 8 / 4 / 2 row
- * pairs 8 4K frames encode in 642 / 645 / 700 us and one frame in 155 / 147 /
- * 150 us, a 256x64 frame there and back takes 174 us at 8 and 157 at 1.
+ * takes the time.  Fewer cost rows read twice (3 per warp): at 8 / 4 / 2 / 1
+ * row pairs on every level 8 4K frames encode in 508 / 512 / 531 / 571 us and
+ * decode in 433 / 438 / 460 / 536, one frame in 118 / 112 / 114 / 117 and 93 /
+ * 90 / 93 / 99 us, a 256x64 frame there and back takes 120 / 111 / 106 / 103.
  * The levels with int32 low bands on their other side (`deep`) read twice as
  * much per row again, and 8 warps on each SM do for them: level 1 of a 4K frame
  * at 4 / 1 row pairs takes 10.9 / 11.9 us forward and 10.4 / 12.3 inverse. */
